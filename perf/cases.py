@@ -184,6 +184,7 @@ class State:
         if case["mode"] == "host":
             self._host_buffers(fc)
         if case["call"] == "frame":
+            self.outputs = _frame_outputs(self)
             return
         pipe.build("graph")
         torch.cuda.synchronize()
@@ -194,8 +195,14 @@ class State:
             hits = _hits(case, pipe, scene, rng)
             self.hits = torch.from_numpy(hits.view(np.uint8).reshape(-1)).cuda()
             self.decoded = torch.zeros(len(hits) * L.BaseHit.itemsize, dtype=torch.uint8, device="cuda")
+            rec = self.decoded.view(torch.int32).view(-1, 10)
+            self.outputs = {"ids": rec[:, :5], "parts": rec[:, 8:], "barycentrics": rec.view(torch.float32)[:, 5:8]}
         else:
-            self.raster, self.raster_bufs = pipe.state.raster_outputs()
+            self.raster, b = pipe.state.raster_outputs()
+            self.outputs = {"counts": b["counts"].handle.view(torch.int32), "batches": _as(b["batches"], torch.int32, 6),
+                            "clip": _as(b["clipPositions"], torch.float32, 4),
+                            "world": _as(b["worldPositions"], torch.float32, 3),
+                            "indices": b["indices"].handle, "primitives": b["primitiveIDs"].handle.view(torch.int32)}
 
     def _host_buffers(self, fc):
         """The frame's inputs as one pinned block, which the frame's arguments mirror on the device."""
@@ -315,6 +322,8 @@ def _frame_outputs(s):
         out["build_vertices"] = _as(st.trans_builds, torch.int16, 32)[:, 16]
         out["build_instances"] = st.trans_instance_ids.handle.view(torch.int32)
         out["build_addresses"] = st.trans_cluster_addresses.handle.view(torch.int64)
+    if s.case["mode"] == "host":
+        out["host_readback"] = s.readback.view(torch.int32)
     return out
 
 
@@ -326,25 +335,20 @@ def run(s):
         return {"vertices": v.detach(), "grads": list(grads)}
     if call == "decode":
         pipe.decode_hits_device(s.hits, s.decoded)
-        rec = s.decoded.view(torch.int32).view(-1, 10)
-        return {"ids": rec[:, :5], "parts": rec[:, 8:], "barycentrics": rec.view(torch.float32)[:, 5:8]}
+        return s.outputs
     if call == "raster":
         pipe.stage("raster_batches", ctypes.byref(s.raster))
-        b = s.raster_bufs
-        return {"counts": b["counts"].handle.view(torch.int32), "batches": _as(b["batches"], torch.int32, 6),
-                "clip": _as(b["clipPositions"], torch.float32, 4), "world": _as(b["worldPositions"], torch.float32, 3),
-                "indices": b["indices"].handle, "primitives": b["primitiveIDs"].handle.view(torch.int32)}
+        return s.outputs
     if mode == "host":
         # the frame before has ended (the wait below), so its staging block is free to be written
         s.staging_np[:] = s.inputs
         pipe.build_host(s.staging.data_ptr(), s.base, s.inputs.size, s.readback.data_ptr())
         torch.cuda.current_stream().synchronize()
-        return dict(_frame_outputs(s), host_readback=s.readback.view(torch.int32))
-    if mode == "stages":
+    elif mode == "stages":
         _stages(pipe)
     else:
         pipe.build(mode)
-    return _frame_outputs(s)
+    return s.outputs
 
 
 # ---------------------------------------------------------------------------
@@ -381,7 +385,7 @@ def work(case):
     if case["call"] == "decode":
         return {"bytes": 64 * case["hits"] + 24 * parts + geometry - 32 * base_vertices, "flops": 40 * case["hits"]}
     run(s)
-    batches, rv, rt = (int(x) for x in s.raster_bufs["counts"].read(np.uint32, 3))
+    batches, rv, rt = (int(x) for x in s.outputs["counts"][:3].cpu())
     return {"bytes": geometry + maps + 24 * parts + 24 * batches + 28 * rv + 7 * rt, "flops": 100 * rv}
 
 
