@@ -1,0 +1,62 @@
+"""Kernels whose mapping depends on sizes or alignment, at the edges of each
+form, against the CPU oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests.conftest import cuda_available
+from tests.parity import vertex_tolerance
+from vk_tessellated_clusters_gb300 import layouts as L
+from vk_tessellated_clusters_gb300 import scene as S
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_available(), reason="needs a CUDA GPU")]
+
+FLAGS = L.FLAG_CULLING | L.FLAG_WRITE_FULLCLUSTERS
+
+
+# part counts at which k_raster_write's warps (4 per block, 8 blocks per SM, 152 SMs: 4,864; with PN or the ripple
+# half of that) share a group four ways, two ways and not at all
+@pytest.mark.parametrize("instances,pixels,flags,parts", [(24, 4.0, 0, (1, 38912)), (170, 4.0, 0, (38913, 77824)),
+                                                          (256, 3.0, 0, (77825, 1 << 20)),
+                                                          (170, 4.0, L.FLAG_PN, (38913, 1 << 20))])
+def test_raster_group_sharing(oracle, instances, pixels, flags, parts):
+    """Whole outputs against the oracle (positions to the vertex tolerance times the largest instance scale), then
+    the same call on outputs one float off 16-byte alignment and too small by a few vertices and triangles: the same
+    values up to the capacity, nothing past it, and the capacity bit."""
+    import torch
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_batched(num_instances=instances, map_size=64)
+    cam = S.camera_orbit(5, tess_rate_pixels=pixels)
+    caps = L.default_caps(vertex_bits=23)
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS | flags)
+    want = oracle.raster_batches(ref_state)
+    pipe = TessellationPipeline(sc, caps, FLAGS | flags)
+    pipe.set_cameras(cam)
+    pipe.build("graph")
+    got = pipe.raster_batches()
+    n = int(pipe.state.scene_building()["partTriangleCounter"])
+    assert parts[0] <= n <= parts[1], n
+    assert pipe.device_errors() == 0 and got["counts"] == want["counts"]
+    for f in ("batches", "indices", "primitiveIDs"):
+        assert got[f].tobytes() == want[f].tobytes(), f
+    scale = max(float(np.abs(np.asarray(i.world)[:3, :3]).sum(axis=1).max()) for i in sc.instances)
+    assert np.abs(got["worldPositions"].astype(np.float64) - want["worldPositions"]).max() <= vertex_tolerance(sc) * scale
+    nv, nt = got["counts"][1] - 5, got["counts"][2] - 7
+    ro, bufs = pipe.state.raster_outputs()
+    small = type(ro).from_buffer_copy(ro)
+    clip = torch.full((4 * nv + 64,), -7.0, device="cuda")
+    small.clipPositions, small.maxVertices, small.maxTriangles = clip.data_ptr() + 4, nv, nt
+    for b in ("worldPositions", "indices", "primitiveIDs"):
+        bufs[b].handle.fill_(0xAB)
+    pipe.stage("raster_batches", ctypes.byref(small))
+    assert pipe.device_errors() == 8  # TC_DEVERR_CAPACITY
+    c = clip.cpu().numpy()
+    assert c[1:1 + 4 * nv].tobytes() == got["clipPositions"][:nv].tobytes()
+    assert c[0] == -7.0 and (c[1 + 4 * nv:] == -7.0).all()
+    cut = {"worldPositions": (np.float32, 3 * nv), "indices": (np.uint8, 3 * nt), "primitiveIDs": (np.uint32, nt)}
+    for f, (dtype, count) in cut.items():
+        raw = bufs[f].read(np.uint8, min(bufs[f].nbytes, count * dtype().itemsize + 64))
+        size = count * dtype().itemsize
+        assert raw[:size].tobytes() == got[f].reshape(-1)[:count].tobytes() and (raw[size:] == 0xAB).all(), f
+    pipe.close()

@@ -7,8 +7,8 @@
 //
 // Three launches: per group of 32 parts (one warp) its batch, vertex and
 // triangle counts; one block scans the groups' counts into offsets; per group
-// again (four warps, a quarter of the parts each) the batch records, then part
-// by part the vertices (lanes over the part's vertices) and triangles.
+// again the batch records, then the group's vertices and triangles, each as
+// one contiguous range over which the lanes take consecutive elements.
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
@@ -17,21 +17,9 @@ namespace tc {
 
 namespace {
 
-constexpr u32 kRasterBlock   = 256;
-constexpr u32 kWarpsPerGroup = 4;  // k_raster_write: warps per group of 32 parts
-constexpr u32 kPartsPerWarp  = 32 / kWarpsPerGroup;
-
-// what the vertex and triangle loops of one part need
-struct RasterPart
-{
-  f3                     bp[3], bn[3], bb[3];
-  f2                     bt[3];
-  tc_DisplacementTexture tx;
-  const float*           world;
-  float                  scale, offset, size;
-  u32                    cfg, triID, inst, partID, v0, t0, vs;
-  bool                   hasTx;
-};
+constexpr u32 kRasterBlock = 256;  // counts
+constexpr u32 kWriteBlock  = 128;  // k_raster_write: its part records fill the shared memory of a block
+constexpr u32 kWriteWarps  = kWriteBlock / 32;
 
 // the group's parts: per lane (part g0 + lane) its inclusive vertex and
 // triangle sums; lanes past the parts count as a full batch (they never fit)
@@ -106,22 +94,32 @@ __global__ void __launch_bounds__(kRasterBlock) k_raster_counts(StageCtx c, uint
   }
 }
 
-// one block: exclusive scan of the groups' counts, in place; totals to counts[3]
+// one block: exclusive scan of the groups' counts, in place; totals to
+// counts[3]. Four consecutive groups per thread and round: a round costs two
+// barriers and a memory round trip, so a frame of 160,000 parts (5,100 groups)
+// takes two rounds.
+constexpr u32 kScanGroups = 4;
+
 __global__ void __launch_bounds__(1024) k_raster_scan(StageCtx c, uint4* groups, u32* counts)
 {
   stage_prologue();
-  __shared__ uint4 s_warp[32];
-  __shared__ uint4 s_carry;
+  __shared__ uint3 s_warp[2][33];
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 ngroups = (num_parts(c) + 31) / 32;
-  if(threadIdx.x == 0)
-    s_carry = make_uint4(0, 0, 0, 0);
-  __syncthreads();
-  for(u32 base = 0; base < ngroups; base += blockDim.x)
+  uint3     carry   = make_uint3(0, 0, 0);
+  u32       round   = 0;
+  for(u32 base = 0; base < ngroups; base += blockDim.x * kScanGroups, round ^= 1)
   {
-    const u32 i = base + threadIdx.x;
-    uint4     v = i < ngroups ? groups[i] : make_uint4(0, 0, 0, 0);
-    uint4     inc = v;
+    const u32 i = base + threadIdx.x * kScanGroups;
+    uint4     v[kScanGroups];
+    uint3     sum = make_uint3(0, 0, 0);
+#pragma unroll
+    for(u32 k = 0; k < kScanGroups; k++)
+      v[k] = i + k < ngroups ? groups[i + k] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for(u32 k = 0; k < kScanGroups; k++)
+      sum.x += v[k].x, sum.y += v[k].y, sum.z += v[k].z;
+    uint3 inc = sum;
 #pragma unroll
     for(int d = 1; d < 32; d <<= 1)
     {
@@ -131,11 +129,12 @@ __global__ void __launch_bounds__(1024) k_raster_scan(StageCtx c, uint4* groups,
         inc.x += a, inc.y += b, inc.z += e;
     }
     if(lane == 31)
-      s_warp[warp] = inc;
+      s_warp[round][warp] = inc;
     __syncthreads();
     if(warp == 0)
     {
-      uint4 w = s_warp[lane], wi = w;
+      const uint3 w  = s_warp[round][lane];
+      uint3       wi = w;
 #pragma unroll
       for(int d = 1; d < 32; d <<= 1)
       {
@@ -144,52 +143,76 @@ __global__ void __launch_bounds__(1024) k_raster_scan(StageCtx c, uint4* groups,
         if(lane >= (u32)d)
           wi.x += a, wi.y += b, wi.z += e;
       }
-      s_warp[lane] = make_uint4(wi.x - w.x, wi.y - w.y, wi.z - w.z, 0u);
+      s_warp[round][lane] = make_uint3(wi.x - w.x, wi.y - w.y, wi.z - w.z);
+      if(lane == 31)
+        s_warp[round][32] = wi;
     }
     __syncthreads();
-    const uint4 cw = s_carry, ww = s_warp[warp];
-    if(i < ngroups)
-      groups[i] = make_uint4(cw.x + ww.x + inc.x - v.x, cw.y + ww.y + inc.y - v.y, cw.z + ww.z + inc.z - v.z, 0u);
-    __syncthreads();
-    if(threadIdx.x == blockDim.x - 1)
-      s_carry = make_uint4(cw.x + ww.x + inc.x, cw.y + ww.y + inc.y, cw.z + ww.z + inc.z, 0u);
-    __syncthreads();
+    // (the next round writes the other copy; its first barrier orders the one after)
+    const uint3 ww = s_warp[round][warp], tot = s_warp[round][32];
+    uint3       ex = make_uint3(carry.x + ww.x + inc.x - sum.x, carry.y + ww.y + inc.y - sum.y, carry.z + ww.z + inc.z - sum.z);
+#pragma unroll
+    for(u32 k = 0; k < kScanGroups; k++)
+    {
+      if(i + k < ngroups)
+        groups[i + k] = make_uint4(ex.x, ex.y, ex.z, 0u);
+      ex.x += v[k].x, ex.y += v[k].y, ex.z += v[k].z;
+    }
+    carry.x += tot.x, carry.y += tot.y, carry.z += tot.z;
   }
   if(threadIdx.x == 0)
   {
-    counts[0] = s_carry.x, counts[1] = s_carry.y, counts[2] = s_carry.z;
+    counts[0] = carry.x, counts[1] = carry.y, counts[2] = carry.z;
   }
 }
 
-__global__ void __launch_bounds__(kRasterBlock) k_raster_write(StageCtx c, const uint4* groups, tc_raster_outputs o)
+// Bound by instruction issue and the latency of a group's dependent loads.
+// A part has about five vertices and four triangles, so a warp that takes its
+// parts one by one uses a sixth of its lanes; here every part of the group is
+// set up once in shared memory, one part per lane (its affine form as in the
+// vertex kernels, tc_vertex.cuh, and its world matrix), and the lanes walk the
+// group's vertices, then its triangles, in order. When the frame has fewer
+// groups than the grid has warps, several warps share a group, each walking a
+// part of its parts. Measured on a GB300, 105,000 parts (497,000 vertices) of
+// 256 instances: the kernel 104 -> 36 us, the call 112 -> 46 us.
+// Deform: with PN triangles or the ripple.
+template <bool Deform>
+__global__ void __launch_bounds__(kWriteBlock) k_raster_write(StageCtx c, const uint4* groups, tc_raster_outputs o)
 {
   stage_prologue();
-  __shared__ RasterPart      s_parts[kRasterBlock / 32][kPartsPerWarp];
-  const u32                  lane = threadIdx.x & 31, n = num_parts(c), ngroups = (n + 31) / 32;
+  __shared__ PartAffine s_part[kWriteWarps][32];
+  __shared__ float4     s_world[kWriteWarps][32][3];  // rows of the world matrix
+  __shared__ PartPn     s_pn[Deform ? kWriteWarps : 1][Deform ? 32 : 1];
+  const u32                  lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32                  n = num_parts(c), ngroups = (n + 31) / 32;
   const tc_TessTriangleInfo* parts = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->partTriangles);
   tc_raster_batch*           batches = reinterpret_cast<tc_raster_batch*>(o.batches);
   float*                     clip    = reinterpret_cast<float*>(o.clipPositions);
   float*                     world   = reinterpret_cast<float*>(o.worldPositions);
   uint8_t*                   idx     = reinterpret_cast<uint8_t*>(o.indices);
   u32*                       prim    = reinterpret_cast<u32*>(o.primitiveIDs);
+  const bool                 clip16 = (o.clipPositions & 15) == 0;
   const bool                 visTriangles = c.view->visualize == TC_VISUALIZE_TRIANGLES;
-  const bool                 pn = (c.flags & TC_FLAG_PN) != 0;
-  const RippleParams         rp = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
+  const bool                 pn = Deform && (c.flags & TC_FLAG_PN) != 0;
+  const RippleParams         rp = ripple_params(*c.view, Deform && (c.flags & TC_FLAG_RIPPLE) != 0);
   float                      vp[16];
 #pragma unroll
   for(int q = 0; q < 16; q++)
     vp[q] = c.view->viewProjMatrix.m[q];
-  bool overflow = false;
-  // kWarpsPerGroup warps share a group, each taking a quarter of its parts
-  // (the batch layout is recomputed by each, the first writes the records)
-  for(u32 gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gw < ngroups * kWarpsPerGroup;
-      gw += (gridDim.x * blockDim.x) >> 5)
+  PartAffine* sp       = s_part[warp];
+  const u32   below    = (2u << lane) - 2u;
+  bool        overflow = false;
+  // warps per group: as many of 1, 2 and 4 as the grid has warps for
+  const u32 nwarps   = (gridDim.x * blockDim.x) >> 5;
+  const u32 share    = ngroups * 4 <= nwarps ? 4u : (ngroups * 2 <= nwarps ? 2u : 1u);
+  const u32 perShare = 32 / share;
+  for(u32 gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gw < ngroups * share; gw += nwarps)
   {
-    const u32       g = gw / kWarpsPerGroup, sub = gw % kWarpsPerGroup;
+    const u32       g = gw / share, sub = gw % share;
     const u32       g0 = g * 32, local = min(32u, n - g0);
     const uint4     off = groups[g];  // batches, vertices, triangles before this group
     const GroupSums s   = group_sums(c, g0, local);
-    // per part: the vertex count before its batch (its batch-local vertex start)
+    // the vertex count before this lane's part's batch: its batch-local vertex start
     u32 batchStartV = 0;
     group_batches(s, local, [&](u32 q, u32 start, u32 end, u32 lastV, u32 lastT) {
       const u32 ev = __shfl_sync(0xFFFFFFFFu, s.sumV, end), et = __shfl_sync(0xFFFFFFFFu, s.sumT, end);
@@ -213,103 +236,132 @@ __global__ void __launch_bounds__(kRasterBlock) k_raster_write(StageCtx c, const
           overflow = true;
       }
     });
-    // mesh.glsl:190-435: lanes 0..7 set up the warp's parts at once (their
-    // dependent loads overlap), then part by part lanes take its vertices
-    // and triangles
-    const u32 pBegin = sub * kPartsPerWarp, pEnd = min(local, pBegin + kPartsPerWarp);
-    RasterPart* rec = s_parts[threadIdx.x >> 5];
-    // lane l < kPartsPerWarp sets up part pBegin + l: its exclusive sums and
-    // its first vertex within its batch, from that part's lane
-    const u32 src = pBegin + (lane & (kPartsPerWarp - 1));
-    const u32 exV = __shfl_sync(0xFFFFFFFFu, s.sumV - s.v, src), exT = __shfl_sync(0xFFFFFFFFu, s.sumT - s.t, src);
-    const u32 vsP = __shfl_sync(0xFFFFFFFFu, s.sumV - s.v - batchStartV, src);
-    if(pBegin + lane < pEnd && lane < kPartsPerWarp)
+    // mesh.glsl:190-435: this warp's parts [pBegin, pEnd) of the group, one per lane
+    const u32  pBegin = min(local, sub * perShare), pEnd = min(local, pBegin + perShare);
+    const bool owner = lane >= pBegin && lane < pEnd;
+    const u32  exV = s.sumV - s.v, exT = s.sumT - s.t;  // vertices and triangles before this lane's part
+    u32        tvBase = 0, triBase = 0, meta = 0, inst = 0;
+    float      size = 0.0f;
+    if(owner)
     {
-      const u32                 i   = pBegin + lane;
-      const tc_TessTriangleInfo pt  = parts[g0 + i];
-      RasterPart&               r   = rec[lane];
-      r.cfg                         = pt.subTriangle.triangleID_config >> 16;
-      r.triID                       = pt.subTriangle.triangleID_config & 0xFFFFu;
-      r.inst                        = pt.cluster.instanceID;
-      r.v0                          = off.y + exV;
-      r.t0                          = off.z + exT;
-      r.vs                          = vsP;
-      const tc_RenderInstance& in   = c.instances[pt.cluster.instanceID];
-      const tc_Cluster         cl   = reinterpret_cast<const tc_Cluster*>(in.clusters)[pt.cluster.clusterID];
-      const uint8_t* lt = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle;
-      u32            partID = 0;
-      for(int v = 0; v < 3; v++)
-      {
-        const u32 vi = cl.firstLocalVertex + lt[r.triID * 3 + v];
-        r.bp[v]      = ldg3(reinterpret_cast<const float*>(in.positions), vi);
-        r.bn[v]      = normalize3(ldg3(reinterpret_cast<const float*>(in.normals), vi));
-        r.bt[v]      = ldg2(reinterpret_cast<const float*>(in.texcoords), vi);
-        r.bb[v]      = decode_bary(pt.subTriangle.vtxEncoded[v]);
-        partID ^= (pt.subTriangle.vtxEncoded[v] >> 20) | ((pt.subTriangle.vtxEncoded[v] >> 4) & 0xFFFu);
-      }
-      r.partID = partID;
-      r.hasTx  = false;
+      const uint2*            raw = reinterpret_cast<const uint2*>(parts + g0 + lane);
+      const uint2             r0 = __ldg(raw), r1 = __ldg(raw + 1), r2 = __ldg(raw + 2);
+      const u32               cfg = r2.y >> 16, tri = r2.y & 0xFFFFu;
+      const tc_TessTableEntry e   = table_entry(c.table, cfg);
+      const tc_RenderInstance& in = c.instances[r0.x];
+      const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in.clusters)[r0.y];
+      const uint8_t* lt = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle + tri * 3;
+      const u32      corner[3] = {r1.x, r1.y, r2.x};
+      tc_DisplacementTexture tx = {};
       if(c.numTextures > 0 && c.textures != nullptr && in.displacementIndex >= 0)
       {
         if((u32)in.displacementIndex < c.numTextures)
         {
-          r.tx    = c.textures[in.displacementIndex];
-          r.hasTx = true;
+          tx = c.textures[in.displacementIndex];
+          if(tx.width == 0)  // an empty map samples as 0: the offsets still displace
+            tx.width = 1, tx.height = 0;
         }
         else
           atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
       }
-      r.scale  = in.displacementScale;
-      r.offset = in.displacementOffset;
-      r.size   = in.geoHi.w;
-      r.world  = in.worldMatrix.m;
+      const float* pos = reinterpret_cast<const float*>(in.positions);
+      const float* nrm = reinterpret_cast<const float*>(in.normals);
+      part_affine(sp[lane], corner, cfg_flipped(cfg), pos, nrm, reinterpret_cast<const float*>(in.texcoords),
+                  cl.firstLocalVertex, lt, e.firstVertex, tx, in.displacementScale * c.view->displacementScale,
+                  in.displacementOffset + c.view->displacementOffset);
+      if constexpr(Deform)
+        if(pn)
+        {
+          const u32 i0 = cl.firstLocalVertex + lt[0], i1 = cl.firstLocalVertex + lt[1], i2 = cl.firstLocalVertex + lt[2];
+          write_part_pn(s_pn[warp][lane], corner, cfg_flipped(cfg),
+                        setup_pn(ldg3(pos, i0), ldg3(pos, i1), ldg3(pos, i2), normalize3(ldg3(nrm, i0)),
+                                 normalize3(ldg3(nrm, i1)), normalize3(ldg3(nrm, i2))));
+        }
+      const float* m = in.worldMatrix.m;
+#pragma unroll
+      for(int r = 0; r < 3; r++)
+        s_world[warp][lane][r] = make_float4(__ldg(m + r), __ldg(m + 4 + r), __ldg(m + 8 + r), __ldg(m + 12 + r));
+      u32 partID = 0;
+#pragma unroll
+      for(int v = 0; v < 3; v++)
+        partID ^= (corner[v] >> 20) | ((corner[v] >> 4) & 0xFFFu);
+      tvBase  = e.firstVertex - exV;    // table vertex of group vertex j: tvBase + j
+      triBase = e.firstTriangle - exT;  // table triangle of group triangle j: triBase + j
+      meta    = (exV - batchStartV) | ((tri & 0xFFu) << 8) | (partID << 16) | (cfg_flipped(cfg) ? 1u << 28 : 0u);
+      inst    = r0.x;
+      size    = in.geoHi.w;
     }
     __syncwarp();
-    for(u32 i = pBegin; i < pEnd; i++)
+    if(pBegin < pEnd)
     {
-      const RasterPart&       r = rec[i - pBegin];
-      const tc_TessTableEntry e = table_entry(c.table, r.cfg);
-      BasePN                  basis = {};
-      if(pn)
-        basis = setup_pn(r.bp[0], r.bp[1], r.bp[2], r.bn[0], r.bn[1], r.bn[2]);
-      for(u32 vert = lane; vert < e.numVertices; vert += 32)
+      const u32 vBegin = __shfl_sync(0xFFFFFFFFu, exV, pBegin), vEnd = __shfl_sync(0xFFFFFFFFu, s.sumV, pEnd - 1);
+      const u32 vFit = o.maxVertices > off.y ? min(vEnd, o.maxVertices - off.y) : 0u;
+      overflow |= vFit < vEnd;
+#pragma unroll 2  // two steps in flight: their loads overlap
+      for(u32 base = vBegin; base < vFit; base += 32)
       {
-        if(r.v0 + vert >= o.maxVertices)
+        // lane's part: those starting at or before the step's first vertex,
+        // plus those starting inside the step up to the lane (one bit each)
+        const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && exV <= base));
+        const u32 inside =
+            __reduce_or_sync(0xFFFFFFFFu, (owner && exV > base && exV < base + 32) ? 1u << (exV - base) : 0u);
+        const u32 pi = (pBegin + before - 1 + __popc(inside & below)) & 31;
+        const u32 jj = base + lane;
+        const u32 tvIdx = __shfl_sync(0xFFFFFFFFu, tvBase, pi);
+        u32       vInst = 0;
+        float     vSize = 0.0f;
+        if constexpr(Deform)
         {
-          overflow = true;
-          break;
+          vInst = __shfl_sync(0xFFFFFFFFu, inst, pi);
+          vSize = __shfl_sync(0xFFFFFFFFu, size, pi);
         }
-        const f3 w   = interp3(r.bb[0], r.bb[1], r.bb[2], cfg_vertex(c.table, e, r.cfg, vert));
-        f3       pos = pn ? get_pn(basis, w) : interp3(r.bp[0], r.bp[1], r.bp[2], w);
-        if(r.hasTx)
-          pos = displace(pos, interp3(r.bn[0], r.bn[1], r.bn[2], w),
-                         sample_bilinear(r.tx, interp2(r.bt[0], r.bt[1], r.bt[2], w)), r.scale,
-                         c.view->displacementScale, r.offset, c.view->displacementOffset);
-        if(rp.enabled)
-          pos = ripple(pos, r.inst, r.size, rp);
-        float m[16];
-#pragma unroll
-        for(int q = 0; q < 16; q++)
-          m[q] = __ldg(r.world + q);
-        const f3 wp = xform_point(m, pos);
-        const f3 cp = xform_point(vp, wp);
-        float*   wo = world + 3 * (u64)(r.v0 + vert);
-        float*   co = clip + 4 * (u64)(r.v0 + vert);
-        wo[0] = wp.x, wo[1] = wp.y, wo[2] = wp.z;
-        co[0] = cp.x, co[1] = cp.y, co[2] = cp.z;
-        co[3] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(vp[3], wp.x), __fmul_rn(vp[7], wp.y)), __fmul_rn(vp[11], wp.z)), vp[15]);
+        if(jj < vFit)
+        {
+          const u32 tv = __ldg(c.table.vertices + (tvIdx + jj));
+          f3        p;
+          if(pn)
+            p = affine_displace(sp[pi], tv, part_pn_position(s_pn[Deform ? warp : 0][Deform ? pi : 0], tv));
+          else
+            p = affine_vertex(sp[pi], tv);
+          if(rp.enabled)
+            p = ripple(p, vInst, vSize, rp);
+          const float4 mx = s_world[warp][pi][0], my = s_world[warp][pi][1], mz = s_world[warp][pi][2];
+          const f3     wp = {((mx.x * p.x + mx.y * p.y) + mx.z * p.z) + mx.w, ((my.x * p.x + my.y * p.y) + my.z * p.z) + my.w,
+                             ((mz.x * p.x + mz.y * p.y) + mz.z * p.z) + mz.w};
+          const f3     cp = xform_point(vp, wp);
+          const float  cw = ((vp[3] * wp.x + vp[7] * wp.y) + vp[11] * wp.z) + vp[15];
+          float*       wo = world + 3 * (u64)(off.y + jj);
+          float*       co = clip + 4 * (u64)(off.y + jj);
+          wo[0] = wp.x, wo[1] = wp.y, wo[2] = wp.z;
+          if(clip16)
+            *reinterpret_cast<float4*>(co) = make_float4(cp.x, cp.y, cp.z, cw);
+          else
+            co[0] = cp.x, co[1] = cp.y, co[2] = cp.z, co[3] = cw;
+        }
       }
-      for(u32 tri = lane; tri < e.numTriangles; tri += 32)
+      const u32 tBegin = __shfl_sync(0xFFFFFFFFu, exT, pBegin), tEnd = __shfl_sync(0xFFFFFFFFu, s.sumT, pEnd - 1);
+      const u32 tFit = o.maxTriangles > off.z ? min(tEnd, o.maxTriangles - off.z) : 0u;
+      overflow |= tFit < tEnd;
+#pragma unroll 2
+      for(u32 base = tBegin; base < tFit; base += 32)
       {
-        if(r.t0 + tri >= o.maxTriangles)
+        const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && exT <= base));
+        const u32 inside =
+            __reduce_or_sync(0xFFFFFFFFu, (owner && exT > base && exT < base + 32) ? 1u << (exT - base) : 0u);
+        const u32 pi = (pBegin + before - 1 + __popc(inside & below)) & 31;
+        const u32 jj = base + lane;
+        const u32 tb = __shfl_sync(0xFFFFFFFFu, triBase, pi), mt = __shfl_sync(0xFFFFFFFFu, meta, pi);
+        const u32 first = __shfl_sync(0xFFFFFFFFu, exT, pi);
+        if(jj < tFit)
         {
-          overflow = true;
-          break;
+          const u32 packed = __ldg(c.table.triangles + (tb + jj));
+          const u32 a = packed & 0xFF, b1 = (packed >> 8) & 0xFF, b2 = (packed >> 16) & 0xFF;
+          const bool flip = (mt >> 28) != 0;  // tessellation.glsl:165-176 (flip -> .xzy)
+          const u32  vs = mt & 0xFF, ID = visTriangles ? (jj - first) * 3 : (mt >> 16) & 0xFFFu;
+          uint8_t*   d = idx + 3 * (u64)(off.z + jj);
+          d[0] = (uint8_t)(a + vs), d[1] = (uint8_t)((flip ? b2 : b1) + vs), d[2] = (uint8_t)((flip ? b1 : b2) + vs);
+          prim[off.z + jj] = ((mt >> 8) & 0xFFu) | ((ID | 1u) << 8);
         }
-        const uint3 ct = cfg_triangle(c.table, e, r.cfg, tri);
-        uint8_t*    d  = idx + 3 * (u64)(r.t0 + tri);
-        d[0] = (uint8_t)(ct.x + r.vs), d[1] = (uint8_t)(ct.y + r.vs), d[2] = (uint8_t)(ct.z + r.vs);
-        prim[r.t0 + tri] = (r.triID & 0xFFu) | (((visTriangles ? tri * 3 : r.partID) | 1u) << 8);
       }
     }
     __syncwarp();  // the records are rewritten by the warp's next group
@@ -325,14 +377,19 @@ cudaError_t launch_raster_batches(const StageCtx& c, uint4* groups, const tc_ras
 {
   const u32   ngroups = std::max(1u, (maxParts + 31) / 32);
   const u32   grid    = std::max(1u, std::min((ngroups + 7) / 8, numSMs * 8));
-  const u32   wgrid   = std::max(1u, std::min((ngroups * kWarpsPerGroup + 7) / 8, numSMs * 8));
+  // one wave of the write blocks (their shared memory lets eight share an SM,
+  // four with the PN records); small capacities get four warps per group
+  const bool  deform = (c.flags & (TC_FLAG_PN | TC_FLAG_RIPPLE)) != 0;
+  const u32   wgrid  = std::max(1u, std::min(ngroups, numSMs * (deform ? 4u : 8u)));
   cudaError_t e       = launch_pdl(k_raster_counts, grid, kRasterBlock, s, c, groups);
   if(e != cudaSuccess)
     return e;
   e = launch_pdl(k_raster_scan, 1u, 1024u, s, c, groups, reinterpret_cast<u32*>(o.counts));
   if(e != cudaSuccess)
     return e;
-  return launch_pdl(k_raster_write, wgrid, kRasterBlock, s, c, const_cast<const uint4*>(groups), o);
+  if(deform)
+    return launch_pdl(k_raster_write<true>, wgrid, kWriteBlock, s, c, const_cast<const uint4*>(groups), o);
+  return launch_pdl(k_raster_write<false>, wgrid, kWriteBlock, s, c, const_cast<const uint4*>(groups), o);
 }
 
 }  // namespace tc

@@ -438,4 +438,98 @@ __device__ __forceinline__ f3 ripple(f3 p, u32 seed, float size, const RipplePar
   return {p.x + dir.x * (amp * wave.x), p.y + dir.y * (amp * wave.y), p.z + dir.z * (amp * wave.z)};
 }
 
+// ---------------------------------------------------------------------------
+// The PN-triangle cubic of a part in per-part form (TC_FLAG_PN): the base
+// triangle's control points with the cubic's binomial factors multiplied in
+// (the same first product as get_pn's), and the base barycentrics of a table
+// vertex w = (1 - a - b, a, b) as W0 + a W1 + b W2 (the composition with the
+// sub-triangle's corners, exact up to one rounding per term: the corners are
+// multiples of 2^-15). A vertex takes ten weights shared by x, y and z and
+// three fused multiply-adds for each control point, in place of get_pn's
+// separate products per component.
+// ---------------------------------------------------------------------------
+
+// 176-byte stride: records of an array start in different bank groups.
+struct __align__(16) PartPn
+{
+  float4 q[11];
+  // q[0]..q[7].y: b300, b030, b003, 3 b210, 3 b120, 3 b201, 3 b021, 3 b102, 3 b012, 6 b111 (xyz each)
+  // q[7].zw, q[8].x: W0; q[8].yzw: W1; q[9].xyz: W2
+};
+
+__device__ __forceinline__ void write_part_pn(PartPn& r, const u32 corner[3], bool flipped, const BasePN& b)
+{
+  f3 c0 = decode_bary(corner[0]), c1 = decode_bary(corner[1]), c2 = decode_bary(corner[2]);
+  if(flipped)
+  {
+    const f3 t = c0;
+    c0         = c1;
+    c1         = t;
+  }
+  const f3 w1 = sub3(c1, c0), w2 = sub3(c2, c0);
+  const f3 b210 = mul3(b.b210, 3.0f), b120 = mul3(b.b120, 3.0f), b201 = mul3(b.b201, 3.0f), b021 = mul3(b.b021, 3.0f),
+           b102 = mul3(b.b102, 3.0f), b012 = mul3(b.b012, 3.0f), b111 = mul3(b.b111, 6.0f);
+  r.q[0] = make_float4(b.b300.x, b.b300.y, b.b300.z, b.b030.x);
+  r.q[1] = make_float4(b.b030.y, b.b030.z, b.b003.x, b.b003.y);
+  r.q[2] = make_float4(b.b003.z, b210.x, b210.y, b210.z);
+  r.q[3] = make_float4(b120.x, b120.y, b120.z, b201.x);
+  r.q[4] = make_float4(b201.y, b201.z, b021.x, b021.y);
+  r.q[5] = make_float4(b021.z, b102.x, b102.y, b102.z);
+  r.q[6] = make_float4(b012.x, b012.y, b012.z, b111.x);
+  r.q[7] = make_float4(b111.y, b111.z, c0.x, c0.y);
+  r.q[8] = make_float4(c0.z, w1.x, w1.y, w1.z);
+  r.q[9] = make_float4(w2.x, w2.y, w2.z, 0.0f);
+}
+
+// Position on the cubic at table vertex `tableVertex` (displacement.glsl:80-104)
+__device__ __forceinline__ f3 part_pn_position(const PartPn& r, u32 tableVertex)
+{
+  const float  a  = __uint2float_rn(tableVertex & 0xFFFFu) * (1.0f / 32768.0f);
+  const float  b  = __uint2float_rn(tableVertex >> 16) * (1.0f / 32768.0f);
+  const float4 q7 = r.q[7], q8 = r.q[8], q9 = r.q[9];
+  const float  u = __fmaf_rn(b, q9.x, __fmaf_rn(a, q8.y, q7.z)), v = __fmaf_rn(b, q9.y, __fmaf_rn(a, q8.z, q7.w)),
+               w = __fmaf_rn(b, q9.z, __fmaf_rn(a, q8.w, q8.x));
+  const float u2 = u * u, v2 = v * v, w2 = w * w;
+  f3          p;
+  {
+    const float4 q0 = r.q[0], q1 = r.q[1];
+    const float  k300 = w2 * w, k030 = u2 * u, k003 = v2 * v;
+    const float4 q2 = r.q[2];
+    p = {k300 * q0.x, k300 * q0.y, k300 * q0.z};
+    p = fma3(k030, {q0.w, q1.x, q1.y}, p);
+    p = fma3(k003, {q1.z, q1.w, q2.x}, p);
+    p = fma3(w2 * u, {q2.y, q2.z, q2.w}, p);
+  }
+  {
+    const float4 q3 = r.q[3], q4 = r.q[4];
+    p = fma3(w * u2, {q3.x, q3.y, q3.z}, p);
+    p = fma3(w2 * v, {q3.w, q4.x, q4.y}, p);
+    const float4 q5 = r.q[5];
+    p = fma3(u2 * v, {q4.z, q4.w, q5.x}, p);
+    p = fma3(w * v2, {q5.y, q5.z, q5.w}, p);
+  }
+  const float4 q6 = r.q[6];
+  p = fma3(u * v2, {q6.x, q6.y, q6.z}, p);
+  return fma3((w * u) * v, {q6.w, q7.x, q7.y}, p);
+}
+
+// Displacement of the part in `r` at table vertex `tableVertex` added to `P`
+// (its map, scale and offset from the record).
+__device__ __forceinline__ f3 affine_displace(const PartAffine& r, u32 tableVertex, f3 P)
+{
+  const u32 kind = affine_kind_of(r);
+  if(kind == kAffineFlat)
+    return P;
+  const float  a  = __uint2float_rn(tableVertex & 0xFFFFu) * (1.0f / 32768.0f);
+  const float  b  = __uint2float_rn(tableVertex >> 16) * (1.0f / 32768.0f);
+  const float4 q2 = r.q[2], q3 = r.q[3], q4 = r.q[4], q5 = r.q[5], q6 = r.q[6];
+  const f3     N = {__fmaf_rn(b, q3.w, __fmaf_rn(a, q3.x, q2.y)), __fmaf_rn(b, q4.x, __fmaf_rn(a, q3.y, q2.z)),
+                    __fmaf_rn(b, q4.y, __fmaf_rn(a, q3.z, q2.w))};
+  const float  u      = __fmaf_rn(b, q5.z, __fmaf_rn(a, q5.x, q4.z));
+  const float  v      = __fmaf_rn(b, q5.w, __fmaf_rn(a, q5.y, q4.w));
+  const float  height = __fmaf_rn(sample_kind(kind, r.q[7], r.q[8], u, v), q6.x, q6.y);
+  const float  k      = height * rsqrtf(__fmaf_rn(N.z, N.z, __fmaf_rn(N.y, N.y, N.x * N.x)));
+  return fma3(k, N, P);
+}
+
 }  // namespace tc
