@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from tests.conftest import cuda_available
-from tests.parity import vertex_tolerance
+from tests.parity import assert_same, vertex_tolerance
 from vk_tessellated_clusters_gb300 import layouts as L
 from vk_tessellated_clusters_gb300 import scene as S
 
@@ -59,4 +59,27 @@ def test_raster_group_sharing(oracle, instances, pixels, flags, parts):
         raw = bufs[f].read(np.uint8, min(bufs[f].nbytes, count * dtype().itemsize + 64))
         size = count * dtype().itemsize
         assert raw[:size].tobytes() == got[f].reshape(-1)[:count].tobytes() and (raw[size:] == 0xAB).all(), f
+    pipe.close()
+
+
+# 80 to 20,480 parts on grids of 608 and 152 blocks: chunks of 1, 2, 4, 8, 16 and 32 parts, some cut by the end
+@pytest.mark.parametrize("subdivisions,pixels", [(1, 6.0), (2, 5.0), (3, 8.0), (4, 5.0), (5, 8.0)])
+@pytest.mark.parametrize("grid", [0, 1])
+def test_vertex_chunk_widths(oracle, subdivisions, pixels, grid):
+    """Frame graph and stage entry points against the oracle, integers bit-exact and positions to the vertex
+    tolerance, whatever number of parts a warp takes at a time."""
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_icosphere(subdivisions=subdivisions, map_size=64)
+    cam = S.Camera(eye=(0.3, 0.2, 2.5), center=(0.0, 0.0, 0.0), tess_rate_pixels=pixels)
+    caps = L.default_caps(visible_bits=12, part_bits=17, split_bits=14, vertex_bits=21, megs=256)
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    want = ref_state.outputs(oracle.entries)
+    pipe = TessellationPipeline(sc, caps, FLAGS, schedule={"vertexGridPerSM": grid})
+    pipe.set_cameras(cam)
+    pipe.build("graph")
+    assert_same(pipe.outputs(), want, "graph", vertex_tol=vertex_tolerance(sc))
+    pipe.state.gen_vertices.handle.zero_()
+    pipe.build("plain")  # k_instantiate_parts, one launch per instance and run
+    assert_same(pipe.outputs(), want, "stages", vertex_tol=vertex_tolerance(sc))
+    assert pipe.device_errors() == 0
     pipe.close()

@@ -18,10 +18,11 @@
 //               reference counts and statistics.
 //   vertices  : 12 B written per generated vertex. A warp takes chunks of 32
 //               consecutive parts (its first by index, the rest from a
-//               ticket): every part's affine vertex form (tc_vertex.cuh) is
-//               set up once in shared memory, one part per lane, then the
-//               lanes walk the chunk's contiguous vertex range on consecutive
-//               vertices.
+//               ticket; fewer parts per chunk when the frame has fewer
+//               chunks than the grid has warps): every part's affine vertex
+//               form (tc_vertex.cuh) is set up once in shared memory, one part
+//               per lane, then the lanes walk the chunk's contiguous vertex
+//               range on consecutive vertices.
 #include <algorithm>
 
 #include "tc_kernels.h"
@@ -624,6 +625,23 @@ __device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffi
 #undef TC_CHUNK
 }
 
+// Parts per chunk of a launch with `n` parts and `nwarps` warps: 32 (a lane
+// sets up one part), halved while the chunks still take no more than half of
+// the warps. The parts of a small frame have up to 78 vertices each, so 32 of
+// them in a row keep one warp busy for 50 us while most of the chip idles:
+// 1,280 parts of 36 vertices took 54.7 us in 40 chunks of 32 and take 11.7 us
+// in 1,280 chunks of one (the frame 69.8 -> 48.3 us). Near a chunk per warp
+// the split gains nothing: the full clusters' vertices and the allocations
+// beside it use the rest of the chip (60,000 parts in 16s: the frame 0.5 %
+// slower).
+__device__ __forceinline__ u32 chunk_parts(u32 n, u32 nwarps)
+{
+  u32 w = kPartsPerWarp;
+  while(w > 1 && (n + w / 2 - 1) / (w / 2) <= nwarps / 2)
+    w >>= 1;
+  return w;
+}
+
 // cp.async: 4- and 8-byte global -> shared copies (the next chunk's part
 // records and vertex offsets, fetched while the current chunk is generated)
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem, int bytes)
@@ -664,14 +682,15 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_vertices(Stag
   const tc_TessTriangleInfo* parts     = reinterpret_cast<const tc_TessTriangleInfo*>(b->partTriangles);
   float*                     gv        = reinterpret_cast<float*>(b->genVertices);
   const u32                  nwarps    = (gridDim.x * blockDim.x) >> 5;
-  const u32                  numChunks = (n + kPartsPerWarp - 1) / kPartsPerWarp;
+  const u32                  width     = chunk_parts(n, nwarps);
+  const u32                  numChunks = (n + width - 1) / width;
   PartAffine*                sp        = s_part[warp];
   ChunkStage&                stage     = s_stage[warp];
 
   // stage chunk `ck`'s records (each lane its own part; no other lane reads them)
   auto prefetch = [&](u32 ck) {
-    const u32 q = ck * kPartsPerWarp + lane;
-    if(ck < numChunks && q < n)
+    const u32 q = ck * width + lane;
+    if(ck < numChunks && lane < width && q < n)
     {
       const uint2* raw = reinterpret_cast<const uint2*>(parts + begin + q);
       cp_async(&stage.rec[0][lane], raw, 8);
@@ -746,7 +765,9 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
   const tc_caps&             k         = c.caps;
   const u64                  maxData   = (u64)k.maxGeneratedClusterMegs * 1024ull * 1024ull;
   const u32                  nwarps    = (gridDim.x * blockDim.x) >> 5;
-  const u32                  numChunks = (n + kPartsPerWarp - 1) / kPartsPerWarp;
+  const u32                  width     = chunk_parts(n, nwarps);
+  const u32                  share     = kPartsPerWarp / width;  // chunks per 32 parts (the allocation's chunks)
+  const u32                  numChunks = (n + width - 1) / width;
   const u32                  numTiles  = clamp_tiles(c, (n + kTile - 1) / kTile);
   const u32                  stride    = c.scratch.lbStride;
   const u64                  genBase   = c.scratch.totals[0];
@@ -758,8 +779,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
 
   // stage chunk `ck`'s records; vo marks the lanes with a part (0) or none (~0)
   auto prefetch = [&](u32 ck) {
-    const u32 q = ck * kPartsPerWarp + lane;
-    if(ck < numChunks && q < n && (ck / kChunksPerTile) < numTiles)
+    const u32 q = ck * width + lane;
+    if(ck < numChunks && lane < width && q < n && q / kTile < numTiles)
     {
       const uint2* raw = reinterpret_cast<const uint2*>(parts + begin + q);
       cp_async(&stage.rec[0][lane], raw, 8);
@@ -787,14 +808,23 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
     const u32   cfg = r2.y >> 16;
     const u64   own = valid ? part_packed(c, cfg) : 0ull;
 
-    // ---- offsets: tile + chunk within the tile + lane within the chunk ------
-    const u32 tile = chunk / kChunksPerTile, w = chunk % kChunksPerTile;
-    const u64 cs   = ib.chunkSums[tile * kChunksPerTile + lane];
-    const u64 csi  = warp_inclusive<u64>(cs, lane);
-    const u64 pre  = __shfl_sync(0xFFFFFFFFu, csi - cs, w);
-    const u64 inc  = warp_inclusive<u64>(own, lane);
-    const u64 within       = pre + inc - own;
-    const u32 q            = chunk * kPartsPerWarp + lane;
+    // ---- offsets: tile + 32 parts within the tile + lane within those -------
+    const u32 group = chunk / share, tile = group / kChunksPerTile, w = group % kChunksPerTile;
+    const u64 cs    = ib.chunkSums[tile * kChunksPerTile + lane];
+    const u64 csi   = warp_inclusive<u64>(cs, lane);
+    const u64 pre   = __shfl_sync(0xFFFFFFFFu, csi - cs, w);
+    u64       before = 0;  // the chunk's parts before the lane's
+    if(share == 1)
+      before = warp_inclusive<u64>(own, lane) - own;
+    else
+    {
+      const u32 qa  = group * kPartsPerWarp + lane;
+      const u64 all = qa < n ? part_packed(c, part_cfg(parts, begin + qa)) : 0ull;
+      const u64 ex  = warp_inclusive<u64>(all, lane) - all;
+      before        = __shfl_sync(0xFFFFFFFFu, ex, (chunk % share) * width + lane);
+    }
+    const u64 within       = pre + before;
+    const u32 q            = chunk * width + lane;
     const u32 nvPart       = (u32)(own & kPackMask);
     const u32 ds           = (u32)(own >> kPackShift);
     const u64 genOffset    = genBase + q;
