@@ -83,3 +83,41 @@ def test_vertex_chunk_widths(oracle, subdivisions, pixels, grid):
     assert_same(pipe.outputs(), want, "stages", vertex_tol=vertex_tolerance(sc))
     assert pipe.device_errors() == 0
     pipe.close()
+
+
+def _ripple(cam):
+    fc = S.frame_constants(cam)
+    fc["animationRippleAmplitude"], fc["animationRippleFrequency"] = 0.02, 8.0
+    fc["animationRippleSpeed"], fc["animationState"] = 1.5, 0.7
+    return fc
+
+
+# with PN or the ripple: 320 to 20,480 parts (chunks of 1 to 16 parts); 2X batches below and above one per warp
+@pytest.mark.parametrize("case", ["ico2_pn", "ico4_pn_ripple", "ico5_ripple", "transient_24", "transient_256"])
+def test_deform_chunk_widths(oracle, case):
+    """Integers bit-exact against the oracle, positions to the vertex tolerance; an empty displacement map still
+    displaces by the offsets (ico5_ripple)."""
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    flags = FLAGS
+    if case.startswith("ico"):
+        sc = S.scene_icosphere(subdivisions=int(case[3]), map_size=64)
+        cam = S.Camera(eye=(0.3, 0.2, 2.5), center=(0.0, 0.0, 0.0), tess_rate_pixels=6.0)
+        flags |= (L.FLAG_PN if "pn" in case else 0) | (L.FLAG_RIPPLE if "ripple" in case else 0)
+        if case == "ico5_ripple":
+            sc.textures[0] = S.Texture(np.zeros((0, 0), np.float32), L.TEXEL_F32)
+            sc.instances[0].displacement_offset = 0.125
+    else:
+        sc, cam = S.scene_batched(num_instances=int(case[10:]), map_size=64), S.camera_orbit(0)
+        flags |= L.FLAG_TRANSIENT_1X | L.FLAG_TRANSIENT_2X | L.FLAG_PN | L.FLAG_RIPPLE
+    fc = _ripple(cam)
+    caps = L.default_caps(vertex_bits=22)
+    ref_state, _ = oracle.frame(sc, fc, caps, flags)
+    want = ref_state.outputs(oracle.entries)
+    if case == "transient_256":
+        assert len(want["transBuilds"]) > 152 * 7 * 4  # more builds than the kernel's warps: two per warp
+    pipe = TessellationPipeline(sc, caps, flags)
+    pipe.set_cameras(fc)
+    pipe.build("graph")
+    assert_same(pipe.outputs(), want, case, vertex_tol=vertex_tolerance(sc))
+    assert pipe.device_errors() == 0
+    pipe.close()

@@ -25,6 +25,7 @@
 //           the records write leaves (a launch of its own, beside later work)
 #include <algorithm>
 
+#include "tc_deform.cuh"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
@@ -1010,69 +1011,7 @@ __device__ __forceinline__ void store_clas_build(tc_ClasBuildInfo* dst, u32 mode
   d[3]     = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// cluster_classify.comp.glsl:810-878: one base triangle of a 2X batch (its
-// word's config and corner rotation): its 3 to 6 vertices at its batch slot
-__device__ inline void mini_vertices(const StageCtx& c, const tc_RenderInstance* in, const tc_Cluster& cl, u32 inst,
-                                     u32 tri, u32 word, u32 rel, u32 vertexOffset, const RippleParams& rp)
-{
-  tc_SceneBuilding* b   = c.build;
-  const u32         cfg = word & 0xFFFFu;
-  const tc_TessTableEntry e = table_entry(c.table, cfg);
-  u32               enc[3] = {0u, TC_TESSTABLE_COORD_MAX, TC_TESSTABLE_COORD_MAX << 16};
-  const u32         rot    = (word >> 16) & 3;
-  if(rot == 1)
-  {
-    const u32 t0 = enc[0];
-    enc[0] = enc[1], enc[1] = enc[2], enc[2] = t0;
-  }
-  else if(rot == 2)
-  {
-    const u32 t2 = enc[2];
-    enc[2] = enc[1], enc[1] = enc[0], enc[0] = t2;
-  }
-  const uint8_t* lt = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
-  f3             bp[3], bn[3], bb[3];
-  f2             bt[3];
-  for(int q = 0; q < 3; q++)
-  {
-    const u32 vi = cl.firstLocalVertex + lt[tri * 3 + q];
-    bp[q]        = ldg3(reinterpret_cast<const float*>(in->positions), vi);
-    bn[q]        = normalize3(ldg3(reinterpret_cast<const float*>(in->normals), vi));
-    bt[q]        = ldg2(reinterpret_cast<const float*>(in->texcoords), vi);
-    bb[q]        = decode_bary(enc[q]);
-  }
-  tc_DisplacementTexture tx    = {};
-  bool                   hasTx = false;
-  if(c.numTextures > 0 && c.textures != nullptr && in->displacementIndex >= 0)
-  {
-    if((u32)in->displacementIndex < c.numTextures)
-    {
-      tx    = c.textures[in->displacementIndex];
-      hasTx = true;
-    }
-    else
-      atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
-  }
-  const bool pn    = (c.flags & TC_FLAG_PN) != 0;
-  BasePN     basis = {};
-  if(pn)
-    basis = setup_pn(bp[0], bp[1], bp[2], bn[0], bn[1], bn[2]);
-  float* gv = reinterpret_cast<float*>(b->genVertices);
-  for(u32 vert = 0; vert < e.numVertices; vert++)
-  {
-    const f3 w   = interp3(bb[0], bb[1], bb[2], cfg_vertex(c.table, e, cfg, vert));
-    f3       pos = pn ? get_pn(basis, w) : interp3(bp[0], bp[1], bp[2], w);
-    if(hasTx)
-      pos = displace(pos, interp3(bn[0], bn[1], bn[2], w), sample_bilinear(tx, interp2(bt[0], bt[1], bt[2], w)),
-                     in->displacementScale, c.view->displacementScale, in->displacementOffset, c.view->displacementOffset);
-    if(rp.enabled)
-      pos = ripple(pos, inst, in->geoHi.w, rp);
-    float* d = gv + 3 * ((u64)vertexOffset + rel * TC_2X_MINI_VERTICES + vert);
-    d[0] = pos.x, d[1] = pos.y, d[2] = pos.z;
-  }
-}
-
-// the same base triangle's u16 map entries and u8 indices (:880-903)
+// a 2X batch's base triangle: its u16 map entries and u8 indices (:880-903)
 __device__ inline void mini_indices(const StageCtx& c, u32 tri, u32 word, u32 rel, u32 baseTris, u32 vertexOffset,
                                     u32 partOffset)
 {
@@ -1209,13 +1148,8 @@ __device__ inline void write_cluster_transient(const StageCtx& c, const Classify
   }
   else if(lane == 0)
     cs.fullRecs[v] = make_uint2(kRejected, 0u);
-  u32 miniChunk[4] = {0u, 0u, 0u, 0u};  // per chunk: first batch vertex, accepted batches
   if(full)
-  {
-    if(lane == 0)
-      reinterpret_cast<uint4*>(cs.counts)[v] = make_uint4(0u, 0u, 0u, 0u);
     return;
-  }
 
   // ---- :543-905 the other triangles, one 32-triangle chunk at a time -------------
   const u32*   tw  = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
@@ -1316,21 +1250,9 @@ __device__ inline void write_cluster_transient(const StageCtx& c, const Classify
         }
         mini_indices(c, tri, word, rel, incl - ntris - first, vq, po);
       }
-      // for k_classify_mini_vertices: the chunk's first batch vertex and its accepted batches
-      u32 okMask = 0;
-      for(u32 qq = 0; qq < nb; qq++)
-        okMask |= fits_q(qq) ? 1u << qq : 0u;
-      if(lane == 0)
-      {
-        miniChunk[2 * (t0 >> 5)]     = vo;
-        miniChunk[2 * (t0 >> 5) + 1] = okMask;
-      }
-      __syncwarp();
       g += nb, vo += kMiniVertexSize * nb, d += dataSize * nb, tr += nb, y += kMiniPartSlots * nb;
     }
   }
-  if(lane == 0)  // (counts of this cluster were read into shared memory before)
-    reinterpret_cast<uint4*>(cs.counts)[v] = make_uint4(miniChunk[0], miniChunk[1], miniChunk[2], miniChunk[3]);
 }
 
 // The offsets at which block `blockIdx.x` of the write launch starts, with
@@ -1451,48 +1373,84 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
   }
 }
 
-// cluster_classify.comp.glsl:810-878: the vertices of the accepted 2X
-// batches, from what k_classify_write_transient left per cluster (each
-// chunk's first batch vertex and accepted batches, in place of its counts).
-// One warp per cluster, one lane per base triangle.
-__global__ void __launch_bounds__(kBlock, 2) k_classify_mini_vertices(StageCtx c, ClassifyScratch cs)
+// cluster_classify.comp.glsl:810-878: the vertices of the launch's accepted 2X
+// batches, from their build records: the batch's base triangles are the first
+// entries of its triangle map (table triangle 0), whose edge factors give the
+// configuration. A warp takes two builds at a time (one lane per base
+// triangle), one when there are not enough for every warp, then one lane per
+// vertex (3 to 6 per base triangle; tc_deform.cuh).
+__global__ void __launch_bounds__(kDeformBlock, kDeformBlocksPerSM) k_classify_mini_vertices(StageCtx c, ClassifyScratch cs)
 {
   stage_prologue();
-  __shared__ u32        s_range[2];
-  __shared__ FlatStarts s_starts;
-  if(threadIdx.x == 0)
-    window_range(c, s_range[0], s_range[1]);
-  __syncthreads();
-  const u32*            starts = stage_flat_starts(c, s_starts);
-  const u32             lane = threadIdx.x & 31, ltm = (1u << lane) - 1u;
-  const u32             begin = s_range[0];
-  const u32             n     = min(s_range[1] - s_range[0], c.scratch.itemCapacity);
-  const tc_ClusterInfo* vis   = reinterpret_cast<const tc_ClusterInfo*>(c.build->visibleClusters);
-  const RippleParams    rp    = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
-  const u32             nwarps = (gridDim.x * blockDim.x) >> 5;
-  for(u32 v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps)
+  __shared__ DeformRecords s_rec[kDeformWarps];
+  __shared__ uint4         s_lane[kDeformWarps][32];
+  const u32                lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ltm = (1u << lane) - 1u;
+  const tc_SceneBuilding*  b      = c.build;
+  const tc_ClasBuildInfo*  builds = reinterpret_cast<const tc_ClasBuildInfo*>(b->transBuilds);
+  const uint8_t*           ptb    = reinterpret_cast<const uint8_t*>(b->partTriangles);
+  float*                   gv     = reinterpret_cast<float*>(b->genVertices);
+  const bool               pn     = (c.flags & TC_FLAG_PN) != 0;
+  const RippleParams       rp     = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
+  // accepted builds take consecutive slots after those before the launch
+  const u32 first = reinterpret_cast<const TransBases*>(cs.bases + 1)->trans;
+  const u32 count = max(b->transBuildCounter, first) - first;
+  const u32 nwarps = (gridDim.x * blockDim.x) >> 5;
+  u32       per    = kDeformParts / kMiniBatch;
+  while(per > 1 && (count + per / 2 - 1) / (per / 2) <= nwarps)
+    per >>= 1;
+  DeformRecords& rec = s_rec[warp];
+  for(u32 k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k * per < count; k += nwarps)
   {
-    const uint4 m = reinterpret_cast<const uint4*>(cs.counts)[v];
-    if((m.y | m.w) == 0)
-      continue;
-    const tc_ClusterInfo     ci = visible_cluster(c, starts, vis, begin + v);
-    const tc_RenderInstance* in = c.instances + ci.instanceID;
-    const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
-    const u32                nt = min((u32)cl.numTriangles, TC_MAX_CLUSTER_TRIANGLES);
-    const u32*               tw = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
-    for(u32 q = 0; q < 2; q++)
+    // lane's base triangle: number lane % 8 of build lane / 8
+    const u32 j    = k * per + lane / kMiniBatch, rel = lane % kMiniBatch;
+    u32       part = 0, vo = 0, ntri = 0;
+    bool      take = false;
+    if(lane / kMiniBatch < per && j < count)
     {
-      const u32 ok = q ? m.w : m.y, vo = q ? m.z : m.x;
-      if(ok == 0)
-        continue;
-      const u32  tri  = 32 * q + lane;
-      const u32  word = tri < nt ? tw[tri] : 0u;
-      const bool mini = tri < nt && (word & kWordMini);
-      const u32  rank = __popc(__ballot_sync(0xFFFFFFFFu, mini) & ltm);
-      const u32  qb   = rank / kMiniBatch;
-      if(mini && ((ok >> qb) & 1u))
-        mini_vertices(c, in, cl, ci.instanceID, tri, word, rank % kMiniBatch, vo + kMiniVertexSize * qb, rp);
+      const tc_ClasBuildInfo& bi = builds[first + j];
+      part = bi.clusterID & 0x3FFFFFFFu;
+      ntri = bi.packed & 0x1FFu;
+      vo   = (u32)((bi.vertexBuffer - b->genVertices) / 12);
+      take = bi.clusterID >> 30 == TC_RT_CLUSTER_MODE_2X_BATCHED_TESSELLATED;
     }
+    // the rel-th of the map's entries that start a base triangle: each of the
+    // build's lanes tests four of the 32 entries
+    const uint16_t* map    = reinterpret_cast<const uint16_t*>(ptb + (u64)part * kTessInfoBytes + kClusterInfoBytes);
+    u32             starts = 0;
+    if(take)
+    {
+      const uint2 e = reinterpret_cast<const uint2*>(map)[rel];
+#pragma unroll
+      for(u32 i = 0; i < 4; i++)
+        if(4 * rel + i < ntri && (((i & 2 ? e.y : e.x) >> (16 * (i & 1) + 8)) & 3u) == 0)
+          starts |= 1u << (4 * rel + i);
+    }
+    starts = __reduce_or_sync(0xFFu << (lane & 24u), starts);
+    for(u32 i = 0; i < rel; i++)
+      starts &= starts - 1;
+    const bool found = starts != 0;
+    const u32  word  = found ? map[__ffs(starts) - 1] : 0u;
+    const u32 tm = __ballot_sync(0xFFFFFFFFu, found);
+    if(found)
+    {
+      const uint2              hdr = *reinterpret_cast<const uint2*>(ptb + (u64)part * kTessInfoBytes);
+      const tc_RenderInstance& in  = c.instances[hdr.x];
+      const tc_Cluster         cl  = reinterpret_cast<const tc_Cluster*>(in.clusters)[hdr.y];
+      u32                      corner[3] = {0u, TC_TESSTABLE_COORD_MAX, TC_TESSTABLE_COORD_MAX << 16};
+      const u32                cfg = get_config(make_uint3(1u + ((word >> 12) & 1u), 1u + ((word >> 13) & 1u), 1u + ((word >> 14) & 1u)),
+                                                corner[0], corner[1], corner[2]);
+      const tc_TessTableEntry  e    = table_entry(c.table, cfg);
+      const u32                slot = __popc(tm & ltm);
+      setup_deform(c, in, cl, word & 0xFFu, cfg, corner, e.firstVertex, pn, rec.affine[slot], rec.pn[slot]);
+      s_lane[warp][slot] = make_uint4(e.firstVertex | (u32)e.numVertices << 16, vo + rel * TC_2X_MINI_VERTICES, hdr.x,
+                                      __float_as_uint(in.geoHi.w));
+    }
+    __syncwarp();
+    const u32        owners = __popc(tm);
+    const uint4      l      = lane < owners ? s_lane[warp][lane] : make_uint4(0u, 0u, 0u, 0u);
+    const DeformLane d      = {l.x >> 16, l.x & 0xFFFFu, l.y, l.z, __uint_as_float(l.w)};
+    deform_walk(c, rec, owners, d, pn, rp, gv);
+    __syncwarp();  // the records are rewritten by the warp's next builds
   }
 }
 
@@ -1667,9 +1625,10 @@ cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffe
                                      : launch_pdl(k_classify_full_vertices<4>, grid, kBlock, s, c, cs);
   if(e != cudaSuccess || !(c.flags & TC_FLAG_TRANSIENT_2X))
     return e;
-  // the 2X batches' vertices (one warp per visible cluster of the window)
-  const u32 miniGrid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * 8));
-  return launch_pdl(k_classify_mini_vertices, miniGrid, kBlock, s, c, cs);
+  // the 2X batches' vertices (at most eight builds per cluster): warps stride
+  // over the builds, one resident wave of the kernel's blocks
+  const u32 miniGrid = std::max(1u, std::min((maxClusters * 8 + kDeformWarps - 1) / kDeformWarps, numSMs * (u32)kDeformBlocksPerSM));
+  return launch_pdl(k_classify_mini_vertices, miniGrid, kDeformBlock, s, c, cs);
 }
 
 u32 classify_max_blocks(u32 maxClusters) { return std::max(1u, (maxClusters + kWarps - 1) / kWarps); }

@@ -25,6 +25,7 @@
 //               range on consecutive vertices.
 #include <algorithm>
 
+#include "tc_deform.cuh"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
@@ -625,21 +626,40 @@ __device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffi
 #undef TC_CHUNK
 }
 
-// Parts per chunk of a launch with `n` parts and `nwarps` warps: 32 (a lane
-// sets up one part), halved while the chunks still take no more than half of
-// the warps. The parts of a small frame have up to 78 vertices each, so 32 of
-// them in a row keep one warp busy for 50 us while most of the chip idles:
-// 1,280 parts of 36 vertices took 54.7 us in 40 chunks of 32 and take 11.7 us
-// in 1,280 chunks of one (the frame 69.8 -> 48.3 us). Near a chunk per warp
-// the split gains nothing: the full clusters' vertices and the allocations
-// beside it use the rest of the chip (60,000 parts in 16s: the frame 0.5 %
-// slower).
-__device__ __forceinline__ u32 chunk_parts(u32 n, u32 nwarps)
+// Parts per chunk of a launch with `n` parts, `vertices` vertices in all (about)
+// and `nwarps` warps: `most` (a lane sets up one part), halved
+//  - while the chunks still take no more than half of the warps. The parts of
+//    a small frame have up to 78 vertices each, so 32 of them in a row keep
+//    one warp busy for 50 us while most of the chip idles: 1,280 parts of 36
+//    vertices took 54.7 us in 40 chunks of 32 and take 11.7 us in 1,280 chunks
+//    of one (the frame 69.8 -> 48.3 us);
+//  - while there are fewer than two chunks per warp for the ticket to even
+//    out, as long as a chunk keeps 256 vertices (eight steps of the walk) for
+//    its set-up: 25,600 parts of 70 vertices, with PN, took 70.7 us in 800
+//    chunks of 32.
+// Parts of five vertices stay at 32 (60,000 of them in 16s: the frame 0.5 %
+// slower; the full clusters' vertices and the allocations run beside).
+__device__ __forceinline__ u32 chunk_parts(u32 n, u32 vertices, u32 nwarps, u32 most)
 {
-  u32 w = kPartsPerWarp;
-  while(w > 1 && (n + w / 2 - 1) / (w / 2) <= nwarps / 2)
+  u32 w = most;
+  while(w > 1)
+  {
+    const u32 chunks = (n + w / 2 - 1) / (w / 2);
+    if(chunks > nwarps / 2 && (chunks > 2 * nwarps || vertices / chunks < 256))
+      break;
     w >>= 1;
+  }
   return w;
+}
+
+// The vertices of parts [begin, begin + n) from their offsets (0: unknown,
+// some were not accepted).
+__device__ __forceinline__ u32 parts_vertices(const InstantiateBuffers& ib, u32 begin, u32 n)
+{
+  if(n < 2)
+    return 0;
+  const u32 first = ib.vertexOffset[begin], last = ib.vertexOffset[begin + n - 1];
+  return last != ~0u ? last - first : 0u;
 }
 
 // cp.async: 4- and 8-byte global -> shared copies (the next chunk's part
@@ -671,10 +691,14 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_vertices(Stag
   stage_prologue();
   __shared__ PartAffine s_part[kWarps][kPartsPerWarp];
   __shared__ ChunkStage s_stage[kWarps];
-  __shared__ u32        s_range[2];
+  __shared__ u32        s_range[2], s_width;
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if(threadIdx.x == 0)
+  {
     part_range(c, s_range[0], s_range[1]);
+    const u32 count = s_range[1] - s_range[0];
+    s_width = chunk_parts(count, parts_vertices(ib, s_range[0], count), gridDim.x * kWarps, kPartsPerWarp);
+  }
   __syncthreads();
   const u32 begin = s_range[0], n = s_range[1] - s_range[0];
 
@@ -682,7 +706,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_vertices(Stag
   const tc_TessTriangleInfo* parts     = reinterpret_cast<const tc_TessTriangleInfo*>(b->partTriangles);
   float*                     gv        = reinterpret_cast<float*>(b->genVertices);
   const u32                  nwarps    = (gridDim.x * blockDim.x) >> 5;
-  const u32                  width     = chunk_parts(n, nwarps);
+  const u32                  width     = s_width;
   const u32                  numChunks = (n + width - 1) / width;
   PartAffine*                sp        = s_part[warp];
   ChunkStage&                stage     = s_stage[warp];
@@ -765,11 +789,13 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
   const tc_caps&             k         = c.caps;
   const u64                  maxData   = (u64)k.maxGeneratedClusterMegs * 1024ull * 1024ull;
   const u32                  nwarps    = (gridDim.x * blockDim.x) >> 5;
-  const u32                  width     = chunk_parts(n, nwarps);
-  const u32                  share     = kPartsPerWarp / width;  // chunks per 32 parts (the allocation's chunks)
-  const u32                  numChunks = (n + width - 1) / width;
   const u32                  numTiles  = clamp_tiles(c, (n + kTile - 1) / kTile);
   const u32                  stride    = c.scratch.lbStride;
+  // (the last tile's vertices, not in its own offset, don't change the rule)
+  const u32                  vertices  = numTiles < 2 ? 0u : (u32)(c.scratch.lbState[2 * stride + numTiles - 1] - c.scratch.lbState[2 * stride]);
+  const u32                  width     = chunk_parts(n, vertices, nwarps, kPartsPerWarp);
+  const u32                  share     = kPartsPerWarp / width;  // chunks per 32 parts (the allocation's chunks)
+  const u32                  numChunks = (n + width - 1) / width;
   const u64                  genBase   = c.scratch.totals[0];
   const u64                  tempBase  = c.scratch.totals[1];
   PartAffine*                sp        = s_part[warp];
@@ -943,77 +969,59 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
 }
 
 // triangle_tess_template_instantiate.comp.glsl:295-371 with TESS_USE_PN and /
-// or DO_ANIMATION: eight lanes per part triangle over its vertices; the
-// PN basis and the base attributes stay in registers. Written like the CPU
-// restatement (tess_interpolate of the base barycentrics, the reference-order
-// sampling and displacement) rather than in the affine form of the fast path.
-__global__ void __launch_bounds__(kBlock) k_instantiate_vertices_deform(StageCtx c, InstantiateBuffers ib)
+// or DO_ANIMATION: chunks of up to 32 parts per warp as in
+// k_instantiate_vertices, records and vertex walk of tc_deform.cuh.
+__global__ void __launch_bounds__(kDeformBlock, kDeformBlocksPerSM) k_instantiate_vertices_deform(StageCtx c, InstantiateBuffers ib)
 {
   stage_prologue();
-  __shared__ u32 s_range[2];
-  const u32 lane = threadIdx.x & 31;
+  __shared__ DeformRecords s_rec[kDeformWarps];
+  __shared__ u32           s_range[2], s_width;
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if(threadIdx.x == 0)
-    part_range(c, s_range[0], s_range[1]);
-  __syncthreads();
-  const u32                  begin = s_range[0], end = s_range[1];
-  const tc_SceneBuilding*    b     = c.build;
-  const tc_TessTriangleInfo* parts = reinterpret_cast<const tc_TessTriangleInfo*>(b->partTriangles);
-  float*                     gv    = reinterpret_cast<float*>(b->genVertices);
-  const bool                 pn    = (c.flags & TC_FLAG_PN) != 0;
-  const RippleParams         rp    = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
-  // eight lanes per part (parts average a handful of vertices), four parts per warp
-  const u32                  subLane = lane & 7;
-  const u32                  nsubs  = (gridDim.x * blockDim.x) >> 3;
-  for(u32 p = begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 3); p < end; p += nsubs)
   {
-    const u32 vo = ib.vertexOffset[p];
-    if(vo == ~0u)
-      break;  // accepted parts form a prefix of the part order
-    const tc_TessTriangleInfo pt  = parts[p];
-    const u32                 cfg = pt.subTriangle.triangleID_config >> 16;
-    const u32                 tri = pt.subTriangle.triangleID_config & 0xFFFFu;
-    const tc_TessTableEntry   e   = table_entry(c.table, cfg);
-    const tc_RenderInstance&  in  = c.instances[pt.cluster.instanceID];
-    const tc_Cluster          cl  = reinterpret_cast<const tc_Cluster*>(in.clusters)[pt.cluster.clusterID];
-    const uint8_t*            lt  = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle;
-    f3                        bp[3], bn[3], bb[3];
-    f2                        bt[3];
-    for(int v = 0; v < 3; v++)
+    part_range(c, s_range[0], s_range[1]);
+    const u32 count = s_range[1] - s_range[0];
+    s_width = chunk_parts(count, parts_vertices(ib, s_range[0], count), gridDim.x * kDeformWarps, kDeformParts);
+  }
+  __syncthreads();
+  const u32                  begin = s_range[0], n = s_range[1] - s_range[0];
+  const tc_SceneBuilding*    b      = c.build;
+  const tc_TessTriangleInfo* parts  = reinterpret_cast<const tc_TessTriangleInfo*>(b->partTriangles);
+  float*                     gv     = reinterpret_cast<float*>(b->genVertices);
+  const bool                 pn     = (c.flags & TC_FLAG_PN) != 0;
+  const RippleParams         rp     = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
+  const u32                  nwarps = (gridDim.x * blockDim.x) >> 5;
+  const u32                  width  = s_width;
+  const u32                  numChunks = (n + width - 1) / width;
+  DeformRecords&             rec    = s_rec[warp];
+  u32                        chunk  = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  while(chunk < numChunks)
+  {
+    u32 following = 0;
+    if(lane == 0)
+      following = nwarps + atomicAdd(c.scratch.ticket, 1u);
+    const u32  q = chunk * width + lane, p = begin + q;
+    const u32  vo       = lane < width && q < n ? ib.vertexOffset[p] : ~0u;
+    const bool accepted = vo != ~0u;
+    const u32  count    = __popc(__ballot_sync(0xFFFFFFFFu, accepted));  // accepted parts form a prefix of the part order
+    if(count == 0)
+      break;
+    DeformLane d = {0u, 0u, vo, 0u, 0.0f};
+    if(accepted)
     {
-      const u32 vi = cl.firstLocalVertex + lt[tri * 3 + v];
-      bp[v]        = ldg3(reinterpret_cast<const float*>(in.positions), vi);
-      bn[v]        = normalize3(ldg3(reinterpret_cast<const float*>(in.normals), vi));  // :329
-      bt[v]        = ldg2(reinterpret_cast<const float*>(in.texcoords), vi);
-      bb[v]        = decode_bary(pt.subTriangle.vtxEncoded[v]);
+      const uint2*             raw = reinterpret_cast<const uint2*>(parts + p);
+      const uint2              r0 = raw[0], r1 = raw[1], r2 = raw[2];
+      const u32                cfg = r2.y >> 16, corner[3] = {r1.x, r1.y, r2.x};
+      const tc_TessTableEntry  e   = table_entry(c.table, cfg);
+      const tc_RenderInstance& in  = c.instances[r0.x];
+      const tc_Cluster         cl  = reinterpret_cast<const tc_Cluster*>(in.clusters)[r0.y];
+      setup_deform(c, in, cl, r2.y & 0xFFFFu, cfg, corner, e.firstVertex, pn, rec.affine[lane], rec.pn[lane]);
+      d = {e.numVertices, e.firstVertex, vo, r0.x, in.geoHi.w};
     }
-    tc_DisplacementTexture tx    = {};
-    bool                   hasTx = false;
-    if(c.numTextures > 0 && c.textures != nullptr && in.displacementIndex >= 0)
-    {
-      if((u32)in.displacementIndex < c.numTextures)
-      {
-        tx    = c.textures[in.displacementIndex];
-        hasTx = true;
-      }
-      else if(subLane == 0)
-        atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
-    }
-    BasePN basis = {};
-    if(pn)
-      basis = setup_pn(bp[0], bp[1], bp[2], bn[0], bn[1], bn[2]);
-    for(u32 vert = subLane; vert < e.numVertices; vert += 8)
-    {
-      const f3 w   = interp3(bb[0], bb[1], bb[2], cfg_vertex(c.table, e, cfg, vert));
-      f3       pos = pn ? get_pn(basis, w) : interp3(bp[0], bp[1], bp[2], w);
-      if(hasTx)
-        pos = displace(pos, interp3(bn[0], bn[1], bn[2], w), sample_bilinear(tx, interp2(bt[0], bt[1], bt[2], w)),
-                       in.displacementScale, c.view->displacementScale, in.displacementOffset,
-                       c.view->displacementOffset);
-      if(rp.enabled)
-        pos = ripple(pos, pt.cluster.instanceID, in.geoHi.w, rp);
-      float* d = gv + 3 * ((u64)vo + vert);
-      d[0] = pos.x, d[1] = pos.y, d[2] = pos.z;
-    }
+    __syncwarp();
+    deform_walk(c, rec, count, d, pn, rp, gv);
+    __syncwarp();  // the warp's records are rewritten by its next chunk
+    chunk = __shfl_sync(0xFFFFFFFFu, following, 0);
   }
 }
 
@@ -1086,9 +1094,9 @@ cudaError_t launch_instantiate_vertices(const StageCtx& c, const InstantiateBuff
                                         u32 vertexBlocksPerSM, u32 vertexGridPerSM, cudaStream_t s)
 {
   const u32 chunks = (maxParts + kPartsPerWarp - 1) / kPartsPerWarp;
-  if(c.flags & (TC_FLAG_PN | TC_FLAG_RIPPLE))  // the deformation path: one warp per part
-    return launch_pdl(k_instantiate_vertices_deform, std::max(1u, std::min((maxParts + 4 * kWarps - 1) / (4 * kWarps), numSMs * 8)),
-                      kBlock, s, c, buf);
+  if(c.flags & (TC_FLAG_PN | TC_FLAG_RIPPLE))  // one resident wave of the deformation kernel's blocks
+    return launch_pdl(k_instantiate_vertices_deform,
+                      std::max(1u, std::min((chunks + kDeformWarps - 1) / kDeformWarps * 8, numSMs * (u32)kDeformBlocksPerSM)), kDeformBlock, s, c, buf);
   // warps stride over the 32-part chunks; the grid is sized to the machine,
   // not to the capacity (blocks with no chunk would only add a tail), by
   // default one resident wave; vertexBlocksPerSM picks the register budget

@@ -9,6 +9,7 @@
 // triangle counts; one block scans the groups' counts into offsets; per group
 // again the batch records, then the group's vertices and triangles, each as
 // one contiguous range over which the lanes take consecutive elements.
+#include "tc_deform.cuh"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
@@ -250,33 +251,8 @@ __global__ void __launch_bounds__(kWriteBlock) k_raster_write(StageCtx c, const 
       const tc_TessTableEntry e   = table_entry(c.table, cfg);
       const tc_RenderInstance& in = c.instances[r0.x];
       const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in.clusters)[r0.y];
-      const uint8_t* lt = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle + tri * 3;
-      const u32      corner[3] = {r1.x, r1.y, r2.x};
-      tc_DisplacementTexture tx = {};
-      if(c.numTextures > 0 && c.textures != nullptr && in.displacementIndex >= 0)
-      {
-        if((u32)in.displacementIndex < c.numTextures)
-        {
-          tx = c.textures[in.displacementIndex];
-          if(tx.width == 0)  // an empty map samples as 0: the offsets still displace
-            tx.width = 1, tx.height = 0;
-        }
-        else
-          atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
-      }
-      const float* pos = reinterpret_cast<const float*>(in.positions);
-      const float* nrm = reinterpret_cast<const float*>(in.normals);
-      part_affine(sp[lane], corner, cfg_flipped(cfg), pos, nrm, reinterpret_cast<const float*>(in.texcoords),
-                  cl.firstLocalVertex, lt, e.firstVertex, tx, in.displacementScale * c.view->displacementScale,
-                  in.displacementOffset + c.view->displacementOffset);
-      if constexpr(Deform)
-        if(pn)
-        {
-          const u32 i0 = cl.firstLocalVertex + lt[0], i1 = cl.firstLocalVertex + lt[1], i2 = cl.firstLocalVertex + lt[2];
-          write_part_pn(s_pn[warp][lane], corner, cfg_flipped(cfg),
-                        setup_pn(ldg3(pos, i0), ldg3(pos, i1), ldg3(pos, i2), normalize3(ldg3(nrm, i0)),
-                                 normalize3(ldg3(nrm, i1)), normalize3(ldg3(nrm, i2))));
-        }
+      const u32               corner[3] = {r1.x, r1.y, r2.x};
+      setup_deform(c, in, cl, tri, cfg, corner, e.firstVertex, pn, sp[lane], s_pn[Deform ? warp : 0][Deform ? lane : 0]);
       const float* m = in.worldMatrix.m;
 #pragma unroll
       for(int r = 0; r < 3; r++)
@@ -318,13 +294,7 @@ __global__ void __launch_bounds__(kWriteBlock) k_raster_write(StageCtx c, const 
         if(jj < vFit)
         {
           const u32 tv = __ldg(c.table.vertices + (tvIdx + jj));
-          f3        p;
-          if(pn)
-            p = affine_displace(sp[pi], tv, part_pn_position(s_pn[Deform ? warp : 0][Deform ? pi : 0], tv));
-          else
-            p = affine_vertex(sp[pi], tv);
-          if(rp.enabled)
-            p = ripple(p, vInst, vSize, rp);
+          const f3  p  = deform_vertex(sp[pi], s_pn[Deform ? warp : 0][Deform ? pi : 0], tv, pn, vInst, vSize, rp);
           const float4 mx = s_world[warp][pi][0], my = s_world[warp][pi][1], mz = s_world[warp][pi][2];
           const f3     wp = {((mx.x * p.x + mx.y * p.y) + mx.z * p.z) + mx.w, ((my.x * p.x + my.y * p.y) + my.z * p.z) + my.w,
                              ((mz.x * p.x + mz.y * p.y) + mz.z * p.z) + mz.w};

@@ -352,63 +352,10 @@ __device__ __forceinline__ u32 affine_first_vertex(const PartAffine& r) { return
 namespace tc {
 
 // ---------------------------------------------------------------------------
-// PN-triangle displacement and the ripple deformation (displacement.glsl),
-// written like the CPU restatement: separate IEEE multiplies, adds and
-// divisions in the shader's order.
+// The ripple deformation (displacement.glsl), written like the CPU
+// restatement: separate IEEE multiplies, adds and divisions in the shader's
+// order.
 // ---------------------------------------------------------------------------
-
-__device__ __forceinline__ f3 add3(f3 a, f3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ f3 mul3(f3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ f3 div3(f3 a, float s) { return {__fdiv_rn(a.x, s), __fdiv_rn(a.y, s), __fdiv_rn(a.z, s)}; }
-
-// displacement.glsl:40-45
-__device__ __forceinline__ f3 project_to_plane(f3 p, f3 plane, f3 n) { return sub3(p, mul3(n, dot3(sub3(p, plane), n))); }
-
-// displacement.glsl:27-38 (b030 = base vertex 0, b003 = vertex 1, b300 = vertex 2)
-struct BasePN
-{
-  f3 b030, b003, b300, b021, b012, b102, b201, b210, b120, b111;
-};
-
-// displacement.glsl:47-78 deform_setupPN; n: normalised base normals
-__device__ __forceinline__ BasePN setup_pn(f3 v0, f3 v1, f3 v2, f3 n0, f3 n1, f3 n2)
-{
-  BasePN   b;
-  b.b030         = v0;
-  b.b003         = v1;
-  b.b300         = v2;
-  const f3 e300  = sub3(b.b003, b.b030);
-  const f3 e030  = sub3(b.b300, b.b003);
-  const f3 e003  = sub3(b.b030, b.b300);
-  b.b021         = project_to_plane(add3(b.b030, div3(e300, 3.0f)), b.b030, n0);
-  b.b012         = project_to_plane(add3(b.b030, div3(mul3(e300, 2.0f), 3.0f)), b.b003, n1);
-  b.b102         = project_to_plane(add3(b.b003, div3(e030, 3.0f)), b.b003, n1);
-  b.b201         = project_to_plane(add3(b.b003, div3(mul3(e030, 2.0f), 3.0f)), b.b300, n2);
-  b.b210         = project_to_plane(add3(b.b300, div3(e003, 3.0f)), b.b300, n2);
-  b.b120         = project_to_plane(add3(b.b300, div3(mul3(e003, 2.0f), 3.0f)), b.b030, n0);
-  const f3 center = div3(add3(add3(b.b003, b.b030), b.b300), 3.0f);
-  b.b111 = div3(add3(add3(add3(add3(add3(b.b021, b.b012), b.b102), b.b201), b.b210), b.b120), 6.0f);
-  b.b111 = add3(b.b111, div3(sub3(b.b111, center), 2.0f));
-  return b;
-}
-
-// displacement.glsl:80-104 deform_getPN (the powers as products)
-__device__ __forceinline__ f3 get_pn(const BasePN& b, f3 bary)
-{
-  const float u = bary.x, v = bary.y, w = bary.z;
-  const float u3 = u * u * u, v3 = v * v * v, w3 = w * w * w, u2 = u * u, v2 = v * v, w2 = w * w;
-  f3          r = mul3(b.b300, w3);
-  r             = add3(r, mul3(b.b030, u3));
-  r             = add3(r, mul3(b.b003, v3));
-  r             = add3(r, mul3(mul3(mul3(b.b210, 3.0f), w2), u));
-  r             = add3(r, mul3(mul3(mul3(b.b120, 3.0f), w), u2));
-  r             = add3(r, mul3(mul3(mul3(b.b201, 3.0f), w2), v));
-  r             = add3(r, mul3(mul3(mul3(b.b021, 3.0f), u2), v));
-  r             = add3(r, mul3(mul3(mul3(b.b102, 3.0f), w), v2));
-  r             = add3(r, mul3(mul3(mul3(b.b012, 3.0f), u), v2));
-  r             = add3(r, mul3(mul3(mul3(mul3(b.b111, 6.0f), w), u), v));
-  return r;
-}
 
 // the FrameConstants terms of displacement.glsl:106-120
 struct RippleParams
@@ -440,14 +387,25 @@ __device__ __forceinline__ f3 ripple(f3 p, u32 seed, float size, const RipplePar
 
 // ---------------------------------------------------------------------------
 // The PN-triangle cubic of a part in per-part form (TC_FLAG_PN): the base
-// triangle's control points with the cubic's binomial factors multiplied in
-// (the same first product as get_pn's), and the base barycentrics of a table
-// vertex w = (1 - a - b, a, b) as W0 + a W1 + b W2 (the composition with the
-// sub-triangle's corners, exact up to one rounding per term: the corners are
-// multiples of 2^-15). A vertex takes ten weights shared by x, y and z and
-// three fused multiply-adds for each control point, in place of get_pn's
-// separate products per component.
+// triangle's control points with the cubic's binomial factors multiplied in,
+// and the base barycentrics of a table vertex w = (1 - a - b, a, b) as
+// W0 + a W1 + b W2 (the composition with the sub-triangle's corners, exact up
+// to one rounding per term: the corners are multiples of 2^-15). A vertex
+// takes ten weights shared by x, y and z and three fused multiply-adds for
+// each control point (displacement.glsl:80-104 deform_getPN). The control
+// points (displacement.glsl:47-78 deform_setupPN) take the thirds of an edge
+// as fused products with 1/3 and 2/3: one rounding where the shader's
+// division and addition have two, without 21 divisions per part.
 // ---------------------------------------------------------------------------
+
+// a + (b - a) t, moved along n into the plane of `plane` and n
+__device__ __forceinline__ f3 pn_edge_point(f3 a, f3 edge, float t, f3 plane, f3 n)
+{
+  const f3    p = fma3(t, edge, a);
+  const f3    d = sub3(p, plane);
+  const float k = __fmaf_rn(d.z, n.z, __fmaf_rn(d.y, n.y, d.x * n.x));
+  return fma3(-k, n, p);
+}
 
 // 176-byte stride: records of an array start in different bank groups.
 struct __align__(16) PartPn
@@ -457,7 +415,8 @@ struct __align__(16) PartPn
   // q[7].zw, q[8].x: W0; q[8].yzw: W1; q[9].xyz: W2
 };
 
-__device__ __forceinline__ void write_part_pn(PartPn& r, const u32 corner[3], bool flipped, const BasePN& b)
+// v, n: the base triangle's positions and normalised normals
+__device__ __forceinline__ void write_part_pn(PartPn& r, const u32 corner[3], bool flipped, const f3 v[3], const f3 n[3])
 {
   f3 c0 = decode_bary(corner[0]), c1 = decode_bary(corner[1]), c2 = decode_bary(corner[2]);
   if(flipped)
@@ -466,16 +425,25 @@ __device__ __forceinline__ void write_part_pn(PartPn& r, const u32 corner[3], bo
     c0         = c1;
     c1         = t;
   }
-  const f3 w1 = sub3(c1, c0), w2 = sub3(c2, c0);
-  const f3 b210 = mul3(b.b210, 3.0f), b120 = mul3(b.b120, 3.0f), b201 = mul3(b.b201, 3.0f), b021 = mul3(b.b021, 3.0f),
-           b102 = mul3(b.b102, 3.0f), b012 = mul3(b.b012, 3.0f), b111 = mul3(b.b111, 6.0f);
-  r.q[0] = make_float4(b.b300.x, b.b300.y, b.b300.z, b.b030.x);
-  r.q[1] = make_float4(b.b030.y, b.b030.z, b.b003.x, b.b003.y);
-  r.q[2] = make_float4(b.b003.z, b210.x, b210.y, b210.z);
-  r.q[3] = make_float4(b120.x, b120.y, b120.z, b201.x);
-  r.q[4] = make_float4(b201.y, b201.z, b021.x, b021.y);
-  r.q[5] = make_float4(b021.z, b102.x, b102.y, b102.z);
-  r.q[6] = make_float4(b012.x, b012.y, b012.z, b111.x);
+  const f3        w1 = sub3(c1, c0), w2 = sub3(c2, c0);
+  constexpr float kThird = 1.0f / 3.0f, kTwoThirds = 2.0f / 3.0f;
+  // b030 = v0, b003 = v1, b300 = v2
+  const f3 e300 = sub3(v[1], v[0]), e030 = sub3(v[2], v[1]), e003 = sub3(v[0], v[2]);
+  const f3 b021 = pn_edge_point(v[0], e300, kThird, v[0], n[0]), b012 = pn_edge_point(v[0], e300, kTwoThirds, v[1], n[1]);
+  const f3 b102 = pn_edge_point(v[1], e030, kThird, v[1], n[1]), b201 = pn_edge_point(v[1], e030, kTwoThirds, v[2], n[2]);
+  const f3 b210 = pn_edge_point(v[2], e003, kThird, v[2], n[2]), b120 = pn_edge_point(v[2], e003, kTwoThirds, v[0], n[0]);
+  // 6 b111 = 6 (E + (E - V) / 2), E = the six points' mean, V = the corners' = 1.5 (6 E) - 3 V
+  const f3 six  = {((((b021.x + b012.x) + b102.x) + b201.x) + b210.x) + b120.x,
+                   ((((b021.y + b012.y) + b102.y) + b201.y) + b210.y) + b120.y,
+                   ((((b021.z + b012.z) + b102.z) + b201.z) + b210.z) + b120.z};
+  const f3 b111 = fma3(1.5f, six, {-((v[1].x + v[0].x) + v[2].x), -((v[1].y + v[0].y) + v[2].y), -((v[1].z + v[0].z) + v[2].z)});
+  r.q[0] = make_float4(v[2].x, v[2].y, v[2].z, v[0].x);
+  r.q[1] = make_float4(v[0].y, v[0].z, v[1].x, v[1].y);
+  r.q[2] = make_float4(v[1].z, 3.0f * b210.x, 3.0f * b210.y, 3.0f * b210.z);
+  r.q[3] = make_float4(3.0f * b120.x, 3.0f * b120.y, 3.0f * b120.z, 3.0f * b201.x);
+  r.q[4] = make_float4(3.0f * b201.y, 3.0f * b201.z, 3.0f * b021.x, 3.0f * b021.y);
+  r.q[5] = make_float4(3.0f * b021.z, 3.0f * b102.x, 3.0f * b102.y, 3.0f * b102.z);
+  r.q[6] = make_float4(3.0f * b012.x, 3.0f * b012.y, 3.0f * b012.z, b111.x);
   r.q[7] = make_float4(b111.y, b111.z, c0.x, c0.y);
   r.q[8] = make_float4(c0.z, w1.x, w1.y, w1.z);
   r.q[9] = make_float4(w2.x, w2.y, w2.z, 0.0f);
