@@ -49,7 +49,7 @@ struct Plan
   u32    segRows;     // runs
   size_t runOffset;   // run starts (u32 x kMaxRuns+2)
   u32    classifyCap; // clusters the classify scratch holds
-  size_t clsCountsOffset, clsTriWordsOffset, clsBlockSumsOffset, clsFullRecsOffset;
+  size_t clsCountsOffset, clsTriWordsOffset, clsBlockSumsOffset, clsFullRecsOffset, clsTransRecsOffset;
   size_t rasterOffset;
   size_t partVertexOffset;  // u32 per part triangle
   size_t chunkSumsOffset;   // u64 per 32 part triangles
@@ -205,8 +205,10 @@ Plan make_plan(const tc_context_desc& d)
   off                 = align_up(off + (size_t)p.classifyCap * TC_MAX_CLUSTER_TRIANGLES * 4, 256);
   p.clsBlockSumsOffset = off;  // the counter bases
   off = align_up(off + sizeof(ClusterOffsets) + sizeof(TransBases), 256);
-  p.clsFullRecsOffset = off;  // per full cluster, then the slot range
-  off = align_up(off + (size_t)p.classifyCap * 8 + 8, 256);
+  p.clsFullRecsOffset = off;  // per full cluster, then the slot range and the transient records' count
+  off = align_up(off + (size_t)p.classifyCap * 8 + 16, 256);
+  p.clsTransRecsOffset = off;
+  off = align_up(off + (size_t)p.classifyCap * 48, 256);
   p.partVertexOffset  = off;
   off                 = align_up(off + (size_t)std::max(1u, k.maxPartTriangles) * 4, 256);
   p.chunkSumsOffset   = off;
@@ -298,7 +300,8 @@ ClassifyBuffers classify_buffers(tc_context* ctx)
           reinterpret_cast<RangeSums*>(ctx->dScratch + p.slots[p.slotClassify].stateOffset),
           reinterpret_cast<ClusterOffsets*>(ctx->dScratch + p.clsBlockSumsOffset),
           reinterpret_cast<uint2*>(ctx->dScratch + p.clsFullRecsOffset),
-          reinterpret_cast<u32*>(ctx->dScratch + p.clsFullRecsOffset + (size_t)p.classifyCap * 8)};
+          reinterpret_cast<u32*>(ctx->dScratch + p.clsFullRecsOffset + (size_t)p.classifyCap * 8),
+          reinterpret_cast<uint4*>(ctx->dScratch + p.clsTransRecsOffset)};
 }
 
 InstantiateBuffers instantiate_buffers(tc_context* ctx)
@@ -318,6 +321,15 @@ u32 frame_begin_grid(const tc_context* ctx, const tc_frame_args* a)
   return std::max(1u, std::min(ctx->numSMs * 2, ceil_div((u64)a->caps.maxSplitTriangles * 6, 256)));
 }
 
+// whether cluster_classify launches a kernel of its own for the clusters with
+// part or split triangles
+bool emits_clusters(const tc_context* ctx, const tc_frame_args* a)
+{
+  return (a->flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)) != 0
+         || classify_lists_clusters(std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
+                                    ctx->schedule.classifyBlocksPerSM);
+}
+
 // kernels one batched frame launches (the BLAS set-up is fused for up to
 // kBlasSetupFusedMax instances)
 uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
@@ -325,7 +337,8 @@ uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
   return kFrameFixedLaunches + (ctx->schedule.splitPerPass ? split_passes(a->caps.splitFactor) : 1)
          - (a->numInstances <= kBlasSetupFusedMax ? 1 : 0)
          - (ctx->schedule.frameShape == 1 ? 4 : 0)  // one allocation + vertex launch instead of two
-         + ((a->flags & TC_FLAG_TRANSIENT_2X) ? 1 : 0);  // the 2X batches' vertices
+         + (emits_clusters(ctx, a) ? 1 : 0)              // the clusters with part or split triangles
+         + ((a->flags & TC_FLAG_TRANSIENT_2X) ? 1 : 0);                           // the 2X batches' vertices
 }
 
 u32 insert_grid(const tc_context* ctx, const tc_frame_args* a)
@@ -1013,7 +1026,7 @@ tc_status tc_cluster_classify(tc_context* ctx, const tc_frame_args* a, uint32_t 
   TC_CHECK_CUDA(launch_classify_full_vertices(c, classify_buffers(ctx),
                                               std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
                                               4, reinterpret_cast<cudaStream_t>(stream)));
-  ctx->launches += (a->flags & TC_FLAG_TRANSIENT_2X) ? 4 : 3;
+  ctx->launches += 3 + (emits_clusters(ctx, a) ? 1 : 0) + ((a->flags & TC_FLAG_TRANSIENT_2X) ? 1 : 0);
   return TC_OK;
 }
 

@@ -102,9 +102,10 @@ struct ClassifyScratch
   RangeSums*      rangeSums;  // per write block's range: the counts' sums, zero before count
   ClusterOffsets* bases;      // the counters before the launch
   u32             writeBlocks;  // the write launch's grid (its blocks' ranges)
-  u32             _pad;
+  u32             listed;       // k_classify_write leaves the clusters with parts to k_classify_emit
   uint2*          fullRecs;   // per full cluster (generated-cluster slot - first slot): visible index, first vertex
-  u32*            fullRange;  // [2]: the launch's generated-cluster slots [begin, end)
+  u32*            fullRange;  // [2]: the launch's generated-cluster slots [begin, end); [2]: transRecs' count
+  uint4*          transRecs;  // per cluster left to k_classify_emit (two words) or k_classify_emit_transient (three)
 };
 
 constexpr u32 kRejected = 0xFFFFFFFFu;  // fullRecs: a full cluster that did not fit the capacities
@@ -447,6 +448,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_count(StageCtx c
   const u32               wordOnes = classify_triangle(make_uint3(1u, 1u, 1u), sf);  // a triangle of factors 1
   if(blockIdx.x == 0 && threadIdx.x == 0)  // the offsets continue from the counters' current values
   {
+    cs.fullRange[2] = 0;
     if constexpr(Trans)
     {
       // parts from the front of the two-sided counter (build.glsl:52-82)
@@ -735,6 +737,83 @@ __device__ __forceinline__ void full_steps_uniform(const FullRecord& u, bool own
   }
 }
 
+// cluster_classify.comp.glsl:543-666: the part and split triangles of one
+// cluster by one warp, from the words of triangles lane and lane + 32. The
+// cluster's parts are consecutive records of 24 bytes: they are put together
+// in the warp's `stage` and stored as consecutive 8-byte words (a lane that
+// stores its own record touches 24 sectors per store instruction, eight when
+// the lanes' words are consecutive).
+__device__ __forceinline__ void emit_cluster(const StageCtx& c, const tc_ClusterInfo& ci, u32 nt, u32 offPart,
+                                             u32 offSplit, u32 w0, u32 w1, uint2* stage)
+{
+  const tc_SceneBuilding* b      = c.build;
+  const tc_caps&          k      = c.caps;
+  tc_TessTriangleInfo*    splits = reinterpret_cast<tc_TessTriangleInfo*>(b->splitTriangles);
+  tc_TessTriangleInfo*    parts  = reinterpret_cast<tc_TessTriangleInfo*>(b->partTriangles);
+  const u32  lane = threadIdx.x & 31, ltm = (1u << lane) - 1u;
+  const bool s0  = lane < nt && (w0 >> 18) != 0, p0 = lane < nt && (w0 >> 18) == 0;
+  const bool s1  = lane + 32 < nt && (w1 >> 18) != 0, p1 = lane + 32 < nt && (w1 >> 18) == 0;
+  const u32  bs0 = __ballot_sync(0xFFFFFFFFu, s0), bp0 = __ballot_sync(0xFFFFFFFFu, p0);
+  const u32  bs1 = __ballot_sync(0xFFFFFFFFu, s1), bp1 = __ballot_sync(0xFFFFFFFFu, p1);
+  tc_TessTriangleInfo* local = reinterpret_cast<tc_TessTriangleInfo*>(stage);
+  if(p0)
+    emit_triangle(local + __popc(bp0 & ltm), ci, lane, w0);
+  if(p1)
+    emit_triangle(local + __popc(bp0) + __popc(bp1 & ltm), ci, lane + 32, w1);
+  __syncwarp();
+  const u32 np   = min((u32)__popc(bp0) + (u32)__popc(bp1), k.maxPartTriangles - min(offPart, k.maxPartTriangles));
+  uint2*    dst  = reinterpret_cast<uint2*>(parts + offPart);
+  for(u32 q = lane; q < 3 * np; q += 32)
+    dst[q] = stage[q];
+  __syncwarp();  // the stage is rewritten by the warp's next cluster
+  if((bs0 | bs1) == 0)
+    return;
+  // split items also carry their base triangle's world positions (read by
+  // every split pass instead of the instance / cluster / vertex chain)
+  const tc_RenderInstance* in = c.instances + ci.instanceID;
+  const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
+  float                    m[16];
+#pragma unroll
+  for(int j = 0; j < 16; j++)
+    m[j] = __ldg(in->worldMatrix.m + j);
+  auto split = [&](u64 o, u32 tri, u32 w) {
+    if(o >= k.maxSplitTriangles)
+      return;
+    emit_triangle(splits + o, ci, tri, w);
+    if(!c.splitBase)
+      return;
+    const uint8_t* lt  = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
+    const float*   pos = reinterpret_cast<const float*>(in->positions);
+    float*         d   = c.splitBase + 9 * o;
+#pragma unroll
+    for(int vv = 0; vv < 3; vv++)
+    {
+      const f3 wp = xform_point(m, ldg3(pos, cl.firstLocalVertex + lt[tri * 3 + vv]));
+      d[3 * vv + 0] = wp.x, d[3 * vv + 1] = wp.y, d[3 * vv + 2] = wp.z;
+    }
+  };
+  if(s0)
+    split((u64)offSplit + __popc(bs0 & ltm), lane, w0);
+  if(s1)
+    split((u64)offSplit + __popc(bs0) + __popc(bs1 & ltm), lane + 32, w1);
+}
+
+// the words of cluster v's triangles lane and lane + 32
+__device__ __forceinline__ uint2 cluster_words(const ClassifyScratch& cs, u32 v, u32 nt)
+{
+  const u32  lane = threadIdx.x & 31;
+  const u32* tw   = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
+  return make_uint2(lane < nt ? tw[lane] : 0u, lane + 32 < nt ? tw[lane + 32] : 0u);
+}
+
+// Listed: the clusters with part or split triangles go to a list that
+// k_classify_emit's warps stride over, instead of being written by their
+// range's block. The visible clusters of an instance lie next to each other,
+// so of the 608 ranges of 341 clusters of a frame with 207,360 clusters, 4,694
+// of them tessellated, a few hold them all: from the count's end to the last
+// write 39 us in one kernel, 22 us in two (terrain of 32,768 clusters, nearly
+// all tessellated: 36 -> 23 us). Ranges of up to 32 clusters, four per warp,
+// are written at once: the second launch costs what it gains.
 template <int MinBlocks>
 __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c, ClassifyScratch cs)
 {
@@ -744,6 +823,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
   __shared__ ClusterOffsets s_off[kBlock];  // offsets of the chunk's clusters
   __shared__ uint2          s_cnt[kBlock];  // counts of the chunk's clusters
   __shared__ tc_ClusterInfo s_ci[kBlock];   // the chunk's clusters
+  __shared__ uint2          s_stage[kWarps][3 * TC_MAX_CLUSTER_TRIANGLES];
   __shared__ FlatStarts     s_starts;
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if(threadIdx.x == 0)
@@ -757,8 +837,6 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
   const tc_caps&        k            = c.caps;
   const tc_ClusterInfo* vis          = reinterpret_cast<const tc_ClusterInfo*>(b->visibleClusters);
   const u64             maxData      = (u64)k.maxGeneratedClusterMegs * 1024ull * 1024ull;
-  tc_TessTriangleInfo*  splits       = reinterpret_cast<tc_TessTriangleInfo*>(b->splitTriangles);
-  tc_TessTriangleInfo*  parts        = reinterpret_cast<tc_TessTriangleInfo*>(b->partTriangles);
   tc_BlasBuildInfo*     blas         = reinterpret_cast<tc_BlasBuildInfo*>(b->blasBuildInfos);
   const u32             ltm          = (1u << lane) - 1u;
   u32                   statTris = 0, statTemp = 0;
@@ -794,81 +872,30 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
     const u32 perW = (len + kWarps - 1) / kWarps;
     const u32 lo = min(len, warp * perW), hi = min(len, lo + perW);
 
-    // ---- phase 1: part and split triangles, one cluster at a time -------------
-    for(u32 i = lo; i < hi; i++)
+    // ---- phase 1: part and split triangles ------------------------------------
+    const u32  mine  = lo + lane;
+    const bool cut   = mine < hi && !cnt_full(s_cnt[min(mine, kBlock - 1)]);
+    u32        left  = __ballot_sync(0xFFFFFFFFu, cut);
+    if(cs.listed && left)
     {
-      const uint2 cnt = s_cnt[i];
-      if(cnt_full(cnt))
-        continue;  // phase 2 (no part or split triangles)
-      const u32 v = c0 + i, offPart = s_off[i].part, offSplit = s_off[i].split;
-      const tc_ClusterInfo ci = s_ci[i];
+      u32 at = 0;
+      if(lane == 0)
+        at = atomicAdd(cs.fullRange + 2, __popc(left));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(left & ltm);
+      if(cut)
       {
-        // cluster_classify.comp.glsl:543-666: part and split triangles
-        const u32  nt  = cnt_parts(cnt) + cnt_splits(cnt);
-        const u32* tw  = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
-        const u32  w0  = lane < nt ? tw[lane] : 0u;
-        const u32  w1  = lane + 32 < nt ? tw[lane + 32] : 0u;
-        const bool s0  = lane < nt && (w0 >> 18) != 0, p0 = lane < nt && (w0 >> 18) == 0;
-        const bool s1  = lane + 32 < nt && (w1 >> 18) != 0, p1 = lane + 32 < nt && (w1 >> 18) == 0;
-        const u32  bs0 = __ballot_sync(0xFFFFFFFFu, s0), bp0 = __ballot_sync(0xFFFFFFFFu, p0);
-        const u32  bs1 = __ballot_sync(0xFFFFFFFFu, s1), bp1 = __ballot_sync(0xFFFFFFFFu, p1);
-        // split items also carry their base triangle's world positions (read by
-        // every split pass instead of the instance / cluster / vertex chain)
-        const tc_RenderInstance* in  = nullptr;
-        tc_Cluster               cl  = {};
-        float                    m[16];
-        if(bs0 | bs1)
-        {
-          in = c.instances + ci.instanceID;
-          cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
-#pragma unroll
-          for(int j = 0; j < 16; j++)
-            m[j] = __ldg(in->worldMatrix.m + j);
-        }
-        auto split_base = [&](u64 o, u32 tri) {
-          if(!c.splitBase)
-            return;
-          const uint8_t* lt  = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
-          const float*   pos = reinterpret_cast<const float*>(in->positions);
-          float*         d   = c.splitBase + 9 * o;
-#pragma unroll
-          for(int vv = 0; vv < 3; vv++)
-          {
-            const f3 wp = xform_point(m, ldg3(pos, cl.firstLocalVertex + lt[tri * 3 + vv]));
-            d[3 * vv + 0] = wp.x, d[3 * vv + 1] = wp.y, d[3 * vv + 2] = wp.z;
-          }
-        };
-        if(s0)
-        {
-          const u64 o = (u64)offSplit + __popc(bs0 & ltm);
-          if(o < k.maxSplitTriangles)
-          {
-            emit_triangle(splits + o, ci, lane, w0);
-            split_base(o, lane);
-          }
-        }
-        else if(p0)
-        {
-          const u64 o = (u64)offPart + __popc(bp0 & ltm);
-          if(o < k.maxPartTriangles)
-            emit_triangle(parts + o, ci, lane, w0);
-        }
-        if(s1)
-        {
-          const u64 o = (u64)offSplit + __popc(bs0) + __popc(bs1 & ltm);
-          if(o < k.maxSplitTriangles)
-          {
-            emit_triangle(splits + o, ci, lane + 32, w1);
-            split_base(o, lane + 32);
-          }
-        }
-        else if(p1)
-        {
-          const u64 o = (u64)offPart + __popc(bp0) + __popc(bp1 & ltm);
-          if(o < k.maxPartTriangles)
-            emit_triangle(parts + o, ci, lane + 32, w1);
-        }
+        uint4* rec = cs.transRecs + 2 * (u64)at;
+        rec[0] = make_uint4(s_ci[mine].instanceID, s_ci[mine].clusterID, s_off[mine].part, s_off[mine].split);
+        rec[1] = make_uint4(c0 + mine, cnt_parts(s_cnt[mine]) + cnt_splits(s_cnt[mine]), 0u, 0u);
       }
+      left = 0;
+    }
+    for(; left; left &= left - 1)
+    {
+      const u32   i  = lo + (u32)__ffs(left) - 1;
+      const u32   nt = cnt_parts(s_cnt[i]) + cnt_splits(s_cnt[i]);
+      const uint2 w  = cluster_words(cs, c0 + i, nt);
+      emit_cluster(c, s_ci[i], nt, s_off[i].part, s_off[i].split, w.x, w.y, s_stage[warp]);
     }
 
     // ---- phase 2: full clusters of the warp's part, 32 at a time ---------------
@@ -967,6 +994,34 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
   }
 }
 
+// The clusters k_classify_write listed: a warp's next cluster is loaded while
+// the current one is written.
+__global__ void __launch_bounds__(kBlock, 4) k_classify_emit(StageCtx c, ClassifyScratch cs)
+{
+  stage_prologue();
+  __shared__ uint2 s_stage[kWarps][3 * TC_MAX_CLUSTER_TRIANGLES];
+  const u32 count = cs.fullRange[2], warp = threadIdx.x >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  u32       i     = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if(i >= count)
+    return;
+  uint4 a = cs.transRecs[2 * (u64)i], v = cs.transRecs[2 * (u64)i + 1];
+  uint2 w = cluster_words(cs, v.x, v.y);
+  for(;;)
+  {
+    const uint4 ca = a, cv = v;
+    const uint2 cw = w;
+    i += nwarps;
+    if(i < count)
+    {
+      a = cs.transRecs[2 * (u64)i], v = cs.transRecs[2 * (u64)i + 1];
+      w = cluster_words(cs, v.x, v.y);
+    }
+    emit_cluster(c, {ca.x, ca.y}, cv.y, ca.z, ca.w, cw.x, cw.y, s_stage[warp]);
+    if(i >= count)
+      break;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // write, with transient builds
 // ---------------------------------------------------------------------------
@@ -1041,15 +1096,15 @@ __device__ __forceinline__ void warp_zero(void* p, u32 words)
     w[i] = 0u;
 }
 
-// cluster_classify.comp.glsl:254-905 with transient builds, for one cluster,
-// by one warp, in the canonical order: the full-cluster or 1X allocation, then
-// per 32-triangle chunk its parts and splits followed by its 2X batches.
-// Offsets come from the block scan; every allocation is tested like the
-// reference's (the counters advance whether or not it fits). Bytes the
+// cluster_classify.comp.glsl:254-905 with transient builds, for one cluster
+// that is not a full one, by one warp, in the canonical order: the 1X
+// allocation, then per 32-triangle chunk its parts and splits followed by its
+// 2X batches. Offsets come from the block scan; every allocation is tested like
+// the reference's (the counters advance whether or not it fits). Bytes the
 // reference leaves unwritten inside an allocation are written as zeros.
 __device__ inline void write_cluster_transient(const StageCtx& c, const ClassifyScratch& cs, u32 visIndex, u32 v,
-                                               const tc_ClusterInfo& ci, uint4 r, TransOffsets o, u32 genBase,
-                                               const TransBases& tb, u32& statTemp, u32& statTrans, u32& statTris)
+                                               const tc_ClusterInfo& ci, uint4 r, TransOffsets o, u32& statTrans,
+                                               u32& statTris)
 {
   const u32         lane = threadIdx.x & 31, ltm = (1u << lane) - 1u;
   tc_SceneBuilding* b    = c.build;
@@ -1058,7 +1113,7 @@ __device__ inline void write_cluster_transient(const StageCtx& c, const Classify
   const u32*        basic   = reinterpret_cast<const u32*>(b->basicClusterSizes);
   tc_BlasBuildInfo* blas    = reinterpret_cast<tc_BlasBuildInfo*>(b->blasBuildInfos);
   const u32         nt = t_nt(r), nv = t_nv(r), simple = t_simple(r);
-  const bool        full = t_full(r), subset = t_subset(r);
+  const bool        subset = t_subset(r);
   const tc_RenderInstance* in = c.instances + ci.instanceID;
   const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
   u32 x = o.front, y = o.back, s = o.split, g = o.gen, vo = o.vert, tr = o.trans;
@@ -1070,86 +1125,59 @@ __device__ inline void write_cluster_transient(const StageCtx& c, const Classify
   uint8_t* gvb = reinterpret_cast<uint8_t*>(b->genVertices);
   uint8_t* ptb = reinterpret_cast<uint8_t*>(b->partTriangles);
 
-  // ---- :254-437 full cluster or 1X subset ----------------------------------------
-  if(full || subset)
+  // ---- :254-437 1X subset ----------------------------------------------------------
+  if(subset)
   {
-    const u32 vertexSize = full ? nv : subset_vertex_size(nv, simple);
-    const u64 dataSize   = full ? (u64)__ldg(reinterpret_cast<const u32*>(in->clusterTemplateInstantiatonSizes) + ci.clusterID)
-                                : (u64)basic[simple];
-    const u32 partSize   = full ? 0u : subset_part_slots(simple);
-    const u32 partOffset = full ? 0u : back_alloc(x, y, partSize, k.maxPartTriangles);
-    const bool ok        = fits(vertexSize, dataSize, partOffset, partSize);
+    const u32  vertexSize = subset_vertex_size(nv, simple);
+    const u64  dataSize   = (u64)basic[simple];
+    const u32  partSize   = subset_part_slots(simple);
+    const u32  partOffset = back_alloc(x, y, partSize, k.maxPartTriangles);
+    const bool ok         = fits(vertexSize, dataSize, partOffset, partSize);
     if(lane == 0)  // the vertex walk's record, per visible cluster with transient builds
       cs.fullRecs[v] = ok ? make_uint2(visIndex, vo) : make_uint2(kRejected, 0u);
     if(ok)
     {
       if(lane == 0)
       {
-        if(full)
-        {
-          const u32                  tempOffset = tb.temp + (g - genBase) - (tr - tb.trans);
-          tc_TemplateInstantiateInfo ti;
-          ti.clusterIdOffset        = 0;
-          ti.geometryIndexOffset    = 0;
-          ti.clusterTemplateAddress = __ldg(reinterpret_cast<const u64*>(in->clusterTemplateAdresses) + ci.clusterID);
-          ti.vertexBufferAddress    = b->genVertices + (u64)vo * 12ull;
-          ti.vertexBufferStride     = 12;
-          reinterpret_cast<tc_TemplateInstantiateInfo*>(b->tempInstantiations)[tempOffset] = ti;
-          reinterpret_cast<u32*>(b->tempInstanceIDs)[tempOffset]                          = ci.instanceID;
-          reinterpret_cast<u64*>(b->tempClusterAddresses)[tempOffset]                     = b->genClusterData + d;
-          if((c.flags & TC_FLAG_WRITE_FULLCLUSTERS) && b->fullClusters)
-            reinterpret_cast<tc_ClusterInfo*>(b->fullClusters)[tempOffset] = ci;
-          statTemp += 1;
-        }
-        else
-        {
-          store_clas_build(reinterpret_cast<tc_ClasBuildInfo*>(b->transBuilds) + tr, TC_RT_CLUSTER_MODE_1X_SUBSET_CLUSTER,
-                           partOffset, simple, nv, b->positionTruncateBitCount, b->genVertices + (u64)vo * 12ull);
-          reinterpret_cast<u32*>(b->transInstanceIDs)[tr]      = ci.instanceID;
-          reinterpret_cast<u64*>(b->transClusterAddresses)[tr] = b->genClusterData + d;
-          statTrans += 1;
-        }
+        store_clas_build(reinterpret_cast<tc_ClasBuildInfo*>(b->transBuilds) + tr, TC_RT_CLUSTER_MODE_1X_SUBSET_CLUSTER,
+                         partOffset, simple, nv, b->positionTruncateBitCount, b->genVertices + (u64)vo * 12ull);
+        reinterpret_cast<u32*>(b->transInstanceIDs)[tr]      = ci.instanceID;
+        reinterpret_cast<u64*>(b->transClusterAddresses)[tr] = b->genClusterData + d;
+        statTrans += 1;
         statTris += simple;
         atomicAdd(&blas[ci.instanceID].clusterReferencesCount, 1u);
       }
-      if(subset)
+      // :489-535 indices after the vertices, triangle map after the header
+      uint8_t* idx = gvb + ((u64)vo + nv) * 12;
+      uint8_t* map = ptb + (u64)partOffset * kTessInfoBytes;
+      warp_zero(idx, (simple * 3 + 11) / 12 * 3);
+      warp_zero(map, partSize * kTessInfoBytes / 4);
+      __syncwarp();
+      if(lane == 0)
+        *reinterpret_cast<uint2*>(map) = make_uint2(ci.instanceID, ci.clusterID);
+      const u32* tw = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
+      const uint8_t* lt = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
+      u32 out = 0;
+      for(u32 t0 = 0; t0 < nt; t0 += 32)
       {
-        // :489-535 indices after the vertices, triangle map after the header
-        uint8_t* idx = gvb + ((u64)vo + nv) * 12;
-        uint8_t* map = ptb + (u64)partOffset * kTessInfoBytes;
-        warp_zero(idx, (simple * 3 + 11) / 12 * 3);
-        warp_zero(map, partSize * kTessInfoBytes / 4);
-        __syncwarp();
-        if(lane == 0)
-          *reinterpret_cast<uint2*>(map) = make_uint2(ci.instanceID, ci.clusterID);
-        const u32* tw = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
-        const uint8_t* lt = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
-        u32 out = 0;
-        for(u32 t0 = 0; t0 < nt; t0 += 32)
+        const u32  tri = t0 + lane;
+        const bool sub = tri < nt && (tw[tri] & kWordSubset);
+        const u32  bm  = __ballot_sync(0xFFFFFFFFu, sub);
+        if(sub)
         {
-          const u32  tri = t0 + lane;
-          const bool sub = tri < nt && (tw[tri] & kWordSubset);
-          const u32  bm  = __ballot_sync(0xFFFFFFFFu, sub);
-          if(sub)
-          {
-            const u32 q = out + __popc(bm & ltm);
-            map[kClusterInfoBytes + q] = (uint8_t)tri;
-            idx[q * 3 + 0]            = lt[tri * 3 + 0];
-            idx[q * 3 + 1]            = lt[tri * 3 + 1];
-            idx[q * 3 + 2]            = lt[tri * 3 + 2];
-          }
-          out += __popc(bm);
+          const u32 q = out + __popc(bm & ltm);
+          map[kClusterInfoBytes + q] = (uint8_t)tri;
+          idx[q * 3 + 0]            = lt[tri * 3 + 0];
+          idx[q * 3 + 1]            = lt[tri * 3 + 1];
+          idx[q * 3 + 2]            = lt[tri * 3 + 2];
         }
+        out += __popc(bm);
       }
     }
-    g += 1, vo += vertexSize, d += dataSize;
-    if(subset)
-      tr += 1;
+    g += 1, vo += vertexSize, d += dataSize, tr += 1;
   }
   else if(lane == 0)
     cs.fullRecs[v] = make_uint2(kRejected, 0u);
-  if(full)
-    return;
 
   // ---- :543-905 the other triangles, one 32-triangle chunk at a time -------------
   const u32*   tw  = cs.triWords + (u64)v * TC_MAX_CLUSTER_TRIANGLES;
@@ -1284,6 +1312,15 @@ __device__ inline void block_prefix_transient(const ClassifyScratch& cs, u64 (&p
   pre[kTTrans] = t0.trans + tot[kTTrans];
 }
 
+// The offsets of every cluster, the full clusters' arguments (32 clusters at a
+// time, one per lane, like k_classify_write), and a list of the others, which
+// k_classify_emit_transient takes one per warp: a cluster with 1X and 2X builds
+// takes a warp about 10 us of dependent steps, and the visible, tessellated
+// clusters lie next to each other in the list, so a block that wrote its own
+// range's clusters had up to 57 of them while most blocks had none.
+// Measured on a GB300, 51,840 clusters of 256 instances, 1,217 of them partly
+// tessellated: 79 us from the count's end to the last write in one kernel,
+// 31 us in two.
 __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx c, ClassifyScratch cs)
 {
   stage_prologue();
@@ -1303,7 +1340,10 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
   tc_SceneBuilding*     b   = c.build;
   const tc_ClusterInfo* vis = reinterpret_cast<const tc_ClusterInfo*>(b->visibleClusters);
   const uint4*          counts = reinterpret_cast<const uint4*>(cs.counts);
-  u32                   statTemp = 0, statTrans = 0, statTris = 0;
+  const tc_caps&        k       = c.caps;
+  const u64             maxData = (u64)k.maxGeneratedClusterMegs * 1024ull * 1024ull;
+  tc_BlasBuildInfo*     blas    = reinterpret_cast<tc_BlasBuildInfo*>(b->blasBuildInfos);
+  u32                   statTemp = 0, statTris = 0;
 
   u64 pre[kTNum];
   block_prefix_transient(cs, pre, s_warp);
@@ -1333,20 +1373,77 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
     __syncthreads();
     const u32 perW = (len + kWarps - 1) / kWarps;
     const u32 lo = min(len, warp * perW), hi = min(len, lo + perW);
-    for(u32 i = lo; i < hi; i++)
-      write_cluster_transient(c, cs, begin + c0 + i, c0 + i, s_ci[i], s_cnt[i], s_off[i], genBase, tb, statTemp,
-                              statTrans, statTris);
+    for(u32 i0 = lo; i0 < hi; i0 += 32)
+    {
+      const u32  i       = i0 + lane;
+      const bool valid   = i < hi;
+      const uint4 r      = valid ? s_cnt[i] : make_uint4(0u, 0u, 0u, 0u);
+      const bool isFull  = valid && t_full(r);
+      u32        inst    = 0xFFFFFFFFu;
+      bool       full    = false;
+      // cluster_classify.comp.glsl:254-437, full clusters
+      if(isFull)
+      {
+        const TransOffsets o = s_off[i];
+        full = !((u64)o.vert + t_nv(r) > k.maxGeneratedVertices || (u64)o.gen + 1 > k.maxGeneratedClusters
+                 || o.data + r.z > maxData);
+        cs.fullRecs[c0 + i] = full ? make_uint2(begin + c0 + i, o.vert) : make_uint2(kRejected, 0u);
+        if(full)
+        {
+          const tc_ClusterInfo       ci = s_ci[i];
+          const tc_RenderInstance*   in = c.instances + ci.instanceID;
+          const u32                  tempOffset = tb.temp + (o.gen - genBase) - (o.trans - tb.trans);
+          tc_TemplateInstantiateInfo ti;
+          ti.clusterIdOffset        = 0;
+          ti.geometryIndexOffset    = 0;
+          ti.clusterTemplateAddress = __ldg(reinterpret_cast<const u64*>(in->clusterTemplateAdresses) + ci.clusterID);
+          ti.vertexBufferAddress    = b->genVertices + (u64)o.vert * 12ull;
+          ti.vertexBufferStride     = 12;
+          reinterpret_cast<tc_TemplateInstantiateInfo*>(b->tempInstantiations)[tempOffset] = ti;
+          reinterpret_cast<u32*>(b->tempInstanceIDs)[tempOffset]                          = ci.instanceID;
+          reinterpret_cast<u64*>(b->tempClusterAddresses)[tempOffset]                     = b->genClusterData + o.data;
+          if((c.flags & TC_FLAG_WRITE_FULLCLUSTERS) && b->fullClusters)
+            reinterpret_cast<tc_ClusterInfo*>(b->fullClusters)[tempOffset] = ci;
+          statTemp += 1;
+          statTris += t_simple(r);
+          inst = ci.instanceID;
+        }
+      }
+      // CLAS reference counts: one atomic per distinct instance of the batch
+      for(u32 remaining = __ballot_sync(0xFFFFFFFFu, full); remaining;)
+      {
+        const int src = __ffs(remaining) - 1;
+        const u32 gk  = __shfl_sync(0xFFFFFFFFu, inst, src);
+        const u32 sel = __ballot_sync(0xFFFFFFFFu, full && inst == gk);
+        remaining &= ~sel;
+        if((int)lane == src)
+          atomicAdd(&blas[gk].clusterReferencesCount, __popc(sel));
+      }
+      const u32 others = __ballot_sync(0xFFFFFFFFu, valid && !isFull);
+      if(others)
+      {
+        u32 at = 0;
+        if(lane == 0)
+          at = atomicAdd(cs.fullRange + 2, __popc(others));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(others & ((1u << lane) - 1u));
+        if(valid && !isFull)
+        {
+          const TransOffsets o   = s_off[i];
+          uint4*             rec = cs.transRecs + 3 * (u64)at;
+          rec[0]                 = make_uint4(c0 + i, s_ci[i].instanceID, s_ci[i].clusterID, o.front);
+          rec[1]                 = make_uint4(o.split, o.gen, o.vert, o.back);
+          rec[2]                 = make_uint4(o.trans, (u32)o.data, (u32)(o.data >> 32), 0u);
+        }
+      }
+    }
     __syncthreads();
   }
-  statTemp  = __reduce_add_sync(0xFFFFFFFFu, statTemp);
-  statTrans = __reduce_add_sync(0xFFFFFFFFu, statTrans);
-  statTris  = __reduce_add_sync(0xFFFFFFFFu, statTris);
+  statTemp = __reduce_add_sync(0xFFFFFFFFu, statTemp);
+  statTris = __reduce_add_sync(0xFFFFFFFFu, statTris);
   if(lane == 0)
   {
     if(statTemp)
       atomicAdd(&b->tempInstantiateCounter, statTemp);
-    if(statTrans)
-      atomicAdd(&b->transBuildCounter, statTrans);
     if(statTris)
       atomicAdd(&c.readback->numTotalTriangles, statTris);
   }
@@ -1370,6 +1467,37 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
     }
     if(c.fuseSetup != kNoSetup)
       build_setup_apply(c, c.fuseSetup);
+  }
+}
+
+// The clusters k_classify_write_transient listed: warps stride over them.
+__global__ void __launch_bounds__(kBlock, 4) k_classify_emit_transient(StageCtx c, ClassifyScratch cs)
+{
+  stage_prologue();
+  __shared__ u32 s_range[2];
+  if(threadIdx.x == 0)
+    window_range(c, s_range[0], s_range[1]);
+  __syncthreads();
+  const u32 begin = s_range[0], count = cs.fullRange[2];
+  const u32 lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
+  u32       statTrans = 0, statTris = 0;
+  for(u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps)
+  {
+    const uint4*         rec = cs.transRecs + 3 * (u64)i;
+    const uint4          a = rec[0], b = rec[1], d = rec[2];
+    const tc_ClusterInfo ci = {a.y, a.z};
+    const TransOffsets   o  = {a.w, b.x, b.y, b.z, b.w, d.x, (u64)d.y | ((u64)d.z << 32)};
+    write_cluster_transient(c, cs, begin + a.x, a.x, ci, reinterpret_cast<const uint4*>(cs.counts)[a.x], o, statTrans,
+                            statTris);
+  }
+  statTrans = __reduce_add_sync(0xFFFFFFFFu, statTrans);
+  statTris  = __reduce_add_sync(0xFFFFFFFFu, statTris);
+  if(lane == 0)
+  {
+    if(statTrans)
+      atomicAdd(&c.build->transBuildCounter, statTrans);
+    if(statTris)
+      atomicAdd(&c.readback->numTotalTriangles, statTris);
   }
 }
 
@@ -1588,7 +1716,7 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
   // the write launch's blocks own contiguous ranges of clusters, whose count
   // sums the count launch accumulates (its warps stride over the whole list)
   const u32 grid = std::max(1u, std::min(classify_max_blocks(maxClusters), numSMs * std::max(1u, warpBlocksPerSM)));
-  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, grid, 0, buf.fullRecs, buf.fullRange};
+  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, grid, 0, buf.fullRecs, buf.fullRange, buf.transRecs};
   // register budget from the requested residency: 4 or less -> 64, 5-7 -> 40, 8 and more -> 32
   if(c.flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X))
   {
@@ -1600,23 +1728,32 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
     cudaError_t e      = launch_pdl_critical(k_classify_count<4, true>, tgrid, kBlock, s, c, ts);
     if(e != cudaSuccess)
       return e;
-    return launch_pdl_critical(k_classify_write_transient, tgrid, kBlock, s, c, ts);
+    e = launch_pdl_critical(k_classify_write_transient, tgrid, kBlock, s, c, ts);
+    if(e != cudaSuccess)
+      return e;
+    const u32 egrid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * 4));
+    return launch_pdl_critical(k_classify_emit_transient, egrid, kBlock, s, c, ts);
   }
+  cs.listed       = classify_lists_clusters(maxClusters, numSMs, warpBlocksPerSM) ? 1u : 0u;
   const int   occ = warpBlocksPerSM >= 8 ? 8 : (warpBlocksPerSM >= 5 ? 6 : 4);
   cudaError_t e   = occ == 8   ? launch_pdl_critical(k_classify_count<8>, grid, kBlock, s, c, cs)
                     : occ == 6 ? launch_pdl_critical(k_classify_count<6>, grid, kBlock, s, c, cs)
                                : launch_pdl_critical(k_classify_count<4>, grid, kBlock, s, c, cs);
   if(e != cudaSuccess)
     return e;
-  return occ == 8   ? launch_pdl_critical(k_classify_write<8>, grid, kBlock, s, c, cs)
-         : occ == 6 ? launch_pdl_critical(k_classify_write<6>, grid, kBlock, s, c, cs)
-                    : launch_pdl_critical(k_classify_write<4>, grid, kBlock, s, c, cs);
+  e = occ == 8   ? launch_pdl_critical(k_classify_write<8>, grid, kBlock, s, c, cs)
+      : occ == 6 ? launch_pdl_critical(k_classify_write<6>, grid, kBlock, s, c, cs)
+                 : launch_pdl_critical(k_classify_write<4>, grid, kBlock, s, c, cs);
+  if(e != cudaSuccess || !cs.listed)
+    return e;
+  const u32 egrid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * 4));
+  return launch_pdl_critical(k_classify_emit, egrid, kBlock, s, c, cs);
 }
 
 cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffers& buf, u32 maxClusters, u32 numSMs,
                                           u32 blocksPerSM, cudaStream_t s)
 {
-  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, 0, 0, buf.fullRecs, buf.fullRange};
+  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, 0, 0, buf.fullRecs, buf.fullRange, buf.transRecs};
   // every warp of the grid takes a share of the slots
   const u32 grid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * std::max(1u, blocksPerSM)));
   // register budget from the requested residency: 4 or less -> 64, 5-6 -> 40, 7 and more -> 32
@@ -1629,6 +1766,11 @@ cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffe
   // over the builds, one resident wave of the kernel's blocks
   const u32 miniGrid = std::max(1u, std::min((maxClusters * 8 + kDeformWarps - 1) / kDeformWarps, numSMs * (u32)kDeformBlocksPerSM));
   return launch_pdl(k_classify_mini_vertices, miniGrid, kDeformBlock, s, c, cs);
+}
+
+bool classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM)
+{
+  return maxClusters > 32ull * numSMs * std::max(1u, warpBlocksPerSM);
 }
 
 u32 classify_max_blocks(u32 maxClusters) { return std::max(1u, (maxClusters + kWarps - 1) / kWarps); }

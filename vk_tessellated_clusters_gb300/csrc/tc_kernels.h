@@ -45,7 +45,8 @@ struct ClassifyBuffers
   RangeSums*      rangeSums;  // per block: the sums of its range's counts (zero before the launch)
   ClusterOffsets* bases;      // one: the counters before the launch (then one TransBases)
   uint2*          fullRecs;   // per full cluster of the window: visible index, first generated vertex
-  u32*            fullRange;  // [2]: the window's generated-cluster slots
+  u32*            fullRange;  // [2]: the window's generated-cluster slots; [2]: transRecs' count
+  uint4*          transRecs;  // 48 bytes per cluster that is not a full one
 };
 
 cudaError_t launch_frame_begin(const StageCtx& c, u32 grid, cudaStream_t s);
@@ -81,6 +82,10 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
 cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffers& buf, u32 maxClusters, u32 numSMs,
                                           u32 blocksPerSM, cudaStream_t s);
 u32         classify_max_blocks(u32 maxClusters);
+// whether launch_cluster_classify launches a kernel of its own for the
+// clusters with part or split triangles (without transient builds; with them
+// it always does)
+bool        classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM);
 cudaError_t launch_triangle_split(const StageCtx& c, u32 blockSize, u32 grid, cudaStream_t s);
 // every split pass in one launch: per level its look-back rows and control
 // words (a scratch slot each; the ticket of level 0's slot is the launch's)
