@@ -121,3 +121,31 @@ def test_deform_chunk_widths(oracle, case):
     assert_same(pipe.outputs(), want, case, vertex_tol=vertex_tolerance(sc))
     assert pipe.device_errors() == 0
     pipe.close()
+
+
+@pytest.mark.parametrize("count", [1, 31, 256, 257, 1023])
+@pytest.mark.parametrize("offset", [0, 4, 8])
+def test_decode_counts_and_alignment(oracle, count, offset):
+    """Partial blocks of hits at 4-, 8- and 16-byte aligned addresses: field-exact against the oracle, and nothing
+    written past the results."""
+    import torch
+    from vk_tessellated_clusters_gb300.hits import sample_hits
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_batched(num_instances=8, map_size=64)
+    caps = L.default_caps(visible_bits=16, part_bits=18, split_bits=14, vertex_bits=21, megs=256)
+    flags = FLAGS | L.FLAG_TRANSIENT_1X | L.FLAG_TRANSIENT_2X
+    cam = S.frame_constants(S.camera_orbit(0))
+    ref_state, _ = oracle.frame(sc, cam, caps, flags)
+    pipe = TessellationPipeline(sc, caps, flags)
+    pipe.set_cameras(cam)
+    pipe.build("batched")
+    hits = sample_hits(pipe.outputs(), sc, pipe.entries, count, seed=3, bad=0)
+    want = oracle.decode_hits(ref_state, hits)
+    src = torch.zeros(hits.nbytes + 16, dtype=torch.uint8, device="cuda")[offset:offset + hits.nbytes]
+    src.copy_(torch.from_numpy(hits.view(np.uint8).reshape(-1).copy()))
+    whole = torch.full((want.nbytes + 64,), 0xCD, dtype=torch.uint8, device="cuda")
+    pipe.decode_hits_device(src, whole[offset:])
+    got = whole.cpu().numpy()
+    assert got[offset:offset + want.nbytes].tobytes() == want.tobytes()
+    assert (got[:offset] == 0xCD).all() and (got[offset + want.nbytes:] == 0xCD).all()
+    pipe.close()

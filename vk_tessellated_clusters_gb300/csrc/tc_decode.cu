@@ -3,7 +3,13 @@
 // 2X batch hits when the frame was built with those transient builds), as a
 // kernel any CUDA ray tracer can run over its hit records.
 //
-// One thread per hit; every index is checked against the frame's data (a hit
+// One thread per hit. Hits (24 bytes) and results (40 bytes) go through shared
+// memory, so that global memory sees whole 16-byte words in order: a thread
+// that reads and writes its own records touches 24 and 40 sectors per
+// instruction. Bound by the chain of dependent loads (hit, part, instance,
+// cluster, indices, table), so the registers are held to 32 for eight blocks
+// per SM (38 registers, six blocks: 32.3 us). Measured on a GB300, 2,073,600
+// hits: 59.6 -> 29.3 us (133 MB of records, 4.5 TB/s). Every index is checked against the frame's data (a hit
 // from another frame reports TC_HIT_OUT_OF_RANGE instead of reading past a
 // buffer). Barycentric compositions are separate multiplies and adds in the
 // shader's order, so the results equal the CPU restatement's bit for bit.
@@ -27,13 +33,39 @@ __device__ __forceinline__ f3 compose(f3 a, f3 b, f3 c, f3 w)
   return scale_add(r, c, w.z);
 }
 
-__global__ void k_decode_hits(StageCtx c, const tc_hit* hits, u32 count, tc_base_hit* out)
+constexpr u32 kDecodeBlock = 256;
+constexpr u32 kHitWords = sizeof(tc_hit) / 4, kBaseHitWords = sizeof(tc_base_hit) / 4;
+
+// `words` consecutive 32-bit words by the block's threads, as 16-byte words
+// where both sides are aligned; the global side is touched once, so it is
+// marked to leave L2 first (the frame's part records stay).
+__device__ __forceinline__ void block_load(u32* shared, const u32* global, u32 words, bool aligned)
 {
-  stage_prologue();
-  const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= count)
-    return;
-  const tc_hit h = hits[i];
+  u32 q = threadIdx.x;
+  if(aligned)
+  {
+    for(; q < words / 4; q += kDecodeBlock)
+      reinterpret_cast<uint4*>(shared)[q] = __ldcs(reinterpret_cast<const uint4*>(global) + q);
+    q = words / 4 * 4 + threadIdx.x;
+  }
+  for(; q < words; q += kDecodeBlock)
+    shared[q] = __ldcs(global + q);
+}
+__device__ __forceinline__ void block_store(u32* global, const u32* shared, u32 words, bool aligned)
+{
+  u32 q = threadIdx.x;
+  if(aligned)
+  {
+    for(; q < words / 4; q += kDecodeBlock)
+      __stcs(reinterpret_cast<uint4*>(global) + q, reinterpret_cast<const uint4*>(shared)[q]);
+    q = words / 4 * 4 + threadIdx.x;
+  }
+  for(; q < words; q += kDecodeBlock)
+    __stcs(global + q, shared[q]);
+}
+
+__device__ __forceinline__ tc_base_hit decode_hit(const StageCtx& c, const tc_hit& h)
+{
   tc_base_hit  r = {};
   u32          mode = h.clusterID >> 30, clusterID = h.clusterID & 0x3FFFFFFFu;
   u32          triangleID = h.triangleID, subTriangleID = h.triangleID, cfg = 0;
@@ -105,10 +137,7 @@ __global__ void k_decode_hits(StageCtx c, const tc_hit* hits, u32 count, tc_base
       r.status = TC_HIT_OUT_OF_RANGE;
   }
   if(r.status != TC_HIT_OK)
-  {
-    out[i] = r;
-    return;
-  }
+    return r;
   // rchit.glsl:191-200: the base triangle's vertices
   const uint8_t* lt = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
   for(int v = 0; v < 3; v++)
@@ -138,7 +167,26 @@ __global__ void k_decode_hits(StageCtx c, const tc_hit* hits, u32 count, tc_base
   r.barycentrics[1] = base.y;
   r.barycentrics[2] = base.z;
   r.partID          = partID;
-  out[i]            = r;
+  return r;
+}
+
+__global__ void __launch_bounds__(kDecodeBlock, 8) k_decode_hits(StageCtx c, const tc_hit* hits, u32 count, tc_base_hit* out)
+{
+  stage_prologue();
+  // the block's hits, then its results (a record's words stay 8-byte aligned)
+  __shared__ __align__(16) u32 s_io[kDecodeBlock * kBaseHitWords];
+  const u32  first = blockIdx.x * kDecodeBlock, n = min(kDecodeBlock, count - first);
+  // a block's records start at a multiple of 16 bytes from the arrays' start
+  block_load(s_io, reinterpret_cast<const u32*>(hits + first), n * kHitWords, (reinterpret_cast<uintptr_t>(hits) & 15) == 0);
+  __syncthreads();
+  tc_hit h = {};
+  if(threadIdx.x < n)
+    h = reinterpret_cast<const tc_hit*>(s_io)[threadIdx.x];
+  __syncthreads();
+  if(threadIdx.x < n)
+    reinterpret_cast<tc_base_hit*>(s_io)[threadIdx.x] = decode_hit(c, h);
+  __syncthreads();
+  block_store(reinterpret_cast<u32*>(out + first), s_io, n * kBaseHitWords, (reinterpret_cast<uintptr_t>(out) & 15) == 0);
 }
 
 }  // namespace
@@ -147,7 +195,7 @@ cudaError_t launch_decode_hits(const StageCtx& c, const tc_hit* hits, u32 count,
 {
   if(count == 0)
     return cudaSuccess;
-  return launch_pdl(k_decode_hits, (count + 255) / 256, 256u, s, c, hits, count, out);
+  return launch_pdl(k_decode_hits, (count + kDecodeBlock - 1) / kDecodeBlock, kDecodeBlock, s, c, hits, count, out);
 }
 
 }  // namespace tc
