@@ -1212,7 +1212,7 @@ tc_status tc_generate_vertices(tc_context* ctx, const tc_frame_args* a, void* st
      || (a->flags & (TC_FLAG_PN | TC_FLAG_RIPPLE | TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)))
     return TC_ERR_INVALID_ARG;
   StageCtx c = base_ctx(ctx, a);
-  TC_CHECK_CUDA(launch_generate_vertices(c, ctx->numSMs * 8, reinterpret_cast<cudaStream_t>(stream)));
+  TC_CHECK_CUDA(launch_generate_vertices(c, ctx->numSMs * 4, reinterpret_cast<cudaStream_t>(stream)));
   ctx->launches += 1;
   return TC_OK;
 }

@@ -29,6 +29,7 @@
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
+#include "tc_walk.cuh"
 
 namespace tc {
 
@@ -198,19 +199,6 @@ __device__ __forceinline__ FactorParams factor_params(const StageCtx& c)
 // ---------------------------------------------------------------------------
 // scans
 // ---------------------------------------------------------------------------
-
-template <class T>
-__device__ __forceinline__ T warp_inclusive(T x, u32 lane)
-{
-#pragma unroll
-  for(int d = 1; d < 32; d <<= 1)
-  {
-    T y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-    if(lane >= (u32)d)
-      x += y;
-  }
-  return x;
-}
 
 // block-wide exclusive scan of kNumCounters values per thread
 __device__ inline void block_scan5(u64 (&v)[kNumCounters], u64 (&tot)[kNumCounters], u64 (*s_warp)[kNumCounters])
@@ -646,95 +634,6 @@ __device__ __forceinline__ void emit_triangle(tc_TessTriangleInfo* dst, const tc
     v2 = v1, v1 = v0, v0 = t;
   }
   store_tess_info(dst, ci, v0, v1, v2, tri | ((word & 0xFFFFu) << 16));
-}
-
-// what the vertex walk of a full cluster needs (phase 2 of k_classify_write)
-struct FullRecord
-{
-  MapDesc      map;
-  const float* pos;
-  const float* nrm;
-  const float* uvs;
-  u32          first;  // firstLocalVertex
-  float        scale;  // instance x view displacement scale
-  float        offset; // instance + view displacement offset
-  u32          vo;     // first generated vertex
-  u32          nv;     // vertex count
-  u32          inst;   // instance (the ripple's seed)
-  float        size;   // its geometry size (RenderInstance.geoHi.w)
-};
-
-// the vertex walk over a batch of full clusters (records in `rec`), for
-// records of map kind Kind (~0u: any)
-template <u32 Kind>
-__device__ __forceinline__ void full_steps(const FullRecord* rec, bool owner, u32 rStart, u32 rEnd, float* dst,
-                                           const RippleParams& rp)
-{
-  const u32 lane = threadIdx.x & 31;
-#pragma unroll 2  // two steps in flight: their loads overlap
-  for(u32 base = 0; base < rEnd; base += 32)
-  {
-    const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && rStart <= base));
-    const u32 inside = __reduce_or_sync(0xFFFFFFFFu,
-                                        (owner && rStart > base && rStart < base + 32) ? 1u << (rStart - base) : 0u);
-    const u32 ri     = before - 1 + __popc(inside & ((2u << lane) - 2u));
-    const u32 rs     = __shfl_sync(0xFFFFFFFFu, rStart, ri & 31);
-    const u32 jj     = base + lane;
-    const FullRecord& fr = rec[ri];
-    // (transient builds leave index bytes and 2X batches between the ranges)
-    if(jj < rEnd && jj - rs < fr.nv)
-    {
-      const u32 vi = fr.first + (jj - rs);
-      f3                p  = ldg3(fr.pos, vi);
-      if(Kind != kAffineFlat)
-        p = full_vertex_k<Kind>(p, ldg3(fr.nrm, vi), ldg2(fr.uvs, vi), fr.map, fr.scale, fr.offset);
-      if(rp.enabled)  // cluster_classify.comp.glsl:483-485
-        p = ripple(p, fr.inst, fr.size, rp);
-      float* d = dst + (u64)jj * 3;
-      d[0]     = p.x;
-      d[1]     = p.y;
-      d[2]     = p.z;
-    }
-  }
-}
-
-// full_steps for a batch whose records share the attribute arrays, map,
-// displacement scale and offset (and, with the ripple, the instance): those
-// stay in registers (`u`, read once per batch), and each step takes only its
-// record's vertex-index offset and range end from the record's lane (two
-// shuffles) instead of the record from shared memory. Same operations, so the
-// same bits.
-template <u32 Kind>
-__device__ __forceinline__ void full_steps_uniform(const FullRecord& u, bool owner, u32 rStart, u32 rOff, u32 rStop,
-                                                   u32 rEnd, float* dst, const RippleParams& rp)
-{
-  const u32 lane  = threadIdx.x & 31;
-  const u32 below = (2u << lane) - 2u;
-#pragma unroll 2  // two steps in flight: their loads overlap
-  for(u32 base = 0; base < rEnd; base += 32)
-  {
-    const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && rStart <= base));
-    const u32 inside = __reduce_or_sync(0xFFFFFFFFu,
-                                        (owner && rStart > base && rStart < base + 32) ? 1u << (rStart - base) : 0u);
-    const u32 ri     = (before - 1 + __popc(inside & below)) & 31;
-    const u32 off    = __shfl_sync(0xFFFFFFFFu, rOff, ri);
-    const u32 stop   = __shfl_sync(0xFFFFFFFFu, rStop, ri);
-    const u32 jj     = base + lane;
-    // (transient builds leave index bytes and 2X batches between the ranges)
-    if(jj < stop)
-    {
-      const u32 vi = off + jj;
-      f3        p  = ldg3(u.pos, vi);
-      if(Kind != kAffineFlat)
-        p = full_vertex_k<Kind>(p, ldg3(u.nrm, vi), ldg2(u.uvs, vi), u.map, u.scale, u.offset);
-      if(rp.enabled)  // cluster_classify.comp.glsl:483-485
-        p = ripple(p, u.inst, u.size, rp);
-      float* d = dst + (u64)jj * 3;
-      d[0]     = p.x;
-      d[1]     = p.y;
-      d[2]     = p.z;
-    }
-  }
 }
 
 // cluster_classify.comp.glsl:543-666: the part and split triangles of one
@@ -1596,14 +1495,12 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_full_vertices(St
   __shared__ FlatStarts s_starts;
   const u32*            starts = stage_flat_starts(c, s_starts);
   const u32             lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const u32             ltm  = (1u << lane) - 1u;
   const u32             count        = cs.fullRange[1] - cs.fullRange[0];
   const u32             totalWarps   = gridDim.x * kWarps;
   const u32             per          = min(32u, max(1u, (count + totalWarps - 1) / totalWarps));
   const u32             numChunks    = (count + per - 1) / per;
   const tc_SceneBuilding* b          = c.build;
   const tc_ClusterInfo* vis          = reinterpret_cast<const tc_ClusterInfo*>(b->visibleClusters);
-  const bool            haveTextures = c.numTextures > 0 && c.textures != nullptr;
   float*                gv           = reinterpret_cast<float*>(b->genVertices);
   FullRecord*           rec          = s_full[warp];
   const RippleParams    rp           = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
@@ -1618,92 +1515,11 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_full_vertices(St
       const uint2 fs = cs.fullRecs[slot];
       if(fs.x != kRejected)
       {
-        const tc_ClusterInfo     ci = visible_cluster(c, starts, vis, fs.x);
-        const tc_RenderInstance* in = c.instances + ci.instanceID;
-        const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
-        owner                       = true;
-        fr.vo                       = fs.y;
-        fr.nv                       = min((u32)cl.numVertices, TC_MAX_CLUSTER_VERTICES);
-        fr.pos                      = reinterpret_cast<const float*>(in->positions);
-        fr.nrm                      = reinterpret_cast<const float*>(in->normals);
-        fr.uvs                      = reinterpret_cast<const float*>(in->texcoords);
-        fr.first                    = cl.firstLocalVertex;
-        tc_DisplacementTexture tx   = {};
-        if(haveTextures && in->displacementIndex >= 0)
-        {
-          if((u32)in->displacementIndex < c.numTextures)
-            tx = c.textures[in->displacementIndex];
-          else
-            atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
-        }
-        fr.map    = make_map_desc(tx);
-        fr.scale  = in->displacementScale * c.view->displacementScale;
-        fr.offset = in->displacementOffset + c.view->displacementOffset;
-        fr.inst   = ci.instanceID;
-        fr.size   = in->geoHi.w;
+        owner = true;
+        fr    = full_record(c, visible_cluster(c, starts, vis, fs.x), fs.y);
       }
     }
-    // the owners' records in slot order (their vertex ranges follow each
-    // other, with gaps only where transient builds placed other data)
-    const u32 fm = __ballot_sync(0xFFFFFFFFu, owner);
-    if(fm == 0)
-      continue;
-    if(owner)
-      rec[__popc(fm & ltm)] = fr;
-    __syncwarp();
-    // per record (lane r < nrec): first vertex within the batch and vertex count
-    const u32  nrec   = __popc(fm);
-    const u32  vBase  = rec[0].vo;
-    const u32  rStart = lane < nrec ? rec[lane].vo - vBase : 0u;
-    const u32  rCount = lane < nrec ? rec[lane].nv : 0u;
-    const u32  rEnd   = __shfl_sync(0xFFFFFFFFu, rStart + rCount, nrec - 1);
-    const bool own    = lane < nrec;
-    // one specialisation when the batch's clusters share a map kind
-    const u32 kind  = own ? rec[lane].map.kind : 0u;
-    const u32 kind0 = rec[0].map.kind;
-    const u32 kw    = __all_sync(0xFFFFFFFFu, !own || kind == kind0) ? kind0 : ~0u;
-    float*    dst   = gv + (u64)vBase * 3;
-    // the usual batch: consecutive clusters of instances of one mesh and map
-    const FullRecord u    = rec[0];
-    const bool       same = !own
-                      || (rec[lane].pos == u.pos && rec[lane].nrm == u.nrm && rec[lane].uvs == u.uvs
-                          && rec[lane].map.kind == u.map.kind
-                          && __float_as_uint(rec[lane].map.q7.x) == __float_as_uint(u.map.q7.x)
-                          && __float_as_uint(rec[lane].map.q7.y) == __float_as_uint(u.map.q7.y)
-                          && __float_as_uint(rec[lane].map.q7.z) == __float_as_uint(u.map.q7.z)
-                          && __float_as_uint(rec[lane].map.q7.w) == __float_as_uint(u.map.q7.w)
-                          && __float_as_uint(rec[lane].scale) == __float_as_uint(u.scale)
-                          && __float_as_uint(rec[lane].offset) == __float_as_uint(u.offset)
-                          && (!rp.enabled || (rec[lane].inst == u.inst && __float_as_uint(rec[lane].size) == __float_as_uint(u.size))));
-    if(__all_sync(0xFFFFFFFFu, same))
-    {
-      // per record (lane r): vertex index of batch vertex jj is rOff + jj, for jj < rStop
-      const u32 rOff  = own ? rec[lane].first - rStart : 0u;
-      const u32 rStop = own ? rStart + rCount : 0u;
-      switch(u.map.kind)
-      {
-        case affine_kind(TC_TEXEL_F32, true):
-          full_steps_uniform<affine_kind(TC_TEXEL_F32, true)>(u, own, rStart, rOff, rStop, rEnd, dst, rp);
-          break;
-        case affine_kind(TC_TEXEL_F16, true):
-          full_steps_uniform<affine_kind(TC_TEXEL_F16, true)>(u, own, rStart, rOff, rStop, rEnd, dst, rp);
-          break;
-        case kAffineFlat: full_steps_uniform<kAffineFlat>(u, own, rStart, rOff, rStop, rEnd, dst, rp); break;
-        default: full_steps_uniform<~0u>(u, own, rStart, rOff, rStop, rEnd, dst, rp); break;
-      }
-    }
-    else
-      switch(kw)
-      {
-        case affine_kind(TC_TEXEL_F32, true):
-          full_steps<affine_kind(TC_TEXEL_F32, true)>(rec, own, rStart, rEnd, dst, rp);
-          break;
-        case affine_kind(TC_TEXEL_F16, true):
-          full_steps<affine_kind(TC_TEXEL_F16, true)>(rec, own, rStart, rEnd, dst, rp);
-          break;
-        case kAffineFlat: full_steps<kAffineFlat>(rec, own, rStart, rEnd, dst, rp); break;
-        default: full_steps<~0u>(rec, own, rStart, rEnd, dst, rp); break;
-      }
+    full_batch(rec, owner, fr, gv, rp);
     __syncwarp();  // records are rewritten by the next batch
   }
 }

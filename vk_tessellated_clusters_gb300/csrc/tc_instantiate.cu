@@ -29,6 +29,7 @@
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 #include "tc_vertex.cuh"
+#include "tc_walk.cuh"
 
 namespace tc {
 
@@ -38,7 +39,6 @@ constexpr u32 kBlock        = 256;
 constexpr u32 kItems        = 4;
 constexpr u32 kTile         = kBlock * kItems;
 constexpr u32 kWarps        = kBlock / 32;
-constexpr u32 kPartsPerWarp = 32;  // parts staged per warp and chunk: one per lane
 constexpr u32 kScanBlock    = 1024;
 constexpr u32 kChunksPerTile = kTile / kPartsPerWarp;  // 32-part chunks per allocation tile
 static_assert(kChunksPerTile == 32, "one warp reads a tile's chunk sums");
@@ -84,19 +84,6 @@ __device__ inline void part_range(const StageCtx& c, u32& lo, u32& hi)
     lo       = lower_bound_instance(lo, e, c.instBegin, get);
     hi       = e;
   }
-}
-
-template <class T>
-__device__ __forceinline__ T warp_inclusive(T x, u32 lane)
-{
-#pragma unroll
-  for(int d = 1; d < 32; d <<= 1)
-  {
-    T y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-    if(lane >= (u32)d)
-      x += y;
-  }
-  return x;
 }
 
 __device__ __forceinline__ u32 part_cfg(const tc_TessTriangleInfo* parts, u32 p)
@@ -301,38 +288,6 @@ __global__ void __launch_bounds__(kScanBlock) k_instantiate_tile_scan(StageCtx c
 // ---------------------------------------------------------------------------
 // write: arguments, counts, vertices
 // ---------------------------------------------------------------------------
-
-// Uniform: every part of the chunk has the map, scale and offset in `m`,
-// `scale`, `offset` (held in registers; the records' q6-q8 are not read).
-// `tvBase`: per owner lane, its part's first table vertex minus its first
-// vertex within the chunk (table index of chunk vertex jj = tvBase + jj).
-template <u32 Kind, bool Uniform>
-__device__ __forceinline__ void chunk_vertices(const StageCtx& c, const PartAffine* sp, u32 owner, u32 start, u32 tvBase,
-                                               u32 total, float* dst, const MapDesc& m, float scale, float offset)
-{
-  const u32 lane  = threadIdx.x & 31;
-  const u32 below = (2u << lane) - 2u;  // bits 1..lane
-  #pragma unroll 2  // two steps in flight: their loads overlap
-  for(u32 base = 0; base < total; base += 32)
-  {
-    // lane's part: those starting at or before the step's first vertex, plus
-    // those starting inside the step up to the lane (one bit each)
-    const u32         before = __popc(__ballot_sync(0xFFFFFFFFu, owner && start <= base));
-    const u32         inside = __reduce_or_sync(0xFFFFFFFFu,
-                                                (owner && start > base && start < base + 32) ? 1u << (start - base) : 0u);
-    const u32         pi     = before - 1 + __popc(inside & below);
-    const u32         tvIdx  = __shfl_sync(0xFFFFFFFFu, tvBase, pi & 31);
-    const u32         jj     = base + lane;
-    const PartAffine& r      = sp[pi];
-    if(jj < total)
-    {
-      const u32 tv = __ldg(c.table.vertices + (tvIdx + jj));
-      const f3  q  = Uniform ? affine_vertex_u<Kind>(r, tv, m, scale, offset) : affine_vertex_k<Kind>(r, tv);
-      float*   d = dst + 3 * (u64)jj;
-      d[0] = q.x, d[1] = q.y, d[2] = q.z;
-    }
-  }
-}
 
 __global__ void __launch_bounds__(kBlock, 4) k_instantiate_args(StageCtx c, InstantiateBuffers ib)
 {
@@ -541,116 +496,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_instantiate_args(StageCtx c, Inst
 // ---------------------------------------------------------------------------
 // vertices
 // ---------------------------------------------------------------------------
-
-// One lane's part (records r0..r2 of its TessTriangleInfo): its affine
-// record in `rec` (tc_vertex.cuh), vertex count, map kind and description,
-// first table vertex, displacement scale and offset.
-__device__ __forceinline__ void lane_part(const StageCtx& c, uint2 r0, uint2 r1, uint2 r2, PartAffine& rec, u32& nv,
-                                          u32& kind, u32& tvBase, float& scale, float& offset, MapDesc& map)
-{
-  const u32                cfg = r2.y >> 16;
-  const u32                tri = r2.y & 0xFFFFu;
-  const tc_TessTableEntry  e   = table_entry(c.table, cfg);
-  const tc_RenderInstance& in  = c.instances[r0.x];
-  const tc_Cluster         cl  = reinterpret_cast<const tc_Cluster*>(in.clusters)[r0.y];
-  const uint8_t*           lt  = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle;
-  const u32                corner[3] = {r1.x, r1.y, r2.x};
-  tc_DisplacementTexture   tx = {};
-  if(c.numTextures > 0 && c.textures != nullptr && in.displacementIndex >= 0)
-  {
-    if((u32)in.displacementIndex < c.numTextures)
-      tx = c.textures[in.displacementIndex];
-    else
-      atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
-  }
-  scale  = in.displacementScale * c.view->displacementScale;
-  offset = in.displacementOffset + c.view->displacementOffset;
-  part_affine(rec, corner, cfg_flipped(cfg), reinterpret_cast<const float*>(in.positions),
-              reinterpret_cast<const float*>(in.normals), reinterpret_cast<const float*>(in.texcoords),
-              cl.firstLocalVertex, lt + tri * 3, e.firstVertex, tx, scale, offset);
-  map    = make_map_desc(tx);
-  nv     = e.numVertices;
-  kind   = map.kind;
-  tvBase = e.firstVertex;
-}
-
-// The vertices of one chunk, after every lane set up its part's record in
-// `sp[lane]` (nv = 0: no part): lanes walk the chunk's contiguous vertex
-// range (first generated vertex: lane 0's `vo`) on consecutive vertices, with
-// one specialisation for the whole chunk when its parts share a map kind, and
-// the map, scale and offset in registers when they share those too.
-__device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffine* sp, float* gv, u32 vo, u32 nv,
-                                             u32 kind, u32 tvBase, const MapDesc& map, float scale, float offset)
-{
-  const u32 lane = threadIdx.x & 31;
-  const u32  inc   = warp_inclusive<u32>(nv, lane);
-  const u32  start = inc - nv;  // first vertex of this lane's part within the chunk
-  const u32  total = __shfl_sync(0xFFFFFFFFu, inc, kPartsPerWarp - 1);
-  const u32  v0    = __shfl_sync(0xFFFFFFFFu, vo, 0);
-  const bool owner = lane < kPartsPerWarp && nv > 0;
-  tvBase -= start;  // table index of chunk vertex jj: tvBase + jj
-  // one specialisation for the whole chunk when its parts share a map kind
-  const u32 kind0 = __shfl_sync(0xFFFFFFFFu, kind, 0);
-  const u32 kw    = __all_sync(0xFFFFFFFFu, !owner || kind == kind0) ? kind0 : ~0u;
-  // the usual chunk: every part displaced from one map with one scale and
-  // offset (lane 0 always owns a part: accepted parts form a prefix)
-  MapDesc um;
-  um.q7 = make_float4(__shfl_sync(0xFFFFFFFFu, map.q7.x, 0), __shfl_sync(0xFFFFFFFFu, map.q7.y, 0),
-                      __shfl_sync(0xFFFFFFFFu, map.q7.z, 0), __shfl_sync(0xFFFFFFFFu, map.q7.w, 0));
-  um.q8 = make_float4(__shfl_sync(0xFFFFFFFFu, map.q8.x, 0), __shfl_sync(0xFFFFFFFFu, map.q8.y, 0),
-                      __shfl_sync(0xFFFFFFFFu, map.q8.z, 0), __shfl_sync(0xFFFFFFFFu, map.q8.w, 0));
-  um.kind            = kind0;
-  const float uScale = __shfl_sync(0xFFFFFFFFu, scale, 0), uOffset = __shfl_sync(0xFFFFFFFFu, offset, 0);
-  const bool  same   = !owner
-                    || (__float_as_uint(map.q7.x) == __float_as_uint(um.q7.x)
-                        && __float_as_uint(map.q7.y) == __float_as_uint(um.q7.y)
-                        && __float_as_uint(map.q7.z) == __float_as_uint(um.q7.z)
-                        && __float_as_uint(map.q7.w) == __float_as_uint(um.q7.w)
-                        && __float_as_uint(scale) == __float_as_uint(uScale)
-                        && __float_as_uint(offset) == __float_as_uint(uOffset) && kind == kind0);
-  const bool  uni    = __all_sync(0xFFFFFFFFu, same);
-  __syncwarp();
-  float* dst = gv + 3 * (u64)v0;
-#define TC_CHUNK(K)                                                                                                    \
-  (uni ? chunk_vertices<K, true>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset)                       \
-       : chunk_vertices<K, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset))
-  switch(kw)
-  {
-    case affine_kind(TC_TEXEL_F16, true): TC_CHUNK(affine_kind(TC_TEXEL_F16, true)); break;
-    case affine_kind(TC_TEXEL_F32, true): TC_CHUNK(affine_kind(TC_TEXEL_F32, true)); break;
-    case kAffineFlat:
-      chunk_vertices<kAffineFlat, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset);
-      break;
-    default: chunk_vertices<~0u, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset); break;
-  }
-#undef TC_CHUNK
-}
-
-// Parts per chunk of a launch with `n` parts, `vertices` vertices in all (about)
-// and `nwarps` warps: `most` (a lane sets up one part), halved
-//  - while the chunks still take no more than half of the warps. The parts of
-//    a small frame have up to 78 vertices each, so 32 of them in a row keep
-//    one warp busy for 50 us while most of the chip idles: 1,280 parts of 36
-//    vertices took 54.7 us in 40 chunks of 32 and take 11.7 us in 1,280 chunks
-//    of one (the frame 69.8 -> 48.3 us);
-//  - while there are fewer than two chunks per warp for the ticket to even
-//    out, as long as a chunk keeps 256 vertices (eight steps of the walk) for
-//    its set-up: 25,600 parts of 70 vertices, with PN, took 70.7 us in 800
-//    chunks of 32.
-// Parts of five vertices stay at 32 (60,000 of them in 16s: the frame 0.5 %
-// slower; the full clusters' vertices and the allocations run beside).
-__device__ __forceinline__ u32 chunk_parts(u32 n, u32 vertices, u32 nwarps, u32 most)
-{
-  u32 w = most;
-  while(w > 1)
-  {
-    const u32 chunks = (n + w / 2 - 1) / (w / 2);
-    if(chunks > nwarps / 2 && (chunks > 2 * nwarps || vertices / chunks < 256))
-      break;
-    w >>= 1;
-  }
-  return w;
-}
 
 // The vertices of parts [begin, begin + n) from their offsets (0: unknown,
 // some were not accepted).
