@@ -52,16 +52,17 @@ class FrozenFrame:
         self._layout_gradients(scene)
 
     def _layout_gradients(self, scene) -> None:
-        """All gradients of one backward live in one flat float32 buffer; the
-        kernel's pointer tables (per instance dPositions/dNormals, per map
-        texels) point into it once and for all, so a backward is a zero fill,
-        the kernel and one copy out, with no host-to-device transfer."""
+        """All gradients of one backward live in one flat float32 buffer, in
+        parameter order; the kernel's pointer tables (per instance
+        dPositions/dNormals, per map texels) are its address plus these
+        offsets (0 where a gradient is not wanted), so a backward is a zeroed
+        buffer, one addition for the table and the kernel, with no
+        host-to-device transfer and no copy."""
         torch = self.torch
         sizes = [p.numel() for p in self.positions] + [n.numel() for n in self.normals]
         sizes += [t.numel() if t is not None else 0 for t in self.texels]
         starts = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
         self._grad_floats = int(starts[-1])
-        self._grad_starts = starts
         ng = len(self.positions)
         rel = np.zeros((len(self._inst_geo), 2), np.int64)
         rel[:, 0] = 4 * starts[self._inst_geo]
@@ -69,13 +70,12 @@ class FrozenFrame:
         tex = np.array([4 * starts[2 * ng + i] if t is not None else -1 for i, t in enumerate(self.texels)] or [-1],
                        np.int64)
         self._num_targets = rel.size
-        # one persistent gradient buffer and its pointer table (built once);
-        # every backward zeroes it, accumulates into it and hands out a copy
-        self._flat = torch.zeros(self._grad_floats, dtype=torch.float32, device=self.pipe.device)
-        base = self._flat.data_ptr()
-        table = np.concatenate([rel.reshape(-1), tex])
-        table = np.where(table >= 0, table + base, 0).astype(np.int64)
-        self._table = torch.from_numpy(table).to(self.pipe.device)
+        offsets = np.concatenate([rel.reshape(-1), tex])
+        device = self.device = torch.device("cuda", self.pipe.device)
+        self._offsets = torch.from_numpy(np.maximum(offsets, 0)).to(device)
+        self._wanted = torch.from_numpy((offsets >= 0).astype(np.int64)).to(device)
+        self._flat, self._table = None, None  # gradient_buffers()
+        self._vertices = self.pipe.gen_vertices_tensor(self.num_vertices)
 
     def _view(self, buf, shape):
         n = int(np.prod(shape))
@@ -93,11 +93,17 @@ class FrozenFrame:
     def generate(self):
         """Vertices of the frozen frame from the current parameters (a copy)."""
         self.pipe.stage("generate_vertices")
-        return self.pipe.gen_vertices_tensor(self.num_vertices).clone()
+        return self._vertices.clone()
+
+    def _pointer_table(self, flat):
+        return self.torch.add(self._offsets, self._wanted, alpha=flat.data_ptr())
 
     def gradient_buffers(self, device=None):
-        """The persistent flat float32 gradient buffer, zeroed (enqueued on the
+        """A persistent flat float32 gradient buffer, zeroed (enqueued on the
         current stream), and the kernel's pointer table into it."""
+        if self._flat is None:
+            self._flat = self.torch.zeros(self._grad_floats, dtype=self.torch.float32, device=self.device)
+            self._table = self._pointer_table(self._flat)
         self._flat.zero_()
         return self._flat, self._table
 
@@ -105,19 +111,20 @@ class FrozenFrame:
         """tc_instantiate_backward: accumulates dL/dv into the buffer `table` points at."""
         self.pipe.backward(grad_vertices.data_ptr(), table.data_ptr(), table.data_ptr() + 8 * self._num_targets)
 
+    def gradients(self, grad_vertices):
+        """dL/dv -> the gradients of parameters(), in their order; all enqueued
+        on the current stream, no synchronisation."""
+        flat = self.torch.empty(self._grad_floats, dtype=self.torch.float32, device=self.device).zero_()
+        self.launch_backward(grad_vertices.contiguous().float(), self._pointer_table(flat))
+        return self.torch._utils._unflatten_dense_tensors(flat, self.parameters())
+
     def scatter_gradients(self, grad_vertices):
         """dL/dv -> (dPositions, dNormals, dTexels), lists parallel to the
-        parameters; all enqueued on the current stream, no synchronisation."""
-        buf, table = self.gradient_buffers()
-        self.launch_backward(grad_vertices.contiguous().float(), table)
-        flat = buf.clone()
-        st = self._grad_starts
-        ng = len(self.positions)
-        views = [flat[st[i]:st[i + 1]] for i in range(len(st) - 1)]
-        dP = [views[i].view(p.shape) for i, p in enumerate(self.positions)]
-        dN = [views[ng + i].view(n.shape) for i, n in enumerate(self.normals)]
-        dT = [views[2 * ng + i].view(t.shape) if t is not None else None for i, t in enumerate(self.texels)]
-        return dP, dN, dT
+        parameters (None for a map without gradient)."""
+        grads, ng = self.gradients(grad_vertices), len(self.positions)
+        texels = iter(grads[2 * ng:])
+        return (list(grads[:ng]), list(grads[ng:2 * ng]),
+                [next(texels) if t is not None else None for t in self.texels])
 
 
 class _Tessellate:
@@ -137,17 +144,7 @@ class _Tessellate:
 
                 @staticmethod
                 def backward(ctx, grad):
-                    f = ctx.frozen
-                    dP, dN, dT = f.scatter_gradients(grad)
-                    grads = []
-                    for p, g in zip(f.positions, dP):
-                        grads.append(g)
-                    for n, g in zip(f.normals, dN):
-                        grads.append(g)
-                    for t, g in zip(f.texels, dT):
-                        if t is not None:
-                            grads.append(g)
-                    return (None, *grads)
+                    return (None, *ctx.frozen.gradients(grad))
 
             cls.fn = TessellateFunction
         return cls.fn
