@@ -149,3 +149,42 @@ def test_decode_counts_and_alignment(oracle, count, offset):
     assert got[offset:offset + want.nbytes].tobytes() == want.tobytes()
     assert (got[:offset] == 0xCD).all() and (got[offset + want.nbytes:] == 0xCD).all()
     pipe.close()
+
+
+# group sizes below, at and above the kernel's 8 members; instances that share a mesh but not map, scale or offset;
+# no sharing at all (the walk by clusters); a vertex capacity that refuses the last clusters
+@pytest.mark.parametrize("case", ["pairs", "eights", "nines", "mixed", "distinct", "overflow", "mixed_transient"])
+def test_instance_groups(oracle, case):
+    """Integers bit-exact against the oracle and positions to the vertex tolerance, from the graph twice and from the
+    per-instance launches, which use no groups."""
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_batched(num_instances={"pairs": 2, "eights": 32, "nines": 36}.get(case, 48), map_size=64)
+    for i, inst in enumerate(sc.instances):
+        if case == "pairs":
+            inst.geometry, inst.displacement_index = 3, 1
+        if case.startswith("mixed"):
+            # none, map 0, map 1; under the ripple maps only (it has no value at an undisplaced origin)
+            inst.displacement_index = (i // 4) % 3 - (0 if case == "mixed_transient" else 1)
+            inst.displacement_scale = 0.01 * (1 + i // 12 % 2)
+            inst.displacement_offset = 0.005 * (i // 24)
+        if case == "distinct":
+            inst.displacement_scale = 0.001 * (i + 1)
+    flags = FLAGS
+    caps = L.default_caps(vertex_bits=22)
+    if case == "mixed_transient":
+        flags |= L.FLAG_TRANSIENT_1X | L.FLAG_TRANSIENT_2X | L.FLAG_RIPPLE
+    if case == "overflow":
+        caps = dict(caps, maxGeneratedVertices=300000)
+    fc = _ripple(S.camera_orbit(5))
+    ref_state, _ = oracle.frame(sc, fc, caps, flags)
+    want = ref_state.outputs(oracle.entries)
+    if case == "overflow":
+        assert int(want["readback"]["numGenVertices"]) > 300000
+    pipe = TessellationPipeline(sc, caps, flags)
+    pipe.set_cameras(fc)
+    for mode in ("graph", "graph", "plain"):
+        pipe.state.gen_vertices.handle.zero_()
+        pipe.build(mode)
+        assert_same(pipe.outputs(), want, f"{case} {mode}", vertex_tol=vertex_tolerance(sc))
+    assert pipe.device_errors() == 0
+    pipe.close()

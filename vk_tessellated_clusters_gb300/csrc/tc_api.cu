@@ -50,6 +50,8 @@ struct Plan
   size_t runOffset;   // run starts (u32 x kMaxRuns+2)
   u32    classifyCap; // clusters the classify scratch holds
   size_t clsCountsOffset, clsTriWordsOffset, clsBlockSumsOffset, clsFullRecsOffset, clsTransRecsOffset;
+  u32    groupCap;  // instances the group tables hold
+  size_t groupOffset;
   size_t rasterOffset;
   size_t partVertexOffset;  // u32 per part triangle
   size_t chunkSumsOffset;   // u64 per 32 part triangles
@@ -113,6 +115,7 @@ struct tc_context
   // overlaps the split passes (fork / join through the two events)
   cudaStream_t side    = nullptr;  // the first part run's instantiation
   cudaStream_t side2   = nullptr;  // the full clusters' vertices
+  cudaStream_t side3   = nullptr;  // the instance groups they use
   cudaEvent_t  evFork  = nullptr;
   cudaEvent_t  evJoin  = nullptr;  // first part run allocated
   cudaEvent_t  evJoin2 = nullptr;  // full clusters' vertices written
@@ -121,6 +124,7 @@ struct tc_context
   cudaEvent_t  evInst  = nullptr;  // instances classified
   cudaEvent_t  evScan0 = nullptr;  // first part run's offsets (and the counters after it)
   cudaEvent_t  evCull  = nullptr;  // clusters_cull done (on the second side stream)
+  cudaEvent_t  evGroup = nullptr;  // instance groups done
 
   // graph cache
   cudaGraphExec_t graphExec = nullptr;
@@ -209,6 +213,9 @@ Plan make_plan(const tc_context_desc& d)
   off = align_up(off + (size_t)p.classifyCap * 8 + 16, 256);
   p.clsTransRecsOffset = off;
   off = align_up(off + (size_t)p.classifyCap * 48, 256);
+  p.groupCap    = std::min(kGroupInstances, std::max(1u, d.maxInstances));
+  p.groupOffset = off;  // head, subgroups, members
+  off           = align_up(off + 16 + (size_t)p.groupCap * 24, 256);
   p.partVertexOffset  = off;
   off                 = align_up(off + (size_t)std::max(1u, k.maxPartTriangles) * 4, 256);
   p.chunkSumsOffset   = off;
@@ -301,7 +308,11 @@ ClassifyBuffers classify_buffers(tc_context* ctx)
           reinterpret_cast<ClusterOffsets*>(ctx->dScratch + p.clsBlockSumsOffset),
           reinterpret_cast<uint2*>(ctx->dScratch + p.clsFullRecsOffset),
           reinterpret_cast<u32*>(ctx->dScratch + p.clsFullRecsOffset + (size_t)p.classifyCap * 8),
-          reinterpret_cast<uint4*>(ctx->dScratch + p.clsTransRecsOffset)};
+          reinterpret_cast<uint4*>(ctx->dScratch + p.clsTransRecsOffset),
+          nullptr,
+          reinterpret_cast<u32*>(ctx->dScratch + p.groupOffset + 16 + (size_t)p.groupCap * 16),
+          p.groupCap,
+          reinterpret_cast<u32*>(ctx->dScratch + p.groupOffset)};
 }
 
 InstantiateBuffers instantiate_buffers(tc_context* ctx)
@@ -330,6 +341,13 @@ bool emits_clusters(const tc_context* ctx, const tc_frame_args* a)
                                     ctx->schedule.classifyBlocksPerSM);
 }
 
+// whether a batched frame writes its full clusters' vertices once per group of
+// instances (RT semantics only: the visible list is every cluster in instance order)
+bool groups_instances(const tc_frame_args* a)
+{
+  return (a->flags & TC_FLAG_RASTER_CULL) == 0 && a->numInstances >= 2 && a->numInstances <= kGroupInstances;
+}
+
 // kernels one batched frame launches (the BLAS set-up is fused for up to
 // kBlasSetupFusedMax instances)
 uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
@@ -338,6 +356,7 @@ uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
          - (a->numInstances <= kBlasSetupFusedMax ? 1 : 0)
          - (ctx->schedule.frameShape == 1 ? 4 : 0)  // one allocation + vertex launch instead of two
          + (emits_clusters(ctx, a) ? 1 : 0)              // the clusters with part or split triangles
+         + (groups_instances(a) ? 1 : 0)
          + ((a->flags & TC_FLAG_TRANSIENT_2X) ? 1 : 0);                           // the 2X batches' vertices
 }
 
@@ -418,6 +437,9 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   // clusters_cull (which writes it out, with its counter and set-up) runs on
   // the second side stream, joined at the frame's end.
   const bool flat = (a->flags & TC_FLAG_RASTER_CULL) == 0;
+  ClassifyBuffers cb = classify_buffers(ctx);
+  if(groups_instances(a))
+    cb.groups = reinterpret_cast<uint4*>(ctx->dScratch + p.groupOffset + 16);
   {
     StageCtx cc = c;
     bind_slot(ctx, cc, p.slotCull, false);
@@ -428,6 +450,12 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
       TC_CHECK_CUDA(cudaEventRecord(ctx->evInst, s));
       TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evInst, 0));
       cs = ctx->side2;
+      if(cb.groups)  // beside the cull, for the full clusters' vertices
+      {
+        TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side3, ctx->evInst, 0));
+        TC_CHECK_CUDA(launch_instance_groups(c, cb, ctx->side3));
+        TC_CHECK_CUDA(cudaEventRecord(ctx->evGroup, ctx->side3));
+      }
     }
     TC_CHECK_CUDA(
         launch_clusters_cull(cc, persistent_grid(ctx, ceil_div(a->totalClusters, kCullTile), 4), kCullTile, cs, flat));
@@ -438,7 +466,7 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
 
   bind_slot(ctx, c, p.slotClassify, false);
   c.fuseSetup = TC_BUILD_SETUP_SPLIT;
-  TC_CHECK_CUDA(launch_cluster_classify(c, classify_buffers(ctx), std::min(a->totalClusters, a->caps.maxVisibleClusters),
+  TC_CHECK_CUDA(launch_cluster_classify(c, cb, std::min(a->totalClusters, a->caps.maxVisibleClusters),
                                         ctx->numSMs, sched.classifyBlocksPerSM, s));
 
   // The parts classify produced (run 0) come first in the instantiation order
@@ -452,7 +480,9 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   // The full clusters' vertices depend on classify alone and nothing later in
   // the frame reads them: they run on a second side stream, joined at the end.
   TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evFork, 0));
-  TC_CHECK_CUDA(launch_classify_full_vertices(c, classify_buffers(ctx),
+  if(cb.groups)
+    TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evGroup, 0));
+  TC_CHECK_CUDA(launch_classify_full_vertices(c, cb,
                                               std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
                                               sched.fullVertexBlocksPerSM, ctx->side2));
   TC_CHECK_CUDA(cudaEventRecord(ctx->evJoin2, ctx->side2));
@@ -672,10 +702,10 @@ namespace {
 void destroy_streams(tc_context* ctx)
 {
   for(cudaEvent_t* e : {&ctx->evFork, &ctx->evJoin, &ctx->evJoin2, &ctx->evArgs1, &ctx->evVerts, &ctx->evInst,
-                        &ctx->evScan0, &ctx->evCull})
+                        &ctx->evScan0, &ctx->evCull, &ctx->evGroup})
     if(*e)
       cudaEventDestroy(*e), *e = nullptr;
-  for(cudaStream_t* st : {&ctx->side, &ctx->side2})
+  for(cudaStream_t* st : {&ctx->side, &ctx->side2, &ctx->side3})
     if(*st)
       cudaStreamDestroy(*st), *st = nullptr;
 }
@@ -704,6 +734,7 @@ tc_status tc_context_create(const tc_context_desc* desc, tc_context** outCtx)
   ctx->numSMs   = (u32)std::max(1, sms);
   if(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess
      || cudaStreamCreateWithFlags(&ctx->side2, cudaStreamNonBlocking) != cudaSuccess
+     || cudaStreamCreateWithFlags(&ctx->side3, cudaStreamNonBlocking) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evFork, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evJoin, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evJoin2, cudaEventDisableTiming) != cudaSuccess
@@ -711,7 +742,8 @@ tc_status tc_context_create(const tc_context_desc* desc, tc_context** outCtx)
      || cudaEventCreateWithFlags(&ctx->evVerts, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evInst, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evScan0, cudaEventDisableTiming) != cudaSuccess
-     || cudaEventCreateWithFlags(&ctx->evCull, cudaEventDisableTiming) != cudaSuccess)
+     || cudaEventCreateWithFlags(&ctx->evCull, cudaEventDisableTiming) != cudaSuccess
+     || cudaEventCreateWithFlags(&ctx->evGroup, cudaEventDisableTiming) != cudaSuccess)
   {
     destroy_streams(ctx);
     delete ctx;

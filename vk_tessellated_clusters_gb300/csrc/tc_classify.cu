@@ -106,6 +106,9 @@ struct ClassifyScratch
   u32             listed;       // k_classify_write leaves the clusters with parts to k_classify_emit
   uint2*          fullRecs;   // per full cluster (generated-cluster slot - first slot): visible index, first vertex
   u32*            fullRange;  // [2]: the launch's generated-cluster slots [begin, end); [2]: transRecs' count
+  const uint4*    groups;     // instance groups, or null; with them fullRecs are per visible cluster
+  const u32*      members;
+  const u32*      groupHead;
   uint4*          transRecs;  // per cluster left to k_classify_emit (two words) or k_classify_emit_transient (three)
 };
 
@@ -816,7 +819,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
           const u32            v   = c0 + i;
           full = !((u64)off.vert + cnt_verts(r) > k.maxGeneratedVertices || (u64)off.gen + 1 > k.maxGeneratedClusters
                    || off.data + r.y > maxData);
-          cs.fullRecs[off.gen - genBase] = full ? make_uint2(begin + v, off.vert) : make_uint2(kRejected, 0u);
+          cs.fullRecs[cs.groups ? v : off.gen - genBase] = full ? make_uint2(begin + v, off.vert) : make_uint2(kRejected, 0u);
           if(full)
           {
             const tc_ClusterInfo     ci = s_ci[i];
@@ -840,6 +843,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
             inst = ci.instanceID;
           }
         }
+        else if(cs.groups)
+          cs.fullRecs[c0 + i] = make_uint2(kRejected, 0u);
       }
       const u32 fm = __ballot_sync(0xFFFFFFFFu, full);
       // CLAS reference counts: one atomic per distinct instance of the batch
@@ -875,8 +880,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
   // counters after count took their values
   if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
   {
-    cs.fullRange[0] = genBase;
-    cs.fullRange[1] = (u32)pre[kCntGen];
+    cs.fullRange[0] = cs.groups ? 0u : genBase;
+    cs.fullRange[1] = cs.groups ? n : (u32)pre[kCntGen];
     if(n)
     {
       const ClusterOffsets b0  = *cs.bases;
@@ -1481,30 +1486,121 @@ __global__ void __launch_bounds__(kDeformBlock, kDeformBlocksPerSM) k_classify_m
   }
 }
 
-// cluster_classify.comp.glsl:457-482: the displaced vertices of the full
-// clusters the write launch accepted. A warp takes `per` <= 32 consecutive
-// generated-cluster slots (per: the slots spread over all of the grid's
-// warps): one lane per cluster sets up its record, then the clusters' vertex
-// ranges, contiguous in genVertices, are walked on consecutive lanes. Its own
-// launch so that it can overlap other work.
-template <int MinBlocks>
-__global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_full_vertices(StageCtx c, ClassifyScratch cs)
+// ---------------------------------------------------------------------------
+// full clusters' vertices
+// ---------------------------------------------------------------------------
+
+// what the vertices of an instance's full clusters depend on
+struct GroupKey
+{
+  u64   positions, normals, texcoords, clusters;
+  int   map;
+  float scale, offset;
+  u32   numClusters;
+};
+
+__device__ __forceinline__ GroupKey group_key(const tc_RenderInstance& in)
+{
+  return {in.positions, in.normals, in.texcoords, in.clusters, in.displacementIndex, in.displacementScale,
+          in.displacementOffset, in.numClusters};
+}
+
+__device__ __forceinline__ bool same_key(const GroupKey& a, const GroupKey& b)
+{
+  return a.positions == b.positions && a.normals == b.normals && a.texcoords == b.texcoords && a.clusters == b.clusters
+         && a.map == b.map && __float_as_uint(a.scale) == __float_as_uint(b.scale)
+         && __float_as_uint(a.offset) == __float_as_uint(b.offset) && a.numClusters == b.numClusters;
+}
+
+// One block: the frame's instances grouped by key (a hash table of their
+// indices in shared memory), the groups cut into subgroups of at most
+// kGroupMembers, and a task per cluster of every subgroup. It runs beside the
+// classification and reads the instance records alone. Grouping is left out
+// (head[2] = 0) when instances have fewer than two in a group on average.
+// 256 threads: a block of 1,024 would need an SM to itself, which it does not
+// get until the classification ends.
+constexpr u32 kGroupBlock = 256, kGroupTable = 2 * kGroupInstances;
+
+// `members` has room for a second array of as many words
+__global__ void __launch_bounds__(kGroupBlock, 4) k_instance_groups(StageCtx c, uint4* groups, u32* members, u32 cap, u32* head)
 {
   stage_prologue();
-  __shared__ FullRecord s_full[kWarps][32];
-  __shared__ FlatStarts s_starts;
-  const u32*            starts = stage_flat_starts(c, s_starts);
+  __shared__ unsigned short s_table[kGroupTable];
+  __shared__ u32            s_count[kGroupInstances], s_scan[33];
+  constexpr unsigned short  kEmpty = 0xFFFF;
+  const u32                 n      = min(c.numInstances, min(cap, kGroupInstances));
+  u32*                      place  = members + cap;  // per instance: representative | rank << 16
+  for(u32 i = threadIdx.x; i < kGroupTable; i += kGroupBlock)
+    s_table[i] = kEmpty;
+  for(u32 i = threadIdx.x; i < kGroupInstances; i += kGroupBlock)
+    s_count[i] = 0;
+  __syncthreads();
+  for(u32 i = threadIdx.x; i < n; i += kGroupBlock)
+  {
+    const GroupKey key = group_key(c.instances[i]);
+    u64            h   = key.positions ^ (key.clusters << 1) ^ ((u64)(u32)key.map << 40) ^ ((u64)__float_as_uint(key.scale) << 8);
+    h *= 0x9E3779B97F4A7C15ull;  // Fibonacci hashing: the high bits of a multiple of 2^64 / golden ratio
+    u32 rep = ~0u;
+    for(u32 slot = (u32)(h >> 40) % kGroupTable; rep == ~0u; slot = (slot + 1) % kGroupTable)
+    {
+      // (the table has twice as many slots as instances)
+      const unsigned short found = atomicCAS(&s_table[slot], kEmpty, (unsigned short)i);
+      if(found == kEmpty)
+        rep = i;
+      else if(same_key(key, group_key(c.instances[found])))
+        rep = found;
+    }
+    place[i] = rep | atomicAdd(&s_count[rep], 1u) << 16;
+  }
+  __syncthreads();
+  // the representatives' members, subgroups and tasks, scanned in instance order
+  const u32 per = (n + kGroupBlock - 1) / kGroupBlock;
+  const u32 i0 = min(n, threadIdx.x * per), i1 = min(n, i0 + per);
+  u32       sumM = 0, sumS = 0, sumT = 0, reps = 0;
+  for(u32 i = i0; i < i1; i++)
+    if((place[i] & 0xFFFFu) == i)
+    {
+      const u32 m = s_count[i], subs = (m + kGroupMembers - 1) / kGroupMembers;
+      sumM += m, sumS += subs, sumT += subs * c.instances[i].numClusters, reps++;
+    }
+  u32 totalM, totalS, totalT, totalR;
+  u32 atM = block_exclusive_scan(sumM, s_scan, &totalM);
+  u32 atS = block_exclusive_scan(sumS, s_scan, &totalS);
+  u32 atT = block_exclusive_scan(sumT, s_scan, &totalT);
+  block_exclusive_scan(reps, s_scan, &totalR);
+  for(u32 i = i0; i < i1; i++)
+    if((place[i] & 0xFFFFu) == i)
+    {
+      const u32 m = s_count[i];
+      s_count[i]  = atM;  // now the group's first member
+      for(u32 k = 0; k < m; k += kGroupMembers)
+      {
+        groups[atS++] = make_uint4(atT, atM + k, min(kGroupMembers, m - k), i);
+        atT += c.instances[i].numClusters;
+      }
+      atM += m;
+    }
+  __syncthreads();
+  for(u32 i = threadIdx.x; i < n; i += kGroupBlock)
+    members[s_count[place[i] & 0xFFFFu] + (place[i] >> 16)] = i;
+  if(threadIdx.x == 0)
+    head[0] = totalS, head[1] = totalT, head[2] = n >= 2 * totalR ? 1u : 0u;
+}
+
+// cluster_classify.comp.glsl:457-482: the displaced vertices of the full
+// clusters the write launch accepted. A warp takes `per` <= 32 consecutive
+// records (per: the records spread over all of the grid's warps): one lane per
+// cluster, then the clusters' vertex ranges, contiguous in genVertices, are
+// walked on consecutive lanes.
+__device__ __forceinline__ void full_slots(const StageCtx& c, const ClassifyScratch& cs, const u32* starts,
+                                           FullRecord* rec, float* gv, const RippleParams& rp)
+{
   const u32             lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32             count        = cs.fullRange[1] - cs.fullRange[0];
   const u32             totalWarps   = gridDim.x * kWarps;
   const u32             per          = min(32u, max(1u, (count + totalWarps - 1) / totalWarps));
   const u32             numChunks    = (count + per - 1) / per;
-  const tc_SceneBuilding* b          = c.build;
-  const tc_ClusterInfo* vis          = reinterpret_cast<const tc_ClusterInfo*>(b->visibleClusters);
-  float*                gv           = reinterpret_cast<float*>(b->genVertices);
-  FullRecord*           rec          = s_full[warp];
-  const RippleParams    rp           = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
-
+  const tc_ClusterInfo* vis          = reinterpret_cast<const tc_ClusterInfo*>(c.build->visibleClusters);
   for(u32 chunk = blockIdx.x * kWarps + warp; chunk < numChunks; chunk += totalWarps)
   {
     const u32  slot  = chunk * per + lane;
@@ -1524,6 +1620,160 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_full_vertices(St
   }
 }
 
+// Its own launch so that it can overlap other work.
+template <int MinBlocks>
+__global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_full_vertices(StageCtx c, ClassifyScratch cs)
+{
+  stage_prologue();
+  __shared__ FullRecord s_full[kWarps][32];
+  __shared__ FlatStarts s_starts;
+  const u32*            starts = stage_flat_starts(c, s_starts);
+  full_slots(c, cs, starts, s_full[threadIdx.x >> 5], reinterpret_cast<float*>(c.build->genVertices),
+             ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0));
+}
+
+// The same vertices by instance groups (k_instance_groups). They are in object
+// space, so instances of one mesh, map, scale and offset have the same ones:
+// a warp evaluates a cluster's vertices once for a subgroup and stores them for
+// each member whose cluster is a full one, as consecutive words. One at a
+// time, the walk above reads 32 bytes of attributes and its texel sectors for
+// each vertex through L2, which bounds it (about 9 TB/s). Measured on a GB300:
+// 2.4 M vertices of 256 instances 34 -> 14 us, 9.9 M of 1,024 instances
+// 115 -> 35 us (the frames 109 -> 101 and 287 -> 233 us). Under the ripple,
+// which differs by instance, the lanes take (member, vertex) pairs.
+__global__ void __launch_bounds__(kBlock, 4) k_classify_full_groups(StageCtx c, ClassifyScratch cs)
+{
+  stage_prologue();
+  __shared__ union
+  {
+    FullRecord full[kWarps][32];
+    float      words[kWarps][3 * TC_MAX_CLUSTER_VERTICES];
+  } s;
+  __shared__ uint2      s_member[kWarps][kGroupMembers];
+  __shared__ FlatStarts s_starts;
+  const u32*            starts = stage_flat_starts(c, s_starts);
+  const u32             lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float*                gv   = reinterpret_cast<float*>(c.build->genVertices);
+  const RippleParams    rp   = ripple_params(*c.view, (c.flags & TC_FLAG_RIPPLE) != 0);
+  if(cs.groupHead[2] == 0)
+  {
+    full_slots(c, cs, starts, s.full[warp], gv, rp);
+    return;
+  }
+  const u32 subs = cs.groupHead[0], tasks = cs.groupHead[1], n = cs.fullRange[1];
+  const u32 gwarp = blockIdx.x * kWarps + warp, nwarps = gridDim.x * kWarps;
+  float*    words = s.words[warp];
+  for(u32 t0 = gwarp; t0 < tasks; t0 += 32 * nwarps)
+  {
+    // lane's task t0 + lane * nwarps: its representative instance, cluster and
+    // the members' first vertices (~0: the cluster is not a full one there)
+    u32        rep = 0, firstV = 0, nv = 0, member = 0;
+    u32        vo[kGroupMembers];
+    const u64  t     = (u64)t0 + (u64)lane * nwarps;
+    const bool valid = t < tasks;
+#pragma unroll
+    for(u32 m = 0; m < kGroupMembers; m++)
+      vo[m] = ~0u;
+    if(valid)
+    {
+      u32 lo = 0, hi = subs;  // the last subgroup whose first task is at most t
+      while(hi - lo > 1)
+      {
+        const u32 mid = (lo + hi) >> 1;
+        if(cs.groups[mid].x <= (u32)t)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      const uint4      g  = cs.groups[lo];
+      const u32        k  = (u32)t - g.x;
+      const tc_Cluster cl = reinterpret_cast<const tc_Cluster*>(c.instances[g.w].clusters)[k];
+      rep = g.w, member = g.y, firstV = cl.firstLocalVertex;
+      nv  = min((u32)cl.numVertices, TC_MAX_CLUSTER_VERTICES);
+      u32 v[kGroupMembers];
+#pragma unroll
+      for(u32 m = 0; m < kGroupMembers; m++)
+        v[m] = m < g.z ? starts[cs.members[g.y + m]] + k : ~0u;
+#pragma unroll
+      for(u32 m = 0; m < kGroupMembers; m++)
+        if(v[m] < n)
+        {
+          const uint2 r = cs.fullRecs[v[m]];
+          vo[m]         = r.x != kRejected ? r.y : ~0u;
+        }
+    }
+    bool any = false;
+#pragma unroll
+    for(u32 m = 0; m < kGroupMembers; m++)
+      any |= vo[m] != ~0u;
+    for(u32 left = __ballot_sync(0xFFFFFFFFu, any); left; left &= left - 1)
+    {
+      const int  src = __ffs(left) - 1;
+      const u32  cv  = __shfl_sync(0xFFFFFFFFu, nv, src);
+      FullRecord fr  = full_attributes(c, __shfl_sync(0xFFFFFFFFu, rep, src));
+      fr.first       = __shfl_sync(0xFFFFFFFFu, firstV, src);
+      for(u32 i = lane; i < cv; i += 32)
+      {
+        const f3 p = full_vertex(fr, i);
+        words[3 * i] = p.x, words[3 * i + 1] = p.y, words[3 * i + 2] = p.z;
+      }
+      if(rp.enabled)  // cluster_classify.comp.glsl:483-485: by instance; the lanes take (member, vertex) pairs
+      {
+        u32 count = 0;
+#pragma unroll
+        for(u32 m = 0; m < kGroupMembers; m++)
+          if((int)lane == src && vo[m] != ~0u)
+            s_member[warp][count++] = make_uint2(vo[m], member + m);
+        count = __shfl_sync(0xFFFFFFFFu, count, src);
+        __syncwarp();
+        u32   first = 0, inst = 0;
+        float size = 0.0f;
+        if(lane < count)
+        {
+          first = s_member[warp][lane].x;
+          inst  = cs.members[s_member[warp][lane].y];
+          size  = c.instances[inst].geoHi.w;
+        }
+        u32 m = 0, i = lane;
+        for(u32 base = 0; base < count * cv; base += 32, i += 32)
+        {
+          for(; i >= cv; i -= cv)
+            m++;
+          const u32   mFirst = __shfl_sync(0xFFFFFFFFu, first, m & 31), mInst = __shfl_sync(0xFFFFFFFFu, inst, m & 31);
+          const float mSize  = __shfl_sync(0xFFFFFFFFu, size, m & 31);
+          if(m < count)
+          {
+            const f3 q = ripple({words[3 * i], words[3 * i + 1], words[3 * i + 2]}, mInst, mSize, rp);
+            float*   d = gv + 3 * ((u64)mFirst + i);
+            d[0] = q.x, d[1] = q.y, d[2] = q.z;
+          }
+        }
+      }
+      else
+      {
+        __syncwarp();
+        float w[6];
+#pragma unroll
+        for(u32 q = 0; q < 6; q++)
+          w[q] = lane + 32 * q < 3 * cv ? words[lane + 32 * q] : 0.0f;
+#pragma unroll
+        for(u32 m = 0; m < kGroupMembers; m++)
+        {
+          const u32 first = __shfl_sync(0xFFFFFFFFu, vo[m], src);
+          if(first == ~0u)
+            continue;
+          float* dst = gv + 3 * (u64)first;
+#pragma unroll
+          for(u32 q = 0; q < 6; q++)
+            if(lane + 32 * q < 3 * cv)
+              dst[lane + 32 * q] = w[q];
+        }
+      }
+      __syncwarp();  // the words are rewritten by the warp's next cluster
+    }
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& buf, u32 maxClusters, u32 numSMs,
@@ -1532,7 +1782,8 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
   // the write launch's blocks own contiguous ranges of clusters, whose count
   // sums the count launch accumulates (its warps stride over the whole list)
   const u32 grid = std::max(1u, std::min(classify_max_blocks(maxClusters), numSMs * std::max(1u, warpBlocksPerSM)));
-  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, grid, 0, buf.fullRecs, buf.fullRange, buf.transRecs};
+  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, grid, 0, buf.fullRecs, buf.fullRange, buf.groups,
+                     buf.members, buf.groupHead, buf.transRecs};
   // register budget from the requested residency: 4 or less -> 64, 5-7 -> 40, 8 and more -> 32
   if(c.flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X))
   {
@@ -1566,14 +1817,22 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
   return launch_pdl_critical(k_classify_emit, egrid, kBlock, s, c, cs);
 }
 
+cudaError_t launch_instance_groups(const StageCtx& c, const ClassifyBuffers& buf, cudaStream_t s)
+{
+  return launch_kernel(k_instance_groups, 1u, kGroupBlock, high_launch_priority(), false, s, c, buf.groups, buf.members,
+                       buf.groupCap, buf.groupHead);
+}
+
 cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffers& buf, u32 maxClusters, u32 numSMs,
                                           u32 blocksPerSM, cudaStream_t s)
 {
-  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, 0, 0, buf.fullRecs, buf.fullRange, buf.transRecs};
+  ClassifyScratch cs{buf.counts, buf.triWords, buf.rangeSums, buf.bases, 0, 0, buf.fullRecs, buf.fullRange, buf.groups,
+                     buf.members, buf.groupHead, buf.transRecs};
   // every warp of the grid takes a share of the slots
   const u32 grid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * std::max(1u, blocksPerSM)));
   // register budget from the requested residency: 4 or less -> 64, 5-6 -> 40, 7 and more -> 32
-  cudaError_t e = blocksPerSM >= 7   ? launch_pdl(k_classify_full_vertices<8>, grid, kBlock, s, c, cs)
+  cudaError_t e = cs.groups          ? launch_pdl(k_classify_full_groups, grid, kBlock, s, c, cs)
+                  : blocksPerSM >= 7 ? launch_pdl(k_classify_full_vertices<8>, grid, kBlock, s, c, cs)
                   : blocksPerSM >= 5 ? launch_pdl(k_classify_full_vertices<6>, grid, kBlock, s, c, cs)
                                      : launch_pdl(k_classify_full_vertices<4>, grid, kBlock, s, c, cs);
   if(e != cudaSuccess || !(c.flags & TC_FLAG_TRANSIENT_2X))

@@ -47,7 +47,18 @@ struct ClassifyBuffers
   uint2*          fullRecs;   // per full cluster of the window: visible index, first generated vertex
   u32*            fullRange;  // [2]: the window's generated-cluster slots; [2]: transRecs' count
   uint4*          transRecs;  // 48 bytes per cluster that is not a full one
+  uint4*          groups;     // instance groups (launch_instance_groups), or null: none this frame
+  u32*            members;    // [2 * groupCap]: their instances, and scratch
+  u32             groupCap;
+  u32*            groupHead;  // [4]: subgroups, tasks, whether grouping pays
 };
+
+// Instances that share their mesh, displacement map, scale and offset, and so
+// the vertices of their full clusters: found for frames of 2 to
+// kGroupInstances instances, in subgroups of at most kGroupMembers.
+constexpr u32 kGroupInstances = 4096;
+constexpr u32 kGroupMembers   = 8;
+cudaError_t launch_instance_groups(const StageCtx& c, const ClassifyBuffers& buf, cudaStream_t s);
 
 cudaError_t launch_frame_begin(const StageCtx& c, u32 grid, cudaStream_t s);
 cudaError_t launch_decode_hits(const StageCtx& c, const tc_hit* hits, u32 count, tc_base_hit* out, cudaStream_t s);

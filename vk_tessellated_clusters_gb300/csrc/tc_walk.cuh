@@ -151,10 +151,11 @@ __device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffi
 //    one warp busy for 50 us while most of the chip idles: 1,280 parts of 36
 //    vertices took 54.7 us in 40 chunks of 32 and take 11.7 us in 1,280 chunks
 //    of one (the frame 69.8 -> 48.3 us);
+//  - while there are no more chunks than warps and a chunk keeps 64 vertices
+//    (two steps of the walk);
 //  - while there are fewer than two chunks per warp for the ticket to even
-//    out, as long as a chunk keeps 256 vertices (eight steps of the walk) for
-//    its set-up: 25,600 parts of 70 vertices, with PN, took 70.7 us in 800
-//    chunks of 32.
+//    out, as long as a chunk keeps 256 vertices for its set-up: 25,600 parts of
+//    70 vertices, with PN, took 70.7 us in 800 chunks of 32.
 // Parts of five vertices stay at 32 (60,000 of them in 16s: the frame 0.5 %
 // slower; the full clusters' vertices and the allocations run beside).
 __device__ __forceinline__ u32 chunk_parts(u32 n, u32 vertices, u32 nwarps, u32 most)
@@ -163,7 +164,7 @@ __device__ __forceinline__ u32 chunk_parts(u32 n, u32 vertices, u32 nwarps, u32 
   while(w > 1)
   {
     const u32 chunks = (n + w / 2 - 1) / (w / 2);
-    if(chunks > nwarps / 2 && (chunks > 2 * nwarps || vertices / chunks < 256))
+    if(chunks > nwarps / 2 && (chunks > 2 * nwarps || vertices / chunks < (chunks > nwarps ? 256u : 64u)))
       break;
     w >>= 1;
   }
@@ -263,18 +264,14 @@ __device__ __forceinline__ void full_steps_uniform(const FullRecord& u, bool own
   }
 }
 
-// the record of full cluster `ci` whose first generated vertex is `vo`
-__device__ __forceinline__ FullRecord full_record(const StageCtx& c, const tc_ClusterInfo& ci, u32 vo)
+// what the vertices of instance `inst`'s full clusters share
+__device__ __forceinline__ FullRecord full_attributes(const StageCtx& c, u32 inst)
 {
-  const tc_RenderInstance* in = c.instances + ci.instanceID;
-  const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
-  FullRecord               fr;
-  fr.vo                     = vo;
-  fr.nv                     = min((u32)cl.numVertices, TC_MAX_CLUSTER_VERTICES);
+  const tc_RenderInstance* in = c.instances + inst;
+  FullRecord               fr = {};
   fr.pos                    = reinterpret_cast<const float*>(in->positions);
   fr.nrm                    = reinterpret_cast<const float*>(in->normals);
   fr.uvs                    = reinterpret_cast<const float*>(in->texcoords);
-  fr.first                  = cl.firstLocalVertex;
   tc_DisplacementTexture tx = {};
   if(c.numTextures > 0 && c.textures != nullptr && in->displacementIndex >= 0)
   {
@@ -286,9 +283,29 @@ __device__ __forceinline__ FullRecord full_record(const StageCtx& c, const tc_Cl
   fr.map    = make_map_desc(tx);
   fr.scale  = in->displacementScale * c.view->displacementScale;
   fr.offset = in->displacementOffset + c.view->displacementOffset;
-  fr.inst   = ci.instanceID;
+  fr.inst   = inst;
   fr.size   = in->geoHi.w;
   return fr;
+}
+
+// the record of full cluster `ci` whose first generated vertex is `vo`
+__device__ __forceinline__ FullRecord full_record(const StageCtx& c, const tc_ClusterInfo& ci, u32 vo)
+{
+  const tc_Cluster cl = reinterpret_cast<const tc_Cluster*>(c.instances[ci.instanceID].clusters)[ci.clusterID];
+  FullRecord       fr = full_attributes(c, ci.instanceID);
+  fr.vo               = vo;
+  fr.nv               = min((u32)cl.numVertices, TC_MAX_CLUSTER_VERTICES);
+  fr.first            = cl.firstLocalVertex;
+  return fr;
+}
+
+// vertex i of the cluster in `fr`, before the ripple
+__device__ __forceinline__ f3 full_vertex(const FullRecord& fr, u32 i)
+{
+  const u32 vi = fr.first + i;
+  const f3  p  = ldg3(fr.pos, vi);
+  return fr.map.kind == kAffineFlat ? p
+                                    : full_vertex_k<~0u>(p, ldg3(fr.nrm, vi), ldg2(fr.uvs, vi), fr.map, fr.scale, fr.offset);
 }
 
 // The vertices of up to 32 full clusters: owner lanes hold their record `fr`,
