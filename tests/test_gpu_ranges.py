@@ -151,17 +151,25 @@ def test_decode_counts_and_alignment(oracle, count, offset):
     pipe.close()
 
 
-# group sizes below, at and above the kernel's 8 members; instances that share a mesh but not map, scale or offset;
-# no sharing at all (the walk by clusters); a vertex capacity that refuses the last clusters
-@pytest.mark.parametrize("case", ["pairs", "eights", "nines", "mixed", "distinct", "overflow", "mixed_transient"])
+# Frames of 16,384 clusters and more group their instances: groups of 24 and 25 (subgroups of 8 with and without a
+# rest), a pair (grouped, but with too many distinct clusters for bounds), instances that share a mesh but not map,
+# scale or offset, no sharing at all; capacities that refuse the last clusters, and an instance short of the limit
+@pytest.mark.parametrize("case", ["groups24", "groups25", "pair", "mixed", "distinct", "vertices", "visible", "below",
+                                  "mixed_transient"])
 def test_instance_groups(oracle, case):
     """Integers bit-exact against the oracle and positions to the vertex tolerance, from the graph twice and from the
-    per-instance launches, which use no groups."""
+    direct launches; the per-instance launches, which use no groups, give the same bytes."""
     from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
-    sc = S.scene_batched(num_instances={"pairs": 2, "eights": 32, "nines": 36}.get(case, 48), map_size=64)
+    if case == "pair":
+        mesh = S.clusterize(S.grid(512, 512, 4.0, 4.0), 0)
+        sc = S.scene_batched(num_instances=2, map_size=64)
+        sc.geometries = [mesh]
+        for inst in sc.instances:
+            inst.geometry, inst.displacement_index = 0, 1
+    else:
+        sc = S.scene_batched(num_instances={"groups25": 100, "below": 80}.get(case, 96), map_size=64)
+    assert (sc.total_clusters >= 16384) == (case != "below")
     for i, inst in enumerate(sc.instances):
-        if case == "pairs":
-            inst.geometry, inst.displacement_index = 3, 1
         if case.startswith("mixed"):
             # none, map 0, map 1; under the ripple maps only (it has no value at an undisplaced origin)
             inst.displacement_index = (i // 4) % 3 - (0 if case == "mixed_transient" else 1)
@@ -173,18 +181,24 @@ def test_instance_groups(oracle, case):
     caps = L.default_caps(vertex_bits=22)
     if case == "mixed_transient":
         flags |= L.FLAG_TRANSIENT_1X | L.FLAG_TRANSIENT_2X | L.FLAG_RIPPLE
-    if case == "overflow":
-        caps = dict(caps, maxGeneratedVertices=300000)
+    if case == "vertices":
+        caps = dict(caps, maxGeneratedVertices=700000)
+    if case == "visible":
+        caps = dict(caps, maxVisibleClusters=10000)
     fc = _ripple(S.camera_orbit(5))
     ref_state, _ = oracle.frame(sc, fc, caps, flags)
     want = ref_state.outputs(oracle.entries)
-    if case == "overflow":
-        assert int(want["readback"]["numGenVertices"]) > 300000
+    if case == "vertices":
+        assert int(want["readback"]["numGenVertices"]) > 700000
     pipe = TessellationPipeline(sc, caps, flags)
     pipe.set_cameras(fc)
-    for mode in ("graph", "graph", "plain"):
+    first = None
+    for mode in ("graph", "graph", "batched", "plain"):
         pipe.state.gen_vertices.handle.zero_()
         pipe.build(mode)
-        assert_same(pipe.outputs(), want, f"{case} {mode}", vertex_tol=vertex_tolerance(sc))
+        got = pipe.outputs()
+        assert_same(got, want, f"{case} {mode}", vertex_tol=vertex_tolerance(sc))
+        first = first or got
+        assert got["genVertices"].tobytes() == first["genVertices"].tobytes()
     assert pipe.device_errors() == 0
     pipe.close()

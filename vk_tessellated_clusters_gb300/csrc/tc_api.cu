@@ -52,6 +52,8 @@ struct Plan
   size_t clsCountsOffset, clsTriWordsOffset, clsBlockSumsOffset, clsFullRecsOffset, clsTransRecsOffset;
   u32    groupCap;  // instances the group tables hold
   size_t groupOffset;
+  u32    boundsCap;  // clusters with bounds
+  size_t boundsOffset;
   size_t rasterOffset;
   size_t partVertexOffset;  // u32 per part triangle
   size_t chunkSumsOffset;   // u64 per 32 part triangles
@@ -115,7 +117,6 @@ struct tc_context
   // overlaps the split passes (fork / join through the two events)
   cudaStream_t side    = nullptr;  // the first part run's instantiation
   cudaStream_t side2   = nullptr;  // the full clusters' vertices
-  cudaStream_t side3   = nullptr;  // the instance groups they use
   cudaEvent_t  evFork  = nullptr;
   cudaEvent_t  evJoin  = nullptr;  // first part run allocated
   cudaEvent_t  evJoin2 = nullptr;  // full clusters' vertices written
@@ -124,7 +125,6 @@ struct tc_context
   cudaEvent_t  evInst  = nullptr;  // instances classified
   cudaEvent_t  evScan0 = nullptr;  // first part run's offsets (and the counters after it)
   cudaEvent_t  evCull  = nullptr;  // clusters_cull done (on the second side stream)
-  cudaEvent_t  evGroup = nullptr;  // instance groups done
 
   // graph cache
   cudaGraphExec_t graphExec = nullptr;
@@ -214,8 +214,11 @@ Plan make_plan(const tc_context_desc& d)
   p.clsTransRecsOffset = off;
   off = align_up(off + (size_t)p.classifyCap * 48, 256);
   p.groupCap    = std::min(kGroupInstances, std::max(1u, d.maxInstances));
-  p.groupOffset = off;  // head, subgroups, members
-  off           = align_up(off + 16 + (size_t)p.groupCap * 24, 256);
+  p.groupOffset = off;  // head, then per instance: subgroup, representative, members and scratch, first bound
+  off           = align_up(off + 32 + (size_t)p.groupCap * (16 + 8 + 8 + 4), 256);
+  p.boundsCap    = std::max(1u, p.classifyCap / 4);  // more are not used (find_groups)
+  p.boundsOffset = off;
+  off            = align_up(off + (size_t)p.boundsCap * 32, 256);
   p.partVertexOffset  = off;
   off                 = align_up(off + (size_t)std::max(1u, k.maxPartTriangles) * 4, 256);
   p.chunkSumsOffset   = off;
@@ -309,10 +312,38 @@ ClassifyBuffers classify_buffers(tc_context* ctx)
           reinterpret_cast<uint2*>(ctx->dScratch + p.clsFullRecsOffset),
           reinterpret_cast<u32*>(ctx->dScratch + p.clsFullRecsOffset + (size_t)p.classifyCap * 8),
           reinterpret_cast<uint4*>(ctx->dScratch + p.clsTransRecsOffset),
-          nullptr,
-          reinterpret_cast<u32*>(ctx->dScratch + p.groupOffset + 16 + (size_t)p.groupCap * 16),
+          {}};
+}
+
+// From this many clusters on a frame finds its instance groups and bounds their
+// clusters (a longer first kernel and two more launches, one of which takes
+// clusters_cull's place): 48 instances of the batched scene (9,720 clusters)
+// 62.8 us a frame without and 66.8 with, 96 instances 75.2 and 71.8, 1,024
+// instances from host buffers 298 and 162.
+constexpr u32 kGroupMinClusters = 16384;
+
+// whether a batched frame groups its instances (RT semantics only: the visible
+// list is every cluster in instance order)
+bool groups_instances(const tc_frame_args* a)
+{
+  return (a->flags & TC_FLAG_RASTER_CULL) == 0 && a->numInstances >= 2 && a->numInstances <= kGroupInstances
+         && a->totalClusters >= kGroupMinClusters;
+}
+
+// the instance groups' tables
+GroupTables group_tables(tc_context* ctx)
+{
+  const Plan& p    = ctx->plan;
+  char*       base = reinterpret_cast<char*>(ctx->dScratch) + p.groupOffset;
+  const size_t n   = p.groupCap;
+  return {reinterpret_cast<uint4*>(base + 32),
+          reinterpret_cast<u32*>(base + 32 + n * 24),
+          reinterpret_cast<u32*>(base),
+          reinterpret_cast<uint2*>(base + 32 + n * 16),
+          reinterpret_cast<u32*>(base + 32 + n * 32),
+          reinterpret_cast<float4*>(ctx->dScratch + p.boundsOffset),
           p.groupCap,
-          reinterpret_cast<u32*>(ctx->dScratch + p.groupOffset)};
+          p.boundsCap};
 }
 
 InstantiateBuffers instantiate_buffers(tc_context* ctx)
@@ -341,13 +372,6 @@ bool emits_clusters(const tc_context* ctx, const tc_frame_args* a)
                                     ctx->schedule.classifyBlocksPerSM);
 }
 
-// whether a batched frame writes its full clusters' vertices once per group of
-// instances (RT semantics only: the visible list is every cluster in instance order)
-bool groups_instances(const tc_frame_args* a)
-{
-  return (a->flags & TC_FLAG_RASTER_CULL) == 0 && a->numInstances >= 2 && a->numInstances <= kGroupInstances;
-}
-
 // kernels one batched frame launches (the BLAS set-up is fused for up to
 // kBlasSetupFusedMax instances)
 uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
@@ -356,7 +380,7 @@ uint64_t frame_launches(const tc_context* ctx, const tc_frame_args* a)
          - (a->numInstances <= kBlasSetupFusedMax ? 1 : 0)
          - (ctx->schedule.frameShape == 1 ? 4 : 0)  // one allocation + vertex launch instead of two
          + (emits_clusters(ctx, a) ? 1 : 0)              // the clusters with part or split triangles
-         + (groups_instances(a) ? 1 : 0)
+         + (groups_instances(a) ? 1 : 0)                 // two kernels for the groups' bounds, without clusters_cull
          + ((a->flags & TC_FLAG_TRANSIENT_2X) ? 1 : 0);                           // the 2X batches' vertices
 }
 
@@ -407,6 +431,9 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   c.zeroBase           = reinterpret_cast<uint4*>(ctx->dScratch + zeroOff);
   c.zeroN16            = (p.frameBytes - zeroOff) / 16;
   const u32 beginGrid = std::max(frame_begin_grid(ctx, a), ceil_div(a->numInstances, kInstanceTile));
+  ClassifyBuffers cb = classify_buffers(ctx);
+  if(groups_instances(a))
+    cb.groups = group_tables(ctx);
   if(io.bytes)
   {
     const HostUpload up = {io.hostIn, io.devIn, io.bytes};
@@ -419,16 +446,16 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
       ch.view        = reinterpret_cast<const tc_FrameConstants*>(host(a->view));
       ch.viewLast    = reinterpret_cast<const tc_FrameConstants*>(host(a->viewLast));
       ch.instances   = reinterpret_cast<const tc_RenderInstance*>(host(a->instances));
-      TC_CHECK_CUDA(launch_frame_begin_instances_upload(ch, up, beginGrid, s));
+      TC_CHECK_CUDA(launch_frame_begin_instances_upload(ch, cb.groups, up, beginGrid, s));
     }
     else
     {
       TC_CHECK_CUDA(launch_host_upload(up, ctx->numSMs, s));
-      TC_CHECK_CUDA(launch_frame_begin_instances(c, beginGrid, s));
+      TC_CHECK_CUDA(launch_frame_begin_instances(c, cb.groups, beginGrid, s));
     }
   }
   else
-    TC_CHECK_CUDA(launch_frame_begin_instances(c, beginGrid, s));
+    TC_CHECK_CUDA(launch_frame_begin_instances(c, cb.groups, beginGrid, s));
   c.zeroBase = nullptr;
   c.zeroN16  = 0;
 
@@ -437,9 +464,13 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   // clusters_cull (which writes it out, with its counter and set-up) runs on
   // the second side stream, joined at the frame's end.
   const bool flat = (a->flags & TC_FLAG_RASTER_CULL) == 0;
-  ClassifyBuffers cb = classify_buffers(ctx);
-  if(groups_instances(a))
-    cb.groups = reinterpret_cast<uint4*>(ctx->dScratch + p.groupOffset + 16);
+  c.flatVisible = flat ? 1u : 0u;
+  if(cb.groups.groups)
+  {
+    // k_classify_whole, the first of launch_cluster_classify's kernels, writes the list
+    TC_CHECK_CUDA(launch_cluster_bounds(c, cb.groups, ctx->numSMs, s));
+  }
+  else
   {
     StageCtx cc = c;
     bind_slot(ctx, cc, p.slotCull, false);
@@ -450,19 +481,12 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
       TC_CHECK_CUDA(cudaEventRecord(ctx->evInst, s));
       TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evInst, 0));
       cs = ctx->side2;
-      if(cb.groups)  // beside the cull, for the full clusters' vertices
-      {
-        TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side3, ctx->evInst, 0));
-        TC_CHECK_CUDA(launch_instance_groups(c, cb, ctx->side3));
-        TC_CHECK_CUDA(cudaEventRecord(ctx->evGroup, ctx->side3));
-      }
     }
     TC_CHECK_CUDA(
         launch_clusters_cull(cc, persistent_grid(ctx, ceil_div(a->totalClusters, kCullTile), 4), kCullTile, cs, flat));
     if(flat && io.hostRb)
       TC_CHECK_CUDA(cudaEventRecord(ctx->evCull, cs));
   }
-  c.flatVisible = flat ? 1u : 0u;
 
   bind_slot(ctx, c, p.slotClassify, false);
   c.fuseSetup = TC_BUILD_SETUP_SPLIT;
@@ -480,8 +504,6 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   // The full clusters' vertices depend on classify alone and nothing later in
   // the frame reads them: they run on a second side stream, joined at the end.
   TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evFork, 0));
-  if(cb.groups)
-    TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->evGroup, 0));
   TC_CHECK_CUDA(launch_classify_full_vertices(c, cb,
                                               std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
                                               sched.fullVertexBlocksPerSM, ctx->side2));
@@ -565,7 +587,7 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
     // second side stream, whose fused set-up writes numVisibleClusters; the
     // vertex kernels still running beside write none. So the copy to the host
     // waits for the cull alone and overlaps the vertex kernels' tails.
-    if(flat)
+    if(flat && !cb.groups.groups)
       TC_CHECK_CUDA(cudaStreamWaitEvent(s, ctx->evCull, 0));
     TC_CHECK_CUDA(launch_host_readback(c.readback, io.hostRb, s));
   }
@@ -702,10 +724,10 @@ namespace {
 void destroy_streams(tc_context* ctx)
 {
   for(cudaEvent_t* e : {&ctx->evFork, &ctx->evJoin, &ctx->evJoin2, &ctx->evArgs1, &ctx->evVerts, &ctx->evInst,
-                        &ctx->evScan0, &ctx->evCull, &ctx->evGroup})
+                        &ctx->evScan0, &ctx->evCull})
     if(*e)
       cudaEventDestroy(*e), *e = nullptr;
-  for(cudaStream_t* st : {&ctx->side, &ctx->side2, &ctx->side3})
+  for(cudaStream_t* st : {&ctx->side, &ctx->side2})
     if(*st)
       cudaStreamDestroy(*st), *st = nullptr;
 }
@@ -734,7 +756,6 @@ tc_status tc_context_create(const tc_context_desc* desc, tc_context** outCtx)
   ctx->numSMs   = (u32)std::max(1, sms);
   if(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess
      || cudaStreamCreateWithFlags(&ctx->side2, cudaStreamNonBlocking) != cudaSuccess
-     || cudaStreamCreateWithFlags(&ctx->side3, cudaStreamNonBlocking) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evFork, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evJoin, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evJoin2, cudaEventDisableTiming) != cudaSuccess
@@ -742,8 +763,7 @@ tc_status tc_context_create(const tc_context_desc* desc, tc_context** outCtx)
      || cudaEventCreateWithFlags(&ctx->evVerts, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evInst, cudaEventDisableTiming) != cudaSuccess
      || cudaEventCreateWithFlags(&ctx->evScan0, cudaEventDisableTiming) != cudaSuccess
-     || cudaEventCreateWithFlags(&ctx->evCull, cudaEventDisableTiming) != cudaSuccess
-     || cudaEventCreateWithFlags(&ctx->evGroup, cudaEventDisableTiming) != cudaSuccess)
+     || cudaEventCreateWithFlags(&ctx->evCull, cudaEventDisableTiming) != cudaSuccess)
   {
     destroy_streams(ctx);
     delete ctx;

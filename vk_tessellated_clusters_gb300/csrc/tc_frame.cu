@@ -2,6 +2,7 @@
 // the standalone build_setup kernel.
 #include <algorithm>
 
+#include "tc_groups.cuh"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 
@@ -222,9 +223,12 @@ __global__ void k_instances_classify(StageCtx c)
 // Both in one launch (the batched frame): instances_classify reads nothing the
 // per-frame reset writes, so every block does its share of the reset and then
 // takes instance tiles.
-__global__ void k_frame_begin_instances(StageCtx c)
+// The last block first finds the instance groups (tc_groups.cuh), if any.
+__global__ void k_frame_begin_instances(StageCtx c, GroupTables g)
 {
   stage_prologue();
+  if(g.groups && blockIdx.x == gridDim.x - 1)
+    find_groups(c, g);
   frame_begin_body(c);
   instances_classify_body(c);
 }
@@ -391,9 +395,11 @@ __global__ void k_host_upload(HostUpload u)
 // its share of the input block, and the frame's own reads of the frame
 // constants and instance records (c points them into the host block) go to
 // the host memory directly. Kernels after it read the device copy.
-__global__ void k_frame_begin_instances_upload(StageCtx c, HostUpload u)
+__global__ void k_frame_begin_instances_upload(StageCtx c, GroupTables g, HostUpload u)
 {
   stage_prologue();
+  if(g.groups && blockIdx.x == gridDim.x - 1)
+    find_groups(c, g);
   host_upload_body(u);
   frame_begin_body(c);
   instances_classify_body(c);
@@ -417,9 +423,10 @@ cudaError_t launch_host_upload(const HostUpload& u, u32 maxGrid, cudaStream_t s)
   return launch_side(k_host_upload, grid, 256, s, u);
 }
 
-cudaError_t launch_frame_begin_instances_upload(const StageCtx& c, const HostUpload& u, u32 grid, cudaStream_t s)
+cudaError_t launch_frame_begin_instances_upload(const StageCtx& c, const GroupTables& g, const HostUpload& u, u32 grid,
+                                                cudaStream_t s)
 {
-  return launch_pdl(k_frame_begin_instances_upload, grid, kInstanceTile, s, c, u);
+  return launch_pdl(k_frame_begin_instances_upload, grid + (g.groups ? 1 : 0), kInstanceTile, s, c, g, u);
 }
 
 cudaError_t launch_host_readback(const tc_Readback* src, void* dst, cudaStream_t s)
@@ -449,9 +456,9 @@ cudaError_t launch_instances_classify(const StageCtx& c, u32 grid, u32 block, cu
   return launch_pdl(k_instances_classify, grid, block, s, c);
 }
 
-cudaError_t launch_frame_begin_instances(const StageCtx& c, u32 grid, cudaStream_t s)
+cudaError_t launch_frame_begin_instances(const StageCtx& c, const GroupTables& g, u32 grid, cudaStream_t s)
 {
-  return launch_pdl(k_frame_begin_instances, grid, kInstanceTile, s, c);
+  return launch_pdl(k_frame_begin_instances, grid + (g.groups ? 1 : 0), kInstanceTile, s, c, g);
 }
 
 cudaError_t launch_clusters_cull(const StageCtx& c, u32 grid, u32 block, cudaStream_t s, bool side)

@@ -36,6 +36,33 @@ struct RangeSums
   unsigned long long partsSplits, fullVerts, data, backTrans;
 };
 
+// Instances that share their mesh, displacement map, scale and offset, and so
+// the vertices of their full clusters: found by the batched frame's first
+// kernel (tc_groups.cuh) for up to kGroupInstances instances, in subgroups of
+// at most kGroupMembers, with object-space bounds of their clusters when many
+// instances share them.
+constexpr u32 kGroupInstances = 4096;
+constexpr u32 kGroupMembers   = 8;
+enum : int
+{
+  kHeadSubgroups = 0,
+  kHeadTasks,
+  kHeadGrouped,  // whether the full clusters' vertices are written by groups
+  kHeadBounds,   // clusters with bounds; 0: none are used
+  kHeadReps,     // groups
+  kHeadList,     // visible clusters left to k_classify_count (bounds in use)
+};
+struct GroupTables
+{
+  uint4*  groups;      // per subgroup: first task, first member, members, representative instance; null: no groups
+  u32*    members;     // [2 * cap]: the groups' instances, and scratch
+  u32*    head;        // kHead* words
+  uint2*  reps;        // per group: its first entry of bounds, representative
+  u32*    instBounds;  // per instance: its first entry of bounds
+  float4* bounds;      // [2] per cluster of a group
+  u32     cap, boundsCap;
+};
+
 // cluster_classify scratch: per visible cluster of a launch's window, and per
 // block of the classify grid (each write block owns a contiguous range of clusters)
 struct ClassifyBuffers
@@ -47,24 +74,17 @@ struct ClassifyBuffers
   uint2*          fullRecs;   // per full cluster of the window: visible index, first generated vertex
   u32*            fullRange;  // [2]: the window's generated-cluster slots; [2]: transRecs' count
   uint4*          transRecs;  // 48 bytes per cluster that is not a full one
-  uint4*          groups;     // instance groups (launch_instance_groups), or null: none this frame
-  u32*            members;    // [2 * groupCap]: their instances, and scratch
-  u32             groupCap;
-  u32*            groupHead;  // [4]: subgroups, tasks, whether grouping pays
+  GroupTables     groups;     // instance groups, or all null: none this frame
 };
-
-// Instances that share their mesh, displacement map, scale and offset, and so
-// the vertices of their full clusters: found for frames of 2 to
-// kGroupInstances instances, in subgroups of at most kGroupMembers.
-constexpr u32 kGroupInstances = 4096;
-constexpr u32 kGroupMembers   = 8;
-cudaError_t launch_instance_groups(const StageCtx& c, const ClassifyBuffers& buf, cudaStream_t s);
 
 cudaError_t launch_frame_begin(const StageCtx& c, u32 grid, cudaStream_t s);
 cudaError_t launch_decode_hits(const StageCtx& c, const tc_hit* hits, u32 count, tc_base_hit* out, cudaStream_t s);
 cudaError_t launch_instances_classify(const StageCtx& c, u32 grid, u32 block, cudaStream_t s);
 // frame_begin and instances_classify in one launch (block = kInstanceTile)
-cudaError_t launch_frame_begin_instances(const StageCtx& c, u32 grid, cudaStream_t s);
+// (with groups: one more block, which finds the instance groups)
+cudaError_t launch_frame_begin_instances(const StageCtx& c, const GroupTables& g, u32 grid, cudaStream_t s);
+// the bounds of the groups' clusters, before launch_cluster_classify
+cudaError_t launch_cluster_bounds(const StageCtx& c, const GroupTables& g, u32 numSMs, cudaStream_t s);
 // side: launched on a side stream beside classify (an ordinary launch, see
 // launch_side); otherwise programmatically after the kernel before it
 cudaError_t launch_clusters_cull(const StageCtx& c, u32 grid, u32 block, cudaStream_t s, bool side = false);
@@ -82,7 +102,8 @@ struct HostUpload
 // kernel (launch_frame_begin_instances with the upload; c's frame constants
 // and instance records point into the host block)
 cudaError_t launch_host_upload(const HostUpload& u, u32 maxGrid, cudaStream_t s);
-cudaError_t launch_frame_begin_instances_upload(const StageCtx& c, const HostUpload& u, u32 grid, cudaStream_t s);
+cudaError_t launch_frame_begin_instances_upload(const StageCtx& c, const GroupTables& g, const HostUpload& u, u32 grid,
+                                                cudaStream_t s);
 cudaError_t launch_host_readback(const tc_Readback* src, void* dst, cudaStream_t s);
 // the bounded look-back wait on its own (state: 3 words, zeroed here)
 cudaError_t launch_lookback_probe(unsigned long long* state, u32 published, u32* errorWord, u32 spinLimit,
