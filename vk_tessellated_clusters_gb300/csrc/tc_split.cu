@@ -27,13 +27,14 @@
 //   k_triangle_split_levels every pass in one launch (the batched frame and
 //                           its graph): the persistent blocks take tiles of
 //                           all levels from one ticket, level by level; the
-//                           block that completes a level's last tile applies
-//                           that pass's build_setup (what the multipass
-//                           kernel's last block does) and publishes the next
-//                           level's item range, for which the blocks holding
-//                           later tickets wait (bounded). An empty first
-//                           level leaves every level empty: one block then
-//                           runs the passes' set-ups and the others return.
+//                           block that completes a level's last tile publishes
+//                           the next level's item range, for which the blocks
+//                           holding later tickets wait (bounded); the one that
+//                           completes the last level applies every pass's
+//                           build_setup (what the multipass kernel's last
+//                           block does). An empty first level leaves every
+//                           level empty: one block then runs the passes'
+//                           set-ups and the others return.
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 
@@ -148,11 +149,12 @@ struct SplitShared
 
 // One tile: T items of the level [begin, end) starting at begin + tile * T,
 // their children classified, ordered after every earlier tile of the level
-// (look-back on `lbState` rows of `lbStride`, tile 0 from the counters'
-// current values) and written. The last tile publishes the level's totals.
+// (look-back on `lbState` rows of `lbStride`, tile 0 from the counters' values
+// before the pass: `bases`) and written. The last tile publishes the level's totals.
 template <int T, int B>
 __device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u32 begin, u32 end, u32 numTiles,
-                           u64* lbState, u32 lbStride, u64* totals, const FactorParams& fp, u32 sf, u32 partCap)
+                           u64* lbState, u32 lbStride, u64* totals, const u32* bases, const FactorParams& fp, u32 sf,
+                           u32 partCap)
 {
   using S                  = SplitShared<T, B>;
   constexpr u32 kW         = S::kW;
@@ -300,7 +302,7 @@ __device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u
     const u32 agg  = __shfl_sync(0xFFFFFFFFu, incl, 31);
     u64       base = 0;
     if(tile == 0)  // the counters as the previous pass left them (through L2: see above)
-      base = q == kCntSplit ? __ldcg(&b->splitWriteCounter) : part_base(c);
+      base = bases ? __ldcg(bases + q) : (q == kCntSplit ? __ldcg(&b->splitWriteCounter) : part_base(c));
     const u64 ex = warp_lookback_exclusive(lbState + (u64)q * lbStride, tile, agg, base, c.errorWord, c.spinLimit);
     if(lane == 0)
     {
@@ -436,8 +438,8 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
     const u32 tile = next_tile(c, &sm.tile);
     if(tile >= numTiles)
       break;
-    split_tile<T, B>(c, sm, tile, begin, end, numTiles, c.scratch.lbState, c.scratch.lbStride, c.scratch.totals, fp,
-                     sf, partCap);
+    split_tile<T, B>(c, sm, tile, begin, end, numTiles, c.scratch.lbState, c.scratch.lbStride, c.scratch.totals,
+                     nullptr, fp, sf, partCap);
   }
 
   if(last_block_done(c, &sm.flag))
@@ -457,11 +459,13 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
 // ---------------------------------------------------------------------------
 
 // Per-level control words, in the level's scratch slot (zeroed with the
-// frame): [1] tiles done, [2..] u64 totals (split, part), [12] next level's
-// range published, [13] finalised, [14] start, [15] end. Level 0's [0] is
-// the ticket all levels share; the last level's [12] marks the end.
+// frame): [1] tiles done, [2..] u64 totals (split, part), [6] / [7] the split
+// and part counters before the level, [12] next level's range published,
+// [13] finalised, [14] start, [15] end. Level 0's [0] is the ticket all levels
+// share.
 __device__ __forceinline__ u32* lv_done(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 1; }
 __device__ __forceinline__ u64* lv_totals(const SplitLevels& lv, u32 L) { return reinterpret_cast<u64*>(lv.ctrl[L] + 2); }
+__device__ __forceinline__ u32* lv_bases(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 6; }
 __device__ __forceinline__ u32* lv_ready(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 12; }
 __device__ __forceinline__ u32* lv_final(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 13; }
 
@@ -470,22 +474,81 @@ __device__ __forceinline__ void st_release_u32(u32* p, u32 v)
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Level L is complete (every tile done, or none): the pass's counters and
-// set-up, then the next level's item range, published with release
-// semantics. Run by one thread.
-__device__ void finalize_level(const StageCtx& c, const SplitLevels& lv, u32 L, u32 numTiles, u32 partCap)
+// Every level is complete: the counters and set-ups of all passes
+// (split_pass_counters and TC_BUILD_SETUP_SPLIT_PASS for each, then the fused
+// set-up), from the levels' totals, by one thread. Done here once, in
+// registers: at each level's end it kept the next level's tiles waiting for
+// five dependent accesses. `tilesOf(L, begin, end)`: the level's tiles; with
+// no split item at all (levels empty) nothing but the set-ups is left, 7 us of
+// every frame without splits, now 3.
+template <class TilesOf>
+__device__ void finalize_levels(const StageCtx& c, const SplitLevels& lv, u32 partCap, TilesOf&& tilesOf)
 {
-  tc_SceneBuilding* b = c.build;
-  split_pass_counters(c, numTiles, lv_totals(lv, L), partCap);
-  const bool last = L + 1 >= lv.levels;
-  const u32  mode = last ? c.fuseSetup : (u32)TC_BUILD_SETUP_SPLIT_PASS;
-  if(mode != kNoSetup)
-    build_setup_apply(c, mode);
-  if(!last)
+  tc_SceneBuilding* b     = c.build;
+  const u32         most  = c.caps.maxSplitTriangles;
+  const bool        trans = (c.flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)) != 0;
+  u32 write = b->splitWriteCounter, start = b->splitPassStart, end = b->splitPassEnd, pass = b->splitPass;
+  u32 part  = b->partTriangleCounter;
+  u64 dual  = b->dualPartTriangleCounter;
+  for(u32 L = 0; L < lv.levels; L++)
   {
-    lv.ctrl[L + 1][14] = min(b->splitPassStart, c.caps.maxSplitTriangles);
-    lv.ctrl[L + 1][15] = min(b->splitPassEnd, c.caps.maxSplitTriangles);
+    const u32 last = min(end, most), first = min(start, last);
+    if(tilesOf(first, last))
+    {
+      // split_pass_counters
+      write           = (u32)__ldcg(lv_totals(lv, L) + kCntSplit);
+      const u32 total = (u32)__ldcg(lv_totals(lv, L) + kCntPart);
+      if(trans)
+      {
+        const u32 from = (u32)dual, written = min(total, partCap);
+        dual           = (dual & 0xFFFFFFFF00000000ull) | total;
+        if(written > from)
+          part = max(part, written);
+      }
+      else
+        part = total;
+    }
+    if(L + 1 == lv.levels)
+      break;
+    // TC_BUILD_SETUP_SPLIT_PASS (build_setup_apply)
+    pass++;
+    start = min(end, most);
+    end   = min(write, most);
+    if(pass + 1 <= kMaxRuns)
+      c.runStarts[pass + 1] = part;
   }
+  b->splitWriteCounter   = write;
+  b->partTriangleCounter = part;
+  if(trans)
+    b->dualPartTriangleCounter = dual;
+  if(lv.levels > 1)
+  {
+    b->splitPass             = pass;
+    b->splitPassStart        = start;
+    b->splitPassEnd          = end;
+    b->dispatchTriangleSplit = {(end - start + 63) / 64, 1, 1};
+  }
+  if(c.fuseSetup != kNoSetup)
+    build_setup_apply(c, c.fuseSetup);
+}
+
+// Level L, of items up to `end`, is complete (every tile done, or none): the
+// next level's item range and counters, published with release semantics.
+// Run by one thread.
+__device__ void publish_level(const StageCtx& c, const SplitLevels& lv, u32 L, u32 end, u32 numTiles)
+{
+  if(L + 1 >= lv.levels)
+    return;
+  const u32 most = c.caps.maxSplitTriangles;
+  // another block's last tile wrote the totals: read them through L2
+  u32 write, part;
+  if(numTiles)
+    write = (u32)__ldcg(lv_totals(lv, L) + kCntSplit), part = (u32)__ldcg(lv_totals(lv, L) + kCntPart);
+  else  // (not level 0: without split items no level is published)
+    write = __ldcg(lv_bases(lv, L) + kCntSplit), part = __ldcg(lv_bases(lv, L) + kCntPart);
+  u32* next = lv.ctrl[L + 1];
+  next[6 + kCntSplit] = write, next[6 + kCntPart] = part;
+  next[14] = min(end, most), next[15] = min(write, most);
   __threadfence();
   st_release_u32(lv_ready(lv, L), 1u);
 }
@@ -511,8 +574,7 @@ __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLe
   {
     // no split item: every level is empty; one block runs the passes' set-ups
     if(blockIdx.x == 0 && threadIdx.x == 0)
-      for(u32 L = 0; L < levels; L++)
-        finalize_level(c, lv, L, 0, partCap);
+      finalize_levels(c, lv, partCap, tiles_of);
     return;
   }
   if(threadIdx.x == 0 && (end - begin + T - 1) / T > lv.stride)
@@ -531,7 +593,9 @@ __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLe
         if(numTiles == 0 && atomicCAS(lv_final(lv, level), 0u, 1u) == 0u)
         {
           __threadfence();
-          finalize_level(c, lv, level, 0, partCap);
+          publish_level(c, lv, level, end, 0);
+          if(level + 1 == levels)
+            finalize_levels(c, lv, partCap, tiles_of);
         }
         first += numTiles;
         if(++level >= levels)
@@ -570,16 +634,18 @@ __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLe
     begin    = sm.range[0];
     end      = sm.range[1];
     const u32 tile = g - first;
-    split_tile<T, B>(c, sm, tile, begin, end, numTiles, lv.lbState[level], lv.stride, lv_totals(lv, level), fp, sf,
-                     partCap);
-    // the block completing the level's last tile finalises it
+    split_tile<T, B>(c, sm, tile, begin, end, numTiles, lv.lbState[level], lv.stride, lv_totals(lv, level),
+                     level ? lv_bases(lv, level) : nullptr, fp, sf, partCap);
+    // the block completing the level's last tile publishes the next level
     if(threadIdx.x == 0)
     {
       __threadfence();
       if(atomicAdd(lv_done(lv, level), 1u) == numTiles - 1)
       {
         __threadfence();
-        finalize_level(c, lv, level, numTiles, partCap);
+        publish_level(c, lv, level, end, numTiles);
+        if(level + 1 == levels)
+          finalize_levels(c, lv, partCap, tiles_of);
       }
     }
     __syncthreads();
