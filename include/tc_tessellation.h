@@ -467,7 +467,8 @@ typedef struct tc_schedule {
                                    * it runs beside the rest of the frame (fewer blocks leave room for it);
                                    * 0: the default (4) */
   uint32_t vertexGridPerSM;     /* grid of the part vertex kernel = SMs x this (grid-stride over 32-part chunks);
-                                 * 0: one resident wave (the blocks vertexBlocksPerSM allows) */
+                                 * 0: one resident wave (the blocks vertexBlocksPerSM allows), and one block per SM
+                                 * less for the first part run of a frame that allocates two */
   uint32_t lookbackSpinLimit;   /* polls a bounded look-back wait makes before it gives up, sets
                                  * TC_DEVERR_LOOKBACK_TIMEOUT and goes on with what it has (the frame's offsets are
                                  * then unreliable); 0: the default, 2^22 polls (seconds, with back-off) */

@@ -522,7 +522,7 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
                                           sched.scanBlocksPerSM, ctx->side));
     TC_CHECK_CUDA(cudaEventRecord(ctx->evJoin, ctx->side));
     TC_CHECK_CUDA(launch_instantiate_vertices(c0, instantiate_buffers(ctx), a->caps.maxPartTriangles, ctx->numSMs,
-                                              sched.vertexBlocksPerSM, sched.vertexGridPerSM, ctx->side));
+                                              sched.vertexBlocksPerSM, sched.vertexGridPerSM, true, ctx->side));
   }
 
   const u32 sb     = split_block(sched);
@@ -568,7 +568,7 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
   TC_CHECK_CUDA(cudaEventRecord(ctx->evArgs1, s));
   TC_CHECK_CUDA(cudaStreamWaitEvent(ctx->side, ctx->evArgs1, 0));
   TC_CHECK_CUDA(launch_instantiate_vertices(c, instantiate_buffers(ctx), a->caps.maxPartTriangles, ctx->numSMs,
-                                            sched.vertexBlocksPerSM, sched.vertexGridPerSM, ctx->side));
+                                            sched.vertexBlocksPerSM, sched.vertexGridPerSM, false, ctx->side));
   TC_CHECK_CUDA(cudaEventRecord(ctx->evVerts, ctx->side));
 
   bind_slot(ctx, c, p.slotBlas, false);

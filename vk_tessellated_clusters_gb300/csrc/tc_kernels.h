@@ -155,7 +155,7 @@ cudaError_t launch_instantiate_prefix(const StageCtx& c, const InstantiateBuffer
 cudaError_t launch_instantiate_args(const StageCtx& c, const InstantiateBuffers& buf, u32 maxParts, u32 numSMs,
                                     u32 scanBlocksPerSM, cudaStream_t s);
 cudaError_t launch_instantiate_vertices(const StageCtx& c, const InstantiateBuffers& buf, u32 maxParts, u32 numSMs,
-                                        u32 vertexBlocksPerSM, u32 vertexGridPerSM, cudaStream_t s);
+                                        u32 vertexBlocksPerSM, u32 vertexGridPerSM, bool leaveRoom, cudaStream_t s);
 u32         instantiate_alloc_tiles(u32 maxParts);
 // the stage entry point's form: tile sums, tile scan, then arguments and
 // vertices in one kernel (PN / ripple: launch_triangle_instantiate)
