@@ -458,11 +458,12 @@ typedef enum tc_status {
 typedef struct tc_schedule {
   uint32_t classifyBlocksPerSM; /* grid of the per-cluster classify kernels = SMs x this (256 threads); 4 or less:
                                  * 64 registers per thread, 5-7: 40, 8 and more: 32 */
-  uint32_t splitBlockSize;      /* split tile: 128 (16 items), 256 or 512 (32 items) threads */
+  uint32_t splitBlockSize;      /* split tile: 128, 256 or 512 children, one per thread (default 512) */
   uint32_t vertexBlocksPerSM;   /* register budget of the vertex-generation kernel (one 32-part chunk per warp):
                                  * 4 or less: 64 registers per thread, 5: 48, 6 and more: 40 */
   uint32_t scanBlocksPerSM;     /* grid of the instantiate allocation kernels (tile sums, arguments) = SMs x this */
-  uint32_t blocksPerSM;         /* persistent grid of the split kernel = SMs x this x (512 / splitBlockSize) */
+  uint32_t blocksPerSM;         /* persistent grid of the split kernel = SMs x this x (512 / splitBlockSize), twice
+                                 * that for tc_triangle_split */
   uint32_t fullVertexBlocksPerSM; /* grid of the full-cluster vertex kernel = SMs x this (at most 4 resident);
                                    * it runs beside the rest of the frame (fewer blocks leave room for it);
                                    * 0: the default (4) */

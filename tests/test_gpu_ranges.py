@@ -123,6 +123,38 @@ def test_deform_chunk_widths(oracle, case):
     pipe.close()
 
 
+# split items of the first level, their children and the queue's capacity: indexed by every block for itself (320), by
+# all (1,280 with 128 and 256 threads, 5,120), one chunk of children to a tile or, where a small queue's rows hold fewer
+# tiles, up to 8 (320 and 512 places; what does not fit is dropped like the oracle's)
+@pytest.mark.parametrize("subdivisions,eye,pixels,capacity,several", [(2, 1.08, 2.0, 320, True), (2, 1.08, 2.0, 512, True),
+                                                                      (2, 1.08, 2.0, 17468, False),
+                                                                      (3, 1.08, 1.5, 66984, False),
+                                                                      (4, 1.3, 1.5, 32496, False)])
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_split_tiles(oracle, subdivisions, eye, pixels, capacity, several, block):
+    """All passes in one launch, one per launch, and one per launch and instance window, against the oracle."""
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_icosphere(subdivisions=subdivisions, map_size=64)
+    cam = S.Camera(eye=(0.0, 0.0, eye), center=(0.0, 0.0, 0.0), tess_rate_pixels=pixels, near=0.01, far=10.0)
+    caps = dict(L.default_caps(visible_bits=12, part_bits=18, vertex_bits=23, megs=256), maxSplitTriangles=capacity)
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    want = ref_state.outputs(oracle.entries)
+    items = want["splitTriangles"][:min(capacity, int(want["readback"]["numSplitTriangles"]))]
+    first = np.isin(items["vtxEncoded"], (0, 1 << 15, 1 << 31)).all(axis=1)  # whole base triangles
+    children = int(oracle.entries["numTriangles"][(items["triangleID_config"][first] >> 16) & 0x7FFF].sum())
+    chunks = -(-children // block)
+    assert (chunks > -(-capacity // 16)) == several
+    pipe = TessellationPipeline(sc, caps, FLAGS, schedule={"splitBlockSize": block})
+    pipe.set_cameras(cam)
+    for mode, per_pass in (("graph", 0), ("graph", 1), ("plain", 0)):
+        pipe.set_schedule({**pipe.schedule(), "splitPerPass": per_pass})
+        pipe.state.gen_vertices.handle.zero_()
+        pipe.build(mode)
+        assert_same(pipe.outputs(), want, f"{mode} {per_pass}", vertex_tol=vertex_tolerance(sc))
+    assert pipe.device_errors() == 0
+    pipe.close()
+
+
 @pytest.mark.parametrize("count", [1, 31, 256, 257, 1023])
 @pytest.mark.parametrize("offset", [0, 4, 8])
 def test_decode_counts_and_alignment(oracle, count, offset):

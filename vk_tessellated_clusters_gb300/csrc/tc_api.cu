@@ -58,6 +58,7 @@ struct Plan
   size_t partVertexOffset;  // u32 per part triangle
   size_t chunkSumsOffset;   // u64 per 32 part triangles
   size_t splitBaseOffset;   // 9 floats per split item: its base triangle's world positions
+  size_t splitEndsOffset, splitFirstOffset, splitFirstStride;  // StageCtx::splitEnds, splitFirst
   size_t instOffset;  // instance cluster prefix (u32 x maxInstances+1)
   size_t errOffset;   // device error word
   size_t totalBytes;
@@ -176,9 +177,9 @@ Plan make_plan(const tc_context_desc& d)
   p.slotCull        = add(ceil_div(d.maxTotalClusters, kCullTile), 1);
   p.classifyCap     = (u32)std::max<u64>(1, std::min<u64>(k.maxVisibleClusters, d.maxTotalClusters));
   p.slotClassify    = add(classify_max_blocks(p.classifyCap), 4);  // the range sums (zeroed with the frame)
-  p.slotSplit0      = add(ceil_div(k.maxSplitTriangles, kSplitMinItems), 2);
+  p.slotSplit0      = add(ceil_div(k.maxSplitTriangles, kSplitRowItems), 4);
   for(u32 i = 1; i < passes; i++)
-    add(ceil_div(k.maxSplitTriangles, kSplitMinItems), 2);
+    add(ceil_div(k.maxSplitTriangles, kSplitRowItems), 4);
   p.slotInstantiate = add(instantiate_alloc_tiles(k.maxPartTriangles), 3);
   p.slotInstantiate0 = add(instantiate_alloc_tiles(k.maxPartTriangles), 3);
   p.slotBlas        = add(ceil_div(d.maxInstances, kInstanceTile), 1);
@@ -225,6 +226,12 @@ Plan make_plan(const tc_context_desc& d)
   off                 = align_up(off + (size_t)ceil_div(std::max(1u, k.maxPartTriangles), 1024) * 32 * 8, 256);
   p.splitBaseOffset   = off;
   off                 = align_up(off + (size_t)std::max(1u, k.maxSplitTriangles) * 36, 256);
+  // the children of a split level's items (at most 121 each, tiles of 128 or more)
+  p.splitEndsOffset   = off;
+  off                 = align_up(off + (size_t)std::max(1u, k.maxSplitTriangles) * 4, 256);
+  p.splitFirstOffset  = off;
+  p.splitFirstStride  = (size_t)ceil_div((u64)k.maxSplitTriangles * TC_TESSTABLE_SIZE * TC_TESSTABLE_SIZE, 128) + 1;
+  off                 = align_up(off + p.splitFirstStride * 3 * 4, 256);
   p.rasterOffset      = off;  // raster batching: per group of 32 parts its counts, then offsets
   off                 = align_up(off + (size_t)ceil_div(std::max(1u, k.maxPartTriangles), 32) * 16, 256);
   p.totalBytes        = off;
@@ -282,6 +289,9 @@ StageCtx base_ctx(tc_context* ctx, const tc_frame_args* a)
   c.runStarts               = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.runOffset);
   c.instClusterStart        = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.instOffset);
   c.splitBase               = reinterpret_cast<float*>(ctx->dScratch + ctx->plan.splitBaseOffset);
+  c.splitEnds               = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.splitEndsOffset);
+  c.splitFirst              = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.splitFirstOffset);
+  c.splitFirstStride        = ctx->plan.splitFirstStride;
   c.instBegin               = 0;
   c.instEnd                 = a->numInstances;
   c.fuseSetup               = kNoSetup;
@@ -412,7 +422,6 @@ u32 split_block(const tc_schedule& s)
   u32 b = s.splitBlockSize;
   return (b == 128 || b == 256 || b == 512) ? b : 256;
 }
-u32 split_items_per_tile(u32 block) { return block == 128 ? 16 : 32; }
 
 // The batched frame: one persistent launch per stage, build_setup fused into the
 // producers' last block. Graph-capturable (no host synchronisation, no allocation).
@@ -527,7 +536,7 @@ tc_status record_batched_frame(tc_context* ctx, const tc_frame_args* a, cudaStre
 
   const u32 sb     = split_block(sched);
   const u32 passes = split_passes(a->caps.splitFactor);
-  const u32 sgrid  = persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, split_items_per_tile(sb)), bpsm * (512 / sb));
+  const u32 sgrid  = persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, kSplitRowItems), bpsm * (512 / sb));
   if(sched.splitPerPass)
   {
     // one launch per pass, the pass set-up fused into its last block
@@ -769,7 +778,7 @@ tc_status tc_context_create(const tc_context_desc* desc, tc_context** outCtx)
     delete ctx;
     return TC_ERR_CUDA;
   }
-  ctx->schedule = {4, 256, 4, 4, 1, kDefaultFullVertexBlocksPerSM, 0, 0, 0, 0};  // the batched scene's tuned shape
+  ctx->schedule = {4, 512, 4, 4, 1, kDefaultFullVertexBlocksPerSM, 0, 0, 0, 0};  // the batched scene's tuned shape
   ctx->plan     = make_plan(*desc);
   if(cudaMalloc(&ctx->dScratch, ctx->plan.totalBytes) != cudaSuccess
      || cudaMemset(ctx->dScratch, 0, ctx->plan.totalBytes) != cudaSuccess)
@@ -1095,9 +1104,12 @@ tc_status tc_triangle_split(tc_context* ctx, const tc_frame_args* a, uint32_t in
   c.instEnd   = instanceEnd;
   bind_slot(ctx, c, ctx->plan.slotSplit0, true);
   const u32 sb = split_block(ctx->schedule);
+  // twice the frame's grid: no other kernel beside it wants the registers
+  // (73,000 split items in four passes, the whole frame 322 -> 315 us; inside
+  // the batched frame it costs 337 -> 360)
   TC_CHECK_CUDA(launch_triangle_split(c, sb,
-                                      persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, split_items_per_tile(sb)),
-                                                      std::max(1u, ctx->schedule.blocksPerSM) * (512 / sb)),
+                                      persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, kSplitRowItems),
+                                                      std::max(1u, ctx->schedule.blocksPerSM) * 2 * (512 / sb)),
                                       reinterpret_cast<cudaStream_t>(stream)));
   ctx->launches += 1;
   return TC_OK;
@@ -1122,7 +1134,7 @@ tc_status tc_triangle_split_all(tc_context* ctx, const tc_frame_args* a, void* s
   const SplitLevels lv = split_levels(ctx, passes);
   TC_CHECK_CUDA(launch_triangle_split_levels(
       c, lv, sb,
-      persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, split_items_per_tile(sb)),
+      persistent_grid(ctx, ceil_div(a->caps.maxSplitTriangles, kSplitRowItems),
                       std::max(1u, ctx->schedule.blocksPerSM) * (512 / sb)),
       s));
   ctx->launches += 1;

@@ -124,7 +124,7 @@ cudaError_t launch_triangle_split(const StageCtx& c, u32 blockSize, u32 grid, cu
 constexpr u32 kMaxSplitLevels = 16;
 struct SplitLevels
 {
-  unsigned long long* lbState[kMaxSplitLevels];  // [2][stride] per level
+  unsigned long long* lbState[kMaxSplitLevels];  // [4][stride] per level (split, part, next level's children, index)
   u32*                ctrl[kMaxSplitLevels];     // 16 words per level (see tc_split.cu)
   u32                 stride;                    // tiles per level the rows hold
   u32                 levels;                    // split passes
@@ -174,7 +174,7 @@ cudaError_t launch_instantiate_backward(const StageCtx& c, const float* gradVert
 // tiles per launch for each stage (used to size the look-back scratch)
 constexpr u32 kInstanceTile     = 256;  // instances per tile (instances_classify, blas_setup)
 constexpr u32 kCullTile         = 256;  // clusters per tile
-constexpr u32 kSplitMinItems    = 16;   // smallest split items-per-tile variant
+constexpr u32 kSplitRowItems    = 16;   // split items of the capacity per look-back tile of a split level
 constexpr u32 kInstantiateTile  = 1024; // part triangles per instantiate tile
 
 }  // namespace tc

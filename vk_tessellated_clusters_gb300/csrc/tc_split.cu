@@ -7,15 +7,25 @@
 // on the interpolated world positions, and it is appended either to the split
 // queue (next level) or to the part triangles.
 //
-// GB300 mapping: a tile is T parent items; their children are laid out flat
-// across the block (block scan of child counts, binary search child -> parent,
-// the same packing the reference does per subgroup, triangle_split.comp.glsl:350-472).
-// Pass 1 classifies every child, keeps it in shared memory and counts per
-// (chunk, warp); one warp turns the counts into offsets and a decoupled
-// look-back orders the tile's appends after all earlier tiles; pass 2 writes
-// the children in (parent, child) order (recomputing them only when a tile
-// has more than 64 children per item, i.e. split factors above 8), with no
-// block barrier inside either pass. Split items carry their base
+// GB300 mapping: items have from 2 to 64 children and more (a terrain's: half
+// have 2, one in a hundred over 31, and those lie together), so the work is cut
+// by children: a tile is B consecutive children of the level, one per thread,
+// whatever items they belong to. A level's items carry their running child
+// count (StageCtx::splitEnds) and every B-th child its item (splitFirst): the
+// first level's from a scan of its items at the launch's start, a later level's
+// written with the items themselves (a third look-back counter). Tiles of 32
+// items (73 children in the median, 2,048 at most) left most threads of a block
+// idle and a few blocks with eight rounds. With 73,000 items in one launch
+// beside the first part run it took 146 us and takes 96 (the frame 360 -> 338
+// us); in four launches the frame went from 348 to 315 us; a PN close-up's, of
+// 13,000 items, from 143 to 132 us. What bounds a tile is its chain of loads
+// and the look-back, about 10 us, so tiles are large: 512 children rather than
+// 256 took the terrain's frame from 354 to 338 us. (The next ticket fetched
+// ahead costs 90 us: the blocks that start late hold up everyone's look-back.)
+// A thread classifies its child and keeps it in registers; each warp counts its
+// own; one warp per counter turns the counts into offsets and a decoupled
+// look-back orders the tile's appends after all earlier tiles; then the
+// children are written in (parent, child) order. Split items carry their base
 // triangle's world positions in a side array, so a tile's set-up is one load
 // level instead of the instance / cluster / index / vertex chain. Persistent
 // grid, tiles from a ticket.
@@ -46,7 +56,9 @@ enum : int
 {
   kCntSplit = 0,
   kCntPart,
-  kNumCounters
+  kNumCounters,
+  kCntKids = kNumCounters,  // children of the next level's items
+  kRowScan                  // the scan of the first level's items
 };
 
 constexpr u32 kMaxChildrenPerItem = TC_TESSTABLE_SIZE * TC_TESSTABLE_SIZE;  // 121
@@ -59,6 +71,7 @@ struct SplitItem
   f3             bp[3];  // world positions of the base triangle
   u32            firstTriangle;
   u32            firstVertex;
+  u32            count;  // children
 };
 
 struct Child
@@ -126,37 +139,211 @@ __device__ __forceinline__ u32 part_cap(const StageCtx& c)
   return (u64)y + 1 < m ? m - y - 1 : 0u;
 }
 
-// Shared memory of one split tile (kernel-scope; one per block).
-template <int T, int B>
-struct SplitShared
+// Children an item takes in its level's order. At least one: an item whose
+// config has no triangle takes a place without a child, so that B consecutive
+// children never touch more than B items.
+__device__ __forceinline__ u32 child_places(const StageCtx& c, u32 cfg)
 {
-  static constexpr u32 kMaxChildren   = T * kMaxChildrenPerItem;
-  static constexpr u32 kMaxChunks     = (kMaxChildren + B - 1) / B;
-  static constexpr u32 kW             = B / 32;
-  static constexpr u32 kSlots         = kMaxChunks * kW;  // (chunk, warp) count slots, in serial order
-  static constexpr u32 kCacheChildren = T * 64;  // pass 1 keeps its children for pass 2 when they fit
-  static_assert(T <= B && T <= 32, "tile items are set up by warp 0");
-  static_assert(kSlots <= 128, "one warp scans the count slots, four per lane");
+  return min(max((u32)table_entry(c.table, cfg).numTriangles, 1u), kMaxChildrenPerItem);
+}
 
-  uint4     child[kCacheChildren];      // vtx[3], tc
-  u32       splitMask[kSlots];          // per (chunk, warp): which lanes' children are split items
-  SplitItem item[T];
-  u32       pre[T + 1];
-  u32       cnt[kNumCounters][kSlots];  // per (chunk, warp): count, then exclusive offset within the tile
-  u64       excl[kNumCounters];
-  u32       tile, flag, range[2];
+// One level's items [begin, end) by their children.
+struct Level
+{
+  u32        begin, end;
+  u32        total;  // child places of all items
+  u32        tiles;  // of `chunks` x B child places each
+  u32        chunks;
+  const u32* first;  // per B child places: the item the first belongs to (null: level not known yet)
 };
 
-// One tile: T items of the level [begin, end) starting at begin + tile * T,
-// their children classified, ordered after every earlier tile of the level
-// (look-back on `lbState` rows of `lbStride`, tile 0 from the counters' values
-// before the pass: `bases`) and written. The last tile publishes the level's totals.
-template <int T, int B>
-__device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u32 begin, u32 end, u32 numTiles,
-                           u64* lbState, u32 lbStride, u64* totals, const u32* bases, const FactorParams& fp, u32 sf,
-                           u32 partCap)
+// Tiles of B child places; several (up to 16) only where the look-back rows
+// hold fewer tiles than that (stride: one per kSplitRowItems items of the capacity).
+template <int B>
+__device__ __forceinline__ Level make_level(u32 begin, u32 end, u32 total, const u32* first, u32 stride)
 {
-  using S                  = SplitShared<T, B>;
+  const u32 most = (u32)min((u64)(end - begin) * kMaxChildrenPerItem, 0xFFFFFFFFull - B);
+  Level lv     = {begin, end, min(total, most), 0u, 1u, first};
+  const u32 n  = (lv.total + B - 1) / B;
+  lv.chunks    = max(1u, (n + stride - 1) / stride);
+  lv.tiles     = (n + lv.chunks - 1) / lv.chunks;
+  return lv;
+}
+
+// Shared memory of one split tile (kernel-scope; one per block).
+template <int B>
+struct SplitShared
+{
+  static constexpr u32 kW         = B / 32;
+  static constexpr u32 kMaxChunks = (kMaxChildrenPerItem * kSplitRowItems + B - 1) / B;
+  static constexpr u32 kSlots     = kMaxChunks * kW;  // (chunk, warp) count slots, in serial order
+  static_assert(kSlots <= 64, "one warp scans the count slots, two per lane");
+  static_assert(B >= (int)kMaxChildrenPerItem, "an item holds at most one chunk's first child");
+
+  SplitItem item[B];
+  int       end[B];                  // per item: its last child place + 1, relative to the chunk's first
+  u32       cnt[kCntKids + 1][kSlots];  // per (chunk, warp): count, then exclusive offset within the tile
+  u64       excl[kCntKids + 1];
+  u32       scan[33];
+  u32       tile, flag, range[2], total;
+};
+
+// An item's entry in its level's index: its running child count and, where
+// every B-th child is its own, the item's place in `first`.
+template <int B>
+__device__ __forceinline__ void index_item(const StageCtx& c, u32* first, u32 item, u32 start, u32 places)
+{
+  c.splitEnds[item] = start + places;
+  const u32 g       = (start + B - 1) / B;
+  if(g * B < start + places && g < c.splitFirstStride)
+    first[g] = item;
+}
+
+// Items [begin, end)'s index from their configs, by this block alone: B items
+// at a time. Returns the level's child places.
+template <int B>
+__device__ u32 index_local(const StageCtx& c, SplitShared<B>& sm, u32 begin, u32 end)
+{
+  const tc_TessTriangleInfo* queue = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->splitTriangles);
+  u32                        base  = 0;
+  for(u32 i0 = begin; i0 < end; i0 += B)
+  {
+    const u32 item = i0 + threadIdx.x;
+    const u32 n    = item < end ? child_places(c, __ldcg(&reinterpret_cast<const uint2*>(queue + item)[2].y) >> 16) : 0u;
+    u32       total;
+    const u32 excl = block_exclusive_scan(n, sm.scan, &total);
+    if(n)
+      index_item<B>(c, c.splitFirst, item, base + excl, n);
+    base += total;
+  }
+  __syncthreads();  // (the block's own writes, read by its other threads)
+  return base;
+}
+
+// One tile (B items) of the same by all blocks, ordered by a look-back on `row`.
+template <int B>
+__device__ void index_tile(const StageCtx& c, SplitShared<B>& sm, u64* row, u32 tile, u32 begin, u32 end)
+{
+  const tc_TessTriangleInfo* queue = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->splitTriangles);
+  const u32                  item  = begin + tile * B + threadIdx.x;
+  const u32 n = item < end ? child_places(c, __ldcg(&reinterpret_cast<const uint2*>(queue + item)[2].y) >> 16) : 0u;
+  u32       total;
+  const u32 excl = block_exclusive_scan(n, sm.scan, &total);
+  if(threadIdx.x < 32)
+  {
+    const u64 ex = warp_lookback_exclusive(row, tile, total, 0, c.errorWord, c.spinLimit);
+    if(threadIdx.x == 0)
+      sm.excl[0] = ex;
+  }
+  __syncthreads();
+  if(n)
+    index_item<B>(c, c.splitFirst, item, (u32)sm.excl[0] + excl, n);
+  __syncthreads();
+}
+
+// up to this many tiles' items every block indexes for itself, without waiting
+// for the others
+constexpr u32 kIndexLocalTiles = 4;
+
+// Waits (thread 0) until `flag` is set; false after the limit.
+__device__ __forceinline__ bool wait_flag(const StageCtx& c, const u32* flag)
+{
+  u32 spins = 0;
+  while(ld_acquire_u32(flag) == 0u)
+  {
+    if(++spins > c.spinLimit)
+    {
+      atomicOr(c.errorWord, TC_DEVERR_LOOKBACK_TIMEOUT);
+      return false;
+    }
+    __nanosleep(spins > 64 ? 256 : 32);
+  }
+  return true;
+}
+
+__device__ __forceinline__ void st_release_u32(u32* p, u32 v)
+{
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// One child place and its child.
+struct Lane
+{
+  Child child;
+  u32   item;  // within the chunk's items
+  bool  valid;
+};
+
+// Chunk g's items into shared memory, then the thread's child.
+template <int B>
+__device__ __forceinline__ Lane chunk_child(const StageCtx& c, SplitShared<B>& sm, const Level& lv, u32 g,
+                                            const FactorParams& fp, u32 sf)
+{
+  const tc_TessTriangleInfo* queue = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->splitTriangles);
+  const u32                  from = g * B;
+  // the chunk's items: from its first child's to the next chunk's first
+  // child's. (Clamped: after a look-back that ran out they may be anything.)
+  const u32 a = min(max(__ldcg(lv.first + g), lv.begin), lv.end - 1);
+  const u32 z = from + B < lv.total ? min(max(__ldcg(lv.first + g + 1), a), lv.end - 1) : lv.end - 1;
+  const u32 n = min(z - a + 1, (u32)B);
+  __syncthreads();  // the previous chunk's items are no longer read
+  if(threadIdx.x < n)
+  {
+    const u32 item = a + threadIdx.x;
+    // triangle_split.comp.glsl:146-180 fillBaseVertices; the base
+    // triangle's world positions travel with the item (splitBase)
+    // through L2: with every pass in one launch, other blocks wrote these items
+    const uint2* raw = reinterpret_cast<const uint2*>(queue + item);
+    const uint2  r0 = __ldcg(raw), r1 = __ldcg(raw + 1), r2 = __ldcg(raw + 2);
+    SplitItem    it;
+    it.ci     = {r0.x, r0.y};
+    it.vtx[0] = r1.x;
+    it.vtx[1] = r1.y;
+    it.vtx[2] = r2.x;
+    it.tc     = r2.y;
+    sm.end[threadIdx.x] = (int)(__ldcg(c.splitEnds + item) - from);
+    const float* sb     = c.splitBase + 9 * (u64)item;
+#pragma unroll
+    for(int v = 0; v < 3; v++)
+      it.bp[v] = {__ldcg(sb + 3 * v), __ldcg(sb + 3 * v + 1), __ldcg(sb + 3 * v + 2)};
+    const tc_TessTableEntry e = table_entry(c.table, it.tc >> 16);
+    it.firstTriangle     = e.firstTriangle;
+    it.firstVertex       = e.firstVertex;
+    it.count             = min((u32)e.numTriangles, kMaxChildrenPerItem);
+    sm.item[threadIdx.x] = it;
+  }
+  __syncthreads();
+  // the place's item: the first that ends after it
+  u32 lo = 0, hi = n - 1;
+  while(lo < hi)
+  {
+    const u32 mid = (lo + hi) >> 1;
+    if(sm.end[mid] > (int)threadIdx.x)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  const SplitItem& it  = sm.item[lo];
+  const u32        sub = threadIdx.x - (u32)(sm.end[lo] - (int)max(it.count, 1u));
+  Lane             l;
+  l.item        = lo;
+  l.valid       = from + threadIdx.x < lv.total && sub < it.count;
+  l.child.split = false;
+  if(l.valid)
+    l.child = make_child(c.table, it, sub, fp, sf);
+  return l;
+}
+
+// One tile: its children classified, ordered after every earlier tile of the
+// level (look-back on `lbState` rows of `lbStride`, tile 0 from the counters'
+// values before the pass: `bases`) and written. The last tile publishes the
+// level's totals. `next`: where the next level's `first` is written, null in a
+// launch of one pass.
+template <int B>
+__device__ void split_tile(const StageCtx& c, SplitShared<B>& sm, u32 tile, const Level& lv, u64* lbState, u32 lbStride,
+                           u64* totals, const u32* bases, u32* next, const FactorParams& fp, u32 sf, u32 partCap)
+{
+  using S                  = SplitShared<B>;
   constexpr u32 kW         = S::kW;
   const u32     lane       = threadIdx.x & 31;
   const u32     warp       = threadIdx.x >> 5;
@@ -164,125 +351,35 @@ __device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u
   tc_SceneBuilding*    b     = c.build;
   const tc_caps&       k     = c.caps;
   tc_TessTriangleInfo* queue = reinterpret_cast<tc_TessTriangleInfo*>(b->splitTriangles);
+  const u32            g0 = tile * lv.chunks, chunks = min(lv.chunks, (lv.total + B - 1) / B - g0);
 
-  // parent of child j: last item with pre[item] <= j
-  auto parent_of = [&](u32 j) {
-    u32 lo = 0, hi = T;
-    while(hi - lo > 1)
-    {
-      const u32 mid = (lo + hi) >> 1;
-      if(sm.pre[mid] <= j)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    return lo;
-  };
-
-  // ---- tile setup: parents (warp 0) --------------------------------------
-  if(warp == 0)
+  // ---- classify; every warp counts its own slots ----------------------------
+  Lane l;
+  for(u32 ch = 0; ch < chunks; ch++)
   {
-    const u32  item  = begin + tile * T + lane;
-    const bool valid = lane < T && item < end;
-    u32        n     = 0;
-    if(valid)
-    {
-      // triangle_split.comp.glsl:146-180 fillBaseVertices; the base
-      // triangle's world positions travel with the item (splitBase)
-      // through L2: with every pass in one launch, other blocks wrote these items
-      const uint2* raw = reinterpret_cast<const uint2*>(queue + item);
-      uint2        r0 = __ldcg(raw), r1 = __ldcg(raw + 1), r2 = __ldcg(raw + 2);
-      SplitItem    it;
-      it.ci     = {r0.x, r0.y};
-      it.vtx[0] = r1.x;
-      it.vtx[1] = r1.y;
-      it.vtx[2] = r2.x;
-      it.tc     = r2.y;
-      const tc_TessTableEntry e = table_entry(c.table, it.tc >> 16);
-      if(c.splitBase)
-      {
-        const float* sb = c.splitBase + 9 * (u64)item;
-#pragma unroll
-        for(int v = 0; v < 3; v++)
-          it.bp[v] = {__ldcg(sb + 3 * v), __ldcg(sb + 3 * v + 1), __ldcg(sb + 3 * v + 2)};
-      }
-      else
-      {
-        const tc_RenderInstance& in  = c.instances[it.ci.instanceID];
-        const tc_Cluster         cl  = reinterpret_cast<const tc_Cluster*>(in.clusters)[it.ci.clusterID];
-        const uint8_t*           lt  = reinterpret_cast<const uint8_t*>(in.clusterLocalTriangles) + cl.firstLocalTriangle;
-        const u32                tri = it.tc & 0xFFFFu;
-        const float*             pos = reinterpret_cast<const float*>(in.positions);
-        float                    m[16];
-#pragma unroll
-        for(int j = 0; j < 16; j++)
-          m[j] = __ldg(in.worldMatrix.m + j);
-#pragma unroll
-        for(int v = 0; v < 3; v++)
-          it.bp[v] = xform_point(m, ldg3(pos, cl.firstLocalVertex + lt[tri * 3 + v]));
-      }
-      it.firstTriangle = e.firstTriangle;
-      it.firstVertex   = e.firstVertex;
-      n                = min((u32)e.numTriangles, kMaxChildrenPerItem);
-      sm.item[lane]    = it;
-    }
-    // warp inclusive scan of child counts
-    u32 x = n;
-#pragma unroll
-    for(int d = 1; d < 32; d <<= 1)
-    {
-      u32 y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if(lane >= (u32)d)
-        x += y;
-    }
-    if(lane < T)
-      sm.pre[lane + 1] = x;
-    if(lane == 0)
-      sm.pre[0] = 0;
-  }
-  __syncthreads();
-  const u32  numChildren = sm.pre[T];
-  const u32  numChunks   = (numChildren + B - 1) / B;
-  const bool cached      = numChildren <= S::kCacheChildren;
-
-  // ---- pass 1: classify children; every warp counts its own slots ---------
-  for(u32 ch = 0; ch < numChunks; ch++)
-  {
-    const u32  j     = ch * B + threadIdx.x;
-    const bool valid = j < numChildren;
-    bool       split = false;
-    if(valid)
-    {
-      const u32   it    = parent_of(j);
-      const Child child = make_child(c.table, sm.item[it], j - sm.pre[it], fp, sf);
-      split             = child.split;
-      if(cached)
-        sm.child[j] = make_uint4(child.vtx[0], child.vtx[1], child.vtx[2], child.tc);
-    }
-    const u32 bs = __ballot_sync(0xFFFFFFFFu, valid && split), bp = __ballot_sync(0xFFFFFFFFu, valid && !split);
+    l                = chunk_child<B>(c, sm, lv, g0 + ch, fp, sf);
+    const bool split = l.valid && l.child.split;
+    const u32  bs = __ballot_sync(0xFFFFFFFFu, split), bp = __ballot_sync(0xFFFFFFFFu, l.valid && !split);
+    u32        kids = 0;
+    if(next && bs)
+      kids = __reduce_add_sync(0xFFFFFFFFu, split ? child_places(c, l.child.tc >> 16) : 0u);
     if(lane == 0)
     {
       sm.cnt[kCntSplit][ch * kW + warp] = __popc(bs);
       sm.cnt[kCntPart][ch * kW + warp]  = __popc(bp);
-      sm.splitMask[ch * kW + warp]      = bs;
+      sm.cnt[kCntKids][ch * kW + warp]  = kids;
     }
   }
   __syncthreads();
 
-  // ---- slot offsets within the tile, tile totals, look-back ------------------
-  if(warp < kNumCounters)
+  // ---- slot offsets within the tile, tile totals, look-back -----------------
+  if(warp < (next ? kCntKids + 1 : kNumCounters))
   {
     const u32 q     = warp;
-    const u32 slots = numChunks * kW;
-    u32       v[4], sum = 0;
-#pragma unroll
-    for(int r = 0; r < 4; r++)
-    {
-      const u32 i = lane * 4 + r;
-      v[r]        = i < slots ? sm.cnt[q][i] : 0u;
-      sum += v[r];
-    }
-    u32 incl = sum;
+    const u32 slots = chunks * kW;
+    const u32 i0 = 2 * lane, i1 = i0 + 1;
+    const u32 v0 = i0 < slots ? sm.cnt[q][i0] : 0u, v1 = i1 < slots ? sm.cnt[q][i1] : 0u;
+    u32       incl = v0 + v1;
 #pragma unroll
     for(int d = 1; d < 32; d <<= 1)
     {
@@ -290,67 +387,64 @@ __device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u
       if(lane >= (u32)d)
         incl += y;
     }
-    u32 run = incl - sum;
-#pragma unroll
-    for(int r = 0; r < 4; r++)
-    {
-      const u32 i = lane * 4 + r;
-      if(i < slots)
-        sm.cnt[q][i] = run;
-      run += v[r];
-    }
+    const u32 run = incl - v0 - v1;
+    if(i0 < slots)
+      sm.cnt[q][i0] = run;
+    if(i1 < slots)
+      sm.cnt[q][i1] = run + v0;
     const u32 agg  = __shfl_sync(0xFFFFFFFFu, incl, 31);
     u64       base = 0;
-    if(tile == 0)  // the counters as the previous pass left them (through L2: see above)
+    if(tile == 0 && q < kNumCounters)  // the counters as the previous pass left them (through L2: see above)
       base = bases ? __ldcg(bases + q) : (q == kCntSplit ? __ldcg(&b->splitWriteCounter) : part_base(c));
     const u64 ex = warp_lookback_exclusive(lbState + (u64)q * lbStride, tile, agg, base, c.errorWord, c.spinLimit);
     if(lane == 0)
     {
       sm.excl[q] = ex;
-      if(tile == numTiles - 1)
+      if(tile == lv.tiles - 1 && q < kNumCounters)
         totals[q] = ex + agg;
     }
   }
   __syncthreads();
 
-  // ---- pass 2: write, from pass 1's children or recomputed (no block barriers)
-  for(u32 ch = 0; ch < numChunks; ch++)
+  // ---- write (the children of a tile of several chunks once more) -----------
+  for(u32 ch = 0; ch < chunks; ch++)
   {
-    const u32  j     = ch * B + threadIdx.x;
-    const bool valid = j < numChildren;
-    Child      child;
-    u32        item = 0;
-    child.split     = false;
-    if(valid)
+    if(chunks > 1)
+      l = chunk_child<B>(c, sm, lv, g0 + ch, fp, sf);
+    const Child&     child = l.child;
+    const SplitItem& item  = sm.item[l.item];
+    const bool       split = l.valid && child.split, part = l.valid && !child.split;
+    const u32        bs = __ballot_sync(0xFFFFFFFFu, split), bp = __ballot_sync(0xFFFFFFFFu, part);
+    u32              places = 0, before = 0;
+    if(next && bs)
     {
-      item = parent_of(j);
-      if(cached)
+      places = split ? child_places(c, child.tc >> 16) : 0u;
+      before = places;
+#pragma unroll
+      for(int d = 1; d < 32; d <<= 1)
       {
-        const uint4 cc = sm.child[j];
-        child.vtx[0] = cc.x, child.vtx[1] = cc.y, child.vtx[2] = cc.z, child.tc = cc.w;
-        child.split  = (sm.splitMask[ch * kW + warp] >> lane) & 1u;
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, before, d);
+        if(lane >= (u32)d)
+          before += y;
       }
-      else
-        child = make_child(c.table, sm.item[item], j - sm.pre[item], fp, sf);
+      before -= places;
     }
-    const bool split = valid && child.split, part = valid && !child.split;
-    const u32  bs = __ballot_sync(0xFFFFFFFFu, split), bp = __ballot_sync(0xFFFFFFFFu, part);
     if(split)
     {
       const u64 o = sm.excl[kCntSplit] + sm.cnt[kCntSplit][ch * kW + warp] + __popc(bs & ltm);
       if(o < k.maxSplitTriangles)
       {
         uint2* dst = reinterpret_cast<uint2*>(queue + o);
-        dst[0]     = make_uint2(sm.item[item].ci.instanceID, sm.item[item].ci.clusterID);
+        dst[0]     = make_uint2(item.ci.instanceID, item.ci.clusterID);
         dst[1]     = make_uint2(child.vtx[0], child.vtx[1]);
         dst[2]     = make_uint2(child.vtx[2], child.tc);
-        if(c.splitBase)
-        {
-          float* d = c.splitBase + 9 * o;
+        float* d   = c.splitBase + 9 * o;
 #pragma unroll
-          for(int v = 0; v < 3; v++)
-            d[3 * v] = sm.item[item].bp[v].x, d[3 * v + 1] = sm.item[item].bp[v].y, d[3 * v + 2] = sm.item[item].bp[v].z;
-        }
+        for(int v = 0; v < 3; v++)
+          d[3 * v] = item.bp[v].x, d[3 * v + 1] = item.bp[v].y, d[3 * v + 2] = item.bp[v].z;
+        if(next)
+          index_item<B>(c, next, (u32)o, (u32)sm.excl[kCntKids] + sm.cnt[kCntKids][ch * kW + warp] + before,
+                        places);
       }
     }
     else if(part)
@@ -359,13 +453,13 @@ __device__ void split_tile(const StageCtx& c, SplitShared<T, B>& sm, u32 tile, u
       if(o < partCap)
       {
         uint2* dst = reinterpret_cast<uint2*>(reinterpret_cast<tc_TessTriangleInfo*>(b->partTriangles) + o);
-        dst[0]     = make_uint2(sm.item[item].ci.instanceID, sm.item[item].ci.clusterID);
+        dst[0]     = make_uint2(item.ci.instanceID, item.ci.clusterID);
         dst[1]     = make_uint2(child.vtx[0], child.vtx[1]);
         dst[2]     = make_uint2(child.vtx[2], child.tc);
       }
     }
   }
-  __syncthreads();  // the item, prefix and count arrays are rewritten by the next tile
+  __syncthreads();  // the item and count arrays are rewritten by the next tile
 }
 
 // The counters after a pass (triangle_split.comp.glsl:321-328 and the
@@ -402,11 +496,11 @@ __device__ inline FactorParams split_factor_params(const StageCtx& c)
   return fp;
 }
 
-template <int T, int B>
+template <int B>
 __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
 {
   stage_prologue();
-  __shared__ SplitShared<T, B> sm;
+  __shared__ SplitShared<B> sm;
   tc_SceneBuilding* b = c.build;
   // with transient builds a child part fits when it leaves the back's slots
   // and one more free (build.glsl:68-82, one child at a time)
@@ -428,29 +522,61 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
     sm.range[1] = hi;
   }
   __syncthreads();
-  const u32 begin    = sm.range[0], end = sm.range[1];
-  const u32 numTiles = clamp_tiles(c, (end - begin + T - 1) / T);
+  const u32          begin = sm.range[0], end = sm.range[1];
   const FactorParams fp = split_factor_params(c);
   const u32          sf = clamp_split_factor(c.caps.splitFactor);
+  u32*               indexed  = c.scratch.ticket + 8;  // index tiles done; index complete
+  const u32          own      = (end - begin) <= kIndexLocalTiles * B;
+  const u32          idxTiles = own ? 0u : (end - begin + B - 1) / B;
+  Level              lv       = {};
+  if(own && end > begin)
+    lv = make_level<B>(begin, end, index_local<B>(c, sm, begin, end), c.splitFirst, c.scratch.lbStride);
 
   for(;;)
   {
-    const u32 tile = next_tile(c, &sm.tile);
-    if(tile >= numTiles)
+    u32 tile = next_tile(c, &sm.tile);
+    if(tile < idxTiles)
+    {
+      index_tile<B>(c, sm, c.scratch.lbState + (u64)kRowScan * c.scratch.lbStride, tile, begin, end);
+      if(threadIdx.x == 0)
+      {
+        __threadfence();
+        if(atomicAdd(indexed, 1u) == idxTiles - 1)
+          st_release_u32(indexed + 1, 1u);
+      }
+      continue;
+    }
+    tile -= idxTiles;
+    if(idxTiles && lv.first == nullptr)
+    {
+      if(threadIdx.x == 0)
+        sm.total = wait_flag(c, indexed + 1) ? __ldcg(c.splitEnds + end - 1) : 0u;
+      __syncthreads();
+      lv = make_level<B>(begin, end, sm.total, c.splitFirst, c.scratch.lbStride);
+    }
+    if(tile >= lv.tiles)
       break;
-    split_tile<T, B>(c, sm, tile, begin, end, numTiles, c.scratch.lbState, c.scratch.lbStride, c.scratch.totals,
-                     nullptr, fp, sf, partCap);
+    split_tile<B>(c, sm, tile, lv, c.scratch.lbState, c.scratch.lbStride, c.scratch.totals, nullptr, nullptr, fp, sf,
+                  partCap);
   }
 
   if(last_block_done(c, &sm.flag))
   {
     if(threadIdx.x == 0)
     {
-      split_pass_counters(c, numTiles, c.scratch.totals, partCap);
+      split_pass_counters(c, lv.tiles, c.scratch.totals, partCap);
       if(c.fuseSetup != kNoSetup)
         build_setup_apply(c, c.fuseSetup);
     }
-    scratch_release(c, numTiles, kNumCounters);
+    // (without the index, its wait having run out, what the others used is not known)
+    scratch_release(c, end > begin && lv.tiles == 0 ? c.scratch.lbStride : lv.tiles, kNumCounters);
+    if(c.scratch.selfClean)
+    {
+      for(u32 t = threadIdx.x; t < idxTiles; t += B)
+        c.scratch.lbState[(u64)kRowScan * c.scratch.lbStride + t] = 0;
+      if(threadIdx.x == 0)
+        indexed[0] = indexed[1] = 0;
+    }
   }
 }
 
@@ -460,30 +586,27 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
 
 // Per-level control words, in the level's scratch slot (zeroed with the
 // frame): [1] tiles done, [2..] u64 totals (split, part), [6] / [7] the split
-// and part counters before the level, [12] next level's range published,
-// [13] finalised, [14] start, [15] end. Level 0's [0] is the ticket all levels
-// share.
+// and part counters before the level, [10] the level's child places, [11] next
+// level's range published, [12] finalised, [13] start, [14] end. Level 0's [0]
+// is the ticket all levels share, its [8] counts index tiles, its [9] is set
+// with the index complete, and its [15] before the set-ups are written.
 __device__ __forceinline__ u32* lv_done(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 1; }
 __device__ __forceinline__ u64* lv_totals(const SplitLevels& lv, u32 L) { return reinterpret_cast<u64*>(lv.ctrl[L] + 2); }
 __device__ __forceinline__ u32* lv_bases(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 6; }
-__device__ __forceinline__ u32* lv_ready(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 12; }
-__device__ __forceinline__ u32* lv_final(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 13; }
-
-__device__ __forceinline__ void st_release_u32(u32* p, u32 v)
-{
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
+__device__ __forceinline__ u32* lv_ready(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 11; }
+__device__ __forceinline__ u32* lv_final(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 12; }
 
 // Every level is complete: the counters and set-ups of all passes
 // (split_pass_counters and TC_BUILD_SETUP_SPLIT_PASS for each, then the fused
 // set-up), from the levels' totals, by one thread. Done here once, in
 // registers: at each level's end it kept the next level's tiles waiting for
-// five dependent accesses. `tilesOf(L, begin, end)`: the level's tiles; with
-// no split item at all (levels empty) nothing but the set-ups is left, 7 us of
-// every frame without splits, now 3.
-template <class TilesOf>
-__device__ void finalize_levels(const StageCtx& c, const SplitLevels& lv, u32 partCap, TilesOf&& tilesOf)
+// five dependent accesses. With no split item at all (levels empty) nothing
+// but the set-ups is left, 7 us of every frame without splits, now 3.
+__device__ void finalize_levels(const StageCtx& c, const SplitLevels& lv, u32 partCap)
 {
+  // a block that starts only now must not take the range written below for level 0's
+  st_release_u32(lv.ctrl[0] + 15, 1u);
+  __threadfence();
   tc_SceneBuilding* b     = c.build;
   const u32         most  = c.caps.maxSplitTriangles;
   const bool        trans = (c.flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)) != 0;
@@ -493,7 +616,7 @@ __device__ void finalize_levels(const StageCtx& c, const SplitLevels& lv, u32 pa
   for(u32 L = 0; L < lv.levels; L++)
   {
     const u32 last = min(end, most), first = min(start, last);
-    if(tilesOf(first, last))
+    if(last > first)
     {
       // split_pass_counters
       write           = (u32)__ldcg(lv_totals(lv, L) + kCntSplit);
@@ -548,104 +671,122 @@ __device__ void publish_level(const StageCtx& c, const SplitLevels& lv, u32 L, u
     write = __ldcg(lv_bases(lv, L) + kCntSplit), part = __ldcg(lv_bases(lv, L) + kCntPart);
   u32* next = lv.ctrl[L + 1];
   next[6 + kCntSplit] = write, next[6 + kCntPart] = part;
-  next[14] = min(end, most), next[15] = min(write, most);
+  const u32 first = min(end, most), last = min(write, most);
+  next[10] = last > first ? __ldcg(c.splitEnds + last - 1) : 0u;
+  next[13] = first, next[14] = last;
   __threadfence();
   st_release_u32(lv_ready(lv, L), 1u);
 }
 
-template <int T, int B>
+template <int B>
 __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLevels lv)
 {
   stage_prologue();
-  __shared__ SplitShared<T, B> sm;
-  __shared__ u32               s_level[4];  // level, its first ticket, its tiles, status (1: stop)
-  tc_SceneBuilding* b        = c.build;
-  const u32         partCap  = part_cap(c);
-  const FactorParams fp      = split_factor_params(c);
-  const u32          sf      = clamp_split_factor(c.caps.splitFactor);
-  const u32          levels  = lv.levels;
-  auto tiles_of = [&](u32 lo, u32 hi) { return min((hi - min(lo, hi) + T - 1) / T, lv.stride); };
+  __shared__ SplitShared<B> sm;
+  __shared__ Level          s_lv;
+  __shared__ u32            s_level[3];  // level, its first ticket, status (1: stop)
+  const u32          partCap  = part_cap(c);
+  const FactorParams fp       = split_factor_params(c);
+  const u32          sf       = clamp_split_factor(c.caps.splitFactor);
+  const u32          levels   = lv.levels;
+  u32*               indexed  = lv.ctrl[0] + 8;
 
-  // level 0: the range the classify set-up (BUILD_SETUP_SPLIT) left
-  u32 begin = min(min(b->splitPassStart, c.caps.maxSplitTriangles), min(b->splitPassEnd, c.caps.maxSplitTriangles));
-  u32 end   = min(b->splitPassEnd, c.caps.maxSplitTriangles);
-  u32 level = 0, first = 0, numTiles = tiles_of(begin, end);
-  if(numTiles == 0)
+  // level 0: the range the classify set-up (BUILD_SETUP_SPLIT) left, unless
+  // the launch is complete and the range already the last level's (the flag is
+  // read after the range, and set before it changes)
+  if(threadIdx.x == 0)
+  {
+    const volatile tc_SceneBuilding* b = c.build;
+    const u32 hi = min(b->splitPassEnd, c.caps.maxSplitTriangles), lo = min(b->splitPassStart, hi);
+    __threadfence();
+    sm.range[0] = lo, sm.range[1] = hi;
+    sm.flag = ld_acquire_u32(lv.ctrl[0] + 15);
+  }
+  __syncthreads();
+  const u32 begin0 = sm.range[0], end0 = sm.range[1];
+  if(sm.flag)
+    return;
+  if(begin0 == end0)
   {
     // no split item: every level is empty; one block runs the passes' set-ups
     if(blockIdx.x == 0 && threadIdx.x == 0)
-      finalize_levels(c, lv, partCap, tiles_of);
+      finalize_levels(c, lv, partCap);
     return;
   }
-  if(threadIdx.x == 0 && (end - begin + T - 1) / T > lv.stride)
-    atomicOr(c.errorWord, TC_DEVERR_CAPACITY);
+  const bool own      = end0 - begin0 <= kIndexLocalTiles * B;
+  const u32  idxTiles = own ? 0u : (end0 - begin0 + B - 1) / B;
+  Level      cur      = {};
+  u32        level    = 0, first = idxTiles;
+  if(own)
+    cur = make_level<B>(begin0, end0, index_local<B>(c, sm, begin0, end0), c.splitFirst, lv.stride);
 
   for(;;)
   {
-    const u32 g = next_tile(c, &sm.tile);  // one ticket over all levels
+    const u32 g = next_tile(c, &sm.tile);  // one ticket over the index and all levels
+    if(g < idxTiles)
+    {
+      index_tile<B>(c, sm, lv.lbState[0] + (u64)kRowScan * lv.stride, g, begin0, end0);
+      if(threadIdx.x == 0)
+      {
+        __threadfence();
+        if(atomicAdd(indexed, 1u) == idxTiles - 1)
+          st_release_u32(indexed + 1, 1u);
+      }
+      continue;
+    }
     // the level of ticket g (later levels wait for the earlier ones' completion)
     if(threadIdx.x == 0)
     {
       u32 stop = 0;
-      while(g >= first + numTiles)
+      if(cur.first == nullptr)  // level 0's index
+      {
+        stop = wait_flag(c, indexed + 1) ? 0u : 1u;
+        if(!stop)
+          cur = make_level<B>(begin0, end0, __ldcg(c.splitEnds + end0 - 1), c.splitFirst, lv.stride);
+      }
+      while(!stop && g >= first + cur.tiles)
       {
         // level `level` has no tile for this ticket: move on to the next one
-        if(numTiles == 0 && atomicCAS(lv_final(lv, level), 0u, 1u) == 0u)
+        if(cur.tiles == 0 && atomicCAS(lv_final(lv, level), 0u, 1u) == 0u)
         {
           __threadfence();
-          publish_level(c, lv, level, end, 0);
+          publish_level(c, lv, level, cur.end, 0);
           if(level + 1 == levels)
-            finalize_levels(c, lv, partCap, tiles_of);
+            finalize_levels(c, lv, partCap);
         }
-        first += numTiles;
-        if(++level >= levels)
+        first += cur.tiles;
+        if(++level >= levels || !wait_flag(c, lv_ready(lv, level - 1)))
         {
           stop = 1;
           break;
         }
-        u32 spins = 0;
-        while(ld_acquire_u32(lv_ready(lv, level - 1)) == 0u)
-        {
-          if(++spins > c.spinLimit)
-          {
-            atomicOr(c.errorWord, TC_DEVERR_LOOKBACK_TIMEOUT);
-            stop = 1;
-            break;
-          }
-          __nanosleep(spins > 64 ? 256 : 32);
-        }
-        if(stop)
-          break;
-        begin    = __ldcg(lv.ctrl[level] + 14);
-        end      = __ldcg(lv.ctrl[level] + 15);
-        numTiles = tiles_of(begin, end);
-        if((end - min(begin, end) + T - 1) / T > lv.stride)
-          atomicOr(c.errorWord, TC_DEVERR_CAPACITY);
+        const u32* w = lv.ctrl[level];
+        const u32  lo = __ldcg(w + 13), hi = __ldcg(w + 14);
+        cur = make_level<B>(lo, hi, __ldcg(w + 10), c.splitFirst + c.splitFirstStride * (1 + (level & 1)), lv.stride);
       }
-      s_level[0] = level, s_level[1] = first, s_level[2] = numTiles, s_level[3] = stop;
-      sm.range[0] = begin, sm.range[1] = end;
+      s_lv       = cur;
+      s_level[0] = level, s_level[1] = first, s_level[2] = stop;
     }
     __syncthreads();
-    if(s_level[3])
+    if(s_level[2])
       break;
-    level    = s_level[0];
-    first    = s_level[1];
-    numTiles = s_level[2];
-    begin    = sm.range[0];
-    end      = sm.range[1];
-    const u32 tile = g - first;
-    split_tile<T, B>(c, sm, tile, begin, end, numTiles, lv.lbState[level], lv.stride, lv_totals(lv, level),
-                     level ? lv_bases(lv, level) : nullptr, fp, sf, partCap);
+    cur   = s_lv;
+    level = s_level[0];
+    first = s_level[1];
+    split_tile<B>(c, sm, g - first, cur, lv.lbState[level], lv.stride, lv_totals(lv, level),
+                  level ? lv_bases(lv, level) : nullptr,
+                  level + 1 < levels ? c.splitFirst + c.splitFirstStride * (1 + ((level + 1) & 1)) : nullptr, fp, sf,
+                  partCap);
     // the block completing the level's last tile publishes the next level
     if(threadIdx.x == 0)
     {
       __threadfence();
-      if(atomicAdd(lv_done(lv, level), 1u) == numTiles - 1)
+      if(atomicAdd(lv_done(lv, level), 1u) == cur.tiles - 1)
       {
         __threadfence();
-        publish_level(c, lv, level, end, numTiles);
+        publish_level(c, lv, level, cur.end, cur.tiles);
         if(level + 1 == levels)
-          finalize_levels(c, lv, partCap, tiles_of);
+          finalize_levels(c, lv, partCap);
       }
     }
     __syncthreads();
@@ -660,11 +801,11 @@ cudaError_t launch_triangle_split_levels(const StageCtx& c, const SplitLevels& l
   switch(blockSize)
   {
     case 128:
-      return launch_pdl_prio(k_triangle_split_levels<16, 128>, grid, 128, prio, s, c, lv);
+      return launch_pdl_prio(k_triangle_split_levels<128>, grid, 128, prio, s, c, lv);
     case 512:
-      return launch_pdl_prio(k_triangle_split_levels<32, 512>, grid, 512, prio, s, c, lv);
+      return launch_pdl_prio(k_triangle_split_levels<512>, grid, 512, prio, s, c, lv);
     default:
-      return launch_pdl_prio(k_triangle_split_levels<32, 256>, grid, 256, prio, s, c, lv);
+      return launch_pdl_prio(k_triangle_split_levels<256>, grid, 256, prio, s, c, lv);
   }
 }
 
@@ -676,11 +817,11 @@ cudaError_t launch_triangle_split(const StageCtx& c, u32 blockSize, u32 grid, cu
   switch(blockSize)
   {
     case 128:
-      return launch_pdl_prio(k_triangle_split<16, 128>, grid, 128, prio, s, c);
+      return launch_pdl_prio(k_triangle_split<128>, grid, 128, prio, s, c);
     case 512:
-      return launch_pdl_prio(k_triangle_split<32, 512>, grid, 512, prio, s, c);
+      return launch_pdl_prio(k_triangle_split<512>, grid, 512, prio, s, c);
     default:
-      return launch_pdl_prio(k_triangle_split<32, 256>, grid, 256, prio, s, c);
+      return launch_pdl_prio(k_triangle_split<256>, grid, 256, prio, s, c);
   }
 }
 
