@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_generate_vertices(StageCtx c
         vo               = first_vertex(j);
         lane_part(c, raw[0], raw[1], raw[2], rec.part[lane], nv, kind, tvBase, scale, offset, map);
       }
-      chunk_generate(c, rec.part, gv, vo, nv, kind, tvBase, map, scale, offset);
+      chunk_generate<2>(c, rec.part, gv, vo, nv, kind, tvBase, map, scale, offset);
     }
     __syncwarp();  // the records are rewritten by the warp's next batch
   }

@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_vertices(Stag
                 offset, map);
     const u32  next  = __shfl_sync(0xFFFFFFFFu, following, 0);
     prefetch(next);  // this lane's staged record is in registers now
-    chunk_generate(c, sp, gv, vo, nv, kind, tvBase, map, scale, offset);
+    chunk_generate<4>(c, sp, gv, vo, nv, kind, tvBase, map, scale, offset);
     __syncwarp();  // the warp's part records are rewritten by its next chunk
     chunk = next;
   }
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
       lane_part(c, r0, r1, r2, sp[lane], nv, kind, tvBase, scale, offset, map);
     const u32 next = __shfl_sync(0xFFFFFFFFu, following, 0);
     prefetch(next);
-    chunk_generate(c, sp, gv, (u32)vertexOffset, nv, kind, tvBase, map, scale, offset);
+    chunk_generate<1>(c, sp, gv, (u32)vertexOffset, nv, kind, tvBase, map, scale, offset);
     __syncwarp();  // the warp's part records are rewritten by its next chunk
     chunk = next;
   }

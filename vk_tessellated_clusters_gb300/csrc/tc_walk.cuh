@@ -32,13 +32,20 @@ __device__ __forceinline__ T warp_inclusive(T x, u32 lane)
 // `scale`, `offset` (held in registers; the records' q6-q8 are not read).
 // `tvBase`: per owner lane, its part's first table vertex minus its first
 // vertex within the chunk (table index of chunk vertex jj = tvBase + jj).
-template <u32 Kind, bool Uniform>
+// Bound by instruction issue (185 for each 32 vertices, a seventh of them the
+// parts' set-up) and the latency of the texel and table loads. Steps: steps of
+// 32 vertices unrolled. No lane branches: those past the end repeat the last
+// vertex, so that the steps' loads overlap. With a branch around each vertex
+// the frame of a 2 M triangle terrain takes 338 us, without 332 with two steps
+// and 328 with four; the stage kernel, short of registers, is better with one
+// (314 us with the branch, 312 with two, 309 with one).
+template <u32 Kind, bool Uniform, int Steps>
 __device__ __forceinline__ void chunk_vertices(const StageCtx& c, const PartAffine* sp, u32 owner, u32 start, u32 tvBase,
                                                u32 total, float* dst, const MapDesc& m, float scale, float offset)
 {
   const u32 lane  = threadIdx.x & 31;
   const u32 below = (2u << lane) - 2u;  // bits 1..lane
-  #pragma unroll 2  // two steps in flight: their loads overlap
+#pragma unroll Steps
   for(u32 base = 0; base < total; base += 32)
   {
     // lane's part: those starting at or before the step's first vertex, plus
@@ -48,15 +55,12 @@ __device__ __forceinline__ void chunk_vertices(const StageCtx& c, const PartAffi
                                                 (owner && start > base && start < base + 32) ? 1u << (start - base) : 0u);
     const u32         pi     = before - 1 + __popc(inside & below);
     const u32         tvIdx  = __shfl_sync(0xFFFFFFFFu, tvBase, pi & 31);
-    const u32         jj     = base + lane;
+    const u32         jj     = min(base + lane, total - 1);
     const PartAffine& r      = sp[pi];
-    if(jj < total)
-    {
-      const u32 tv = __ldg(c.table.vertices + (tvIdx + jj));
-      const f3  q  = Uniform ? affine_vertex_u<Kind>(r, tv, m, scale, offset) : affine_vertex_k<Kind>(r, tv);
-      float*   d = dst + 3 * (u64)jj;
-      d[0] = q.x, d[1] = q.y, d[2] = q.z;
-    }
+    const u32         tv     = __ldg(c.table.vertices + (tvIdx + jj));
+    const f3          q      = Uniform ? affine_vertex_u<Kind>(r, tv, m, scale, offset) : affine_vertex_k<Kind>(r, tv);
+    float*            d      = dst + 3 * (u64)jj;
+    d[0] = q.x, d[1] = q.y, d[2] = q.z;
   }
 }
 
@@ -97,6 +101,7 @@ __device__ __forceinline__ void lane_part(const StageCtx& c, uint2 r0, uint2 r1,
 // range (first generated vertex: lane 0's `vo`) on consecutive vertices, with
 // one specialisation for the whole chunk when its parts share a map kind, and
 // the map, scale and offset in registers when they share those too.
+template <int Steps>
 __device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffine* sp, float* gv, u32 vo, u32 nv,
                                              u32 kind, u32 tvBase, const MapDesc& map, float scale, float offset)
 {
@@ -130,16 +135,16 @@ __device__ __forceinline__ void chunk_generate(const StageCtx& c, const PartAffi
   __syncwarp();
   float* dst = gv + 3 * (u64)v0;
 #define TC_CHUNK(K)                                                                                                    \
-  (uni ? chunk_vertices<K, true>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset)                       \
-       : chunk_vertices<K, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset))
+  (uni ? chunk_vertices<K, true, Steps>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset)                       \
+       : chunk_vertices<K, false, Steps>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset))
   switch(kw)
   {
     case affine_kind(TC_TEXEL_F16, true): TC_CHUNK(affine_kind(TC_TEXEL_F16, true)); break;
     case affine_kind(TC_TEXEL_F32, true): TC_CHUNK(affine_kind(TC_TEXEL_F32, true)); break;
     case kAffineFlat:
-      chunk_vertices<kAffineFlat, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset);
+      chunk_vertices<kAffineFlat, false, Steps>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset);
       break;
-    default: chunk_vertices<~0u, false>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset); break;
+    default: chunk_vertices<~0u, false, Steps>(c, sp, owner, start, tvBase, total, dst, um, uScale, uOffset); break;
   }
 #undef TC_CHUNK
 }
