@@ -234,3 +234,70 @@ def test_instance_groups(oracle, case):
         assert got["genVertices"].tobytes() == first["genVertices"].tobytes()
     assert pipe.device_errors() == 0
     pipe.close()
+
+
+# one instance; several below the instance groups' clusters; groups of 18 with some instances apart by offset or by
+# their gradients' place; gradients 0 and 1 floats off 8-byte alignment, maps of odd width
+@pytest.mark.parametrize("case", ["single", "few", "groups", "targets", "shared_map"])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_backward_groups(oracle, case, shift):
+    """Each gradient (positions and normals per mesh, texels per map) against the FP64 adjoint, twice with another
+    frame in between: relative error of its norm within 1e-4, as for the frame the backward is specified on."""
+    import torch
+    from oracle.binding import lib as olib
+    from vk_tessellated_clusters_gb300.autograd import FrozenFrame
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    rng = np.random.default_rng(7)
+    if case == "single":
+        sc = S.scene_icosphere(subdivisions=4, map_size=64)
+        cams = [S.Camera(eye=(0.0, 0.0, d), center=(0.0, 0.0, 0.0), tess_rate_pixels=8.0) for d in (8.0, 7.8)]
+    else:
+        sc = S.scene_batched(num_instances=8 if case == "few" else 72, map_size=64)
+        cams = [S.camera_orbit(0), S.camera_orbit(40, tess_rate_pixels=6.0)]
+        for i in (9, 30, 31):
+            sc.instances[i % len(sc.instances)].displacement_offset = 0.01
+        if case == "shared_map":  # one map for two meshes
+            for i in sc.instances:
+                i.displacement_index = min(i.displacement_index, 1)
+    sc.textures[:] = [S.Texture(rng.random((37, 53), np.float32), L.TEXEL_F32) for _ in sc.textures]
+    caps = L.default_caps(vertex_bits=22)
+    pipe = TessellationPipeline(sc, caps, FLAGS)
+    for cam in cams:
+        pipe.set_cameras(cam)
+        pipe.build("graph")
+        frozen = FrozenFrame(pipe)
+        ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+        full = pipe.outputs()["tempInstantiations"]["clusterIdOffset"] >> 30 == L.RT_CLUSTER_MODE_FULL_CLUSTER
+        assert full.any() and (not full.all() or cam is cams[0])
+        g = rng.normal(0, 1, (frozen.num_vertices, 3)).astype(np.float32)
+        buf = torch.zeros(2 * frozen._grad_floats + 1, device="cuda")
+        flat = buf[shift:shift + frozen._grad_floats]
+        table = frozen._pointer_table(flat)
+        own = [4, 13] if case == "targets" else []  # instances with gradients of their own, past the others
+        apart = buf[frozen._grad_floats + shift:]
+        for i in own:
+            table[2 * i] = apart.data_ptr()
+        frozen.launch_backward(torch.from_numpy(g).cuda(), table)
+        dP = [np.zeros(m.positions.shape) for m in sc.geometries]
+        dN = [np.zeros(m.normals.shape) for m in sc.geometries]
+        dT = [np.zeros(t.texels.shape) for t in sc.textures]
+        mesh = [i.geometry for i in sc.instances]
+        assert not own or len({mesh[i] for i in own}) == 2
+        ptr = lambda a: (ctypes.c_void_p * len(a))(*[x.ctypes.data for x in a])
+        big = np.zeros((max(len(p) for p in dP), 3))
+        g64 = g.astype(np.float64)
+        olib().tco_backward_f64(ctypes.byref(oracle.table), ctypes.byref(ref_state.args), g64.ctypes.data,
+                                ptr([big if i in own else dP[m] for i, m in enumerate(mesh)]),
+                                ptr([dN[m] for m in mesh]), ptr(dT))
+        got = flat.double().cpu().numpy()
+        at = 0
+        for name, want in [("positions", w) for w in dP] + [("normals", w) for w in dN] + [("texels", w) for w in dT]:
+            part = got[at:at + want.size].reshape(want.shape)
+            at += want.size
+            norm = np.linalg.norm(want)
+            assert np.linalg.norm(part - want) <= 1e-4 * norm, (name, np.linalg.norm(part - want) / norm)
+        if own:
+            part = apart[:big.size].double().cpu().numpy().reshape(big.shape)
+            assert np.linalg.norm(part - big) <= 1e-4 * np.linalg.norm(big)
+    assert pipe.device_errors() == 0
+    pipe.close()

@@ -59,6 +59,8 @@ struct Plan
   size_t chunkSumsOffset;   // u64 per 32 part triangles
   size_t splitBaseOffset;   // 9 floats per split item: its base triangle's world positions
   size_t splitEndsOffset, splitFirstOffset, splitFirstStride;  // StageCtx::splitEnds, splitFirst
+  size_t backOffset, backSlotsOffset;  // BackGroups
+  u32    backCap;
   size_t instOffset;  // instance cluster prefix (u32 x maxInstances+1)
   size_t errOffset;   // device error word
   size_t totalBytes;
@@ -232,6 +234,11 @@ Plan make_plan(const tc_context_desc& d)
   p.splitFirstOffset  = off;
   p.splitFirstStride  = (size_t)ceil_div((u64)k.maxSplitTriangles * TC_TESSTABLE_SIZE * TC_TESSTABLE_SIZE, 128) + 1;
   off                 = align_up(off + p.splitFirstStride * 3 * 4, 256);
+  p.backCap    = std::min(kBackInstances, std::max(1u, d.maxInstances));
+  p.backOffset = off;  // the adjoint's groups: head, then per instance subgroup, members; then slots
+  off          = align_up(off + 32 + (size_t)p.backCap * (16 + 8), 256);
+  p.backSlotsOffset = off;
+  off               = align_up(off + (size_t)std::max(1u, d.maxTotalClusters) * 4, 256);
   p.rasterOffset      = off;  // raster batching: per group of 32 parts its counts, then offsets
   off                 = align_up(off + (size_t)ceil_div(std::max(1u, k.maxPartTriangles), 32) * 16, 256);
   p.totalBytes        = off;
@@ -339,6 +346,12 @@ bool groups_instances(const tc_frame_args* a)
   return (a->flags & TC_FLAG_RASTER_CULL) == 0 && a->numInstances >= 2 && a->numInstances <= kGroupInstances
          && a->totalClusters >= kGroupMinClusters;
 }
+
+// Clusters from which the adjoint takes full clusters by instance groups, with
+// one launch more (k_backward_index): 48 instances of the batched scene (9,720
+// clusters) 18.7 us without and 19.1 with, 96 instances 43 and 27 us, 256
+// instances 106 and 46.
+constexpr u32 kBackMinClusters = 12288;
 
 // the instance groups' tables
 GroupTables group_tables(tc_context* ctx)
@@ -1258,10 +1271,24 @@ tc_status tc_instantiate_backward(tc_context* ctx, const tc_frame_args* a, uint6
     return TC_ERR_INVALID_ARG;
   if(!(a->flags & TC_FLAG_WRITE_FULLCLUSTERS))
     return TC_ERR_INVALID_ARG;
-  StageCtx c = base_ctx(ctx, a);
+  StageCtx   c = base_ctx(ctx, a);
+  BackGroups g = {};
+  if(a->numInstances >= 2 && a->numInstances <= kBackInstances && a->totalClusters >= kBackMinClusters)
+  {
+    char* base = reinterpret_cast<char*>(ctx->dScratch) + ctx->plan.backOffset;
+    g          = {reinterpret_cast<uint4*>(base + 32),
+                  reinterpret_cast<u32*>(base + 32 + (size_t)ctx->plan.backCap * 16),
+                  reinterpret_cast<u32*>(base),
+                  reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.backSlotsOffset),
+                  ctx->plan.backCap,
+                  std::max(1u, ctx->desc.maxTotalClusters)};
+    TC_CHECK_CUDA(launch_backward_index(c, g, std::min(ctx->numSMs, ceil_div(a->totalClusters, kBackInstances)),
+                                        reinterpret_cast<cudaStream_t>(stream)));
+    ctx->launches += 1;
+  }
   TC_CHECK_CUDA(launch_instantiate_backward(c, reinterpret_cast<const float*>(gradVertices),
                                             reinterpret_cast<const tc_GradTargets*>(gradTargets),
-                                            reinterpret_cast<float* const*>(gradTexels), ctx->numSMs * 8,
+                                            reinterpret_cast<float* const*>(gradTexels), g, ctx->numSMs,
                                             reinterpret_cast<cudaStream_t>(stream)));
   ctx->launches += 1;
   return TC_OK;

@@ -330,17 +330,15 @@ __device__ __forceinline__ Taps bilinear_taps(const tc_DisplacementTexture& tx, 
   t.fy   = y - yf;
   int ix = __float2int_rz(xf), iy = __float2int_rz(yf);
   t.x0   = wrapi(ix, (int)tx.width);
-  t.x1   = wrapi(ix + 1, (int)tx.width);
   t.y0   = wrapi(iy, (int)tx.height);
-  t.y1   = wrapi(iy + 1, (int)tx.height);
+  // (the neighbours, wrapped: REPEAT)
+  t.x1   = t.x0 + 1 == (int)tx.width ? 0 : t.x0 + 1;
+  t.y1   = t.y0 + 1 == (int)tx.height ? 0 : t.y0 + 1;
   return t;
 }
 
-__device__ __forceinline__ float sample_bilinear(const tc_DisplacementTexture& tx, f2 uv)
+__device__ __forceinline__ float sample_taps(const tc_DisplacementTexture& tx, const Taps& b)
 {
-  if(tx.width == 0 || tx.height == 0)
-    return 0.0f;
-  Taps      b  = bilinear_taps(tx, uv);
   const u64 r0 = (u64)b.y0 * tx.width, r1 = (u64)b.y1 * tx.width;
   float     t00, t10, t01, t11;
   if(tx.format == TC_TEXEL_F16)
@@ -370,6 +368,13 @@ __device__ __forceinline__ float sample_bilinear(const tc_DisplacementTexture& t
   float top = gx * t00 + b.fx * t10;
   float bot = gx * t01 + b.fx * t11;
   return (1.0f - b.fy) * top + b.fy * bot;
+}
+
+__device__ __forceinline__ float sample_bilinear(const tc_DisplacementTexture& tx, f2 uv)
+{
+  if(tx.width == 0 || tx.height == 0)
+    return 0.0f;
+  return sample_taps(tx, bilinear_taps(tx, uv));
 }
 
 // height = (h * instScale * viewScale) + instOffset + viewOffset; pos += normalize(n) * height

@@ -29,6 +29,13 @@ __device__ __forceinline__ bool same_key(const GroupKey& a, const GroupKey& b)
          && __float_as_uint(a.offset) == __float_as_uint(b.offset) && a.numClusters == b.numClusters;
 }
 
+// Fibonacci hashing: the high bits of a multiple of 2^64 / golden ratio
+__device__ __forceinline__ u64 group_hash(const GroupKey& k)
+{
+  return (k.positions ^ (k.clusters << 1) ^ ((u64)(u32)k.map << 40) ^ ((u64)__float_as_uint(k.scale) << 8))
+         * 0x9E3779B97F4A7C15ull;
+}
+
 // One block groups the frame's instances by key (a hash table of their indices
 // in shared memory), cuts the groups into subgroups of at most kGroupMembers
 // and makes a task of every cluster of a subgroup. It reads the instance
@@ -66,10 +73,8 @@ __device__ inline void find_groups(const StageCtx& c, const GroupTables& g)
       const u32 i = base + q * blockDim.x;
       if(i >= n)
         continue;
-      u64 h = key[q].positions ^ (key[q].clusters << 1) ^ ((u64)(u32)key[q].map << 40) ^ ((u64)__float_as_uint(key[q].scale) << 8);
-      h *= 0x9E3779B97F4A7C15ull;  // Fibonacci hashing: the high bits of a multiple of 2^64 / golden ratio
       u32 rep = ~0u;
-      for(u32 slot = (u32)(h >> 40) % kGroupTable; rep == ~0u; slot = (slot + 1) % kGroupTable)
+      for(u32 slot = (u32)(group_hash(key[q]) >> 40) % kGroupTable; rep == ~0u; slot = (slot + 1) % kGroupTable)
       {
         // (the table has twice as many slots as instances)
         const unsigned short found = atomicCAS(&s_table[slot], kEmpty, (unsigned short)i);

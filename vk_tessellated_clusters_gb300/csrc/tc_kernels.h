@@ -168,8 +168,19 @@ cudaError_t launch_blas_clusters_insert(const StageCtx& c, u32* segStart, u32* s
 cudaError_t launch_raster_batches(const StageCtx& c, uint4* groups, const tc_raster_outputs& o, u32 maxParts,
                                   u32 numSMs, cudaStream_t s);
 cudaError_t launch_generate_vertices(const StageCtx& c, u32 grid, cudaStream_t s);
+// instance groups of the adjoint's full clusters, in scratch (head null: none)
+constexpr u32 kBackInstances = 1024;  // instances grouped (one block, a thread each)
+struct BackGroups
+{
+  uint4* groups;   // per subgroup: first task, first member, members, representative instance
+  u32*   members;  // [2 * cap]: the groups' instances, then per instance its representative
+  u32*   head;     // subgroups, tasks, whether the groups are used
+  u32*   slots;    // per cluster of the instances: its full cluster (anything where it has none)
+  u32    cap, slotCap;
+};
+cudaError_t launch_backward_index(const StageCtx& c, const BackGroups& g, u32 grid, cudaStream_t s);
 cudaError_t launch_instantiate_backward(const StageCtx& c, const float* gradVertices, const tc_GradTargets* targets,
-                                        float* const* gradTexels, u32 grid, cudaStream_t s);
+                                        float* const* gradTexels, const BackGroups& g, u32 numSMs, cudaStream_t s);
 
 // tiles per launch for each stage (used to size the look-back scratch)
 constexpr u32 kInstanceTile     = 256;  // instances per tile (instances_classify, blas_setup)
