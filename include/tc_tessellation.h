@@ -466,7 +466,7 @@ typedef struct tc_schedule {
                                  * that for tc_triangle_split */
   uint32_t fullVertexBlocksPerSM; /* grid of the full-cluster vertex kernel = SMs x this (at most 4 resident);
                                    * it runs beside the rest of the frame (fewer blocks leave room for it);
-                                   * 0: the default (4) */
+                                   * 0: the default (3) */
   uint32_t vertexGridPerSM;     /* grid of the part vertex kernel = SMs x this (grid-stride over 32-part chunks);
                                  * 0: one resident wave (the blocks vertexBlocksPerSM allows), and one block per SM
                                  * less for the first part run of a frame that allocates two */

@@ -35,7 +35,11 @@ static_assert(8 + 8 * kMaxCounters <= 48, "the split levels' control words start
 // then the others), blas setup, blas insert (2)
 constexpr uint64_t kFrameFixedLaunches = 16;
 
-constexpr u32 kDefaultFullVertexBlocksPerSM = 4;
+// One block per SM less than fit: with every register taken, the first run's
+// allocation, which becomes ready just after, waits for this kernel (1,024
+// instances 165 -> 159 us a frame, 256 instances 85 -> 79.5; with two 157 and 80,
+// but with PN and the ripple 131 -> 143).
+constexpr u32 kDefaultFullVertexBlocksPerSM = 3;
 
 struct Plan
 {

@@ -1980,8 +1980,8 @@ cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffe
   if(e != cudaSuccess || !(c.flags & TC_FLAG_TRANSIENT_2X))
     return e;
   // the 2X batches' vertices (at most eight builds per cluster): warps stride
-  // over the builds, one resident wave of the kernel's blocks
-  const u32 miniGrid = std::max(1u, std::min((maxClusters * 8 + kDeformWarps - 1) / kDeformWarps, numSMs * (u32)kDeformBlocksPerSM));
+  // over the builds, one resident wave of the kernel's blocks (less kDeformRoom)
+  const u32 miniGrid = std::max(1u, std::min((maxClusters * 8 + kDeformWarps - 1) / kDeformWarps, numSMs * (u32)(kDeformBlocksPerSM - kDeformRoom)));
   return launch_pdl(k_classify_mini_vertices, miniGrid, kDeformBlock, s, c, cs);
 }
 

@@ -25,6 +25,9 @@ constexpr u32 kDeformWarps = kDeformBlock / 32;
 // memory, which leaves the registers to bound the resident blocks
 constexpr u32 kDeformParts = 16;
 constexpr int kDeformBlocksPerSM = 7;  // 72 registers per thread
+// blocks per SM left out where kernels of the frame's critical path run beside:
+// room for one of their blocks
+constexpr int kDeformRoom = 2;
 
 // A warp's part records, and what its walk reads of part `lane` by shuffles.
 struct DeformRecords

@@ -941,14 +941,16 @@ cudaError_t launch_instantiate_vertices(const StageCtx& c, const InstantiateBuff
   const u32 chunks = (maxParts + kPartsPerWarp - 1) / kPartsPerWarp;
   if(c.flags & (TC_FLAG_PN | TC_FLAG_RIPPLE))  // one resident wave of the deformation kernel's blocks
     return launch_pdl(k_instantiate_vertices_deform,
-                      std::max(1u, std::min((chunks + kDeformWarps - 1) / kDeformWarps * 8, numSMs * (u32)kDeformBlocksPerSM)), kDeformBlock, s, c, buf);
+                      std::max(1u, std::min((chunks + kDeformWarps - 1) / kDeformWarps * 8, numSMs * (u32)(kDeformBlocksPerSM - (leaveRoom ? kDeformRoom : 0)))), kDeformBlock, s, c, buf);
   // warps stride over the 32-part chunks; the grid is sized to the machine,
   // not to the capacity (blocks with no chunk would only add a tail), by
   // default one resident wave; vertexBlocksPerSM picks the register budget.
   // leaveRoom: one block per SM less, for the kernels on the frame's critical
   // path that run beside: this kernel's blocks stay until its end, and with
   // every register taken the next allocation waits for it (terrain of 2 M
-  // triangles 376 -> 367 us a frame, 256 instances 87.6 -> 84.5).
+  // triangles 376 -> 367 us a frame, 256 instances 87.6 -> 84.5; the deformation
+  // kernel, kDeformRoom blocks less: 256 instances with PN, ripple and transient
+  // builds 131 -> 127.5, with the 2X batches' kernel likewise).
   const u32 resident   = vertexBlocksPerSM >= 6 ? 6u : (vertexBlocksPerSM == 5 ? 5u : 4u);
   const u32 perSM      = vertexGridPerSM ? vertexGridPerSM : resident - (leaveRoom ? 1 : 0);
   const u32 vertexGrid = std::max(1u, std::min((chunks + kWarps - 1) / kWarps, numSMs * perSM));
