@@ -301,6 +301,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_instantiate_args(StageCtx c, Inst
     part_range(c, s_range[0], s_range[1]);
   __syncthreads();
   const u32 begin    = s_range[0], n = s_range[1] - s_range[0];
+  // no part at all (the later runs of a frame without splits): the first block
+  // alone runs the set-ups, without a count of the blocks that are done (none
+  // of what part_range reads is written below): the later runs' arguments of 256
+  // instances 8 -> 4 us, an icosphere's frame 46.5 -> 43.8 us
+  if(n == 0 && blockIdx.x != 0)
+    return;
   const u32 numTiles = clamp_tiles(c, (n + kTile - 1) / kTile);
   const u32 stride   = c.scratch.lbStride;
   const u64 genBase  = c.scratch.totals[0];
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_instantiate_args(StageCtx c, Inst
       atomicAdd(&c.readback->numTotalTriangles, t);
   }
 
-  if(last_block_done(c, &s_flag))
+  if(n == 0 || last_block_done(c, &s_flag))
   {
     if(threadIdx.x == 0 && c.fuseSetup != kNoSetup)
       build_setup_apply(c, c.fuseSetup);
