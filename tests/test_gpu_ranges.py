@@ -155,7 +155,8 @@ def test_split_tiles(oracle, subdivisions, eye, pixels, capacity, several, block
     pipe.close()
 
 
-@pytest.mark.parametrize("count", [1, 31, 256, 257, 1023])
+# up to 8,192 hits without the staging, then partial and whole blocks of 256
+@pytest.mark.parametrize("count", [1, 31, 256, 257, 1023, 8192, 8193, 8447, 8448, 8449])
 @pytest.mark.parametrize("offset", [0, 4, 8])
 def test_decode_counts_and_alignment(oracle, count, offset):
     """Partial blocks of hits at 4-, 8- and 16-byte aligned addresses: field-exact against the oracle, and nothing
