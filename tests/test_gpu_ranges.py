@@ -85,6 +85,37 @@ def test_vertex_chunk_widths(oracle, subdivisions, pixels, grid):
     pipe.close()
 
 
+# every map kind the vertex walk is specialised for, and chunks that mix them
+@pytest.mark.parametrize("dtype,fmt", [(np.float32, L.TEXEL_F32), (np.float16, L.TEXEL_F16), (np.uint16, L.TEXEL_UNORM16)])
+@pytest.mark.parametrize("size", [(37, 53), (64, 32), (1, 1), "mixed"])
+def test_map_kinds(oracle, dtype, fmt, size):
+    """Frame graph and stage entry points against the oracle, integers bit-exact and positions to the vertex tolerance;
+    the frozen frame's forward gives the same bits."""
+    from vk_tessellated_clusters_gb300.autograd import FrozenFrame
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_batched(num_instances=12, map_size=64)
+    rng = np.random.default_rng(3)
+    for i in range(len(sc.textures)):
+        if size != "mixed" or i % 2:
+            shape = (37, 53) if size == "mixed" else size
+            texels = rng.random(shape) * (65535 if dtype == np.uint16 else 1)
+            sc.textures[i] = S.Texture(texels.astype(dtype), fmt)
+    cam = S.camera_orbit(40, tess_rate_pixels=6.0)
+    caps = L.default_caps(vertex_bits=21)
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    want = ref_state.outputs(oracle.entries)
+    pipe = TessellationPipeline(sc, caps, FLAGS)
+    pipe.set_cameras(cam)
+    for mode in ("graph", "plain"):
+        pipe.state.gen_vertices.handle.zero_()
+        pipe.build(mode)
+        assert_same(pipe.outputs(), want, mode, vertex_tol=vertex_tolerance(sc))
+    built = pipe.outputs()["genVertices"]
+    assert FrozenFrame(pipe).generate().cpu().numpy().tobytes() == built.tobytes()
+    assert pipe.device_errors() == 0
+    pipe.close()
+
+
 def _ripple(cam):
     fc = S.frame_constants(cam)
     fc["animationRippleAmplitude"], fc["animationRippleFrequency"] = 0.02, 8.0
