@@ -89,8 +89,8 @@ def test_vertex_chunk_widths(oracle, subdivisions, pixels, grid):
 @pytest.mark.parametrize("dtype,fmt", [(np.float32, L.TEXEL_F32), (np.float16, L.TEXEL_F16), (np.uint16, L.TEXEL_UNORM16)])
 @pytest.mark.parametrize("size", [(37, 53), (64, 32), (1, 1), "mixed"])
 def test_map_kinds(oracle, dtype, fmt, size):
-    """Frame graph and stage entry points against the oracle, integers bit-exact and positions to the vertex tolerance;
-    the frozen frame's forward gives the same bits."""
+    """Frame graph, stage entry points and raster batches against the oracle, integers bit-exact and positions to the
+    vertex tolerance (times the largest instance scale); the frozen frame's forward gives the same bits."""
     from vk_tessellated_clusters_gb300.autograd import FrozenFrame
     from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
     sc = S.scene_batched(num_instances=12, map_size=64)
@@ -112,6 +112,10 @@ def test_map_kinds(oracle, dtype, fmt, size):
         assert_same(pipe.outputs(), want, mode, vertex_tol=vertex_tolerance(sc))
     built = pipe.outputs()["genVertices"]
     assert FrozenFrame(pipe).generate().cpu().numpy().tobytes() == built.tobytes()
+    got, ref = pipe.raster_batches(), oracle.raster_batches(ref_state)
+    assert got["counts"] == ref["counts"] and got["indices"].tobytes() == ref["indices"].tobytes()
+    scale = max(float(np.abs(np.asarray(i.world)[:3, :3]).sum(axis=1).max()) for i in sc.instances)
+    assert np.abs(got["worldPositions"].astype(np.float64) - ref["worldPositions"]).max() <= vertex_tolerance(sc) * scale
     assert pipe.device_errors() == 0
     pipe.close()
 
