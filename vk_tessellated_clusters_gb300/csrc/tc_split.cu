@@ -522,14 +522,23 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
     sm.range[1] = hi;
   }
   __syncthreads();
-  const u32          begin = sm.range[0], end = sm.range[1];
+  const u32 begin = sm.range[0], end = sm.range[1];
+  // no item: nothing is counted or written, the first block runs the set-up (an
+  // empty pass leaves the next one's range empty as well, so a block that reads
+  // it late finds the same)
+  if(begin == end)
+  {
+    if(blockIdx.x == 0 && threadIdx.x == 0 && c.fuseSetup != kNoSetup)
+      build_setup_apply(c, c.fuseSetup);
+    return;
+  }
   const FactorParams fp = split_factor_params(c);
   const u32          sf = clamp_split_factor(c.caps.splitFactor);
   u32*               indexed  = c.scratch.ticket + 8;  // index tiles done; index complete
   const u32          own      = (end - begin) <= kIndexLocalTiles * B;
   const u32          idxTiles = own ? 0u : (end - begin + B - 1) / B;
   Level              lv       = {};
-  if(own && end > begin)
+  if(own)
     lv = make_level<B>(begin, end, index_local<B>(c, sm, begin, end), c.splitFirst, c.scratch.lbStride);
 
   for(;;)
@@ -569,7 +578,7 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
         build_setup_apply(c, c.fuseSetup);
     }
     // (without the index, its wait having run out, what the others used is not known)
-    scratch_release(c, end > begin && lv.tiles == 0 ? c.scratch.lbStride : lv.tiles, kNumCounters);
+    scratch_release(c, lv.tiles == 0 ? c.scratch.lbStride : lv.tiles, kNumCounters);
     if(c.scratch.selfClean)
     {
       for(u32 t = threadIdx.x; t < idxTiles; t += B)
