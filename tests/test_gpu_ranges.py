@@ -88,7 +88,8 @@ def test_vertex_chunk_widths(oracle, subdivisions, pixels, grid):
 # every map kind the vertex walk is specialised for, and chunks that mix them
 @pytest.mark.parametrize("dtype,fmt", [(np.float32, L.TEXEL_F32), (np.float16, L.TEXEL_F16), (np.uint16, L.TEXEL_UNORM16)])
 @pytest.mark.parametrize("size", [(37, 53), (64, 32), (1, 1), "mixed"])
-def test_map_kinds(oracle, dtype, fmt, size):
+@pytest.mark.parametrize("deform", [0, L.FLAG_PN | L.FLAG_RIPPLE])
+def test_map_kinds(oracle, dtype, fmt, size, deform):
     """Frame graph, stage entry points and raster batches against the oracle, integers bit-exact and positions to the
     vertex tolerance (times the largest instance scale); the frozen frame's forward gives the same bits."""
     from vk_tessellated_clusters_gb300.autograd import FrozenFrame
@@ -101,17 +102,18 @@ def test_map_kinds(oracle, dtype, fmt, size):
             texels = rng.random(shape) * (65535 if dtype == np.uint16 else 1)
             sc.textures[i] = S.Texture(texels.astype(dtype), fmt)
     cam = S.camera_orbit(40, tess_rate_pixels=6.0)
+    cam = _ripple(cam) if deform else cam
     caps = L.default_caps(vertex_bits=21)
-    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS | deform)
     want = ref_state.outputs(oracle.entries)
-    pipe = TessellationPipeline(sc, caps, FLAGS)
+    pipe = TessellationPipeline(sc, caps, FLAGS | deform)
     pipe.set_cameras(cam)
     for mode in ("graph", "plain"):
         pipe.state.gen_vertices.handle.zero_()
         pipe.build(mode)
         assert_same(pipe.outputs(), want, mode, vertex_tol=vertex_tolerance(sc))
     built = pipe.outputs()["genVertices"]
-    assert FrozenFrame(pipe).generate().cpu().numpy().tobytes() == built.tobytes()
+    assert deform or FrozenFrame(pipe).generate().cpu().numpy().tobytes() == built.tobytes()
     got, ref = pipe.raster_batches(), oracle.raster_batches(ref_state)
     assert got["counts"] == ref["counts"] and got["indices"].tobytes() == ref["indices"].tobytes()
     scale = max(float(np.abs(np.asarray(i.world)[:3, :3]).sum(axis=1).max()) for i in sc.instances)

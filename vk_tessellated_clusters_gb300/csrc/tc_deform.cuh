@@ -90,13 +90,44 @@ __device__ __forceinline__ void setup_deform(const StageCtx& c, const tc_RenderI
   }
 }
 
+template <u32 Kind>
 __device__ __forceinline__ f3 deform_vertex(const PartAffine& a, const PartPn& p, u32 tv, bool pn, u32 inst, float size,
                                             const RippleParams& rp)
 {
-  f3 q = pn ? affine_displace(a, tv, part_pn_position(p, tv)) : affine_vertex(a, tv);
+  f3 q = pn ? affine_displace<Kind>(a, tv, part_pn_position(p, tv)) : affine_vertex_k<Kind>(a, tv);
   if(rp.enabled)
     q = ripple(q, inst, size, rp);
   return q;
+}
+
+// The vertex walk of deform_walk for parts of map kind Kind (~0u: any), the
+// lanes past the end repeating the last vertex. (One step at a time: with PN two
+// in flight take 129 us instead of 128 a close-up frame, four 150; any kind at
+// run time 130.7.)
+template <u32 Kind>
+__device__ __forceinline__ void deform_steps(const StageCtx& c, const DeformRecords& rec, bool owner, u32 start, u32 total,
+                                             u32 tvBase, u32 dstBase, const DeformLane& d, bool pn,
+                                             const RippleParams& rp, float* gv)
+{
+  const u32 lane  = threadIdx.x & 31;
+  const u32 below = (2u << lane) - 2u;  // bits 1..lane
+  for(u32 base = 0; base < total; base += 32)
+  {
+    // lane's part: those starting at or before the step's first vertex, plus
+    // those starting inside the step up to the lane (one bit each)
+    const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && start <= base));
+    const u32 inside = __reduce_or_sync(0xFFFFFFFFu,
+                                        (owner && start > base && start < base + 32) ? 1u << (start - base) : 0u);
+    const u32   pi   = (before - 1 + __popc(inside & below)) & 31;
+    const u32   jj   = min(base + lane, total - 1);
+    const u32   tvi  = __shfl_sync(0xFFFFFFFFu, tvBase, pi) + jj;
+    const u32   vo   = __shfl_sync(0xFFFFFFFFu, dstBase, pi) + jj;
+    const u32   inst = rp.enabled ? __shfl_sync(0xFFFFFFFFu, d.inst, pi) : 0u;
+    const float size = rp.enabled ? __shfl_sync(0xFFFFFFFFu, d.size, pi) : 0.0f;
+    const f3 q = deform_vertex<Kind>(rec.affine[pi], rec.pn[pi], __ldg(c.table.vertices + tvi), pn, inst, size, rp);
+    float*   o = gv + 3 * (u64)vo;
+    o[0] = q.x, o[1] = q.y, o[2] = q.z;
+  }
 }
 
 // The vertices of the warp's parts: lane l < count owns record l (d.nv > 0).
@@ -104,7 +135,6 @@ __device__ __forceinline__ void deform_walk(const StageCtx& c, const DeformRecor
                                             bool pn, const RippleParams& rp, float* gv)
 {
   const u32  lane  = threadIdx.x & 31;
-  const u32  below = (2u << lane) - 2u;  // bits 1..lane
   const bool owner = lane < count;
   u32        incl  = owner ? d.nv : 0u;
 #pragma unroll
@@ -117,26 +147,22 @@ __device__ __forceinline__ void deform_walk(const StageCtx& c, const DeformRecor
   const u32 start  = incl - (owner ? d.nv : 0u);
   const u32 total  = __shfl_sync(0xFFFFFFFFu, incl, 31);
   const u32 tvBase = d.tvFirst - start, dstBase = d.dst - start;
-  for(u32 base = 0; base < total; base += 32)
+  // one specialisation for the parts when they share a map kind
+  const u32 kind  = owner ? affine_kind_of(rec.affine[lane]) : ~0u;
+  const u32 kind0 = __shfl_sync(0xFFFFFFFFu, kind, 0);
+  const u32 kw    = __all_sync(0xFFFFFFFFu, !owner || kind == kind0) ? kind0 : ~0u;
+#define TC_DEFORM(K) deform_steps<K>(c, rec, owner, start, total, tvBase, dstBase, d, pn, rp, gv)
+  switch(kw)
   {
-    // lane's part: those starting at or before the step's first vertex, plus
-    // those starting inside the step up to the lane (one bit each)
-    const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, owner && start <= base));
-    const u32 inside = __reduce_or_sync(0xFFFFFFFFu,
-                                        (owner && start > base && start < base + 32) ? 1u << (start - base) : 0u);
-    const u32   pi   = (before - 1 + __popc(inside & below)) & 31;
-    const u32   jj   = base + lane;
-    const u32   tvi  = __shfl_sync(0xFFFFFFFFu, tvBase, pi) + jj;
-    const u32   vo   = __shfl_sync(0xFFFFFFFFu, dstBase, pi) + jj;
-    const u32   inst = __shfl_sync(0xFFFFFFFFu, d.inst, pi);
-    const float size = __shfl_sync(0xFFFFFFFFu, d.size, pi);
-    if(jj < total)
-    {
-      const f3 q = deform_vertex(rec.affine[pi], rec.pn[pi], __ldg(c.table.vertices + tvi), pn, inst, size, rp);
-      float*   o = gv + 3 * (u64)vo;
-      o[0] = q.x, o[1] = q.y, o[2] = q.z;
-    }
+    case affine_kind(TC_TEXEL_F16, true): TC_DEFORM(affine_kind(TC_TEXEL_F16, true)); break;
+    case affine_kind(TC_TEXEL_F32, true): TC_DEFORM(affine_kind(TC_TEXEL_F32, true)); break;
+    case affine_kind(TC_TEXEL_UNORM16, true): TC_DEFORM(affine_kind(TC_TEXEL_UNORM16, true)); break;
+    case affine_kind(TC_TEXEL_F16, false): TC_DEFORM(affine_kind(TC_TEXEL_F16, false)); break;
+    case affine_kind(TC_TEXEL_F32, false): TC_DEFORM(affine_kind(TC_TEXEL_F32, false)); break;
+    case affine_kind(TC_TEXEL_UNORM16, false): TC_DEFORM(affine_kind(TC_TEXEL_UNORM16, false)); break;
+    default: TC_DEFORM(~0u); break;
   }
+#undef TC_DEFORM
 }
 
 }  // namespace tc

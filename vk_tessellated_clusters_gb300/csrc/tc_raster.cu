@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_raster_write(StageCtx c, con
           if(jj < vFit)
           {
             const u32 tv = __ldg(c.table.vertices + (tvIdx + jj));
-            const f3  p  = Deform ? deform_vertex(sp[pi], s_pn[Deform ? warp : 0][Deform ? pi : 0], tv, pn, vInst, vSize, rp)
+            const f3  p  = Deform ? deform_vertex<~0u>(sp[pi], s_pn[Deform ? warp : 0][Deform ? pi : 0], tv, pn, vInst, vSize, rp)
                                 : affine_vertex_k<kKind>(sp[pi], tv);
             const float4 mx = s_world[warp][pi][0], my = s_world[warp][pi][1], mz = s_world[warp][pi][2];
             const f3     wp = {((mx.x * p.x + mx.y * p.y) + mx.z * p.z) + mx.w, ((my.x * p.x + my.y * p.y) + my.z * p.z) + my.w,

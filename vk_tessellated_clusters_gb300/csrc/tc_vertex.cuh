@@ -482,10 +482,11 @@ __device__ __forceinline__ f3 part_pn_position(const PartPn& r, u32 tableVertex)
 }
 
 // Displacement of the part in `r` at table vertex `tableVertex` added to `P`
-// (its map, scale and offset from the record).
+// (its map, scale and offset from the record; Kind ~0u: of any kind).
+template <u32 Kind>
 __device__ __forceinline__ f3 affine_displace(const PartAffine& r, u32 tableVertex, f3 P)
 {
-  const u32 kind = affine_kind_of(r);
+  const u32 kind = Kind == ~0u ? affine_kind_of(r) : Kind;
   if(kind == kAffineFlat)
     return P;
   const float  a  = __uint2float_rn(tableVertex & 0xFFFFu) * (1.0f / 32768.0f);
