@@ -63,6 +63,8 @@ class FrozenFrame:
         sizes += [t.numel() if t is not None else 0 for t in self.texels]
         starts = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
         self._grad_floats = int(starts[-1])
+        # parameters without an element (an empty map): gradients() gives their gradients the shape
+        self._empty = [(i, p.shape) for i, p in enumerate(self.parameters()) if p.numel() == 0]
         ng = len(self.positions)
         rel = np.zeros((len(self._inst_geo), 2), np.int64)
         rel[:, 0] = 4 * starts[self._inst_geo]
@@ -116,7 +118,10 @@ class FrozenFrame:
         on the current stream, no synchronisation."""
         flat = self.torch.empty(self._grad_floats, dtype=self.torch.float32, device=self.device).zero_()
         self.launch_backward(grad_vertices.contiguous().float(), self._pointer_table(flat))
-        return self.torch._utils._unflatten_dense_tensors(flat, self.parameters())
+        grads = list(self.torch._utils._unflatten_dense_tensors(flat, self.parameters()))
+        for i, shape in self._empty:  # (given back as vectors of length 0 by some versions)
+            grads[i] = grads[i].view(shape)
+        return grads
 
     def scatter_gradients(self, grad_vertices):
         """dL/dv -> (dPositions, dNormals, dTexels), lists parallel to the
