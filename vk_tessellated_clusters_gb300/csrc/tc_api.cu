@@ -234,7 +234,7 @@ Plan make_plan(const tc_context_desc& d)
   off                 = align_up(off + (size_t)std::max(1u, k.maxSplitTriangles) * 36, 256);
   // the children of a split level's items (at most 121 each, tiles of 128 or more)
   p.splitEndsOffset   = off;
-  off                 = align_up(off + (size_t)std::max(1u, k.maxSplitTriangles) * 4, 256);
+  off                 = align_up(off + (size_t)std::max(1u, k.maxSplitTriangles) * 8, 256);
   p.splitFirstOffset  = off;
   p.splitFirstStride  = (size_t)ceil_div((u64)k.maxSplitTriangles * TC_TESSTABLE_SIZE * TC_TESSTABLE_SIZE, 128) + 1;
   off                 = align_up(off + p.splitFirstStride * 3 * 4, 256);
@@ -300,7 +300,7 @@ StageCtx base_ctx(tc_context* ctx, const tc_frame_args* a)
   c.runStarts               = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.runOffset);
   c.instClusterStart        = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.instOffset);
   c.splitBase               = reinterpret_cast<float*>(ctx->dScratch + ctx->plan.splitBaseOffset);
-  c.splitEnds               = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.splitEndsOffset);
+  c.splitEnds               = reinterpret_cast<u64*>(ctx->dScratch + ctx->plan.splitEndsOffset);
   c.splitFirst              = reinterpret_cast<u32*>(ctx->dScratch + ctx->plan.splitFirstOffset);
   c.splitFirstStride        = ctx->plan.splitFirstStride;
   c.instBegin               = 0;

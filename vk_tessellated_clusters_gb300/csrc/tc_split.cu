@@ -151,7 +151,7 @@ __device__ __forceinline__ u32 child_places(const StageCtx& c, u32 cfg)
 struct Level
 {
   u32        begin, end;
-  u32        total;  // child places of all items
+  u64        total;  // child places of all items (past 2^32 from 35.5 M items of 121 on)
   u32        tiles;  // of `chunks` x B child places each
   u32        chunks;
   const u32* first;  // per B child places: the item the first belongs to (null: level not known yet)
@@ -160,13 +160,12 @@ struct Level
 // Tiles of B child places; several (up to 16) only where the look-back rows
 // hold fewer tiles than that (stride: one per kSplitRowItems items of the capacity).
 template <int B>
-__device__ __forceinline__ Level make_level(u32 begin, u32 end, u32 total, const u32* first, u32 stride)
+__device__ __forceinline__ Level make_level(u32 begin, u32 end, u64 total, const u32* first, u32 stride)
 {
-  const u32 most = (u32)min((u64)(end - begin) * kMaxChildrenPerItem, 0xFFFFFFFFull - B);
-  Level lv     = {begin, end, min(total, most), 0u, 1u, first};
-  const u32 n  = (lv.total + B - 1) / B;
-  lv.chunks    = max(1u, (n + stride - 1) / stride);
-  lv.tiles     = (n + lv.chunks - 1) / lv.chunks;
+  Level     lv = {begin, end, min(total, (u64)(end - begin) * kMaxChildrenPerItem), 0u, 1u, first};
+  const u64 n  = (lv.total + B - 1) / B;
+  lv.chunks    = max(1u, (u32)((n + stride - 1) / stride));
+  lv.tiles     = (u32)((n + lv.chunks - 1) / lv.chunks);
   return lv;
 }
 
@@ -184,17 +183,18 @@ struct SplitShared
   int       end[B];                  // per item: its last child place + 1, relative to the chunk's first
   u32       cnt[kCntKids + 1][kSlots];  // per (chunk, warp): count, then exclusive offset within the tile
   u64       excl[kCntKids + 1];
+  u64       total;
   u32       scan[33];
-  u32       tile, flag, range[2], total;
+  u32       tile, flag, range[2];
 };
 
 // An item's entry in its level's index: its running child count and, where
 // every B-th child is its own, the item's place in `first`.
 template <int B>
-__device__ __forceinline__ void index_item(const StageCtx& c, u32* first, u32 item, u32 start, u32 places)
+__device__ __forceinline__ void index_item(const StageCtx& c, u32* first, u32 item, u64 start, u32 places)
 {
   c.splitEnds[item] = start + places;
-  const u32 g       = (start + B - 1) / B;
+  const u64 g       = (start + B - 1) / B;
   if(g * B < start + places && g < c.splitFirstStride)
     first[g] = item;
 }
@@ -202,10 +202,10 @@ __device__ __forceinline__ void index_item(const StageCtx& c, u32* first, u32 it
 // Items [begin, end)'s index from their configs, by this block alone: B items
 // at a time. Returns the level's child places.
 template <int B>
-__device__ u32 index_local(const StageCtx& c, SplitShared<B>& sm, u32 begin, u32 end)
+__device__ u64 index_local(const StageCtx& c, SplitShared<B>& sm, u32 begin, u32 end)
 {
   const tc_TessTriangleInfo* queue = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->splitTriangles);
-  u32                        base  = 0;
+  u64                        base  = 0;
   for(u32 i0 = begin; i0 < end; i0 += B)
   {
     const u32 item = i0 + threadIdx.x;
@@ -237,7 +237,7 @@ __device__ void index_tile(const StageCtx& c, SplitShared<B>& sm, u64* row, u32 
   }
   __syncthreads();
   if(n)
-    index_item<B>(c, c.splitFirst, item, (u32)sm.excl[0] + excl, n);
+    index_item<B>(c, c.splitFirst, item, sm.excl[0] + excl, n);
   __syncthreads();
 }
 
@@ -280,7 +280,7 @@ __device__ __forceinline__ Lane chunk_child(const StageCtx& c, SplitShared<B>& s
                                             const FactorParams& fp, u32 sf)
 {
   const tc_TessTriangleInfo* queue = reinterpret_cast<const tc_TessTriangleInfo*>(c.build->splitTriangles);
-  const u32                  from = g * B;
+  const u64                  from = (u64)g * B;
   // the chunk's items: from its first child's to the next chunk's first
   // child's. (Clamped: after a look-back that ran out they may be anything.)
   const u32 a = min(max(__ldcg(lv.first + g), lv.begin), lv.end - 1);
@@ -301,7 +301,7 @@ __device__ __forceinline__ Lane chunk_child(const StageCtx& c, SplitShared<B>& s
     it.vtx[1] = r1.y;
     it.vtx[2] = r2.x;
     it.tc     = r2.y;
-    sm.end[threadIdx.x] = (int)(__ldcg(c.splitEnds + item) - from);
+    sm.end[threadIdx.x] = (int)((long long)__ldcg(c.splitEnds + item) - (long long)from);
     const float* sb     = c.splitBase + 9 * (u64)item;
 #pragma unroll
     for(int v = 0; v < 3; v++)
@@ -351,7 +351,7 @@ __device__ void split_tile(const StageCtx& c, SplitShared<B>& sm, u32 tile, cons
   tc_SceneBuilding*    b     = c.build;
   const tc_caps&       k     = c.caps;
   tc_TessTriangleInfo* queue = reinterpret_cast<tc_TessTriangleInfo*>(b->splitTriangles);
-  const u32            g0 = tile * lv.chunks, chunks = min(lv.chunks, (lv.total + B - 1) / B - g0);
+  const u32            g0 = tile * lv.chunks, chunks = min(lv.chunks, (u32)((lv.total + B - 1) / B) - g0);
 
   // ---- classify; every warp counts its own slots ----------------------------
   Lane l;
@@ -443,7 +443,7 @@ __device__ void split_tile(const StageCtx& c, SplitShared<B>& sm, u32 tile, cons
         for(int v = 0; v < 3; v++)
           d[3 * v] = item.bp[v].x, d[3 * v + 1] = item.bp[v].y, d[3 * v + 2] = item.bp[v].z;
         if(next)
-          index_item<B>(c, next, (u32)o, (u32)sm.excl[kCntKids] + sm.cnt[kCntKids][ch * kW + warp] + before,
+          index_item<B>(c, next, (u32)o, sm.excl[kCntKids] + sm.cnt[kCntKids][ch * kW + warp] + before,
                         places);
       }
     }
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
     if(idxTiles && lv.first == nullptr)
     {
       if(threadIdx.x == 0)
-        sm.total = wait_flag(c, indexed + 1) ? __ldcg(c.splitEnds + end - 1) : 0u;
+        sm.total = wait_flag(c, indexed + 1) ? __ldcg(c.splitEnds + end - 1) : 0ull;
       __syncthreads();
       lv = make_level<B>(begin, end, sm.total, c.splitFirst, c.scratch.lbStride);
     }
@@ -595,13 +595,15 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
 
 // Per-level control words, in the level's scratch slot (zeroed with the
 // frame): [1] tiles done, [2..] u64 totals (split, part), [6] / [7] the split
-// and part counters before the level, [10] the level's child places, [11] next
-// level's range published, [12] finalised, [13] start, [14] end. Level 0's [0]
-// is the ticket all levels share, its [8] counts index tiles, its [9] is set
-// with the index complete, and its [15] before the set-ups are written.
+// and part counters before the level, [8] u64 the level's child places (not of
+// level 0), [11] next level's range published, [12] finalised, [13] start, [14]
+// end. Level 0's [0] is the ticket all levels share, its [8] counts index tiles,
+// its [9] is set with the index complete, and its [15] before the set-ups are
+// written.
 __device__ __forceinline__ u32* lv_done(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 1; }
 __device__ __forceinline__ u64* lv_totals(const SplitLevels& lv, u32 L) { return reinterpret_cast<u64*>(lv.ctrl[L] + 2); }
 __device__ __forceinline__ u32* lv_bases(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 6; }
+__device__ __forceinline__ u64* lv_places(const SplitLevels& lv, u32 L) { return reinterpret_cast<u64*>(lv.ctrl[L] + 8); }
 __device__ __forceinline__ u32* lv_ready(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 11; }
 __device__ __forceinline__ u32* lv_final(const SplitLevels& lv, u32 L) { return lv.ctrl[L] + 12; }
 
@@ -681,7 +683,7 @@ __device__ void publish_level(const StageCtx& c, const SplitLevels& lv, u32 L, u
   u32* next = lv.ctrl[L + 1];
   next[6 + kCntSplit] = write, next[6 + kCntPart] = part;
   const u32 first = min(end, most), last = min(write, most);
-  next[10] = last > first ? __ldcg(c.splitEnds + last - 1) : 0u;
+  *lv_places(lv, L + 1) = last > first ? __ldcg(c.splitEnds + last - 1) : 0ull;
   next[13] = first, next[14] = last;
   __threadfence();
   st_release_u32(lv_ready(lv, L), 1u);
@@ -771,7 +773,7 @@ __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLe
         }
         const u32* w = lv.ctrl[level];
         const u32  lo = __ldcg(w + 13), hi = __ldcg(w + 14);
-        cur = make_level<B>(lo, hi, __ldcg(w + 10), c.splitFirst + c.splitFirstStride * (1 + (level & 1)), lv.stride);
+        cur = make_level<B>(lo, hi, __ldcg(lv_places(lv, level)), c.splitFirst + c.splitFirstStride * (1 + (level & 1)), lv.stride);
       }
       s_lv       = cur;
       s_level[0] = level, s_level[1] = first, s_level[2] = stop;

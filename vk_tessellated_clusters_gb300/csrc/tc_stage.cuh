@@ -115,7 +115,7 @@ struct StageCtx
   u32*                          runStarts;         // [kRunStartsSize]: part counter at each run start, the full-cluster count, full attempts
   u32*                          instClusterStart;  // [numInstances + 1] exclusive prefix of numClusters
   float*                        splitBase;         // [maxSplitTriangles][9]: world positions of each split item's base triangle
-  u32*                          splitEnds;         // [maxSplitTriangles]: per split item its level's running child count
+  u64*                          splitEnds;         // [maxSplitTriangles]: per split item its level's running child count
   u32*                          splitFirst;        // [3][splitFirstStride]: per tile of children its first item (level 0; odd, even levels)
   u64                           splitFirstStride;
   LaunchScratch                 scratch;
