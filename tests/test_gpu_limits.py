@@ -51,3 +51,94 @@ def test_level_of_more_than_2_to_the_32_children():
     # every pass in one launch: the later levels only add split items
     got = _first_level(mesh, n, 59000000, True)
     assert got[0] == n * items and got[1] >= n * splits
+
+
+def _many(instances, apart, seed=3):
+    """Small meshes in many places; each instance with a key of its own (apart) or one of six."""
+    rng = np.random.default_rng(seed)
+    meshes = [S.clusterize(S.icosphere(3), 0), S.clusterize(S.torus(1.0, 0.3, 64, 16), 1)]
+    insts = []
+    for i in range(instances):
+        world = S.translate_rotate_scale(rng.random(3) * 40.0, S.random_unit_quaternion(rng), 0.5 + rng.random())
+        offset = 0.0001 * (i + 1) if apart else 0.01 * (i % 3)
+        insts.append(S.Instance(i % 2, world, i % 2, 0.03, offset))
+    textures = [S.Texture(rng.random((37, 53), np.float32), L.TEXEL_F32) for _ in range(2)]
+    return S.Scene("many", meshes, insts, textures)
+
+
+# the instances one round of the grouping block takes (1,024, also the most whose first clusters classify keeps in
+# shared memory), one more, the most that are grouped, one more
+@pytest.mark.parametrize("instances", [1024, 1025, 4096, 4097])
+@pytest.mark.parametrize("apart", [False, True])
+def test_groups_of_many_instances(oracle, instances, apart):
+    """Integers bit-exact against the oracle and positions to the vertex tolerance, from the graph, the direct launches
+    and the graph with its host traffic; the same bytes from all."""
+    import torch
+    from tests.parity import assert_same, vertex_tolerance
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = _many(instances, apart)
+    assert sc.total_clusters >= 16384
+    caps = L.default_caps(part_bits=19, vertex_bits=23)
+    fc = S.frame_constants(S.camera_orbit(5, tess_rate_pixels=6.0))
+    ref_state, _ = oracle.frame(sc, fc, caps, FLAGS)
+    want = ref_state.outputs(oracle.entries)
+    assert len(want["partTriangles"]) > 0 and len(want["fullClusters"]) > 16384 // 2
+    pipe = TessellationPipeline(sc, caps, FLAGS)
+    pipe.set_cameras(fc)
+    block = np.concatenate([np.frombuffer(fc.tobytes(), np.uint8), np.frombuffer(fc.tobytes(), np.uint8),
+                            pipe.state.res.instance_records.view(np.uint8).reshape(-1)])
+    host = torch.empty(block.size, dtype=torch.uint8, pin_memory=True)
+    host.numpy()[:] = block
+    readback = torch.zeros(L.Readback.itemsize, dtype=torch.uint8, pin_memory=True)
+    device = torch.zeros(block.size, dtype=torch.uint8, device="cuda")
+    first = None
+    for mode in ("graph", "batched", "host"):
+        pipe.state.gen_vertices.handle.zero_()
+        if mode == "host":
+            a = pipe.args
+            a.view, a.viewLast = device.data_ptr(), device.data_ptr() + fc.nbytes
+            a.instances = device.data_ptr() + 2 * fc.nbytes
+            pipe.build_host(host.data_ptr(), device.data_ptr(), block.size, readback.data_ptr())
+        else:
+            pipe.build(mode)
+        got = pipe.outputs()
+        assert_same(got, want, mode, vertex_tol=vertex_tolerance(sc))
+        first = first or got
+        assert got["genVertices"].tobytes() == first["genVertices"].tobytes()
+    assert readback.numpy().tobytes() == got["readback"].tobytes()
+    assert pipe.device_errors() == 0
+    pipe.close()
+
+
+# the most instances whose full clusters the adjoint takes by groups, and one more
+@pytest.mark.parametrize("instances", [1024, 1025])
+@pytest.mark.parametrize("apart", [False, True])
+def test_adjoint_of_many_instances(oracle, instances, apart):
+    """Each gradient against the FP64 adjoint: relative error of its norm within 1e-4, as for fewer instances."""
+    import ctypes
+    import torch
+    from oracle.binding import lib as olib
+    from vk_tessellated_clusters_gb300.autograd import FrozenFrame
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = _many(instances, apart)
+    assert sc.total_clusters >= 12288
+    caps = L.default_caps(part_bits=18, vertex_bits=23)
+    cam = S.camera_orbit(5, tess_rate_pixels=6.0)
+    pipe = TessellationPipeline(sc, caps, FLAGS)
+    pipe.set_cameras(cam)
+    pipe.build("graph")
+    frozen = FrozenFrame(pipe)
+    g = np.random.default_rng(1).normal(0, 1, (frozen.num_vertices, 3)).astype(np.float32)
+    dP, dN, dT = frozen.scatter_gradients(torch.from_numpy(g).cuda())
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    want = [[np.zeros(tuple(x.shape)) for x in xs] for xs in (dP, dN, dT)]
+    mesh = [i.geometry for i in sc.instances]
+    ptr = lambda a: (ctypes.c_void_p * len(a))(*[x.ctypes.data for x in a])
+    g64 = g.astype(np.float64)
+    olib().tco_backward_f64(ctypes.byref(oracle.table), ctypes.byref(ref_state.args), g64.ctypes.data,
+                            ptr([want[0][m] for m in mesh]), ptr([want[1][m] for m in mesh]), ptr(want[2]))
+    for got, ref in zip([*dP, *dN, *dT], [*want[0], *want[1], *want[2]]):
+        part, norm = got.double().cpu().numpy(), np.linalg.norm(ref)
+        assert norm > 0 and np.linalg.norm(part - ref) <= 1e-4 * norm, np.linalg.norm(part - ref) / norm
+    assert pipe.device_errors() == 0
+    pipe.close()

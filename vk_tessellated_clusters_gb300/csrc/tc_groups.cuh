@@ -2,38 +2,16 @@
 // offset, grouped by one block of the batched frame's first kernel.
 #pragma once
 
+#include "tc_group_key.h"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
 
 namespace tc {
 
-// what the vertices of an instance's full clusters depend on
-struct GroupKey
-{
-  u64   positions, normals, texcoords, clusters, localTriangles;
-  int   map;
-  float scale, offset;
-  u32   numClusters;
-};
-
 __device__ __forceinline__ GroupKey group_key(const tc_RenderInstance& in)
 {
-  return {in.positions, in.normals, in.texcoords, in.clusters, in.clusterLocalTriangles, in.displacementIndex, in.displacementScale,
-          in.displacementOffset, in.numClusters};
-}
-
-__device__ __forceinline__ bool same_key(const GroupKey& a, const GroupKey& b)
-{
-  return a.positions == b.positions && a.normals == b.normals && a.texcoords == b.texcoords && a.clusters == b.clusters
-         && a.localTriangles == b.localTriangles && a.map == b.map && __float_as_uint(a.scale) == __float_as_uint(b.scale)
-         && __float_as_uint(a.offset) == __float_as_uint(b.offset) && a.numClusters == b.numClusters;
-}
-
-// Fibonacci hashing: the high bits of a multiple of 2^64 / golden ratio
-__device__ __forceinline__ u64 group_hash(const GroupKey& k)
-{
-  return (k.positions ^ (k.clusters << 1) ^ ((u64)(u32)k.map << 40) ^ ((u64)__float_as_uint(k.scale) << 8))
-         * 0x9E3779B97F4A7C15ull;
+  return {in.positions, in.normals, in.texcoords, in.clusters, in.clusterLocalTriangles, (u32)in.displacementIndex, in.numClusters,
+          __float_as_uint(in.displacementScale), __float_as_uint(in.displacementOffset)};
 }
 
 // One block groups the frame's instances by key (a hash table of their indices
@@ -43,13 +21,16 @@ __device__ __forceinline__ u64 group_hash(const GroupKey& k)
 // instances (a block of their launch; as a kernel of its own it would be a
 // second root of the frame's graph, which starts 10 us late). With the records
 // in host memory every access is a round trip over the host link: a thread
-// loads the keys of four instances at once. Grouping is left out (kHeadGrouped 0)
+// loads the keys of four instances at once, and a probe compares 16 bits of the
+// hash in shared memory before it reads a record. Grouping is left out (kHeadGrouped 0)
 // when instances have fewer than two in a group on average.
-constexpr u32 kGroupTable = 2 * kGroupInstances;
+constexpr u32 kGroupTable = 1u << kGroupTableBits;
+static_assert(kGroupTable == 2 * kGroupInstances, "the table is at most half full");
 
 __device__ inline void find_groups(const StageCtx& c, const GroupTables& g)
 {
   __shared__ unsigned short s_table[kGroupTable];
+  __shared__ unsigned short s_print[kGroupInstances];
   __shared__ u32            s_count[kGroupInstances], s_scan[33];
   constexpr unsigned short  kEmpty = 0xFFFF;
   const u32                 n      = min(c.numInstances, min(g.cap, kGroupInstances));
@@ -73,14 +54,18 @@ __device__ inline void find_groups(const StageCtx& c, const GroupTables& g)
       const u32 i = base + q * blockDim.x;
       if(i >= n)
         continue;
+      const u64            hash  = group_hash(key[q]);
+      const unsigned short print = group_print(hash);
+      s_print[i]                 = print;
+      __threadfence_block();  // (before the instance is seen in the table)
       u32 rep = ~0u;
-      for(u32 slot = (u32)(group_hash(key[q]) >> 40) % kGroupTable; rep == ~0u; slot = (slot + 1) % kGroupTable)
+      for(u32 slot = group_slot(hash); rep == ~0u; slot = (slot + 1) % kGroupTable)
       {
         // (the table has twice as many slots as instances)
         const unsigned short found = atomicCAS(&s_table[slot], kEmpty, (unsigned short)i);
         if(found == kEmpty)
           rep = i;
-        else if(same_key(key[q], group_key(c.instances[found])))
+        else if(*(volatile unsigned short*)&s_print[found] == print && same_key(key[q], group_key(c.instances[found])))
           rep = found;
       }
       place[i]        = rep | atomicAdd(&s_count[rep], 1u) << 16;
