@@ -544,29 +544,37 @@ __device__ __forceinline__ void add_full_sums(RangeSums& rs, u32 clusters, u32 v
     atomicAdd(&rs.data, (unsigned long long)data);
 }
 
+// the visible clusters' counter and set-up when every cluster is visible
+__device__ __forceinline__ void visible_set_up(const StageCtx& c)
+{
+  c.build->visibleClusterCounter = c.instClusterStart[c.numInstances];
+  build_setup_apply(c, TC_BUILD_SETUP_CLASSIFY);
+}
+
 // With bounds: one thread per visible cluster writes the visible list (RT
 // semantics: every cluster in instance order, clusters_cull.comp.glsl:112-161,
-// and its set-up; the list is written here also when the frame turns out to
-// have no bounds) and counts the clusters that are full
+// and its set-up) and counts the clusters that are full
 // clusters for certain, without their vertices (of an invisible instance, or
 // too small for their distance by their bounds), and lists the others for
 // k_classify_count. Neighbouring threads take neighbouring clusters, so the
 // instance's matrix is one broadcast load and a warp adds to its range's sums
 // once. Measured on a GB300, 207,360 clusters of 1,024 instances, 10,700 of
 // them listed: the count 88 -> 24 us (bounds 4, this 8, the listed clusters 12),
-// the frame 233 -> 162 us.
+// the frame 233 -> 162 us. A frame that turns out to have no bounds leaves
+// everything to k_classify_count, whose lanes then write the list: written here,
+// in front of the count, it costs 2.5 us of 262 with 1,000 instances that share
+// nothing and 1.6 of 93 with 256 (by clusters_cull on a side stream 17 and 4: its
+// blocks are placed before this kernel's).
 template <bool Trans>
 __global__ void __launch_bounds__(kBlock) k_classify_whole(StageCtx c, ClassifyScratch cs)
 {
   stage_prologue();
   __shared__ FlatStarts s_starts;
-  const u32*         starts  = stage_flat_starts(c, s_starts);
-  const bool         bounded = cs.groupHead[kHeadBounds] != 0;
+  if(cs.groupHead[kHeadBounds] == 0)
+    return;
+  const u32* starts = stage_flat_starts(c, s_starts);
   if(blockIdx.x == 0 && threadIdx.x == 0)
-  {
-    c.build->visibleClusterCounter = c.instClusterStart[c.numInstances];
-    build_setup_apply(c, TC_BUILD_SETUP_CLASSIFY);
-  }
+    visible_set_up(c);
   tc_ClusterInfo*    vis     = reinterpret_cast<tc_ClusterInfo*>(c.build->visibleClusters);
   const u32          n       = min(min(c.instClusterStart[c.numInstances], c.caps.maxVisibleClusters), c.scratch.itemCapacity);
   const u32          lane    = threadIdx.x & 31;
@@ -586,22 +594,17 @@ __global__ void __launch_bounds__(kBlock) k_classify_whole(StageCtx c, ClassifyS
       const tc_ClusterInfo     ci = flat_cluster(starts, c.numInstances, v);
       const tc_RenderInstance* in = c.instances + ci.instanceID;
       reinterpret_cast<uint2*>(vis)[v] = make_uint2(ci.instanceID, ci.clusterID);
-      if(bounded)
-      {
-        const tc_Cluster cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
-        nt = cl.numTriangles, nv = cl.numVertices;
-        data = __ldg(reinterpret_cast<const u32*>(in->clusterTemplateInstantiatonSizes) + ci.clusterID);
-        const float4* bd = cs.bounds + 2 * (u64)(cs.instBounds[ci.instanceID] + ci.clusterID);
-        // (a malformed cluster is k_classify_count's to report)
-        whole = nt <= TC_MAX_CLUSTER_TRIANGLES && nv <= TC_MAX_CLUSTER_VERTICES
-                && ((culling && (states[ci.instanceID] & TC_INSTANCE_VISIBLE_BIT) == 0)
-                    || bounds_factor_one(in->worldMatrix.m, bd[0], bd[1], fp, kRate));
-        if(whole)
-          store_full_counts<Trans>(cs, v, nv, nt, data);
-      }
+      const tc_Cluster cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
+      nt = cl.numTriangles, nv = cl.numVertices;
+      data = __ldg(reinterpret_cast<const u32*>(in->clusterTemplateInstantiatonSizes) + ci.clusterID);
+      const float4* bd = cs.bounds + 2 * (u64)(cs.instBounds[ci.instanceID] + ci.clusterID);
+      // (a malformed cluster is k_classify_count's to report)
+      whole = nt <= TC_MAX_CLUSTER_TRIANGLES && nv <= TC_MAX_CLUSTER_VERTICES
+              && ((culling && (states[ci.instanceID] & TC_INSTANCE_VISIBLE_BIT) == 0)
+                  || bounds_factor_one(in->worldMatrix.m, bd[0], bd[1], fp, kRate));
+      if(whole)
+        store_full_counts<Trans>(cs, v, nv, nt, data);
     }
-    if(!bounded)
-      continue;
     const u32 wm = __ballot_sync(0xFFFFFFFFu, whole), om = __ballot_sync(0xFFFFFFFFu, v < n && !whole);
     // the warp's range (two where one ends inside it)
     for(u32 left = wm; left;)
@@ -684,6 +687,9 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_count(StageCtx c
   const bool bounded = cs.groups != nullptr && cs.groupHead[kHeadBounds] != 0;
   const u32* list    = reinterpret_cast<const u32*>(cs.transRecs);
   const u32  items   = bounded ? cs.groupHead[kHeadList] : n;
+  const bool write   = cs.groups != nullptr && !bounded;  // the visible list
+  if(write && blockIdx.x == 0 && threadIdx.x == 0)
+    visible_set_up(c);
   const u32  cntW   = gw < items ? (items - gw + nwarps - 1) / nwarps : 0u;
   const u32* states = reinterpret_cast<const u32*>(b->instanceStates);
   for(u32 j0 = 0; j0 < cntW; j0 += 32)
@@ -699,6 +705,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_count(StageCtx c
       const tc_RenderInstance* in = c.instances + ci.instanceID;
       const tc_Cluster         cl = reinterpret_cast<const tc_Cluster*>(in->clusters)[ci.clusterID];
       u32                      nt = cl.numTriangles, nv = cl.numVertices;
+      if(write)
+        reinterpret_cast<uint2*>(c.build->visibleClusters)[v] = make_uint2(ci.instanceID, ci.clusterID);
       if(nt > TC_MAX_CLUSTER_TRIANGLES || nv > TC_MAX_CLUSTER_VERTICES)
       {
         atomicOr(c.errorWord, TC_DEVERR_BAD_CLUSTER);
