@@ -414,6 +414,12 @@ __device__ __forceinline__ void count_transient(const StageCtx& c, const Classif
 // bounds of the clusters of instance groups (tc_groups.cuh)
 // ---------------------------------------------------------------------------
 
+// The smallest normal float, added to the squares whose roots bound a length
+// from above: squares of less underflow, by at most 2^-149 for each product. (A
+// mesh of 1e-23 units under a scale of 1e18 had bounds of zero, and its clusters
+// were accepted wherever they lay. A scale whose square overflows fails the test.)
+constexpr float kBoundsTiny = 1.17549435e-38f;
+
 // Object-space bounds of the groups' clusters, one warp each: a sphere around
 // the vertices and the longest triangle edge, both rounded up. They let the
 // count kernel accept a whole cluster of an instance without its vertices
@@ -497,8 +503,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_cluster_bounds(StageCtx c, GroupT
     bad = __any_sync(0xFFFFFFFFu, bad);
     if(lane == 0)
     {
-      // (1e-5 covers the roundings of the differences, dot products and roots)
-      const float r = __fsqrt_rn(r2) * (1.0f + 1e-5f), e = __fsqrt_rn(e2) * (1.0f + 1e-5f);
+      // (1e-5 covers the roundings of the differences, dot products and roots,
+      // kBoundsTiny squares that underflow)
+      const float r = __fsqrt_rn(r2 + kBoundsTiny) * (1.0f + 1e-5f), e = __fsqrt_rn(e2 + kBoundsTiny) * (1.0f + 1e-5f);
       g.bounds[2 * (u64)u]     = make_float4(mid.x, mid.y, mid.z, r);
       g.bounds[2 * (u64)u + 1] = make_float4(bad ? inf : e, (len3(mid) + r) * (1.0f + 1e-5f), 0.0f, 0.0f);
     }
@@ -521,7 +528,7 @@ __device__ __forceinline__ bool bounds_factor_one(const float* m, float4 b0, flo
   const f3    a0 = {m[0], m[1], m[2]}, a1 = {m[4], m[5], m[6]}, a2 = {m[8], m[9], m[10]}, t = {m[12], m[13], m[14]};
   const float g01 = fabsf(dot3(a0, a1)), g02 = fabsf(dot3(a0, a2)), g12 = fabsf(dot3(a1, a2));
   const float s2  = fmaxf(dot3(a0, a0) + g01 + g02, fmaxf(dot3(a1, a1) + g01 + g12, dot3(a2, a2) + g02 + g12));
-  const float s   = __fsqrt_rn(s2) * (1.0f + 1e-5f);
+  const float s   = __fsqrt_rn(s2 + kBoundsTiny) * (1.0f + 1e-5f);
   const float err = 2e-6f * (s * b1.y + len3(t));
   const float d   = dist3(xform_point(m, {b0.x, b0.y, b0.z}), fp.viewPos) - s * b0.w - err;
   return (s * b1.x + err) * kRate < 1.4999f * fmaxf(fp.nearPlane, d * (1.0f - 1e-5f));
