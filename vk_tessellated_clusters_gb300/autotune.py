@@ -5,7 +5,7 @@ grid multipliers of the classify warp kernels and of the instantiate
 allocation, the vertex kernel's register budget, the grid of the
 full-cluster vertex kernel (which runs beside the rest of the frame), the
 split tile size
-(128 threads x 16 items, 256 or 512 threads x 32 items), the split grid, and
+(128, 256 or 512 children, one per thread), the split grid, and
 the frame graph's shape (the first part run allocated beside the split passes,
 or every run after them) and the split passes' form (one launch, or one per
 pass).

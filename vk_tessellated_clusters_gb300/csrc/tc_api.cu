@@ -26,8 +26,8 @@ struct SlotPlan
   size_t ctrlOffset;  // ticket, done (u32 x2) + totals (u64 x kMaxCounters)
 };
 
-constexpr size_t kCtrlBytes = 64;  // ticket, done, totals (u64 x kMaxCounters), then the split levels' words
-static_assert(8 + 8 * kMaxCounters <= 48, "the split levels' control words start at byte 48");
+constexpr size_t kCtrlBytes = 64;  // ticket, done, totals (u64 x kMaxCounters); a split slot's words by tc_split.cu
+static_assert(8 + 8 * kMaxCounters <= kCtrlBytes && 4 * kSplitCtrlWords <= kCtrlBytes, "a slot's control words");
 
 // kernels of a batched frame besides the split launch (every pass in one): frame_begin,
 // frame_begin + instances_classify (one launch), clusters_cull, classify (3),

@@ -205,43 +205,6 @@ __device__ __forceinline__ FactorParams factor_params(const StageCtx& c)
 // scans
 // ---------------------------------------------------------------------------
 
-// block-wide exclusive scan of kNumCounters values per thread
-__device__ inline void block_scan5(u64 (&v)[kNumCounters], u64 (&tot)[kNumCounters], u64 (*s_warp)[kNumCounters])
-{
-  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  u64       inc[kNumCounters];
-#pragma unroll
-  for(int q = 0; q < kNumCounters; q++)
-  {
-    inc[q] = warp_inclusive<u64>(v[q], lane);
-    if(lane == 31)
-      s_warp[warp][q] = inc[q];
-  }
-  __syncthreads();
-  if(warp == 0)
-  {
-#pragma unroll
-    for(int q = 0; q < kNumCounters; q++)
-    {
-      u64 w = lane < nw ? s_warp[lane][q] : 0;
-      u64 s = warp_inclusive<u64>(w, lane);
-      __syncwarp();
-      if(lane < nw)
-        s_warp[lane][q] = s - w;
-      if(lane == 31)
-        s_warp[32][q] = s;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for(int q = 0; q < kNumCounters; q++)
-  {
-    tot[q] = s_warp[32][q];
-    v[q]   = s_warp[warp][q] + inc[q] - v[q];
-  }
-  __syncthreads();
-}
-
 // block-wide exclusive scan of N values per thread (totals in tot)
 template <int N>
 __device__ inline void block_scan_n(u64 (&v)[N], u64 (&tot)[N], u64 (*s_warp)[N])
@@ -300,7 +263,7 @@ __device__ inline void block_prefix(const ClassifyScratch& cs, u64 (&pre)[kNumCo
     x[kCntData] += o.data;
   }
   u64 tot[kNumCounters];
-  block_scan5(x, tot, s_warp);
+  block_scan_n<kNumCounters>(x, tot, s_warp);
   const ClusterOffsets b0 = *cs.bases;
   pre[kCntParts]          = b0.part + tot[kCntParts];
   pre[kCntSplits]         = b0.split + tot[kCntSplits];
@@ -929,8 +892,6 @@ __device__ __forceinline__ void emit_cluster(const StageCtx& c, const tc_Cluster
     if(o >= k.maxSplitTriangles)
       return;
     emit_triangle(splits + o, ci, tri, w);
-    if(!c.splitBase)
-      return;
     const uint8_t* lt  = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
     const float*   pos = reinterpret_cast<const float*>(in->positions);
     float*         d   = c.splitBase + 9 * o;
@@ -1005,7 +966,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_classify_write(StageCtx c
         s_ci[threadIdx.x] = visible_cluster(c, starts, vis, begin + c0 + threadIdx.x);
       u64 x[kNumCounters] = {cnt_parts(r), cnt_splits(r), cnt_full(r), cnt_verts(r), r.y};
       u64 tot[kNumCounters];
-      block_scan5(x, tot, s_warp);
+      block_scan_n<kNumCounters>(x, tot, s_warp);
       s_cnt[threadIdx.x] = r;
       s_off[threadIdx.x] = {(u32)(pre[kCntParts] + x[kCntParts]), (u32)(pre[kCntSplits] + x[kCntSplits]),
                             (u32)(pre[kCntGen] + x[kCntGen]), (u32)(pre[kCntVerts] + x[kCntVerts]),
@@ -1358,21 +1319,18 @@ __device__ inline void write_cluster_transient(const StageCtx& c, const Classify
       if(so < k.maxSplitTriangles)
       {
         emit_triangle(splits + so, ci, tri, word);
-        if(c.splitBase)
+        const uint8_t* lt  = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
+        const float*   pos = reinterpret_cast<const float*>(in->positions);
+        float          m[16];
+#pragma unroll
+        for(int j = 0; j < 16; j++)
+          m[j] = __ldg(in->worldMatrix.m + j);
+        float* dd = c.splitBase + 9 * so;
+#pragma unroll
+        for(int vv = 0; vv < 3; vv++)
         {
-          const uint8_t* lt  = reinterpret_cast<const uint8_t*>(in->clusterLocalTriangles) + cl.firstLocalTriangle;
-          const float*   pos = reinterpret_cast<const float*>(in->positions);
-          float          m[16];
-#pragma unroll
-          for(int j = 0; j < 16; j++)
-            m[j] = __ldg(in->worldMatrix.m + j);
-          float* dd = c.splitBase + 9 * so;
-#pragma unroll
-          for(int vv = 0; vv < 3; vv++)
-          {
-            const f3 wp = xform_point(m, ldg3(pos, cl.firstLocalVertex + lt[tri * 3 + vv]));
-            dd[3 * vv + 0] = wp.x, dd[3 * vv + 1] = wp.y, dd[3 * vv + 2] = wp.z;
-          }
+          const f3 wp = xform_point(m, ldg3(pos, cl.firstLocalVertex + lt[tri * 3 + vv]));
+          dd[3 * vv + 0] = wp.x, dd[3 * vv + 1] = wp.y, dd[3 * vv + 2] = wp.z;
         }
       }
     }

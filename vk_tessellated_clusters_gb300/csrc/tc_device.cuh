@@ -370,23 +370,6 @@ __device__ __forceinline__ float sample_taps(const tc_DisplacementTexture& tx, c
   return (1.0f - b.fy) * top + b.fy * bot;
 }
 
-__device__ __forceinline__ float sample_bilinear(const tc_DisplacementTexture& tx, f2 uv)
-{
-  if(tx.width == 0 || tx.height == 0)
-    return 0.0f;
-  return sample_taps(tx, bilinear_taps(tx, uv));
-}
-
-// height = (h * instScale * viewScale) + instOffset + viewOffset; pos += normalize(n) * height
-// (cluster_classify.comp.glsl:471-478, triangle_tess_template_instantiate.comp.glsl:356-365)
-__device__ __forceinline__ f3 displace(f3 pos, f3 normal, float h, float instScale, float viewScale, float instOffset,
-                                       float viewOffset)
-{
-  h    = ((h * instScale) * viewScale + instOffset) + viewOffset;
-  f3 n = normalize3(normal);
-  return {pos.x + n.x * h, pos.y + n.y * h, pos.z + n.z * h};
-}
-
 // ---------------------------------------------------------------------------
 // memory-model helpers
 // ---------------------------------------------------------------------------

@@ -820,8 +820,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) k_instantiate_parts(StageCt
 }
 
 // triangle_tess_template_instantiate.comp.glsl:295-371 with TESS_USE_PN and /
-// or DO_ANIMATION: chunks of up to 32 parts per warp as in
-// k_instantiate_vertices, records and vertex walk of tc_deform.cuh.
+// or DO_ANIMATION: chunks of up to kDeformParts parts per warp, otherwise as in
+// k_instantiate_vertices; records and vertex walk of tc_deform.cuh.
 __global__ void __launch_bounds__(kDeformBlock, kDeformBlocksPerSM) k_instantiate_vertices_deform(StageCtx c, InstantiateBuffers ib)
 {
   stage_prologue();

@@ -122,10 +122,11 @@ cudaError_t launch_triangle_split(const StageCtx& c, u32 blockSize, u32 grid, cu
 // every split pass in one launch: per level its look-back rows and control
 // words (a scratch slot each; the ticket of level 0's slot is the launch's)
 constexpr u32 kMaxSplitLevels = 16;
+constexpr u32 kSplitCtrlWords = 16;  // of a level's slot
 struct SplitLevels
 {
   unsigned long long* lbState[kMaxSplitLevels];  // [4][stride] per level (split, part, next level's children, index)
-  u32*                ctrl[kMaxSplitLevels];     // 16 words per level (see tc_split.cu)
+  u32*                ctrl[kMaxSplitLevels];     // kSplitCtrlWords per level (see tc_split.cu)
   u32                 stride;                    // tiles per level the rows hold
   u32                 levels;                    // split passes
 };

@@ -375,8 +375,10 @@ cudaError_t launch_raster_batches(const StageCtx& c, uint4* groups, const tc_ras
 {
   const u32   ngroups = std::max(1u, (maxParts + 31) / 32);
   const u32   grid    = std::max(1u, std::min((ngroups + 7) / 8, numSMs * 8));
-  // one wave of the write blocks (their shared memory lets eight share an SM,
-  // four with the PN records); small capacities get four warps per group
+  // Two waves of the write blocks: four are resident per SM (106 registers), and
+  // eight per SM even out the groups (992,000 vertices 35.5 us a call, 42.2 with
+  // one wave; 286,000 24.9 and 30.2). One with PN or the ripple, where the records
+  // take the shared memory of four. Small capacities get four warps per group.
   const bool  deform = (c.flags & (TC_FLAG_PN | TC_FLAG_RIPPLE)) != 0;
   const u32   wgrid  = std::max(1u, std::min(ngroups, numSMs * (deform ? 4u : 8u)));
   cudaError_t e       = launch_pdl(k_raster_counts, grid, kRasterBlock, s, c, groups);

@@ -61,6 +61,11 @@ enum : int
   kRowScan                  // the scan of the first level's items
 };
 
+// k_triangle_split's index words, counted from the slot's first (ticket, done,
+// totals); words 2 to 5 are the totals
+constexpr u32 kIndexWords = 8;
+static_assert(2 + 2 * kNumCounters <= kIndexWords && kIndexWords + 2 <= kSplitCtrlWords, "the index words follow the totals");
+
 constexpr u32 kMaxChildrenPerItem = TC_TESSTABLE_SIZE * TC_TESSTABLE_SIZE;  // 121
 
 struct SplitItem
@@ -534,7 +539,7 @@ __global__ void __launch_bounds__(B) k_triangle_split(StageCtx c)
   }
   const FactorParams fp = split_factor_params(c);
   const u32          sf = clamp_split_factor(c.caps.splitFactor);
-  u32*               indexed  = c.scratch.ticket + 8;  // index tiles done; index complete
+  u32*               indexed  = c.scratch.ticket + kIndexWords;  // index tiles done; index complete
   const u32          own      = (end - begin) <= kIndexLocalTiles * B;
   const u32          idxTiles = own ? 0u : (end - begin + B - 1) / B;
   Level              lv       = {};
@@ -700,7 +705,7 @@ __global__ void __launch_bounds__(B) k_triangle_split_levels(StageCtx c, SplitLe
   const FactorParams fp       = split_factor_params(c);
   const u32          sf       = clamp_split_factor(c.caps.splitFactor);
   const u32          levels   = lv.levels;
-  u32*               indexed  = lv.ctrl[0] + 8;
+  u32*               indexed  = lv.ctrl[0] + kIndexWords;
 
   // level 0: the range the classify set-up (BUILD_SETUP_SPLIT) left, unless
   // the launch is complete and the range already the last level's (the flag is

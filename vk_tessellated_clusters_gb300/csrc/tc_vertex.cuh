@@ -340,13 +340,6 @@ __device__ __forceinline__ f3 affine_vertex_u(const PartAffine& r, u32 tableVert
   return fma3(k, N, P);
 }
 
-__device__ __forceinline__ f3 affine_vertex(const PartAffine& r, u32 tableVertex)
-{
-  return affine_vertex_k<~0u>(r, tableVertex);
-}
-
-__device__ __forceinline__ u32 affine_first_vertex(const PartAffine& r) { return __float_as_uint(r.q[6].z); }
-
 }  // namespace tc
 
 namespace tc {
