@@ -340,7 +340,10 @@ ClassifyBuffers classify_buffers(tc_context* ctx)
 // clusters (a longer first kernel and two more launches, one of which takes
 // clusters_cull's place): 48 instances of the batched scene (9,720 clusters)
 // 62.8 us a frame without and 66.8 with, 96 instances 75.2 and 71.8, 1,024
-// instances from host buffers 298 and 162.
+// instances from host buffers 298 and 162. Whether instances share anything is
+// known on the device only; where none do, 96 instances take 65.6 us without and
+// 67.1 with, 256 94.3 and 93.3 (152 and 157 with every option), 1,000 256.8 and
+// 262.3, 3,000 508 and 518.
 constexpr u32 kGroupMinClusters = 16384;
 
 // whether a batched frame groups its instances (RT semantics only: the visible
@@ -354,7 +357,9 @@ bool groups_instances(const tc_frame_args* a)
 // Clusters from which the adjoint takes full clusters by instance groups, with
 // one launch more (k_backward_index): 48 instances of the batched scene (9,720
 // clusters) 18.7 us without and 19.1 with, 96 instances 43 and 27 us, 256
-// instances 106 and 46.
+// instances 106 and 46; where none share anything, 96 instances 40 and 50, 256
+// 100 and 119, 900 374 and 418 (one warp for each full cluster, as it was before:
+// 52, 127 and 478).
 constexpr u32 kBackMinClusters = 12288;
 
 // the instance groups' tables
