@@ -142,3 +142,47 @@ def test_adjoint_of_many_instances(oracle, instances, apart):
         assert norm > 0 and np.linalg.norm(part - ref) <= 1e-4 * norm, np.linalg.norm(part - ref) / norm
     assert pipe.device_errors() == 0
     pipe.close()
+
+
+@pytest.mark.parametrize("call", ["raster", "frame", "frame_pn", "plain", "frozen"])
+def test_map_of_more_than_2_to_the_32_texels(call):
+    """A map of 65,536 x 65,600 texels, ones in its last 64 rows and zeros elsewhere, read in the middle of those rows:
+    the same bits as from a small map of ones."""
+    import torch
+    from vk_tessellated_clusters_gb300.autograd import FrozenFrame
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    wide, high = 65536, 65600
+    sc = S.scene_icosphere(subdivisions=3, map_size=64)
+    sc.textures[0] = S.Texture(np.full((4, 4), 65535, np.uint16), L.TEXEL_UNORM16)
+    rng = np.random.default_rng(2)
+    for g in sc.geometries:
+        g.texcoords[:, 0] = rng.random(len(g.texcoords))
+        g.texcoords[:, 1] = (high - 32) / high
+    caps = L.default_caps(visible_bits=12, part_bits=17, split_bits=14, vertex_bits=20, megs=64)
+    pipe = TessellationPipeline(sc, caps, FLAGS | (L.FLAG_PN if call == "frame_pn" else 0))
+    # whole clusters and parts
+    pipe.set_cameras(S.Camera(eye=(0.0, 0.0, 3.6), center=(0.0, 0.0, 0.0), tess_rate_pixels=40.0))
+    texels = torch.zeros(wide * high * 2, dtype=torch.uint8, device="cuda")
+    texels[-64 * wide * 2:] = 255
+    record = np.zeros(1, L.DisplacementTexture)
+    got = []
+    for large in (False, True):
+        if large:
+            record[0] = (texels.data_ptr(), wide, high, L.TEXEL_UNORM16, 0)
+            pipe.state.res.textures.write(record)
+        pipe.state.gen_vertices.handle.zero_()
+        pipe.build("plain" if call == "plain" else "graph")
+        out = pipe.outputs()
+        assert len(out["fullClusters"]) > 0 and len(out["partTriangles"]) > 0
+        if call == "raster":
+            got.append(pipe.raster_batches()["worldPositions"])
+        elif call == "frozen":
+            frozen = FrozenFrame(pipe)
+            pipe.state.gen_vertices.handle.zero_()
+            got.append(frozen.generate().cpu().numpy())
+        else:
+            got.append(out["genVertices"])
+    assert np.abs(got[0]).max() > 1.04  # displaced
+    assert got[0].tobytes() == got[1].tobytes()
+    assert pipe.device_errors() == 0
+    pipe.close()

@@ -48,14 +48,16 @@ enum : u32
   kAffineFlat     = 0,  // no displacement map
   kAffineZeroMap  = 1,  // map of height 0: displaced by the offsets only
   kAffineTextured = 2,  // 2 + 2 * format + (1 if both sizes are powers of two)
+  kAffineLarge    = 8,  // 8 + format: 2^32 texels and more (no walk is specialised for these)
 };
 
 __host__ __device__ constexpr u32 affine_kind(u32 format, bool pow2) { return kAffineTextured + 2 * format + (pow2 ? 1 : 0); }
 
 // A displacement map as the vertex code reads it: q7 = texels lo, texels hi,
 // width, height (bits); q8 = width, height (floats), width - 1, height - 1
-// (bits; the wrap masks of power-of-two sizes); kind = affine_kind(format, pow2),
-// kAffineFlat without a map, kAffineZeroMap for a map of height 0.
+// (bits; the wrap masks of power-of-two sizes); kind = affine_kind(format, pow2)
+// or kAffineLarge + format, kAffineFlat without a map, kAffineZeroMap for a map
+// of height 0.
 struct MapDesc
 {
   float4 q7, q8;
@@ -73,7 +75,8 @@ __device__ __forceinline__ MapDesc make_map_desc(const tc_DisplacementTexture& t
   const bool pow2 = w != 0 && h != 0 && (w & (w - 1)) == 0 && (h & (h - 1)) == 0;
   // formats other than fp16 / unorm16 read as fp32, as in every other sampling path
   const u32 fmt = tx.format == TC_TEXEL_F16 || tx.format == TC_TEXEL_UNORM16 ? tx.format : TC_TEXEL_F32;
-  m.kind        = w == 0 ? kAffineFlat : (h == 0 ? kAffineZeroMap : affine_kind(fmt, pow2));
+  const u32 textured = __umulhi(w, h) ? kAffineLarge + fmt : affine_kind(fmt, pow2);
+  m.kind             = w == 0 ? kAffineFlat : (h == 0 ? kAffineZeroMap : textured);
   return m;
 }
 
@@ -230,8 +233,8 @@ __device__ __forceinline__ float texel_at(u64 texels, u64 i)
   return __uint2float_rn(__ldg(reinterpret_cast<const unsigned short*>(texels) + i)) * (1.0f / 65535.0f);
 }
 
-// bilinear sample at (u, v) of the map described by q7 and q8
-template <u32 Format, bool Pow2>
+// bilinear sample at (u, v) of the map described by q7 and q8 (Index: of its texels)
+template <u32 Format, bool Pow2, class Index = u32>
 __device__ __forceinline__ float affine_sample(float4 q7, float4 q8, float u, float v)
 {
   const u32   w = __float_as_uint(q7.z), h = __float_as_uint(q7.w);
@@ -250,7 +253,7 @@ __device__ __forceinline__ float affine_sample(float4 q7, float4 q8, float u, fl
     x0 = wrapi(ix, (int)w), x1 = wrapi(ix + 1, (int)w), y0 = wrapi(iy, (int)h), y1 = wrapi(iy + 1, (int)h);
   }
   const u64   texels = (u64)__float_as_uint(q7.x) | ((u64)__float_as_uint(q7.y) << 32);
-  const u32   r0 = (u32)y0 * w, r1 = (u32)y1 * w;  // maps hold fewer than 2^32 texels
+  const Index r0 = (Index)(u32)y0 * w, r1 = (Index)(u32)y1 * w;
   const float t00 = texel_at<Format>(texels, r0 + (u32)x0), t10 = texel_at<Format>(texels, r0 + (u32)x1);
   const float t01 = texel_at<Format>(texels, r1 + (u32)x0), t11 = texel_at<Format>(texels, r1 + (u32)x1);
   const float top = __fmaf_rn(fx, t10 - t00, t00), bot = __fmaf_rn(fx, t11 - t01, t01);
@@ -270,6 +273,9 @@ __device__ __forceinline__ float sample_kind(u32 kind, float4 q7, float4 q8, flo
     case affine_kind(TC_TEXEL_F16, false): return affine_sample<TC_TEXEL_F16, false>(q7, q8, u, v);
     case affine_kind(TC_TEXEL_UNORM16, true): return affine_sample<TC_TEXEL_UNORM16, true>(q7, q8, u, v);
     case affine_kind(TC_TEXEL_UNORM16, false): return affine_sample<TC_TEXEL_UNORM16, false>(q7, q8, u, v);
+    case kAffineLarge + TC_TEXEL_F32: return affine_sample<TC_TEXEL_F32, false, u64>(q7, q8, u, v);
+    case kAffineLarge + TC_TEXEL_F16: return affine_sample<TC_TEXEL_F16, false, u64>(q7, q8, u, v);
+    case kAffineLarge + TC_TEXEL_UNORM16: return affine_sample<TC_TEXEL_UNORM16, false, u64>(q7, q8, u, v);
     default: return 0.0f;
   }
 }
