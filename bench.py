@@ -246,8 +246,8 @@ LIMITERS = {
     "batched/cluster_classify": "instruction issue and latency, not DRAM: the 256 instances share 4 meshes, so "
                                 "the working set is L2-resident (DRAM 0.3-1.1 %); k_classify_count issue-bound "
                                 "(67 % issue active), k_classify_full_vertices long-scoreboard-bound",
-    "terrain/triangle_instantiate": "L1 data pipe and instruction issue in k_instantiate_parts (61 % issue "
-                                    "active, LSU data pipe 73 %, DRAM 30 %), DRAM traffic below the "
+    "terrain/triangle_instantiate": "L1 data pipe and instruction issue in k_instantiate_parts (59 % issue "
+                                    "active, LSU data pipe 74 %, DRAM 30 %), DRAM traffic below the "
                                     "algorithmic bytes",
 }
 
