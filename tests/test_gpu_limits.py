@@ -186,3 +186,46 @@ def test_map_of_more_than_2_to_the_32_texels(call):
     assert got[0].tobytes() == got[1].tobytes()
     assert pipe.device_errors() == 0
     pipe.close()
+
+
+def test_adjoint_adds_a_part_once(oracle):
+    """224,000 parts of 54 vertices on 320 triangles: the positions' gradients are sums of thousands of parts' terms, and
+    their error is that of adding each part once. Adding n terms of random sign in float32 makes an error of
+    c sqrt(n / 2) of the sum, c <= 2^-24 / sqrt(3); each part in as many pieces as the walk cuts it into (2.7 here) makes
+    1.6 times as much."""
+    import ctypes
+    import torch
+    from oracle.binding import lib as olib
+    from vk_tessellated_clusters_gb300.autograd import FrozenFrame
+    from vk_tessellated_clusters_gb300.pipeline import TessellationPipeline
+    sc = S.scene_icosphere(subdivisions=2, map_size=64)
+    sc.instances[0].displacement_index = -1
+    caps = L.default_caps(visible_bits=12, part_bits=18, split_bits=16, vertex_bits=24, megs=1024)
+    cam = S.Camera(eye=(0.0, 0.0, 1.5), center=(0.0, 0.0, 0.0), tess_rate_pixels=1.0, near=0.01, far=10.0)
+    pipe = TessellationPipeline(sc, caps, FLAGS)
+    pipe.set_cameras(cam)
+    pipe.build("graph")
+    frozen = FrozenFrame(pipe)
+    out = pipe.outputs()
+    g = np.random.default_rng(1).normal(0, 1, (frozen.num_vertices, 3)).astype(np.float32)
+    got = frozen.scatter_gradients(torch.from_numpy(g).cuda())[0][0].double().cpu().numpy()
+    ref_state, _ = oracle.frame(sc, cam, caps, FLAGS)
+    want = [np.zeros(x.shape) for x in (sc.geometries[0].positions, sc.geometries[0].normals)]
+    texels = np.zeros(sc.textures[0].texels.shape)
+    g64 = g.astype(np.float64)
+    ptr = lambda a: (ctypes.c_void_p * 1)(a.ctypes.data)
+    olib().tco_backward_f64(ctypes.byref(oracle.table), ctypes.byref(ref_state.args), g64.ctypes.data, ptr(want[0]),
+                            ptr(want[1]), ptr(texels))
+    # parts on each base vertex
+    parts, geo = out["partTriangles"], sc.geometries[0]
+    assert len(parts) > 200000
+    cluster = geo.clusters[parts["clusterID"]]
+    first = cluster["firstLocalTriangle"].astype(np.int64) + 3 * (parts["triangleID_config"] & 0xFFFF).astype(np.int64)
+    n = np.zeros(len(geo.positions))
+    for k in range(3):
+        np.add.at(n, cluster["firstLocalVertex"].astype(np.int64) + geo.local_triangles.reshape(-1)[first + k], 1)
+    bound = 2.0 ** -24 / 3 ** 0.5 * np.sqrt((n * n / 2).sum() / n.sum())
+    error = np.linalg.norm(got - want[0]) / np.linalg.norm(want[0])
+    assert error <= bound, (error, bound)
+    assert pipe.device_errors() == 0
+    pipe.close()

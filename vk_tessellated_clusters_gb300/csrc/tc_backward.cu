@@ -70,10 +70,14 @@ __device__ __forceinline__ void red_add3(float* base, u64 index, f3 v)
 constexpr u32 kWarps = 8;      // of the forward's blocks
 constexpr u32 kBackWarps = 4;  // of the adjoint's
 constexpr int kBackBlocksPerSM = 7;  // 72 registers per thread
-// Vertices of parts a warp takes at a time: 20,480 parts of 36 vertices 14.2 us
-// with 96, 10.7 with 64 and 8.9 with 32, where 256 instances lose (55 to 63 us).
-constexpr u32 kBackChunk       = 64;
-constexpr u32 kMaxPartVertices = (TC_TESSTABLE_SIZE + 1) * (TC_TESSTABLE_SIZE + 2) / 2;
+// Vertices of parts a warp takes at a time (the parts that start in them), by
+// those of all parts and the number of warps: BACKCHUNKFIG.
+constexpr u32 kBackChunk = 128;
+__device__ __forceinline__ u32 back_chunk(u64 vertices, u32 nwarps)
+{
+  const u32 per = (u32)((vertices + nwarps - 1) / nwarps), rounds = max(1u, (per + kBackChunk / 2) / kBackChunk);
+  return per <= 32 ? 32u : max(64u, (per + rounds - 1) / rounds);
+}
 constexpr int kBackSteps = 2;  // steps of 32 vertices whose loads are in flight together
 
 // number of leading full-cluster instantiations (they precede all parts)
@@ -99,6 +103,8 @@ enum : u32
   kBackTasks,
   kBackGrouped,  // whether instances share enough (two to a group on average)
 };
+
+constexpr u32 kBackTable = 2 * kBackInstances;
 
 // A full cluster's place in `slots`: its number among the instances' clusters
 // (the frame's prefix; ~0 or one taken by another: the cluster is left out of
@@ -144,23 +150,34 @@ __global__ void __launch_bounds__(kBackInstances) k_backward_index(StageCtx c, B
     }
     return;
   }
-  __shared__ u32 s_hash[kBackInstances], s_rep[kBackInstances], s_count[kBackInstances], s_rank[kBackInstances], s_scan[33];
-  const u32      i = threadIdx.x, n = min(c.numInstances, min(g.cap, kBackInstances));
-  GroupKey       key = {};
+  __shared__ unsigned short s_table[kBackTable], s_print[kBackInstances];
+  __shared__ u32 s_first[kBackTable], s_rep[kBackInstances], s_count[kBackInstances], s_rank[kBackInstances], s_scan[33];
+  constexpr unsigned short kEmpty = 0xFFFF;
+  const u32                i = threadIdx.x, n = min(c.numInstances, min(g.cap, kBackInstances));
+  for(u32 k = i; k < kBackTable; k += kBackInstances)
+    s_table[k] = kEmpty, s_first[k] = ~0u;
+  s_count[i] = 0;
+  GroupKey key = {};
   if(i < n)
     key = group_key(c.instances[i]);
-  const u32 hash = group_hash(key) >> 32;
-  s_hash[i]  = hash;
-  s_count[i] = 0;
+  const u64            hash  = group_hash(key);
+  const unsigned short print = group_print(hash);
+  s_print[i]                 = print;
   __syncthreads();
-  u32 rep = i;
-  for(u32 k = 0; i < n && k < i; k++)
-    if(s_hash[k] == hash && same_key(key, group_key(c.instances[k])))
-    {
-      rep = k;
-      break;
-    }
-  s_rep[i] = rep;
+  // the key's slot (as in find_groups), then the first instance with that key
+  u32 slot = group_slot(hash) % kBackTable;
+  for(bool found = i >= n; !found;)
+  {
+    const unsigned short other = atomicCAS(&s_table[slot], kEmpty, (unsigned short)i);
+    found = other == kEmpty || (s_print[other] == print && same_key(key, group_key(c.instances[other])));
+    if(!found)
+      slot = (slot + 1) % kBackTable;
+  }
+  if(i < n)
+    atomicMin(&s_first[slot], i);
+  __syncthreads();
+  const u32 rep = i < n ? s_first[slot] : i;
+  s_rep[i]      = rep;
   __syncthreads();
   if(i < 32)  // ranks in instance order
     for(u32 base = 0; base < n; base += 32)
@@ -384,28 +401,30 @@ struct __align__(16) BackPart
 };
 static_assert(sizeof(BackPart) % 32 == 16, "consecutive records start in different bank groups");
 
-// Vertices of a chunk of the parts' vertices (kBackChunk of them from `from`
-// on): the first lanes own a part each (record `lane`, `nv` vertices of which
-// the first is the chunk's vertex `start`; no part: nv = 0).
-__device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* rec, u32 nv, int start, u64 from,
-                                           const float* gradVertices, float viewScale, float viewOffset)
+// The vertices of up to 32 parts: lane l owns part l (record `lane`, `nv`
+// vertices, of which the first is vertex `start` of a walk of `total`; no part:
+// nv = 0). `carry`: 18 words of the warp. A part's terms are added to
+// memory once, by the lane that has its first vertex in its last step: one
+// addition for each step or chunk a part lies in rounds the sums more often
+// (a frame of 158,000 parts of 46 vertices: 5.1e-7 of the positions' gradients
+// instead of CARRYERR).
+__device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* rec, float* carry, u32 nv, u32 start, u32 total,
+                                           u64 from, const float* gradVertices, float viewScale, float viewOffset)
 {
   const u32 lane = threadIdx.x & 31;
   const u32 upto = (2u << lane) - 1u;  // bits 0..lane
+  bool      open = false;              // the step's first part began in the step before
   __syncwarp();
-  for(u32 base = 0; base < kBackChunk; base += 32)
+  for(u32 base = 0; base < total; base += 32)
   {
     // lane's part, and the lanes that start one (a part that began before the step starts at lane 0)
-    const int before = __popc(__ballot_sync(0xFFFFFFFFu, nv && start <= (int)base));
-    const u32 heads  = 1u | __reduce_or_sync(0xFFFFFFFFu, (nv && start > (int)base && start < (int)base + 32) ? 1u << (start - (int)base) : 0u);
-    const int at     = before - 2 + __popc(heads & upto);
-    const u32 pi     = (u32)max(at, 0) & 31;
+    const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, nv && start <= base));
+    const u32 heads  = 1u | __reduce_or_sync(0xFFFFFFFFu, (nv && start > base && start < base + 32) ? 1u << (start - base) : 0u);
+    const u32 pi     = (before - 2 + __popc(heads & upto)) & 31;
     const u32 jj     = base + lane;
-    const u32 within = jj - (u32)__shfl_sync(0xFFFFFFFFu, start, pi), count = __shfl_sync(0xFFFFFFFFu, nv, pi);
-    const bool on    = at >= 0 && within < count;
-    const u64 v      = from + jj;
-    if(!__any_sync(0xFFFFFFFFu, on))
-      continue;
+    const u32 within = jj - __shfl_sync(0xFFFFFFFFu, start, pi), count = __shfl_sync(0xFFFFFFFFu, nv, pi);
+    const bool on    = within < count;
+    const bool adds  = on || (open && lane == 0);
     const BackPart& r = rec[pi];
     f3 dP[3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, dNh[3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     const bool tex = r.tx.width != 0;
@@ -413,7 +432,7 @@ __device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* re
     const f3     nh[3] = {{q2.y, q2.z, q2.w}, {q3.x, q3.y, q3.z}, {q3.w, q4.x, q4.y}};
     if(on)
     {
-      const f3 g = ldg3(gradVertices, v);
+      const f3 g = ldg3(gradVertices, from + jj);
       f3       w = decode_bary(__ldg(c.table.vertices + (r.tv + jj)));
       if(__float_as_uint(q6.w))
       {
@@ -448,6 +467,13 @@ __device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* re
           scatter_texels(r.dTexels, r.tx, taps, dh * (r.scale * viewScale));
       }
     }
+    if(open && lane == 0)
+#pragma unroll
+      for(int k = 0; k < 3; k++)
+      {
+        dP[k]  = {dP[k].x + carry[6 * k], dP[k].y + carry[6 * k + 1], dP[k].z + carry[6 * k + 2]};
+        dNh[k] = {dNh[k].x + carry[6 * k + 3], dNh[k].y + carry[6 * k + 4], dNh[k].z + carry[6 * k + 5]};
+      }
     // a part's sums within the step to its first lane
     const u32  above = heads & ~upto;
     const u32  last  = above ? (u32)__ffs(above) - 2u : 31u;
@@ -473,25 +499,40 @@ __device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* re
             dNh[k] = {dNh[k].x + o.x, dNh[k].y + o.y, dNh[k].z + o.z};
         }
     }
-    if(on && ((heads >> lane) & 1u))
+    // whether the step's last part goes on in the next one: no part starts there
+    open = base + 32 < total && !__any_sync(0xFFFFFFFFu, nv && start == base + 32);
+    __syncwarp();  // the carry is rewritten
+    if(adds && ((heads >> lane) & 1u))
     {
-      const float rr[3] = {q6.x, q6.y, q6.z};
-#pragma unroll
-      for(int k = 0; k < 3; k++)
+      if(open && last == 31)
       {
-        if(r.dPositions)
-          red_add3(r.dPositions, r.vi[k], dP[k]);
-        if(tex && r.dNormals)
+#pragma unroll
+        for(int k = 0; k < 3; k++)
         {
-          // d normalize(n_k) / dn_k = (I - nh nh^T) / |n_k|
-          const float d = dot3(nh[k], dNh[k]);
-          red_add3(r.dNormals, r.vi[k],
-                   {rr[k] * (dNh[k].x - nh[k].x * d), rr[k] * (dNh[k].y - nh[k].y * d), rr[k] * (dNh[k].z - nh[k].z * d)});
+          carry[6 * k] = dP[k].x, carry[6 * k + 1] = dP[k].y, carry[6 * k + 2] = dP[k].z;
+          carry[6 * k + 3] = dNh[k].x, carry[6 * k + 4] = dNh[k].y, carry[6 * k + 5] = dNh[k].z;
+        }
+      }
+      else
+      {
+        const float rr[3] = {q6.x, q6.y, q6.z};
+#pragma unroll
+        for(int k = 0; k < 3; k++)
+        {
+          if(r.dPositions)
+            red_add3(r.dPositions, r.vi[k], dP[k]);
+          if(tex && r.dNormals)
+          {
+            // d normalize(n_k) / dn_k = (I - nh nh^T) / |n_k|
+            const float d = dot3(nh[k], dNh[k]);
+            red_add3(r.dNormals, r.vi[k],
+                     {rr[k] * (dNh[k].x - nh[k].x * d), rr[k] * (dNh[k].y - nh[k].y * d), rr[k] * (dNh[k].z - nh[k].z * d)});
+          }
         }
       }
     }
+    __syncwarp();
   }
-  __syncwarp();  // the records are rewritten
 }
 
 // What bounds it: the chains of dependent loads (arguments, cluster reference,
@@ -511,6 +552,7 @@ __global__ void __launch_bounds__(kBackWarps * 32, kBackBlocksPerSM) k_instantia
     BackPart   part[kPartsPerWarp];
   };
   __shared__ __align__(16) unsigned char s_records[kBackWarps][sizeof(Records)];
+  __shared__ float  s_carry[kBackWarps][18];
   Records&          records = *reinterpret_cast<Records*>(s_records[threadIdx.x >> 5]);
   const u32         lane  = threadIdx.x & 31;
   const u32         gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -594,29 +636,34 @@ __global__ void __launch_bounds__(kBackWarps * 32, kBackBlocksPerSM) k_instantia
   const tc_TessTriangleInfo* parts = reinterpret_cast<const tc_TessTriangleInfo*>(b->partTriangles);
   auto first_vertex = [&](u32 j) { return (ti[j].vertexBufferAddress - b->genVertices) / 12; };
   // cut by vertices: parts have 3 to 78 of them, and those of an instance near
-  // the camera have the most
+  // the camera have the most. A chunk's parts are those that start in it.
   const u64 vFirst = first_vertex(nfull), vLast = first_vertex(temps - 1);
-  const u64 span   = (vLast > vFirst ? min(vLast - vFirst, (u64)c.caps.maxGeneratedVertices) : 0ull) + kMaxPartVertices;
-  const u32 chunks = (u32)((span + kBackChunk - 1) / kBackChunk);
+  const u64 span   = (vLast > vFirst ? min(vLast - vFirst, (u64)c.caps.maxGeneratedVertices) : 0ull) + 1;
+  const u32 width  = back_chunk(span, nwarp);
+  const u32 chunks = (u32)((span + width - 1) / width);
   for(u32 t = nwarp - 1 - gwarp; t < chunks; t += nwarp)
   {
-    const u64 from = vFirst + (u64)t * kBackChunk;
-    // the last part that starts at or before `from`, among 32 at a time
+    const u64 from = vFirst + (u64)t * width;
+    // the first part that starts at or after `from`, among 32 at a time
     u32 p0 = 0;
-    for(u32 hi = nparts; hi - p0 > 1;)
+    for(u32 hi = nparts; p0 < hi;)
     {
       const u32 step = (hi - p0 + 31) / 32, q = p0 + lane * step;
-      const u32 k    = __popc(__ballot_sync(0xFFFFFFFFu, q < hi && first_vertex(nfull + q) <= from)) - 1;
-      p0 += k * step;
-      hi = min(hi, p0 + step);
+      const u32 k    = __popc(__ballot_sync(0xFFFFFFFFu, q < hi && first_vertex(nfull + q) < from));
+      if(k == 0)
+        break;
+      hi = min(hi, p0 + k * step);
+      p0 += (k - 1) * step + 1;
     }
     for(; p0 < nparts; p0 += 32)
     {
-      const u32  j     = nfull + p0 + lane;
-      const u64  vo    = j < temps ? first_vertex(j) : ~0ull;
-      const bool own   = j < temps && vo < from + kBackChunk;
-      u32        nv    = 0;
-      int        start = 0;
+      const u32  j   = nfull + p0 + lane;
+      const u64  vo  = j < temps ? first_vertex(j) : ~0ull;
+      const bool own = j < temps && vo < from + width;
+      u32        nv  = 0;
+      // (lane 0 owns a part if any does: parts are in the order of their vertices)
+      const u64 walk  = __shfl_sync(0xFFFFFFFFu, vo, 0);
+      const u32 start = (u32)(vo - walk);
       if(own)
       {
         const tc_TessTriangleInfo pt  = parts[ti[j].clusterIdOffset & 0x3FFFFFFFu];
@@ -628,7 +675,6 @@ __global__ void __launch_bounds__(kBackWarps * 32, kBackBlocksPerSM) k_instantia
         const tc_TessTableEntry   e   = table_entry(c.table, cfg);
         const BackRecord          q   = back_record(c, targets, gradTexels, pt.cluster.instanceID);
         BackPart&                 r   = records.part[lane];
-        start                         = (int)(vo - from);
         nv                            = e.numVertices;
         f3    bb[3], nh[3];
         f2    uvb[3];
@@ -650,14 +696,15 @@ __global__ void __launch_bounds__(kBackWarps * 32, kBackBlocksPerSM) k_instantia
         r.q[4]       = make_float4(nh[2].y, nh[2].z, uvb[0].x, uvb[0].y);
         r.q[5]       = make_float4(uvb[1].x, uvb[1].y, uvb[2].x, uvb[2].y);
         r.q[6]       = make_float4(1.0f / nl[0], 1.0f / nl[1], 1.0f / nl[2], __uint_as_float(cfg_flipped(cfg) ? 1u : 0u));
-        r.tv         = e.firstVertex - (u32)start;
+        r.tv         = e.firstVertex - start;
         r.tx         = q.tx;
         r.dPositions = q.dPositions, r.dNormals = q.dNormals, r.dTexels = q.dTexels;
         r.scale = q.scale, r.offset = q.offset;
       }
       if(!__any_sync(0xFFFFFFFFu, own))
         break;
-      back_parts(c, records.part, nv, start, from, gradVertices, viewScale, viewOffset);
+      back_parts(c, records.part, s_carry[threadIdx.x >> 5], nv, start, __reduce_max_sync(0xFFFFFFFFu, nv ? start + nv : 0u), walk,
+                 gradVertices, viewScale, viewOffset);
       if(!__all_sync(0xFFFFFFFFu, own))
         break;
     }
