@@ -355,11 +355,10 @@ bool groups_instances(const tc_frame_args* a)
 }
 
 // Clusters from which the adjoint takes full clusters by instance groups, with
-// one launch more (k_backward_index): 48 instances of the batched scene (9,720
-// clusters) 18.7 us without and 19.1 with, 96 instances 43 and 27 us, 256
-// instances 106 and 46; where none share anything, 96 instances 40 and 50, 256
-// 100 and 119, 900 374 and 418 (one warp for each full cluster, as it was before:
-// 52, 127 and 478).
+// one launch more (k_backward_index): 64 instances of the batched scene (12,960
+// clusters) 29.5 us without and 18.6 with, 96 instances 43 and 27.5, 256 98 and
+// 49.5; where none share anything, 96 instances 43 and 50, 256 98 and 105, 900 372
+// and 368 (one warp for each full cluster, as it was before: 52, 127 and 480).
 constexpr u32 kBackMinClusters = 12288;
 
 // the instance groups' tables
