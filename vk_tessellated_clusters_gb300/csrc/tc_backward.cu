@@ -14,8 +14,8 @@
 // Gradients scattered: dL/dp, dL/dn (per base vertex) and dL/dtexel (the four
 // bilinear taps). Full clusters: up to 32 instantiations per warp, one lane sets
 // up one of them, then the lanes walk their vertices, direct atomics. Part
-// triangles likewise; the per-base-vertex terms of a part's vertices within a
-// step of 32 are summed across the lanes first.
+// triangles likewise; the per-base-vertex terms of a part's vertices are summed
+// first and added once.
 #include "tc_groups.cuh"
 #include "tc_kernels.h"
 #include "tc_stage.cuh"
@@ -71,7 +71,12 @@ constexpr u32 kWarps = 8;      // of the forward's blocks
 constexpr u32 kBackWarps = 4;  // of the adjoint's
 constexpr int kBackBlocksPerSM = 7;  // 72 registers per thread
 // Vertices of parts a warp takes at a time (the parts that start in them), by
-// those of all parts and the number of warps: BACKCHUNKFIG.
+// those of all parts and the number of warps: whole rounds of all warps, of
+// about kBackChunk each, but no less than 64, since the last step of a walk is
+// half empty, or 32 where a round takes no more (a warp's chain of loads is then
+// the time). Measured with 32, 64, 96 and 128: 95,000 vertices 10.8, 11.6, 12.6 and
+// 16.1 us; 1.7 M 111, 87, 81 and 79 (72 in whole rounds); 4.6 M 329, 253, 225 and
+// 225 (216). 312,000 in one round of 74 36.3, in chunks of 64 48.2.
 constexpr u32 kBackChunk = 128;
 __device__ __forceinline__ u32 back_chunk(u64 vertices, u32 nwarps)
 {
@@ -93,8 +98,8 @@ __device__ __forceinline__ u32 full_count(const StageCtx& c, u32 temps)
 // the mesh, map, scale and offset alone: a warp adds up dL/dv over the members
 // of a subgroup and scatters once. Without that the additions in L2 (12 M
 // sectors for 2.4 M vertices) and the reads of the mesh and map are repeated for
-// each instance. Measured on a GB300, 50,600 full clusters of 256 instances and
-// 77,400 parts, both kernels: 106 -> 46 us; of 96 instances 43 -> 27 us.
+// each instance. Measured on a GB300, 50,200 full clusters of 256 instances and
+// 105,000 parts, both kernels: 98 -> 49.5 us; of 96 instances 43 -> 27.5 us.
 // ---------------------------------------------------------------------------
 
 enum : u32
@@ -405,9 +410,9 @@ static_assert(sizeof(BackPart) % 32 == 16, "consecutive records start in differe
 // vertices, of which the first is vertex `start` of a walk of `total`; no part:
 // nv = 0). `carry`: 18 words of the warp. A part's terms are added to
 // memory once, by the lane that has its first vertex in its last step: one
-// addition for each step or chunk a part lies in rounds the sums more often
-// (a frame of 158,000 parts of 46 vertices: 5.1e-7 of the positions' gradients
-// instead of CARRYERR).
+// addition for each step or chunk a part lies in rounds the sums more often (a
+// frame of 158,000 parts of 46 vertices: an error of 5.1e-7 of the positions'
+// gradients instead of 3.7e-7; 224,000 of 54: 2.4e-6 instead of below 2.0e-6).
 __device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* rec, float* carry, u32 nv, u32 start, u32 total,
                                            u64 from, const float* gradVertices, float viewScale, float viewOffset)
 {
@@ -540,7 +545,7 @@ __device__ __forceinline__ void back_parts(const StageCtx& c, const BackPart* re
 // by 32 lanes for as many instantiations, and no access returns a value. A warp
 // for each full cluster and a lane for each part, at 117 registers, took 147 us
 // for 50,600 full clusters and 77,400 parts (2.8 M vertices) and 19.5 us for
-// 20,480 parts; now 47 us after the index's 5 and 10.5 us.
+// 20,480 parts; now 45 us after the index's 5 and 11 us.
 __global__ void __launch_bounds__(kBackWarps * 32, kBackBlocksPerSM) k_instantiate_backward(StageCtx c, const float* gradVertices,
                                                                       const tc_GradTargets* targets,
                                                                       float* const* gradTexels, BackGroups groups)
