@@ -398,9 +398,9 @@ u32 frame_begin_grid(const tc_context* ctx, const tc_frame_args* a)
 // part or split triangles
 bool emits_clusters(const tc_context* ctx, const tc_frame_args* a)
 {
-  return (a->flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)) != 0
-         || classify_lists_clusters(std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
-                                    ctx->schedule.classifyBlocksPerSM);
+  return classify_lists_clusters(std::min(a->totalClusters, a->caps.maxVisibleClusters), ctx->numSMs,
+                                 ctx->schedule.classifyBlocksPerSM,
+                                 (a->flags & (TC_FLAG_TRANSIENT_1X | TC_FLAG_TRANSIENT_2X)) != 0);
 }
 
 // kernels one batched frame launches (the BLAS set-up is fused for up to

@@ -1431,8 +1431,10 @@ __device__ inline void block_prefix_transient(const ClassifyScratch& cs, u64 (&p
 // range's clusters had up to 57 of them while most blocks had none.
 // Measured on a GB300, 51,840 clusters of 256 instances, 1,217 of them partly
 // tessellated: 79 us from the count's end to the last write in one kernel,
-// 31 us in two.
-__global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx c, ClassifyScratch cs)
+// 31 us in two. Not Listed (a range has no more clusters than warps): the range's
+// warps write them, without the second launch (TRANSFIG).
+template <bool Listed>
+__global__ void __launch_bounds__(kBlock, Listed ? 6 : 4) k_classify_write_transient(StageCtx c, ClassifyScratch cs)
 {
   stage_prologue();
   __shared__ u32            s_range[2];
@@ -1454,7 +1456,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
   const tc_caps&        k       = c.caps;
   const u64             maxData = (u64)k.maxGeneratedClusterMegs * 1024ull * 1024ull;
   tc_BlasBuildInfo*     blas    = reinterpret_cast<tc_BlasBuildInfo*>(b->blasBuildInfos);
-  u32                   statTemp = 0, statTris = 0;
+  u32                   statTemp = 0, statTris = 0, statTrans = 0;
 
   u64 pre[kTNum];
   block_prefix_transient(cs, pre, s_warp);
@@ -1531,7 +1533,15 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
           atomicAdd(&blas[gk].clusterReferencesCount, __popc(sel));
       }
       const u32 others = __ballot_sync(0xFFFFFFFFu, valid && !isFull);
-      if(others)
+      if constexpr(!Listed)
+      {
+        for(u32 left = others; left; left &= left - 1)
+        {
+          const u32 k = i0 + (u32)__ffs(left) - 1;
+          write_cluster_transient(c, cs, begin + c0 + k, c0 + k, s_ci[k], s_cnt[k], s_off[k], statTrans, statTris);
+        }
+      }
+      else if(others)
       {
         u32 at = 0;
         if(lane == 0)
@@ -1549,12 +1559,15 @@ __global__ void __launch_bounds__(kBlock, 6) k_classify_write_transient(StageCtx
     }
     __syncthreads();
   }
-  statTemp = __reduce_add_sync(0xFFFFFFFFu, statTemp);
-  statTris = __reduce_add_sync(0xFFFFFFFFu, statTris);
+  statTemp  = __reduce_add_sync(0xFFFFFFFFu, statTemp);
+  statTris  = __reduce_add_sync(0xFFFFFFFFu, statTris);
+  statTrans = __reduce_add_sync(0xFFFFFFFFu, statTrans);
   if(lane == 0)
   {
     if(statTemp)
       atomicAdd(&b->tempInstantiateCounter, statTemp);
+    if(statTrans)
+      atomicAdd(&b->transBuildCounter, statTrans);
     if(statTris)
       atomicAdd(&c.readback->numTotalTriangles, statTris);
   }
@@ -1900,7 +1913,8 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
   {
     // the transient write is latency-bound per cluster: a full wave of its
     // six resident blocks per SM (the count uses the same ranges)
-    const u32 tgrid = std::max(1u, std::min(classify_max_blocks(maxClusters), numSMs * std::max(6u, warpBlocksPerSM)));
+    const u32  tgrid  = std::max(1u, std::min(classify_max_blocks(maxClusters), numSMs * std::max(6u, warpBlocksPerSM)));
+    const bool listed = classify_lists_clusters(maxClusters, numSMs, warpBlocksPerSM, true);
     ClassifyScratch ts = cs;
     ts.writeBlocks     = tgrid;
     cudaError_t e      = cs.groups ? launch_pdl_critical(k_classify_whole<true>, wholeGrid, kBlock, s, c, ts) : cudaSuccess;
@@ -1909,13 +1923,14 @@ cudaError_t launch_cluster_classify(const StageCtx& c, const ClassifyBuffers& bu
     e = launch_pdl_critical(k_classify_count<4, true>, tgrid, kBlock, s, c, ts);
     if(e != cudaSuccess)
       return e;
-    e = launch_pdl_critical(k_classify_write_transient, tgrid, kBlock, s, c, ts);
-    if(e != cudaSuccess)
+    e = listed ? launch_pdl_critical(k_classify_write_transient<true>, tgrid, kBlock, s, c, ts)
+               : launch_pdl_critical(k_classify_write_transient<false>, tgrid, kBlock, s, c, ts);
+    if(e != cudaSuccess || !listed)
       return e;
     const u32 egrid = std::max(1u, std::min((maxClusters + kWarps - 1) / kWarps, numSMs * 4));
     return launch_pdl_critical(k_classify_emit_transient, egrid, kBlock, s, c, ts);
   }
-  cs.listed       = classify_lists_clusters(maxClusters, numSMs, warpBlocksPerSM) ? 1u : 0u;
+  cs.listed       = classify_lists_clusters(maxClusters, numSMs, warpBlocksPerSM, false) ? 1u : 0u;
   const int   occ = warpBlocksPerSM >= 8 ? 8 : (warpBlocksPerSM >= 5 ? 6 : 4);
   cudaError_t e   = cs.groups ? launch_pdl_critical(k_classify_whole<false>, wholeGrid, kBlock, s, c, cs) : cudaSuccess;
   if(e != cudaSuccess)
@@ -1960,9 +1975,10 @@ cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffe
   return launch_pdl(k_classify_mini_vertices, miniGrid, kDeformBlock, s, c, cs);
 }
 
-bool classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM)
+bool classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM, bool transient)
 {
-  return maxClusters > 32ull * numSMs * std::max(1u, warpBlocksPerSM);
+  return transient ? maxClusters > (u64)kWarps * numSMs * std::max(6u, warpBlocksPerSM)
+                   : maxClusters > 32ull * numSMs * std::max(1u, warpBlocksPerSM);
 }
 
 u32 classify_max_blocks(u32 maxClusters) { return std::max(1u, (maxClusters + kWarps - 1) / kWarps); }

@@ -115,9 +115,8 @@ cudaError_t launch_classify_full_vertices(const StageCtx& c, const ClassifyBuffe
                                           u32 blocksPerSM, cudaStream_t s);
 u32         classify_max_blocks(u32 maxClusters);
 // whether launch_cluster_classify launches a kernel of its own for the
-// clusters with part or split triangles (without transient builds; with them
-// it always does)
-bool        classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM);
+// clusters with part or split triangles (or transient builds)
+bool        classify_lists_clusters(u32 maxClusters, u32 numSMs, u32 warpBlocksPerSM, bool transient);
 cudaError_t launch_triangle_split(const StageCtx& c, u32 blockSize, u32 grid, cudaStream_t s);
 // every split pass in one launch: per level its look-back rows and control
 // words (a scratch slot each; the ticket of level 0's slot is the launch's)
